@@ -292,8 +292,7 @@ int iw_run(iw_handle *h, int nsteps, int use_graph);
  * or one CTA per task of <= 4 right-hand sides).  Candidates run on the
  * handle's scratch fields; the state is not changed (the solver tables are
  * built if no step has built them yet).  The stage-A variants and the solve
- * variants 0 and 1 give the same bits; the stage-E variants and the
- * tensor-core products round differently.
+ * variants give the same bits; the stage-E variants round differently.
  * choices (optional, 4 ints): the y-tile width; for stage A and stage E
  * 1 = register-column, 0 = tiled, -1 = not applicable (stage E also 2 =
  * tiled with the input tiles staged by bulk copies, N <= 64); the pressure
@@ -306,8 +305,9 @@ int iw_autotune(iw_handle *h, int *choices);
 #define IW_LAUNCH_STAGE_A 1 /* -1 (size heuristic), 0 tiled, 1 register-column */
 #define IW_LAUNCH_STAGE_E 2 /* as stage A, or 2: tiled, bulk-copied input tiles (N <= 33); 3: the same with
                                its z operators in the constant bank */
-#define IW_LAUNCH_SOLVE 3   /* 1 system-grouped (default), 2 same on the FP64 tensor cores, 0 per task,
-                               3 system-grouped with two rows per thread (u/v, w, rho; the pressure takes 1) */
+#define IW_LAUNCH_SOLVE 3   /* 2 system-grouped on the FP64 tensor cores (default; 1 where it does not apply),
+                               1 system-grouped on the FP64 pipes, 0 per task, 3 system-grouped with two rows
+                               per thread (u/v, w, rho; the pressure takes 1).  All give the same bits. */
 /* one solve role's variant (values as IW_LAUNCH_SOLVE; -1 = the IW_LAUNCH_SOLVE choice) */
 #define IW_LAUNCH_SOLVE_UV 4
 #define IW_LAUNCH_SOLVE_W 5

@@ -5,6 +5,14 @@
 // (-Xcompiler -ffp-contract=off) so the tables equal the ones the reference
 // builds (setup.f, penalty.f param_set) bit for bit.
 
+struct Tables {
+  std::vector<double> zpts, wg, alpol, D, D2, sigma, Lfil;
+};
+
+// One system kind: 0 pressure, 1 u/v, 2 w, 3 rho.
+enum { SYS_P = 0, SYS_U, SYS_W, SYS_T, SYS_KINDS };
+
+#ifndef IW_INST
 namespace {
 
 // --------------------------------------------------------------------------
@@ -90,10 +98,6 @@ void h_jacobl(int n, std::vector<double>& xcol) {
   xcol.assign(n + 1, 0.0);
   for (int k = 0; k <= n; ++k) xcol[k] = xjac[n - k + 1];
 }
-
-struct Tables {
-  std::vector<double> zpts, wg, alpol, D, D2, sigma, Lfil;
-};
 
 Tables h_tables(int N, double p, double amp, double fackc) {
   Tables t;
@@ -264,6 +268,9 @@ FftPlan make_plan(int M) {
   return p;
 }
 
+}  // namespace
+#endif  // IW_INST
+
 template <typename C>
 std::vector<C> twiddles(int n, int count) {  // exp(-2 pi i e / n), e < count
   std::vector<C> w(count);
@@ -274,10 +281,6 @@ std::vector<C> twiddles(int n, int count) {  // exp(-2 pi i e / n), e < count
   }
   return w;
 }
-// One system kind: 0 pressure, 1 u/v, 2 w, 3 rho.
-enum { SYS_P = 0, SYS_U, SYS_W, SYS_T, SYS_KINDS };
-
-}  // namespace
 
 // per-precision device buffers
 template <typename T>
@@ -393,7 +396,8 @@ struct iw_handle {
   Task* dtasks2[SYS_KINDS] = {0, 0, 0, 0};
   int ntask2[SYS_KINDS] = {0, 0, 0, 0};
   int nold[SYS_KINDS] = {0, 0, 0, 0};
-  int use_sys = 1;  // 0: k_solve_cta for every task, 1: k_solve_sys, 2: k_solve_sys on the FP64 tensor cores
+  // 0: k_solve_cta for every task, 1: k_solve_sys, 2: k_solve_tc (k_solve_sys where it does not apply), 3: k_solve_sys2
+  int use_sys = 2;
   int sys_role[4] = {-1, -1, -1, -1};  // per solve role (u/v, w, rho, pressure), set by iw_autotune; -1: use_sys
   double bi_bdfv[SYS_KINDS] = {-1, -1, -1, -1};
   bool bi_fold[SYS_KINDS] = {false, false, false, false};  // Legendre filter folded into ainv
@@ -543,6 +547,7 @@ static void free_fields(FieldSet<T>& fs) {
   cudaFree(fs.Wy);
 }
 
+#ifndef IW_INST
 // ---------------------------------------------------------------------------
 // systems: distinct kx^2+ky^2 (the matrix of a column depends on it only)
 // ---------------------------------------------------------------------------
@@ -910,6 +915,8 @@ static int ensure_factors(iw_handle* h, int cpen) {
   return 0;
 }
 
+#endif  // IW_INST
+
 static SolveTabs solve_tabs(iw_handle* h, int kind) {
   SolveTabs tb;
   tb.ab = h->dab[kind];
@@ -955,7 +962,7 @@ static void launch_stageA_r(iw_handle* h, FieldSet<T>& fs, int proj) {
 }
 
 template <typename T>
-static void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj) {
+void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj) {
   switch (h->tune_a == 0 ? 0 : zop_bucket(h->N)) {
     case 9: launch_stageA_r<T, 9>(h, fs, proj); return;
     case 17: launch_stageA_r<T, 17>(h, fs, proj); return;
@@ -1004,7 +1011,7 @@ static int build_stageE_ops(iw_handle* h) {
 }
 
 template <typename T>
-static void launch_stageE(iw_handle* h, FieldSet<T>& fs) {
+void launch_stageE(iw_handle* h, FieldSet<T>& fs) {
   EArgs<T> a;
   for (int q = 0; q < 4; ++q) {
     a.B[q] = fs.B8[q];
@@ -1131,7 +1138,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
 }
 
 template <typename T>
-static void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int nplanes, bool four) {
+void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int nplanes, bool four) {
   typedef typename cplx_t<T>::type C;
   const int tx = ytx<T>(h, four);
   const int ntile = (h->nxhp + tx - 1) / tx;
@@ -1180,7 +1187,7 @@ static int postp_step(iw_handle* h, FieldSet<T>& fs);
 // K_C: x rows (k_xrow_nl), one CTA per (y, z) row with 256 threads, or 128
 // when the autotuner measured that faster (tune_xthr)
 template <typename T>
-static void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
+void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
   typedef typename cplx_t<T>::type C;
   Geo g = geo(h);
   const int M = h->nx / 2;
@@ -1253,6 +1260,7 @@ static void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
   }
 }
 
+#ifndef IW_INST
 template <typename T>
 static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj) {
   typedef typename cplx_t<T>::type C;
@@ -1404,10 +1412,107 @@ static int adapt_dt(iw_handle* h, FieldSet<T>& fs) {
   return IW_OK;
 }
 
+#endif  // IW_INST
+
+// The solve variant a role resolves to (IW_LAUNCH_SOLVE values): its own
+// choice or the handle's, where the variant applies; 0 where no grouped kernel
+// does (more rows than threads, tables too large for shared memory, a filter
+// that is not folded into the inverses).
+static int role_kind(int role) { return role == 0 ? SYS_U : role == 1 ? SYS_W : role == 2 ? SYS_T : SYS_P; }
 template <typename T>
-static void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int kstart) {
+static int solve_variant(const iw_handle* h, int role, int cpen) {
+  int us = h->sys_role[role] >= 0 ? h->sys_role[role] : h->use_sys;
+  const bool fold = h->bi_fold[role_kind(role)] && cpen;
+  if (!us || h->nz > kSysMaxRows || (cpen && !fold)) return 0;
+  // variant 3 (two rows per thread) exists for u/v, w and rho when a subdomain's
+  // row pairs fit one CTA; otherwise the one-row grouped kernel takes its place
+  if (us == 3 && (role == 3 || (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32 > kSys2MaxThreads)) us = 1;
+  const size_t lim = 200 * 1024;
+  if (us == 2 && (h->N > kTcMaxN || tc_smem<T>(h->nz, h->N, h->ns, h->nb, role == 3).total > lim)) us = 1;
+  if (us != 2 && sys_smem(h->nz, h->N, h->ns, h->nb, role == 3).total * sizeof(double) > lim) us = 0;
+  return us;
+}
+
+static double role_rdiv(const iw_handle* h, int role) {
+  return role == 2 ? h->p.dt * h->p.xkappa : h->p.xnu * h->p.dt;
+}
+// w whose only task without k_solve_tc is the (0,0) column (no system, w = 0):
+// the kernel writes that column itself
+static bool tc_zero00(const iw_handle* h, int role) {
+  const int kind = role_kind(role);
+  return role == 1 && h->nrefine[kind] == 0 && h->nold[kind] == 1 && h->htasks[kind][0].sys < 0 &&
+         h->htasks[kind][0].first == 0 && h->htasks[kind][0].count == 1;
+}
+
+// The system-grouped tensor-core solves of the listed roles (0..2: one launch
+// for all of them; 3: the pressure).  The row tiles of 8 are fixed at compile
+// time; one warp per subdomain.
+template <typename T>
+void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles, int kstart) {
+  const Geo g = geo(h);
+  const int nt = std::max((h->N + 7) / 8, 2);
+  const size_t smem = tc_smem<T>(h->nz, h->N, h->ns, h->nb, roles[0] == 3).total;
+  if (roles[0] == 3) {
+    if (h->ntask2[SYS_P] <= 0) return;
+    const auto& B = h->bi[SYS_P];
+    BlockInv bi;
+    memset(&bi, 0, sizeof bi);
+    bi.ainv = B.ainv;
+    bi.lvec = B.lvec;
+    bi.minv = B.minv;
+    bi.sys = B.sys;
+    bi.nb = h->nb;
+    memcpy(bi.bmap, h->bmap, sizeof bi.bmap);
+    const dim3 grid((unsigned)h->ntask2[SYS_P], 2);
+#define IW_TC_CASE(NT)                                                                                             \
+  case NT:                                                                                                         \
+    cudaFuncSetAttribute(k_press_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
+    k_press_tc<T, NT><<<grid, 32 * h->ns, smem, h->st>>>(g, bi, h->dtasks2[SYS_P], h->dcolorder, fs.F[0], fs.F[1], \
+                                                         fs.F[2], h->dDt, h->dwnl, h->dwvr, kstart);               \
+    break;
+    switch (nt) { IW_TC_CASE(2) IW_TC_CASE(3) IW_TC_CASE(4) IW_TC_CASE(5) }
+#undef IW_TC_CASE
+    return;
+  }
+  TcJobs<T> jobs;
+  memset(&jobs, 0, sizeof jobs);
+  jobs.nb = h->nb;
+  memcpy(jobs.bmap, h->bmap, sizeof jobs.bmap);
+  int nblk = 0;
+  for (int i = 0; i < nroles; ++i) {
+    const int role = roles[i], kind = role_kind(role);
+    if (h->ntask2[kind] <= 0) continue;
+    const auto& B = h->bi[kind];
+    TcJob<T>& j = jobs.j[jobs.n++];
+    j.ainv = (const double*)B.ainv;
+    j.lvec = B.lvec;
+    j.minv = B.minv;
+    j.sys = B.sys;
+    j.tasks = h->dtasks2[kind];
+    j.first = nblk;
+    j.per = role == 0 ? 4 : 2;
+    j.zero00 = tc_zero00(h, role);
+    j.meanu = role == 0 ? h->p.meanu_damping : 0;
+    j.rdiv = role_rdiv(h, role);
+    j.irdiv = 1.0 / j.rdiv;
+    j.F0 = fs.F[role == 0 ? 0 : role + 1];
+    j.F1 = fs.F[1];
+    nblk += h->ntask2[kind];
+  }
+  if (nblk == 0) return;
+#define IW_TC_CASE(NT)                                                                                       \
+  case NT:                                                                                                   \
+    cudaFuncSetAttribute(k_solve_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
+    k_solve_tc<T, NT><<<nblk, 32 * h->ns, smem, h->st>>>(g, jobs, h->dcolorder, h->dmeang);                  \
+    break;
+  switch (nt) { IW_TC_CASE(2) IW_TC_CASE(3) IW_TC_CASE(4) IW_TC_CASE(5) }
+#undef IW_TC_CASE
+}
+
+template <typename T>
+void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int kstart, bool tc_done = false) {
   constexpr int R = 4;
-  const int kind = role == 0 ? SYS_U : role == 1 ? SYS_W : role == 2 ? SYS_T : SYS_P;
+  const int kind = role_kind(role);
   BlockInv bi;
   bi.ainv = h->bi[kind].ainv;
   bi.cvec = h->bi[kind].cvec;
@@ -1435,7 +1540,7 @@ static void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, i
   } else {
     F0 = role == 1 ? fs.F[2] : fs.F[3];
   }
-  const double rd = role == 2 ? h->p.dt * h->p.xkappa : h->p.xnu * h->p.dt;
+  const double rd = role_rdiv(h, role);
   const int meanu = role == 0 ? h->p.meanu_damping : 0;
   if (sm > 48 * 1024) cudaFuncSetAttribute(k_solve_cta<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   // refined prefix, then the rest
@@ -1443,61 +1548,49 @@ static void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, i
   // copy and the filter pass; the rest needs no filter pass.
   const int nref = h->nrefine[kind], nt = h->ntask[kind];
   const bool fold = h->bi_fold[kind] && cpen;
-  // system-grouped kernel for the tasks after the prefix, when it applies
-  // (variant 2: the block products on the FP64 tensor cores, N <= 40)
-  int us = h->sys_role[role] >= 0 ? h->sys_role[role] : h->use_sys;
-  // variant 3 (two rows per thread) exists for u/v, w and rho when a subdomain's
-  // row pairs fit one CTA; otherwise the one-row grouped kernel takes its place
-  const int nthr2 = (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32;
-  if (us == 3 && (role == 3 || nthr2 > kSys2MaxThreads)) us = 1;
-  const bool tc = us == 2 && h->N <= 8 * kTcMT;
-  const SysSmem lay = sys_smem(h->nz, h->N, h->ns, h->nb, role == 3, tc ? kTcRS : kSysRS, tc ? tc_ap(h->N) : 0);
-  const size_t smsys = lay.total * sizeof(double);
-  const bool grouped = us && h->nz <= kSysMaxRows && (!cpen || fold) && smsys <= 200 * 1024;
-  const int nend = grouped ? std::max(h->nold[kind], nref) : nt;
-  if (grouped && h->ntask2[kind] > 0) {
-    const int nthr = (h->nz + 31) / 32 * 32;
+  // a grouped kernel for the tasks after the prefix, when one applies
+  const int us = solve_variant<T>(h, role, cpen);
+  const bool tc = us == 2;
+  int nend = us ? std::max(h->nold[kind], nref) : nt;
+  if (tc && tc_zero00(h, role) && h->ntask2[kind] > 0) nend = 0;
+  if (tc && !tc_done) launch_solve_tc<T>(h, fs, &role, 1, kstart);
+  if (us && !tc && h->ntask2[kind] > 0) {
+    const size_t smsys = sys_smem(h->nz, h->N, h->ns, h->nb, role == 3).total * sizeof(double);
+    const int nthr = (h->nz + 31) / 32 * 32, nthr2 = (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32;
     Geo g = geo(h);
     const double* mg = h->dmeang;
-#define IW_SYS_LAUNCH(RL, TCV)                                                                                    \
-  do {                                                                                                            \
-    cudaFuncSetAttribute(k_solve_sys<T, RL, TCV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smsys);      \
-    k_solve_sys<T, RL, TCV><<<h->ntask2[kind], nthr, smsys, h->st>>>(g, bi, h->dtasks2[kind], h->dcolorder, F0, F1, \
-                                                                    F2, rd, meanu, mg, h->dDt, h->dwnl, h->dwvr,   \
-                                                                    kstart, h->derr);                              \
-  } while (0)
-#define IW_SYS_ROLE(TCV)   \
-  do {                     \
-    if (role == 0)         \
-      IW_SYS_LAUNCH(0, TCV); \
-    else if (role == 1)    \
-      IW_SYS_LAUNCH(1, TCV); \
-    else if (role == 2)    \
-      IW_SYS_LAUNCH(2, TCV); \
-    else                   \
-      IW_SYS_LAUNCH(3, TCV); \
-  } while (0)
+    if (us == 3) {
 #define IW_SYS2_LAUNCH(RL)                                                                                   \
   do {                                                                                                       \
     cudaFuncSetAttribute(k_solve_sys2<T, RL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smsys);      \
     k_solve_sys2<T, RL><<<h->ntask2[kind], nthr2, smsys, h->st>>>(g, bi, h->dtasks2[kind], h->dcolorder, F0, \
                                                                   F1, rd, meanu, mg, h->derr);              \
   } while (0)
-    if (us == 3) {
       if (role == 0)
         IW_SYS2_LAUNCH(0);
       else if (role == 1)
         IW_SYS2_LAUNCH(1);
       else
         IW_SYS2_LAUNCH(2);
-    } else if (tc) {
-      IW_SYS_ROLE(true);
-    } else {
-      IW_SYS_ROLE(false);
-    }
 #undef IW_SYS2_LAUNCH
-#undef IW_SYS_ROLE
+    } else {
+#define IW_SYS_LAUNCH(RL)                                                                                           \
+  do {                                                                                                              \
+    cudaFuncSetAttribute(k_solve_sys<T, RL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smsys);              \
+    k_solve_sys<T, RL><<<h->ntask2[kind], nthr, smsys, h->st>>>(g, bi, h->dtasks2[kind], h->dcolorder, F0, F1, F2, \
+                                                                rd, meanu, mg, h->dDt, h->dwnl, h->dwvr, kstart,   \
+                                                                h->derr);                                          \
+  } while (0)
+      if (role == 0)
+        IW_SYS_LAUNCH(0);
+      else if (role == 1)
+        IW_SYS_LAUNCH(1);
+      else if (role == 2)
+        IW_SYS_LAUNCH(2);
+      else
+        IW_SYS_LAUNCH(3);
 #undef IW_SYS_LAUNCH
+    }
   }
   for (int part = 0; part < 2; ++part) {
     const int t0 = part == 0 ? 0 : nref, cnt = part == 0 ? nref : nend - nref;
@@ -1515,6 +1608,32 @@ static void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, i
                                                           h->dLt, h->dzh, h->dwnl, h->dwvr, kstart);
   }
 }
+
+// The kernels that these launch are compiled in translation units of their own
+// (iw_inst.cu, once per storage type and group), all at the same time.
+#define IW_INST_FFT(X, T)                                                       \
+  X template void launch_y<T>(iw_handle*, FieldSet<T>&, YJobs<T>&, int, int, bool); \
+  X template void launch_xrow<T>(iw_handle*, FieldSet<T>&);
+#define IW_INST_Z(X, T)                                                             \
+  X template void launch_stageA<T>(iw_handle*, FieldSet<T>&, int);                  \
+  X template void launch_stageE<T>(iw_handle*, FieldSet<T>&);                       \
+  X template void launch_solve_tc<T>(iw_handle*, FieldSet<T>&, const int*, int, int); \
+  X template void launch_solve_bi<T>(iw_handle*, FieldSet<T>&, int, int, int, bool);
+#if defined(IW_INST)
+#if IW_INST == 1
+IW_INST_FFT(, float)
+#elif IW_INST == 2
+IW_INST_FFT(, double)
+#elif IW_INST == 3
+IW_INST_Z(, float)
+#else
+IW_INST_Z(, double)
+#endif
+#else
+IW_INST_FFT(extern, float)
+IW_INST_FFT(extern, double)
+IW_INST_Z(extern, float)
+IW_INST_Z(extern, double)
 
 // calcuvwt (calcuvwt_noslip.f / calcuvwt.f) on u*,v*,w*,rho* held in F.
 template <typename T>
@@ -1541,8 +1660,14 @@ static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen) {
   mark(h, 6);
   const double xnudt = h->p.xnu * h->p.dt, dtk = h->p.dt * h->p.xkappa;
   if (h->use_bi) {
+    // one launch for all roles on the tensor-core kernel (separate ones while
+    // the phases are timed)
+    int tcr[3], ntc = 0;
+    for (int role = 0; role < 3 && !h->prof; ++role)
+      if (solve_variant<T>(h, role, cpen) == 2) tcr[ntc++] = role;
+    if (ntc > 0) launch_solve_tc<T>(h, fs, tcr, ntc, kstart);
     for (int role = 0; role < 3; ++role) {
-      launch_solve_bi<T>(h, fs, role, cpen, kstart);
+      launch_solve_bi<T>(h, fs, role, cpen, kstart, !h->prof);
       mark(h, 7 + role);
     }
   } else {
@@ -1735,7 +1860,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
       float best = 0;
       int bestv = 1;
       for (int v = 0; v < 4; ++v) {
-        if (v == 2 && h->N > 8 * kTcMT) continue;
+        if (v == 2 && h->N > kTcMaxN) continue;
         if (v == 3 && (role == 3 || (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32 > kSys2MaxThreads)) continue;
         h->sys_role[role] = v;
         const float t = timeit([&] { launch_solve_bi<T>(h, ts, role, cpen, kstart); });
@@ -2266,7 +2391,7 @@ int iw_set_launch(iw_handle* h, int which, int value) {
       return IW_OK;
     case IW_LAUNCH_SOLVE:
       if (value < 0 || value > 3) return set_err(IW_ERR_CONFIG, "solve variant: 0, 1, 2 or 3");
-      if (value == 2 && h->N > 8 * kTcMT) return set_err(IW_ERR_CONFIG, "tensor-core solve needs N <= 40");
+      if (value == 2 && h->N > kTcMaxN) return set_err(IW_ERR_CONFIG, "tensor-core solve needs N <= 40");
       h->use_sys = value;
       for (int& r : h->sys_role) r = -1;
       return IW_OK;
@@ -2279,7 +2404,7 @@ int iw_set_launch(iw_handle* h, int which, int value) {
     case IW_LAUNCH_SOLVE_RHO:
     case IW_LAUNCH_SOLVE_PRESSURE: {
       if (value < -1 || value > 3) return set_err(IW_ERR_CONFIG, "solve variant: -1, 0, 1, 2 or 3");
-      if (value == 2 && h->N > 8 * kTcMT) return set_err(IW_ERR_CONFIG, "tensor-core solve needs N <= 40");
+      if (value == 2 && h->N > kTcMaxN) return set_err(IW_ERR_CONFIG, "tensor-core solve needs N <= 40");
       const int role = which == IW_LAUNCH_SOLVE_UV ? 0 : which == IW_LAUNCH_SOLVE_W ? 1
                        : which == IW_LAUNCH_SOLVE_RHO ? 2 : 3;
       h->sys_role[role] = value;
@@ -2646,3 +2771,4 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
 #include "iw_restart.inl"
 #include "iw_output.inl"
 #include "iw_postp.inl"
+#endif  // IW_INST

@@ -39,6 +39,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/iw_b200.h"
@@ -1028,7 +1029,7 @@ template <typename T>
 __global__ void __launch_bounds__(kTX* kTW) k_stageE(Geo g, EArgs<T> a, Coefs c) {
   stageE_tile<T>(g, a, c);
 }
-__global__ void __launch_bounds__(kTX* kTW, 8) k_stageE_f32(Geo g, EArgs<float> a, Coefs c) {
+static __global__ void __launch_bounds__(kTX* kTW, 8) k_stageE_f32(Geo g, EArgs<float> a, Coefs c) {
   stageE_tile<float>(g, a, c);
 }
 
@@ -1291,7 +1292,7 @@ __device__ __forceinline__ double& ABr(double* ab, int ldab, int r, int c) {
   return ab[(size_t)(r - 1) + (size_t)ldab * (size_t)(c - 1)];
 }
 
-__global__ void k_factor(Geo g, FactorArgs fa) {
+static __global__ void k_factor(Geo g, FactorArgs fa) {
   const int warps = blockDim.x / 32;
   const int s = blockIdx.x * warps + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
@@ -1449,7 +1450,7 @@ __global__ void k_factor(Geo g, FactorArgs fa) {
 // for nr right-hand sides b[r*n + row] in shared memory; same arithmetic as
 // the reference (no FMA) so results equal the CPU ones bit for bit.
 // ===========================================================================
-__device__ void band_solve_warp(const double* __restrict__ ab, const int* __restrict__ ipiv, double* b, int nr,
+static __device__ void band_solve_warp(const double* __restrict__ ab, const int* __restrict__ ipiv, double* b, int nr,
                                 int n, int kl, int ku, int lane) {
   // The factor entries a step needs do not depend on the data, so they are
   // fetched PF steps ahead into a register ring (indices are compile-time
@@ -1573,7 +1574,7 @@ __device__ void band_solve_warp(const double* __restrict__ ab, const int* __rest
 
 // Legendre filter of solution columns (filtering.f:729-808, filter_legenpen),
 // same order of operations as the reference.  One lane per subdomain column.
-__device__ void legen_filter_cols(double* b, int nr, int n, int N, int ns, const double* __restrict__ wg,
+static __device__ void legen_filter_cols(double* b, int nr, int n, int N, int ns, const double* __restrict__ wg,
                                   const double* __restrict__ alpol, const double* __restrict__ sigma, int lane) {
   const int nzm = N - 1;
   for (int t = lane; t < nr * ns; t += 32) {
@@ -1701,7 +1702,7 @@ struct BlockInv {
 };
 
 // warp per (system, block): invert A_ks from the assembled band
-__global__ void k_block_invert(Geo g, const double* __restrict__ ab, int nsys, double* __restrict__ ainv64,
+static __global__ void k_block_invert(Geo g, const double* __restrict__ ab, int nsys, double* __restrict__ ainv64,
                                double* __restrict__ cvec, double* __restrict__ dvec) {
   extern __shared__ __align__(16) double smi[];
   const int warps = blockDim.x / 32, wid = threadIdx.x / 32, lane = threadIdx.x & 31;
@@ -1770,7 +1771,7 @@ __global__ void k_block_invert(Geo g, const double* __restrict__ ab, int nsys, d
 }
 
 // thread per system: interface matrix M (m = 2(ns-1)) and its inverse
-__global__ void k_iface_matrix(Geo g, int nsys, const double* __restrict__ ainv64, const double* __restrict__ cvec,
+static __global__ void k_iface_matrix(Geo g, int nsys, const double* __restrict__ ainv64, const double* __restrict__ cvec,
                                const double* __restrict__ dvec, double* __restrict__ minv, double* __restrict__ work) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int N = g.N, ns = g.ns, m = 2 * (ns - 1);
@@ -2469,18 +2470,17 @@ constexpr int kSysMaxRows = 512;
 struct SysSmem {  // offsets (doubles) of the shared-memory regions of k_solve_sys
   size_t a, l, m, b, rz, zz, d, total;
 };
-__host__ __device__ inline SysSmem sys_smem(int n, int N, int ns, int nb, bool dmat, int rs = kSysRS, int ap = 0) {
+__host__ __device__ inline SysSmem sys_smem(int n, int N, int ns, int nb, bool dmat) {
   SysSmem o;
   const size_t m = 2 * (size_t)(ns - 1), m1 = m > 0 ? m : 1;
-  if (ap <= 0) ap = N;
   o.a = 0;
-  o.l = ((size_t)nb * N * ap + 3) & ~(size_t)1;  // room for a copy that starts one double early
+  o.l = ((size_t)nb * N * N + 3) & ~(size_t)1;  // room for a copy that starts one double early
   o.m = o.l + m * N;
   o.b = o.m + m * m;
-  o.rz = o.b + (size_t)n * rs;
+  o.rz = o.b + (size_t)n * kSysRS;
   o.zz = o.rz + kSysR * m1;
   o.d = o.zz + kSysR * m1;
-  o.total = o.d + (dmat ? (((size_t)N * ap + 1) & ~(size_t)1) : 0);
+  o.total = o.d + (dmat ? (((size_t)N * N + 1) & ~(size_t)1) : 0);
   return o;
 }
 
@@ -2514,94 +2514,8 @@ __device__ __forceinline__ void row_product16(const double* col, const double* b
   }
 }
 
-// FP64 tensor-core variant of the block products (mma.sync m8n8k4, the FP64
-// matrix instruction of sm_100a; tcgen05 has no FP64 kind).  A warp owns whole
-// subdomains: X_ks[:, 8 nt .. 8 nt + 7] = Op_ks B_ks[:, 8 nt ..] in row tiles
-// of 8, 4 columns of Op per instruction, the padding of the ragged N read as
-// zeros.  Lane (g, t4) = (lane / 4, lane % 4) ends with
-// X[8 mt + g][8 nt + 2 t4 + {0, 1}]: one complex value of one column.  The
-// right-hand-side rows keep the stride of 18 doubles (a B fragment then takes
-// four shared-memory wavefronts instead of two, but a stride of 20 would cost
-// the second resident CTA per SM at C3's sizes); the operators get rows of
-// tc_ap(N) doubles, which makes the five A fragments per step conflict-free.
-constexpr int kTcRS = 18;
-constexpr int kTcMT = 5;  // row tiles per subdomain: N <= 40
-
-// Row stride of the operators staged for the tensor-core products: = 4
-// (mod 8) doubles, so that an A fragment (8 rows x 4 columns of 8 bytes) falls
-// in two shared-memory wavefronts.
-__host__ __device__ inline int tc_ap(int N) {
-  int a = N;
-  while (a % 8 != 4) ++a;
-  return a;
-}
-
-__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(d0), "+d"(d1)
-      : "d"(a), "d"(b));
-}
-
-// acc[mt] = (Op B)[8 mt + g][8 nt + 2 t4 + {0, 1}] for Op(r, c) = op[c ap + r] and
-// B(c, :) = bb[c kTcRS + :], c < N
-__device__ __forceinline__ void tc_block_product(const double* op, int ap, const double* bb, int N, int nt, int lane,
-                                                 double (&acc)[kTcMT][2]) {
-  const int g = lane >> 2, t4 = lane & 3;
-  const int MT = (N + 7) >> 3, KT = (N + 3) >> 2;
-  __syncwarp();  // mma.sync wants the whole warp converged
-#pragma unroll
-  for (int mt = 0; mt < kTcMT; ++mt) acc[mt][0] = acc[mt][1] = 0.0;
-#pragma unroll 3
-  for (int kt = 0; kt < KT; ++kt) {
-    const int c = kt * 4 + t4;
-    const bool cin = c < N;
-    const int cc = cin ? c : N - 1;  // in-range address for the padding
-    const double b = cin ? bb[(size_t)cc * kTcRS + nt * 8 + g] : 0.0;
-#pragma unroll
-    for (int mt = 0; mt < kTcMT; ++mt) {
-      if (mt < MT) {
-        const int r = mt * 8 + g;
-        const bool rin = r < N;
-        const double a = (cin && rin) ? op[(size_t)cc * ap + (rin ? r : N - 1)] : 0.0;
-        dmma884(acc[mt][0], acc[mt][1], a, b);
-      }
-    }
-  }
-}
-// both halves of the 16 right-hand sides at once (each A fragment loaded once)
-__device__ __forceinline__ void tc_block_product2(const double* op, int ap, const double* bb, int N, int lane,
-                                                  double (&acc)[2][kTcMT][2]) {
-  const int g = lane >> 2, t4 = lane & 3;
-  const int MT = (N + 7) >> 3, KT = (N + 3) >> 2;
-  __syncwarp();
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int mt = 0; mt < kTcMT; ++mt) acc[h][mt][0] = acc[h][mt][1] = 0.0;
-#pragma unroll 3
-  for (int kt = 0; kt < KT; ++kt) {
-    const int c = kt * 4 + t4;
-    const bool cin = c < N;
-    const int cc = cin ? c : N - 1;
-    const double b0 = cin ? bb[(size_t)cc * kTcRS + g] : 0.0;
-    const double b1 = cin ? bb[(size_t)cc * kTcRS + 8 + g] : 0.0;
-#pragma unroll
-    for (int mt = 0; mt < kTcMT; ++mt) {
-      if (mt < MT) {
-        const int r = mt * 8 + g;
-        const bool rin = r < N;
-        const double a = (cin && rin) ? op[(size_t)cc * ap + (rin ? r : N - 1)] : 0.0;
-        dmma884(acc[0][mt][0], acc[0][mt][1], a, b0);
-        dmma884(acc[1][mt][0], acc[1][mt][1], a, b1);
-      }
-    }
-  }
-}
-
 // role 0: u/v (4 RHS per column), 1: w, 2: rho, 3: pressure + projection.
-// TC: block products on the FP64 tensor cores (N <= 40), else one row per
-// thread on the FP64 pipes.
-template <typename T, int ROLE, bool TC = false>
+template <typename T, int ROLE>
 __global__ void __maxnreg__(72) k_solve_sys(
     Geo g, BlockInv bi, const Task* __restrict__ tasks, const int* __restrict__ col_order, T* __restrict__ F0,
     T* __restrict__ F1, T* __restrict__ F2, double rdiv, int meanu, const double* __restrict__ meang,
@@ -2611,7 +2525,7 @@ __global__ void __maxnreg__(72) k_solve_sys(
   constexpr int R = kSysR;
   constexpr int PER = ROLE == 0 ? 4 : 2;  // right-hand sides per column
   constexpr int NC = R / PER;             // column slots
-  constexpr int RS = TC ? kTcRS : kSysRS;  // right-hand-side row stride
+  constexpr int RS = kSysRS;  // right-hand-side row stride
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int cj[NC], cii[NC];
@@ -2619,8 +2533,7 @@ __global__ void __maxnreg__(72) k_solve_sys(
   const int n = g.nz, N = g.N, ns = g.ns, m = 2 * (ns - 1), nb = bi.nb;
   const int tid = threadIdx.x;
   const int s = tk.sys;
-  const int AP = TC ? tc_ap(N) : N;  // operator row stride in shared memory
-  const SysSmem L = sys_smem(n, N, ns, nb, ROLE == 3, RS, AP);
+  const SysSmem L = sys_smem(n, N, ns, nb, ROLE == 3);
   double* sA = sm + L.a;
   double* sL = sm + L.l;
   double* sM = sm + L.m;
@@ -2641,32 +2554,15 @@ __global__ void __maxnreg__(72) k_solve_sys(
   }
   __syncthreads();
   if (tid == 0) {
-    // (the tensor-core variant stages the inverse blocks itself, below, in
-    // rows of AP doubles)
-    mbar_expect_tx(&bar, (TC ? 0u : bytesA) + bytesL + bytesM);
-    if (!TC) bulk_g2s(sA, (const void*)(ga - (uintptr_t)offA * 8), bytesA, &bar);
+    mbar_expect_tx(&bar, bytesA + bytesL + bytesM);
+    bulk_g2s(sA, (const void*)(ga - (uintptr_t)offA * 8), bytesA, &bar);
     if (m > 0) {
       bulk_g2s(sL, bi.lvec + (size_t)s * m * N, bytesL, &bar);
       bulk_g2s(sM, bi.minv + (size_t)s * m * m, bytesM, &bar);
     }
   }
-  if (TC) {
-    const double* ag = (const double*)bi.ainv + (size_t)s * nb * N * N;
-    for (int q = tid; q < nb * N * N; q += blockDim.x) {
-      const int c = q / N, r = q - c * N;  // c runs over the blocks' columns
-      sA[(size_t)c * AP + r] = ag[q];
-    }
-  }
-  if (ROLE == 3) {
-    if (TC) {
-      for (int q = tid; q < N * N; q += blockDim.x) {
-        const int c = q / N, r = q - c * N;
-        sD[(size_t)c * AP + r] = Dt[q];
-      }
-    } else {
-      for (int q = tid; q < N * N; q += blockDim.x) sD[q] = Dt[q];
-    }
-  }
+  if (ROLE == 3)
+    for (int q = tid; q < N * N; q += blockDim.x) sD[q] = Dt[q];
   const double eps = bi.sys[s].eps;
   const double dt = g.dt;
   const int k = tid;
@@ -2708,59 +2604,8 @@ __global__ void __maxnreg__(72) k_solve_sys(
     mbar_wait(&bar, 0, 2000000000ull);
     return;
   }
-  const int lane = tid & 31, wid = tid >> 5, nwarp = blockDim.x >> 5;
-  if constexpr (TC) {
-    if (ROLE == 3) {
-      // divergence of u* per subdomain on the tensor cores, the RHS written
-      // over w* in place (a warp reads and writes only its own subdomains)
-      const int gq = lane >> 2, t4 = lane & 3, MT = (N + 7) >> 3;
-      const SysDesc sd = bi.sys[s];
-      for (int ks2 = wid; ks2 < ns; ks2 += nwarp) {
-        double* bb = sb + (size_t)ks2 * N * RS;
-        const double fac = g.hfac[ks2];
-        for (int nt = 0; nt < 2; ++nt) {
-          double tacc[kTcMT][2];
-          tc_block_product(sD, AP, bb, N, nt, lane, tacc);
-          __syncwarp();
-          const int c0 = nt * 8 + 2 * t4, ci = c0 >> 1;
-#pragma unroll
-          for (int mt = 0; mt < kTcMT; ++mt) {
-            const int r = mt * 8 + gq;
-            if (mt >= MT || r >= N) continue;
-            const int kq = ks2 * N + r;
-            double vr = 0.0, vi = 0.0;
-            if (cj[ci] >= 0) {
-              const int j = cj[ci], ii = cii[ci];
-              const size_t pr = fidx<T>(g, 2 * ii, j, kq);
-              const P2 u2 = *(const P2*)(F0 + pr), w2 = *(const P2*)(F1 + pr);
-              const double ur = (double)u2.x, ui = (double)u2.y;
-              const double wr = (double)w2.x, wi = (double)w2.y;
-              const double xw = g.xw[ii], yw = g.yw[j];
-              const double dr = -(xw * ui) - (yw * wi) + tacc[mt][0] * fac;
-              const double di = (xw * ur) + (yw * wr) + tacc[mt][1] * fac;
-              vr = -((dr / dt) * eps);
-              vi = -((di / dt) * eps);
-              if (kq == 0) {
-                const size_t p1 = (size_t)g.nxpp * j + 2 * ii;
-                vr -= (sd.tau1_bot * (wnl[p1] + wvr[p1])) * eps;
-                vi -= (sd.tau1_bot * (wnl[p1 + 1] + wvr[p1 + 1])) * eps;
-              }
-              if (kq == n - 1) {
-                const size_t p2 = (size_t)g.nxpp * (j + g.ny) + 2 * ii;
-                vr += (sd.tau2_top * (wnl[p2] + wvr[p2])) * eps;
-                vi += (sd.tau2_top * (wnl[p2 + 1] + wvr[p2 + 1])) * eps;
-              }
-            }
-            *(double2*)(bb + (size_t)r * RS + c0) = make_double2(vr, vi);
-          }
-          __syncwarp();
-        }
-      }
-      __syncthreads();
-    }
-  }
   double acc[R];
-  if (!TC && ROLE == 3) {
+  if (ROLE == 3) {
     // divergence of u*: i kx u* + i ky v* + (2/h) D w*; RHS = -(div/dt) eps
     // plus the Neumann data at the walls (calcuvwt.f:87-229)
     if (live) {
@@ -2825,115 +2670,6 @@ __global__ void __maxnreg__(72) k_solve_sys(
       szz[q] = z;
     }
     __syncthreads();
-  }
-  if constexpr (TC) {
-    // x = A_ks^-1 b_ks - A_ks^-1 e_0 z_{ks-1} - A_ks^-1 e_{N-1} z_{ns-1+ks} on
-    // the tensor cores; u/v, w, rho are stored, phi goes over the RHS in place
-    const int gq = lane >> 2, t4 = lane & 3, MT = (N + 7) >> 3;
-    for (int ks2 = wid; ks2 < ns; ks2 += nwarp) {
-      double* bb = sb + (size_t)ks2 * N * RS;
-      const double* blk = sA + (size_t)bi.bmap[ks2] * N * AP;
-      // the pressure writes phi over its own right-hand side, half by half;
-      // the other roles store to the fields and take both halves at once
-      double tacc2[2][kTcMT][2];
-      if (ROLE != 3) tc_block_product2(blk, AP, bb, N, lane, tacc2);
-      for (int nt = 0; nt < 2; ++nt) {
-        double tacc[kTcMT][2];
-        if (ROLE == 3) {
-          tc_block_product(blk, AP, bb, N, nt, lane, tacc);
-          __syncwarp();
-        } else {
-#pragma unroll
-          for (int mt = 0; mt < kTcMT; ++mt) {
-            tacc[mt][0] = tacc2[nt][mt][0];
-            tacc[mt][1] = tacc2[nt][mt][1];
-          }
-        }
-        const int c0 = nt * 8 + 2 * t4;
-#pragma unroll
-        for (int mt = 0; mt < kTcMT; ++mt) {
-          const int r = mt * 8 + gq;
-          if (mt >= MT || r >= N) continue;
-          const int kq = ks2 * N + r;
-          const double p = ks2 >= 1 ? blk[r] : 0.0;
-          const double q = ks2 <= ns - 2 ? blk[(size_t)(N - 1) * AP + r] : 0.0;
-          double x0 = tacc[mt][0], x1 = tacc[mt][1];
-          if (ks2 >= 1) {
-            x0 -= p * szz[(size_t)(ks2 - 1) * R + c0];
-            x1 -= p * szz[(size_t)(ks2 - 1) * R + c0 + 1];
-          }
-          if (ks2 <= ns - 2) {
-            x0 -= q * szz[(size_t)(ns - 1 + ks2) * R + c0];
-            x1 -= q * szz[(size_t)(ns - 1 + ks2) * R + c0 + 1];
-          }
-          if (ROLE == 3) {
-            *(double2*)(bb + (size_t)r * RS + c0) = make_double2(x0, x1);
-            continue;
-          }
-          const int ci = c0 / PER;
-          if (cj[ci] < 0) continue;
-          const bool second = ROLE == 0 && (c0 % 4) == 2;  // v of a u/v column
-          if (ROLE == 0 && !second && meanu && cii[ci] == 0 && cj[ci] == 0) {
-            x0 = meang[kq] * x0;
-            x1 = meang[kq] * x1;
-          }
-          P2 o;
-          o.x = (T)x0;
-          o.y = (T)x1;
-          *(P2*)((second ? F1 : F0) + fidx<T>(g, 2 * cii[ci], cj[ci], kq)) = o;
-        }
-        if (ROLE == 3) __syncwarp();
-      }
-    }
-    if (ROLE != 3) return;
-    // (2/h) D phi and the projection, per subdomain (phi of this warp's own
-    // subdomains, written above)
-    for (int ks2 = wid; ks2 < ns; ks2 += nwarp) {
-      const double* bb = sb + (size_t)ks2 * N * RS;
-      const double fac = g.hfac[ks2];
-      for (int nt = 0; nt < 2; ++nt) {
-        double tacc[kTcMT][2];
-        tc_block_product(sD, AP, bb, N, nt, lane, tacc);
-        const int c0 = nt * 8 + 2 * t4, ci = c0 >> 1;
-        if (cj[ci] < 0) continue;
-        const int j = cj[ci], ii = cii[ci];
-#pragma unroll
-        for (int mt = 0; mt < kTcMT; ++mt) {
-          const int r = mt * 8 + gq;
-          if (mt >= MT || r >= N) continue;
-          const int kq = ks2 * N + r;
-          const size_t pr = fidx<T>(g, 2 * ii, j, kq);
-          P2 zu, zv, zw;
-          if (kq < kstart) {
-            zu.x = zu.y = (T)0;
-            *(P2*)(F0 + pr) = zu;
-            *(P2*)(F1 + pr) = zu;
-            *(P2*)(F2 + pr) = zu;
-            continue;
-          }
-          const double phr = bb[(size_t)r * RS + c0], phi = bb[(size_t)r * RS + c0 + 1];
-          const P2 w2 = *(const P2*)(F2 + pr);
-          double wbr = 0, wbi = 0;
-          if (!(ii == 0 && j == 0)) {
-            wbr = (double)w2.x - dt * (tacc[mt][0] * fac);
-            wbi = (double)w2.y - dt * (tacc[mt][1] * fac);
-          }
-          const double dtx = dt * g.xw[ii], dty = dt * g.yw[j];
-          const P2 u2 = *(const P2*)(F0 + pr), v2 = *(const P2*)(F1 + pr);
-          const double ur = (double)u2.x, ui = (double)u2.y, vr = (double)v2.x, vi = (double)v2.y;
-          zu.x = (T)(ur + dtx * phi);
-          zu.y = (T)(ui - dtx * phr);
-          zv.x = (T)(vr + dty * phi);
-          zv.y = (T)(vi - dty * phr);
-          zw.x = (T)wbr;
-          zw.y = (T)wbi;
-          *(P2*)(F0 + pr) = zu;
-          *(P2*)(F1 + pr) = zv;
-          *(P2*)(F2 + pr) = zw;
-        }
-      }
-    }
-    return;
   }
   // x = A_ks^-1 b_ks - A_ks^-1 e_0 z_{ks-1} - A_ks^-1 e_{N-1} z_{ns-1+ks}
   double* x = acc;  // the solution replaces the product in place
@@ -3208,12 +2944,418 @@ __global__ void __launch_bounds__(kSys2MaxThreads, 2) k_solve_sys2(
   }
 }
 
+// ===========================================================================
+// System-grouped solve on the FP64 tensor cores (mma.sync m8n8k4, the FP64
+// matrix instruction of sm_100a; tcgen05 has no FP64 kind).  A task's columns
+// as in k_solve_sys; one warp owns one subdomain.  The products are formed
+// transposed, X^T = B^T Op^T: the right-hand sides are the 8 rows of the A
+// operand, the operator rows the 8 columns of the B operand, 4 operator
+// columns per instruction in ascending order.  The instruction adds its four
+// products one after the other, each with one rounding, so every sum is the
+// FMA chain of k_solve_cta and k_solve_sys and all variants give the same bits.
+// Every warp gathers the columns of its own subdomain (cp.async, in storage
+// precision), so the CTA only meets for the tables and around the interface
+// system: r_e = <lvec_e, b> (a sixth tile next to the block product's, from the
+// same operand loads), z = M^-1 r, x = A^-1 b - A^-1 e_0 z' - A^-1 e_{N-1} z''
+// (one more k step on the accumulators).  The pressure keeps the right-hand
+// side and phi in accumulator registers between its three products (D w*, A^-1,
+// D phi); four shuffles per k step turn them into the next A operand.
+// What bounds it: the shared-memory pipe (an operator fragment is two wavefronts
+// per tile product) and the gather and scatter of single complex values, then the
+// matrix pipe (36.9 TFLOP/s).  B200, 512^2 x (12 x 33) mixed, against the
+// FP64-pipe kernels (a broadcast load per multiply-add): pressure 7.97 -> 4.17 ms,
+// u/v 3.04 -> 2.49, w 2.01 -> 1.32; 256^2 x (8 x 25) FP64: pressure 1.04 -> 0.47 ms.
+// ===========================================================================
+constexpr int kTcMaxN = 40;
+// Operator columns in shared memory are AP = 4 (mod 8) doubles apart: the 4
+// columns x 8 rows of a B fragment then fall in two shared-memory wavefronts.
+__host__ __device__ inline int tc_ap(int N) {
+  int a = N;
+  while (a % 8 != 4) ++a;
+  return a;
+}
+// Staged right-hand sides: [tile][row][8] values of T; of FP64 rows the halves
+// swap places on every other pair of rows, so that an A fragment (4 rows x 8)
+// has no bank conflicts (FP32 fragments are 32 consecutive words as they are).
+template <typename T>
+__device__ __forceinline__ int tc_pos(int r, int g) {
+  return r * 8 + (sizeof(T) == 8 ? g ^ (((r >> 1) & 1) << 2) : g);
+}
+struct TcSmem {  // byte offsets
+  size_t a, l, m, rz, zz, d, raw, total;
+};
+// tiles: staged tiles of 8 right-hand sides (2; the pressure 3: u*, v*, w*)
+template <typename T>
+__host__ __device__ inline TcSmem tc_smem(int n, int N, int ns, int nb, bool press) {
+  TcSmem o;
+  const size_t m = 2 * (size_t)(ns - 1), ap = tc_ap(N), D = sizeof(double), R = press ? 8 : 16;
+  o.a = 0;
+  o.l = o.a + (size_t)nb * N * ap * D;
+  o.m = o.l + m * N * D;
+  o.rz = o.m + m * m * D;
+  o.zz = o.rz + m * R * D;
+  o.d = o.zz + m * R * D;
+  o.raw = o.d + (press ? (size_t)N * ap * D : 0);
+  o.total = o.raw + (press ? 3 : 2) * (size_t)n * 8 * sizeof(T) + 16 * D;  // (room for a fragment past the last column)
+  return o;
+}
+__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void cp_async_8(double* smem, const double* gmem) {
+  cp_async_c<float2>((float2*)smem, (const float2*)gmem);
+}
+// Markstein's division by a constant: y = RN(1 / d).  q within 2 ulp, one
+// correction makes it faithful, the next correctly rounded (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000", 1990).
+__device__ __forceinline__ double div_by(double v, double d, double y) {
+  double q = __dmul_rn(v, y);
+  q = __fma_rn(__fma_rn(-q, d, v), y, q);
+  return __fma_rn(__fma_rn(-q, d, v), y, q);
+}
+// acc[i][nt][h] += sum_c op[c ap + 8 nt + 2 t + h] b_i(c) for right-hand side g of NI
+// tiles: a(i, kt) gives b at row 4 kt + t (0 past N).  Rows past N read what follows
+// the column in shared memory; their sums are not used.  LEFT: also lacc[i]:
+// <l, b> for the left vector l of lane column g (null: 0).
+template <int NT, int NI, bool LEFT, typename A>
+__device__ __forceinline__ void tc_product(const double* op, int ap, int N, int g, int t, A&& a, double (&acc)[NI][NT][2],
+                                           const double* l, double (&lacc)[NI][2]) {
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) acc[i][nt][0] = acc[i][nt][1] = 0.0;
+    lacc[i][0] = lacc[i][1] = 0.0;
+  }
+#pragma unroll
+  for (int kt = 0; kt < 2 * NT; ++kt)
+    if (4 * kt < N) {  // the same for the whole warp
+      const int c = min(4 * kt + t, N - 1);
+      const double* o = op + (size_t)c * ap + g;
+      double b[NI];
+#pragma unroll
+      for (int i = 0; i < NI; ++i) b[i] = a(i, kt);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const double ov = o[8 * nt];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) dmma884(acc[i][nt][0], acc[i][nt][1], b[i], ov);
+      }
+      if (LEFT) {
+        const double lv = l ? l[c] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) dmma884(lacc[i][0], lacc[i][1], b[i], lv);
+      }
+    }
+}
+// acc -= A^-1 e_0 z0 + A^-1 e_{N-1} z1 (z0, z1 of right-hand side g; 0 without that neighbour)
+template <int NT>
+__device__ __forceinline__ void tc_rank2(const double* op, int ap, int N, int g, int t, double z0, double z1,
+                                         double (&acc)[NT][2]) {
+  const double* o = op + (t == 1 ? (size_t)(N - 1) * ap : 0) + g;
+  const double b = t == 0 ? -z0 : t == 1 ? -z1 : 0.0;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) dmma884(acc[nt][0], acc[nt][1], b, o[8 * nt]);
+}
+// Accumulators v[nt][h] (row 8 nt + 2 t + h of lane (g, t)) as the A operand of the next
+// product: row 4 kt + t
+template <int NT>
+__device__ __forceinline__ double tc_next(const double (&v)[NT][2], int kt, int g, int t) {
+  const int src = 4 * g + 2 * (kt & 1) + (t >> 1);
+  const double a = __shfl_sync(0xffffffffu, v[kt >> 1][0], src), b = __shfl_sync(0xffffffffu, v[kt >> 1][1], src);
+  return (t & 1) ? b : a;
+}
+// Lanes of an even and an odd right-hand side (re, im of one column) swap values
+// so that each holds one complex value: row 8 nt + 2 t of the even lane, the next row of
+// the odd one.
+template <typename T>
+__device__ __forceinline__ typename Pair<T>::t tc_pair(T v0, T v1, int g) {
+  const bool odd = g & 1;
+  const T r = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 4);
+  typename Pair<T>::t o;
+  o.x = odd ? r : v0;
+  o.y = odd ? v1 : r;
+  return o;
+}
+// z = M^-1 r for R right-hand sides, [e][r] in shared memory; ends synchronised
+template <int R>
+__device__ __forceinline__ void tc_interface(const double* sM, const double* srz, double* szz, int m, int nr) {
+  __syncthreads();
+  for (int q = threadIdx.x; q < m * R; q += blockDim.x) {
+    const int e = q / R, r = q - e * R;
+    if (r >= nr) continue;
+    const double* mr = sM + (size_t)e * m;
+    double z = 0.0;
+#pragma unroll 4
+    for (int c = 0; c < m; ++c) z = __fma_rn(mr[c], srz[(size_t)c * R + r], z);
+    szz[q] = z;
+  }
+  __syncthreads();
+}
+// the system's inverse blocks (columns AP apart), left vectors and interface matrix
+__device__ __forceinline__ void tc_tables(const double* ag, const double* lg, const double* mg, int nb, int N, int m,
+                                          int ap, double* sA, double* sL, double* sM) {
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < nb * N; c += blockDim.x >> 5)
+    for (int r = lane; r < N; r += 32) cp_async_8(sA + (size_t)c * ap + r, ag + (size_t)c * N + r);
+  for (int q = threadIdx.x; q < m * N; q += blockDim.x) cp_async_8(sL + q, lg + q);
+  for (int q = threadIdx.x; q < m * m; q += blockDim.x) cp_async_8(sM + q, mg + q);
+}
+
+// The u/v, w and rho solves do not depend on one another: one launch takes up
+// to three of them as jobs.
+template <typename T>
+struct TcJob {
+  const double *ainv, *lvec, *minv;
+  const SysDesc* sys;
+  const Task* tasks;
+  int first;     // first CTA of the job
+  int per;       // right-hand sides per column: 4 (u/v) or 2
+  int zero00;    // the (0,0) column has no system and becomes 0 (w)
+  int meanu;     // damp the (0,0) column of F0
+  double rdiv, irdiv;
+  T *F0, *F1;
+};
+template <typename T>
+struct TcJobs {
+  TcJob<T> j[3];
+  int n, nb;
+  int bmap[IW_MAX_SUBD];
+};
+template <typename T, int NT>
+__global__ void __maxnreg__(80) k_solve_tc(Geo g, const __grid_constant__ TcJobs<T> jobs,
+                                                  const int* __restrict__ col_order,
+                                                  const double* __restrict__ meang) {
+  typedef typename Pair<T>::t P2;
+  constexpr int R = 16;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  int ji = 0;
+  while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.j[ji + 1].first) ++ji;
+  const TcJob<T>& J = jobs.j[ji];
+  const Task tk = J.tasks[(int)blockIdx.x - J.first];
+  const int n = g.nz, N = g.N, ns = g.ns, m = 2 * (ns - 1), nb = jobs.nb, s = tk.sys;
+  const int tid = threadIdx.x, lane = tid & 31, ks = tid >> 5, lg = lane >> 2, lt = lane & 3;
+  const int AP = tc_ap(N);
+  const bool uv = J.per == 4;
+  const TcSmem L = tc_smem<T>(n, N, ns, nb, false);
+  double* sA = (double*)(smraw + L.a);
+  double* sL = (double*)(smraw + L.l);
+  double* sM = (double*)(smraw + L.m);
+  double* srz = (double*)(smraw + L.rz);
+  double* szz = (double*)(smraw + L.zz);
+  T* raw = (T*)(smraw + L.raw) + (size_t)ks * N * 8;  // this warp's rows of tile 0
+  const size_t ts = (size_t)n * 8;                    // tile stride
+  const int count = tk.count, nr = count * J.per, nmt = nr > 8 ? 2 : 1;
+  {
+    // complex slot sl of the 8 (2 tiles of 4): column sl (w, rho) or u, v of column sl / 2
+    const int sl = lane & 7, ci = uv ? sl >> 1 : sl;
+    const int c = ci < count ? col_order[tk.first + ci] : -1;
+    const int cj = c / g.nxhp;
+    const T* src = ((uv && (sl & 1)) ? J.F1 : J.F0) + (c < 0 ? 0 : fidx<T>(g, 2 * (c - cj * g.nxhp), cj, ks * N));
+    T* dst = raw + (sl >> 2) * ts;
+    const int p = 2 * (sl & 3);
+    for (int r = lane >> 3; r < N; r += 4) {
+      P2* d = (P2*)(dst + tc_pos<T>(r, p));
+      if (c >= 0)
+        cp_async_c<P2>(d, (const P2*)(src + (size_t)r * g.plane));
+      else
+        *d = P2{0, 0};
+    }
+  }
+  tc_tables(J.ainv + (size_t)s * nb * N * N, J.lvec + (size_t)s * m * N, J.minv + (size_t)s * m * m, nb, N, m, AP, sA, sL,
+            sM);
+  if (J.zero00 && (int)blockIdx.x == J.first)  // (0,0) column: element 0 of every plane
+    for (int k = tid; k < n; k += blockDim.x) *(P2*)(J.F0 + (size_t)k * g.plane) = P2{0, 0};
+  const double eps = J.sys[s].eps, rdiv = J.rdiv, irdiv = J.irdiv;
+  cp_async_wait_all();
+  __syncthreads();
+  const bool lo = ks >= 1, hi = ks <= ns - 2;  // neighbours below and above
+  // left vectors: c_{ks+1} on this block (lane column 0), d_{ks-1} (lane column 1)
+  const double* l = lg == 0 ? (hi ? sL + (size_t)ks * N : nullptr) : lg == 1 && lo ? sL + (size_t)(ns - 2 + ks) * N : nullptr;
+  const double* op = sA + (size_t)jobs.bmap[ks] * N * AP;
+  auto rhs = [&](int i, int kt) -> double {
+    const int r = 4 * kt + lt;
+    return r < N ? __dmul_rn(div_by((double)raw[i * ts + tc_pos<T>(r, lg)], rdiv, irdiv), eps) : 0.0;
+  };
+  auto body = [&](auto ni) {
+    constexpr int NI = decltype(ni)::value;
+    double acc[NI][NT][2], lacc[NI][2];
+    tc_product<NT, NI, true>(op, AP, N, lg, lt, rhs, acc, l, lacc);
+    if (m > 0) {
+      if (lt == 0) {
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+          if (hi) srz[(size_t)ks * R + 8 * i + lg] = lacc[i][0];
+          if (lo) srz[(size_t)(ns - 2 + ks) * R + 8 * i + lg] = lacc[i][1];
+        }
+      }
+      tc_interface<R>(sM, srz, szz, m, 8 * NI);
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        tc_rank2<NT>(op, AP, N, lg, lt, lo ? szz[(size_t)(ks - 1) * R + 8 * i + lg] : 0.0,
+                     hi ? szz[(size_t)(ns - 1 + ks) * R + 8 * i + lg] : 0.0, acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int slot = 4 * i + (lg >> 1), ci = uv ? slot >> 1 : slot;
+      const int c = ci < count ? col_order[tk.first + ci] : -1;
+      const int jj = c / g.nxhp;
+      T* dst = ((uv && (slot & 1)) ? J.F1 : J.F0) + (c < 0 ? 0 : fidx<T>(g, 2 * (c - jj * g.nxhp), jj, ks * N));
+      const bool mean = J.meanu && c == 0 && !(slot & 1);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int r = 8 * nt + 2 * lt, ro = r + (lg & 1);
+        double v0 = acc[i][nt][0], v1 = acc[i][nt][1];
+        if (mean) {
+          v0 = __dmul_rn(meang[ks * N + min(r, N - 1)], v0);
+          v1 = __dmul_rn(meang[ks * N + min(r + 1, N - 1)], v1);
+        }
+        const P2 o = tc_pair<T>((T)v0, (T)v1, lg);
+        if (c >= 0 && ro < N) *(P2*)(dst + (size_t)ro * g.plane) = o;
+      }
+    }
+  };
+  if (nmt == 2)
+    body(std::integral_constant<int, 2>());
+  else
+    body(std::integral_constant<int, 1>());
+}
+
+// Pressure and projection (calcuvwt.f:87-229, 826-901), 4 columns (8 right-hand
+// sides) per CTA; blockIdx.y takes the task's other columns.
+template <typename T, int NT>
+__global__ void __maxnreg__(80) k_press_tc(Geo g, const __grid_constant__ BlockInv bi,
+                                                  const Task* __restrict__ tasks, const int* __restrict__ col_order,
+                                                  T* __restrict__ U, T* __restrict__ V, T* __restrict__ W,
+                                                  const double* __restrict__ Dt, const double* __restrict__ wnl,
+                                                  const double* __restrict__ wvr, int kstart) {
+  typedef typename Pair<T>::t P2;
+  constexpr int R = 8;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const Task tk = tasks[blockIdx.x];
+  const int count = min(tk.count - 4 * (int)blockIdx.y, 4);
+  if (count <= 0) return;
+  const int* cols = col_order + tk.first + 4 * blockIdx.y;
+  const int n = g.nz, N = g.N, ns = g.ns, m = 2 * (ns - 1), nb = bi.nb, s = tk.sys;
+  const int tid = threadIdx.x, lane = tid & 31, ks = tid >> 5, lg = lane >> 2, lt = lane & 3;
+  const int AP = tc_ap(N);
+  const TcSmem L = tc_smem<T>(n, N, ns, nb, true);
+  double* sA = (double*)(smraw + L.a);
+  double* sL = (double*)(smraw + L.l);
+  double* sM = (double*)(smraw + L.m);
+  double* srz = (double*)(smraw + L.rz);
+  double* szz = (double*)(smraw + L.zz);
+  double* sD = (double*)(smraw + L.d);
+  T* raw = (T*)(smraw + L.raw) + (size_t)ks * N * 8;
+  const size_t ts = (size_t)n * 8;
+  {
+    const int ci = lane & 3;
+    const int c = ci < count ? cols[ci] : -1;
+    const int cj = c / g.nxhp;
+    const size_t cb = c < 0 ? 0 : fidx<T>(g, 2 * (c - cj * g.nxhp), cj, ks * N);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const T* src = (f == 0 ? U : f == 1 ? V : W) + cb;
+      for (int r = lane >> 2; r < N; r += 8) {
+        P2* d = (P2*)(raw + f * ts + tc_pos<T>(r, 2 * ci));
+        if (c >= 0)
+          cp_async_c<P2>(d, (const P2*)(src + (size_t)r * g.plane));
+        else
+          *d = P2{0, 0};
+      }
+    }
+  }
+  for (int c = ks; c < N; c += ns)
+    for (int r = lane; r < N; r += 32) cp_async_8(sD + (size_t)c * AP + r, Dt + (size_t)c * N + r);
+  tc_tables((const double*)bi.ainv + (size_t)s * nb * N * N, bi.lvec + (size_t)s * m * N, bi.minv + (size_t)s * m * m, nb, N,
+            m, AP, sA, sL, sM);
+  const double eps = bi.sys[s].eps, dt = g.dt, fac = g.hfac[ks];
+  const int c = (lg >> 1) < count ? cols[lg >> 1] : -1;
+  const bool cok = c >= 0;
+  const int cj = cok ? c / g.nxhp : 0, cii = cok ? c - cj * g.nxhp : 0;
+  const double xw = g.xw[cii], yw = g.yw[cj];
+  cp_async_wait_all();
+  __syncthreads();
+  const bool lo = ks >= 1, hi = ks <= ns - 2, im = lg & 1;
+  const double* l = lg == 0 ? (hi ? sL + (size_t)ks * N : nullptr) : lg == 1 && lo ? sL + (size_t)(ns - 2 + ks) * N : nullptr;
+  const double* op = sA + (size_t)bi.bmap[ks] * N * AP;
+  const T *ru = raw, *rv = raw + ts, *rw = raw + 2 * ts;
+  double acc[1][NT][2], bv[NT][2], lacc[1][2];
+  tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) {
+    const int r = 4 * kt + lt;
+    return r < N ? (double)rw[tc_pos<T>(r, lg)] : 0.0;
+  }, acc, nullptr, lacc);
+  // b = -((i kx u* + i ky v* + (2/h) D w*) / dt) eps and the Neumann data at the walls
+  const double idt = __drcp_rn(dt);
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 8 * nt + 2 * lt + h, k = ks * N + r;
+      double v = 0.0;
+      if (r < N) {
+        const double up = (double)ru[tc_pos<T>(r, lg ^ 1)], vp = (double)rv[tc_pos<T>(r, lg ^ 1)];
+        const double b = __fma_rn(xw, up, __dmul_rn(yw, vp));
+        const double div = __fma_rn(acc[0][nt][h], fac, im ? b : -b);
+        v = -__dmul_rn(div_by(div, dt, idt), eps);
+        if (cok && k == 0) {
+          const size_t p1 = (size_t)g.nxpp * cj + 2 * cii + im;
+          v = __fma_rn(-__dmul_rn(bi.sys[s].tau1_bot, __dadd_rn(wnl[p1], wvr[p1])), eps, v);
+        }
+        if (cok && k == n - 1) {
+          const size_t p2 = (size_t)g.nxpp * (cj + g.ny) + 2 * cii + im;
+          v = __fma_rn(__dmul_rn(bi.sys[s].tau2_top, __dadd_rn(wnl[p2], wvr[p2])), eps, v);
+        }
+      }
+      bv[nt][h] = v;
+    }
+  tc_product<NT, 1, true>(op, AP, N, lg, lt, [&](int, int kt) { return tc_next<NT>(bv, kt, lg, lt); }, acc, l, lacc);
+  if (m > 0) {
+    if (lt == 0) {
+      if (hi) srz[(size_t)ks * R + lg] = lacc[0][0];
+      if (lo) srz[(size_t)(ns - 2 + ks) * R + lg] = lacc[0][1];
+    }
+    tc_interface<R>(sM, srz, szz, m, R);
+    tc_rank2<NT>(op, AP, N, lg, lt, lo ? szz[(size_t)(ks - 1) * R + lg] : 0.0,
+                 hi ? szz[(size_t)(ns - 1 + ks) * R + lg] : 0.0, acc[0]);
+  }
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) bv[nt][h] = 8 * nt + 2 * lt + h < N ? acc[0][nt][h] : 0.0;
+  tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) { return tc_next<NT>(bv, kt, lg, lt); }, acc, nullptr, lacc);
+  const double dtx = __dmul_rn(dt, xw), dty = __dmul_rn(dt, yw);
+  const size_t cb = fidx<T>(g, 2 * cii, cj, ks * N);
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    T u[2], v[2], w[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 8 * nt + 2 * lt + h, p = tc_pos<T>(min(r, N - 1), lg);
+      const double pp = __shfl_xor_sync(0xffffffffu, bv[nt][h], 4);  // the other part of phi
+      u[h] = (T)__fma_rn(im ? -dtx : dtx, pp, (double)ru[p]);
+      v[h] = (T)__fma_rn(im ? -dty : dty, pp, (double)rv[p]);
+      w[h] = (T)__fma_rn(-dt, __dmul_rn(acc[0][nt][h], fac), (double)rw[p]);
+      if (ks * N + r < kstart) u[h] = v[h] = w[h] = (T)0;
+    }
+    const P2 zu = tc_pair<T>(u[0], u[1], lg), zv = tc_pair<T>(v[0], v[1], lg), zw = tc_pair<T>(w[0], w[1], lg);
+    const int ro = 8 * nt + 2 * lt + (lg & 1);
+    if (cok && ro < N) {
+      const size_t p = cb + (size_t)ro * g.plane;
+      *(P2*)(U + p) = zu;
+      *(P2*)(V + p) = zv;
+      *(P2*)(W + p) = zw;
+    }
+  }
+}
+
 // Distinct blocks of each system into compact storage: out[s][b] = in[s][rep[b]],
 // with the Legendre filter folded in when L is given (out = L in, per column).
 struct BlockRep {
   int r[IW_MAX_SUBD];
 };
-__global__ void k_compact_blocks(int N, int nsys, int ns, int nb, BlockRep rep, const double* __restrict__ L,
+static __global__ void k_compact_blocks(int N, int nsys, int ns, int nb, BlockRep rep, const double* __restrict__ L,
                                  const double* __restrict__ in, double* __restrict__ out) {
   const size_t nn = (size_t)N * N, tot = (size_t)nsys * nb * nn;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < tot; q += (size_t)gridDim.x * blockDim.x) {
@@ -3237,7 +3379,7 @@ __global__ void k_compact_blocks(int N, int nsys, int ns, int nb, BlockRep rep, 
 
 // lvec[s][e][c] = sum_k A_blk^-1[k][c] v_e[k]: v_e = c_{e+1} on block e (e < ns-1),
 // d_t on block t+1 (e = ns-1+t).  One thread per (system, e, c).
-__global__ void k_left_vecs(Geo g, int nsys, const double* __restrict__ ainv, const double* __restrict__ cvec,
+static __global__ void k_left_vecs(Geo g, int nsys, const double* __restrict__ ainv, const double* __restrict__ cvec,
                             const double* __restrict__ dvec, double* __restrict__ lvec) {
   const int N = g.N, ns = g.ns, m = 2 * (ns - 1);
   const size_t tot = (size_t)nsys * m * N;
