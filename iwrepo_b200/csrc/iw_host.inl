@@ -351,8 +351,6 @@ struct iw_handle {
   double *dD = 0, *dD2 = 0, *dL = 0, *dh = 0, *dxw = 0, *dyw = 0, *dcf = 0, *dzg = 0, *dzh = 0;
   double *dwg = 0, *dal = 0, *dsig = 0, *dmeang = 0;
   double *dwnl = 0, *dwvr = 0, *dred = 0;
-  unsigned char* deops = 0;  // stage E's padded operators for k_stageE_b (EArgs::ops), built at init
-  unsigned eops_bytes = 0;
   int* dcnt = 0;
   int* dflag = 0;
   int* derr = 0;  // device error words: [0] non-finite state, [1] a bounded device wait gave up
@@ -399,6 +397,7 @@ struct iw_handle {
   // 0: k_solve_cta for every task, 1: k_solve_sys, 2: k_solve_tc (k_solve_sys where it does not apply), 3: k_solve_sys2
   int use_sys = 2;
   int sys_role[4] = {-1, -1, -1, -1};  // per solve role (u/v, w, rho, pressure), set by iw_autotune; -1: use_sys
+  int nsm = 148;  // SMs of the device (persistent kernels)
   double bi_bdfv[SYS_KINDS] = {-1, -1, -1, -1};
   bool bi_fold[SYS_KINDS] = {false, false, false, false};  // Legendre filter folded into ainv
   // distinct subdomain blocks: subdomain ks uses block bmap[ks]; brep[b] is a
@@ -953,6 +952,13 @@ static ZOp<T, NM> make_zop(const iw_handle* h) {
   return op;
 }
 
+// CTAs of the persistent tensor-core z kernels: `occ` per SM, W warps each, no more
+// than there are tiles of 8 points
+static int z_grid(const iw_handle* h, int W, int occ) {
+  const int tiles = (int)((h->plane + 7) / 8) * 4 * h->ns;
+  return std::min((tiles + W - 1) / W, occ * h->nsm);
+}
+
 template <typename T, int NM>
 static void launch_stageA_r(iw_handle* h, FieldSet<T>& fs, int proj) {
   dim3 grid((unsigned)((h->plane + 127) / 128), (unsigned)h->ns, 4);
@@ -963,6 +969,18 @@ static void launch_stageA_r(iw_handle* h, FieldSet<T>& fs, int proj) {
 
 template <typename T>
 void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj) {
+  if (h->tune_a < 0 && h->N <= kTcMaxN) {  // tensor-core kernel
+    const size_t sm = ((size_t)tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);
+    const int blocks = z_grid(h, 16, 2);
+#define IW_ATCASE(NT)                                                                                                   \
+  case NT:                                                                                                              \
+    k_stageA_t<T, NT><<<blocks, 512, sm, h->st>>>(geo(h), fs.F[0], fs.F[1], fs.F[2], fs.F[3], fs.F1[0], fs.F1[1],       \
+                                                  fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], fs.Z4[3], proj,     \
+                                                  h->derr);                                                             \
+    return;
+    switch (tc_nt(h->N)) { IW_ATCASE(2) IW_ATCASE(3) IW_ATCASE(4) IW_ATCASE(5) }
+#undef IW_ATCASE
+  }
   switch (h->tune_a == 0 ? 0 : zop_bucket(h->N)) {
     case 9: launch_stageA_r<T, 9>(h, fs, proj); return;
     case 17: launch_stageA_r<T, 17>(h, fs, proj); return;
@@ -979,39 +997,12 @@ void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj) {
                                                 h->derr);
 }
 
-template <typename T>
-static bool stageE_b_fits(const iw_handle* h, bool cb = false) {
-  const int nm = zop_bucket(h->N);
-  return nm > 0 && eb_smem<T>(h->N, nm, cb) <= 200 * 1024 && (h->plane * sizeof(T)) % 16 == 0;
-}
+// Stage E on the tensor cores: the default where it applies
+static bool stageE_is_t(const iw_handle* h) { return (h->tune_e < 0 || h->tune_e >= 2) && h->N <= kTcMaxN; }
 
-// Stage E's operators zero-padded to the register bucket NM, in the layout of
-// k_stageE_b's shared memory: [NM][NP] doubles of L - I, then [NM][NP] values
-// of D in the storage type, rounded up to 16 bytes (one bulk copy per CTA).
+// cols: u* to whole-column scratch fields (Y12[0..3]) instead of F; only with stageE_is_t
 template <typename T>
-static std::vector<unsigned char> stageE_ops(const iw_handle* h, int NM) {
-  const int N = h->N, NP = eb_np(NM);
-  const size_t nl = (size_t)NM * NP * sizeof(double), nd = (size_t)NM * NP * sizeof(T);
-  std::vector<unsigned char> out((nl + nd + 15) & ~(size_t)15, 0);
-  double* L = (double*)out.data();
-  T* D = (T*)(out.data() + nl);
-  for (int r = 0; r < N; ++r)
-    for (int c = 0; c < N; ++c) {
-      L[(size_t)r * NP + c] = h->tab.Lfil[(size_t)r * N + c] - (r == c ? 1.0 : 0.0);
-      D[(size_t)r * NP + c] = (T)h->tab.D[(size_t)r * N + c];
-    }
-  return out;
-}
-static int build_stageE_ops(iw_handle* h) {
-  const int nm = zop_bucket(h->N);
-  if (nm <= 0) return 0;  // no bulk-staged stage E at this N
-  const std::vector<unsigned char> t = h->mixed ? stageE_ops<float>(h, nm) : stageE_ops<double>(h, nm);
-  h->eops_bytes = (unsigned)t.size();
-  return up(h, &h->deops, t);
-}
-
-template <typename T>
-void launch_stageE(iw_handle* h, FieldSet<T>& fs) {
+void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
   EArgs<T> a;
   for (int q = 0; q < 4; ++q) {
     a.B[q] = fs.B8[q];
@@ -1025,42 +1016,24 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs) {
   }
   a.wnl = h->dwnl;
   a.filter = h->p.ispecfilternl == 1;
-  // the prebuilt operator table holds the handle's storage type
-  const bool own = h->deops && (h->mixed ? sizeof(T) == 4 : sizeof(T) == 8);
-  a.ops = own ? h->deops : nullptr;
-  a.ops_bytes = own ? h->eops_bytes : 0u;
+  if (stageE_is_t(h)) {
+    if (cols)
+      for (int q = 0; q < 4; ++q) a.F[q] = fs.Y12[q];
+    const size_t ops = ((size_t)2 * tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);
+    const int W = (int)std::min<size_t>(sizeof(T) == 4 ? 20 : 16, (226 * 1024 - ops) / ze_buf<T>(h->N));
+    const size_t sm = ops + (size_t)W * ze_buf<T>(h->N);
+    const int blocks = z_grid(h, W, 1), v16 = (h->plane * sizeof(T)) % 16 == 0;
+#define IW_ETCASE(NT)                                                                                        \
+  case NT:                                                                                                   \
+    cudaFuncSetAttribute(k_stageE_t<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);           \
+    k_stageE_t<T, NT><<<blocks, 32 * W, sm, h->st>>>(geo(h), a, h->c, cols, v16);                            \
+    return;
+    switch (tc_nt(h->N)) { IW_ETCASE(2) IW_ETCASE(3) IW_ETCASE(4) IW_ETCASE(5) }
+#undef IW_ETCASE
+  }
   const dim3 rgrid((unsigned)((h->plane + 127) / 128), (unsigned)h->ns, 4);
   // The register-column stage E holds two columns per thread; past these sizes
   // its register count costs more occupancy than the tiled kernel loses.
-  // tune_e = 2: the tiled kernel with its input tiles staged by bulk copies
-  // and its z operators unrolled at the register-column bucket size (N <= 33)
-  // tune_e = 3: the same kernel with its operators in the constant bank
-  const bool cb = h->tune_e == 3;
-  if ((h->tune_e == 2 || cb) && stageE_b_fits<T>(h, cb)) {
-    dim3 grid((unsigned)((h->nxpp + kTX - 1) / kTX), (unsigned)(h->ny * h->ns), 4);
-    const int nm = zop_bucket(h->N);
-    const size_t smem = eb_smem<T>(h->N, nm, cb);
-    switch (nm) {
-#define IW_EBCASE(NM)                                                                                              \
-  case NM:                                                                                                         \
-    if (cb) {                                                                                                      \
-      cudaFuncSetAttribute(k_stageE_b<T, NM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-      k_stageE_b<T, NM, true><<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c, h->derr, make_zop<T, NM>(h));    \
-    } else {                                                                                                       \
-      cudaFuncSetAttribute(k_stageE_b<T, NM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-      k_stageE_b<T, NM, false><<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c, h->derr, make_zop<T, NM>(h));   \
-    }                                                                                                              \
-    return;
-      IW_EBCASE(9)
-      IW_EBCASE(17)
-      IW_EBCASE(21)
-      IW_EBCASE(25)
-      IW_EBCASE(29)
-      IW_EBCASE(33)
-#undef IW_EBCASE
-      default: break;
-    }
-  }
   const int emax = sizeof(T) == 4 ? 25 : 17;
   const bool reg = h->tune_e < 0 ? h->N <= emax : h->tune_e == 1;
   switch (reg ? zop_bucket(h->N) : 0) {
@@ -1262,7 +1235,7 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
 
 #ifndef IW_INST
 template <typename T>
-static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj) {
+static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj, int cols = 0) {
   typedef typename cplx_t<T>::type C;
   Geo g = geo(h);
   const int M = h->nx / 2;
@@ -1308,14 +1281,14 @@ static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj) {
   mark(h, 3);
   // wall pressure BC term (before the histories rotate)
   {
-    long total = (long)h->nxhp * h->ny * 2;
-    k_wviscrot<T><<<(unsigned)((total + 127) / 128), 128, 0, h->st>>>(g, fs.F1[0], fs.F1[1], fs.F1[2], fs.Fn[0],
+    const dim3 wgrid((unsigned)((h->nxhp + 31) / 32), (unsigned)h->ny, 2);
+    k_wviscrot<T><<<wgrid, 192, 0, h->st>>>(g, fs.F1[0], fs.F1[1], fs.F1[2], fs.Fn[0],
                                                                       fs.Fn[1], fs.Fn[2], fs.Fnm[0], fs.Fnm[1],
                                                                       fs.Fnm[2], h->c, h->p.xnu, h->dwvr);
   }
   mark(h, 4);
   // K_E
-  launch_stageE<T>(h, fs);
+  launch_stageE<T>(h, fs, cols);
   mark(h, 5);
   rotate_levels(fs);
   return 0;
@@ -1448,10 +1421,11 @@ static bool tc_zero00(const iw_handle* h, int role) {
 // for all of them; 3: the pressure).  The row tiles of 8 are fixed at compile
 // time; one warp per subdomain.
 template <typename T>
-void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles, int kstart) {
+void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles, int kstart, int cols) {
   const Geo g = geo(h);
-  const int nt = std::max((h->N + 7) / 8, 2);
+  const int nt = tc_nt(h->N);
   const size_t smem = tc_smem<T>(h->nz, h->N, h->ns, h->nb, roles[0] == 3).total;
+  T* const* S = cols ? fs.Y12 : fs.F;  // where stage E left u*, v*, w*, rho*
   if (roles[0] == 3) {
     if (h->ntask2[SYS_P] <= 0) return;
     const auto& B = h->bi[SYS_P];
@@ -1467,8 +1441,8 @@ void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles
 #define IW_TC_CASE(NT)                                                                                             \
   case NT:                                                                                                         \
     cudaFuncSetAttribute(k_press_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-    k_press_tc<T, NT><<<grid, 32 * h->ns, smem, h->st>>>(g, bi, h->dtasks2[SYS_P], h->dcolorder, fs.F[0], fs.F[1], \
-                                                         fs.F[2], h->dDt, h->dwnl, h->dwvr, kstart);               \
+    k_press_tc<T, NT><<<grid, 32 * h->ns, smem, h->st>>>(g, bi, h->dtasks2[SYS_P], h->dcolorder, S[0], S[1], S[2], \
+                                                         h->dDt, h->dwnl, h->dwvr, kstart, cols);                  \
     break;
     switch (nt) { IW_TC_CASE(2) IW_TC_CASE(3) IW_TC_CASE(4) IW_TC_CASE(5) }
 #undef IW_TC_CASE
@@ -1477,6 +1451,7 @@ void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles
   TcJobs<T> jobs;
   memset(&jobs, 0, sizeof jobs);
   jobs.nb = h->nb;
+  jobs.cols = cols;
   memcpy(jobs.bmap, h->bmap, sizeof jobs.bmap);
   int nblk = 0;
   for (int i = 0; i < nroles; ++i) {
@@ -1497,6 +1472,8 @@ void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles
     j.irdiv = 1.0 / j.rdiv;
     j.F0 = fs.F[role == 0 ? 0 : role + 1];
     j.F1 = fs.F[1];
+    j.S0 = S[role == 0 ? 0 : role + 1];
+    j.S1 = S[1];
     nblk += h->ntask2[kind];
   }
   if (nblk == 0) return;
@@ -1510,7 +1487,7 @@ void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles
 }
 
 template <typename T>
-void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int kstart, bool tc_done = false) {
+void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int kstart, int cols, bool tc_done) {
   constexpr int R = 4;
   const int kind = role_kind(role);
   BlockInv bi;
@@ -1530,10 +1507,11 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   const size_t sm = ((size_t)2 * R * h->nz + 2 * R * mm) * sizeof(double) +
                     (role == 3 ? (size_t)3 * R * h->nz * sizeof(T) : 0);
   T *F0, *F1 = nullptr, *F2 = nullptr;
+  T* const* S = cols ? fs.Y12 : fs.F;  // where stage E left u*, v*, w*, rho*
   if (role == 3) {
-    F0 = fs.F[0];
-    F1 = fs.F[1];
-    F2 = fs.F[2];
+    F0 = S[0];
+    F1 = S[1];
+    F2 = S[2];
   } else if (role == 0) {
     F0 = fs.F[0];
     F1 = fs.F[1];
@@ -1553,7 +1531,7 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   const bool tc = us == 2;
   int nend = us ? std::max(h->nold[kind], nref) : nt;
   if (tc && tc_zero00(h, role) && h->ntask2[kind] > 0) nend = 0;
-  if (tc && !tc_done) launch_solve_tc<T>(h, fs, &role, 1, kstart);
+  if (tc && !tc_done) launch_solve_tc<T>(h, fs, &role, 1, kstart, cols);
   if (us && !tc && h->ntask2[kind] > 0) {
     const size_t smsys = sys_smem(h->nz, h->N, h->ns, h->nb, role == 3).total * sizeof(double);
     const int nthr = (h->nz + 31) / 32 * 32, nthr2 = (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32;
@@ -1604,7 +1582,7 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
         cp = 0;
     }
     k_solve_cta<T, R><<<cnt, kSolveThreads, sm, h->st>>>(geo(h), b2, solve_tabs(h, kind), h->dtasks[kind] + t0, F0, F1,
-                                                          F2, rd, role, cp, meanu, part == 0 ? 1 : 0, h->dDt, h->dD2t,
+                                                          F2, S[role == 0 || role == 3 ? 0 : role + 1], S[1], cols, rd, role, cp, meanu, part == 0 ? 1 : 0, h->dDt, h->dD2t,
                                                           h->dLt, h->dzh, h->dwnl, h->dwvr, kstart);
   }
 }
@@ -1616,9 +1594,9 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   X template void launch_xrow<T>(iw_handle*, FieldSet<T>&);
 #define IW_INST_Z(X, T)                                                             \
   X template void launch_stageA<T>(iw_handle*, FieldSet<T>&, int);                  \
-  X template void launch_stageE<T>(iw_handle*, FieldSet<T>&);                       \
-  X template void launch_solve_tc<T>(iw_handle*, FieldSet<T>&, const int*, int, int); \
-  X template void launch_solve_bi<T>(iw_handle*, FieldSet<T>&, int, int, int, bool);
+  X template void launch_stageE<T>(iw_handle*, FieldSet<T>&, int);                  \
+  X template void launch_solve_tc<T>(iw_handle*, FieldSet<T>&, const int*, int, int, int); \
+  X template void launch_solve_bi<T>(iw_handle*, FieldSet<T>&, int, int, int, int, bool);
 #if defined(IW_INST)
 #if IW_INST == 1
 IW_INST_FFT(, float)
@@ -1637,7 +1615,7 @@ IW_INST_Z(extern, double)
 
 // calcuvwt (calcuvwt_noslip.f / calcuvwt.f) on u*,v*,w*,rho* held in F.
 template <typename T>
-static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen) {
+static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen, int cols = 0) {
   Geo g = geo(h);
   const int warps = 4;
   const unsigned nblk = (unsigned)((h->ncol + warps - 1) / warps);
@@ -1645,7 +1623,7 @@ static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen) {
   const int kstart = h->p.bc_variant == IW_BC_NOSLIP ? 1 : 0;
   cudaFuncSetAttribute(k_visc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (h->use_bi) {
-    launch_solve_bi<T>(h, fs, 3, cpen, kstart);
+    launch_solve_bi<T>(h, fs, 3, cpen, kstart, cols, false);
   } else {
   {
     constexpr int G = 2;
@@ -1665,9 +1643,9 @@ static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen) {
     int tcr[3], ntc = 0;
     for (int role = 0; role < 3 && !h->prof; ++role)
       if (solve_variant<T>(h, role, cpen) == 2) tcr[ntc++] = role;
-    if (ntc > 0) launch_solve_tc<T>(h, fs, tcr, ntc, kstart);
+    if (ntc > 0) launch_solve_tc<T>(h, fs, tcr, ntc, kstart, cols);
     for (int role = 0; role < 3; ++role) {
-      launch_solve_bi<T>(h, fs, role, cpen, kstart, !h->prof);
+      launch_solve_bi<T>(h, fs, role, cpen, kstart, cols, !h->prof);
       mark(h, 7 + role);
     }
   } else {
@@ -1719,6 +1697,16 @@ static int iface_avg(iw_handle* h, FieldSet<T>& fs, bool count, int nf = 4) {
   return 0;
 }
 
+// Whether stage E leaves u*, v*, w*, rho* as whole columns in scratch for the
+// solves: all four solve roles on the tensor-core kernel, which then read (and the
+// pressure writes) consecutive rows instead of one value per z-plane.
+template <typename T>
+static int step_cols(const iw_handle* h, int cpen) {
+  bool ok = h->use_bi && stageE_is_t(h);
+  for (int role = 0; role < 4 && ok; ++role) ok = solve_variant<T>(h, role, cpen) == 2;
+  return ok;
+}
+
 template <typename T>
 static int full_step(iw_handle* h, FieldSet<T>& fs) {
   h->istep += 1;
@@ -1733,9 +1721,10 @@ static int full_step(iw_handle* h, FieldSet<T>& fs) {
   const int cpen = (h->p.ispecfilterexp == 1) && (h->istep % h->p.nspecfilterexp == 0);
   r = ensure_factors(h, cpen);
   if (r) return r;
-  convec_impl<T>(h, fs, 1);
+  const int cols = step_cols<T>(h, cpen);
+  convec_impl<T>(h, fs, 1, cols);
   schedule_after_convec(h);
-  calcuvwt_impl<T>(h, fs, cpen);
+  calcuvwt_impl<T>(h, fs, cpen, cols);
   schedule_after_calcuvwt(h);
   h->t = h->t + h->p.dt;
   if (h->nlegspec > 0 && h->istep % h->nlegspec == 0 && (r = legspec_dump<T>(h, fs))) return r;  // main.f:905-910
@@ -1823,24 +1812,29 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
     h->tune_xthr = bestx;
   }
   // stage A and stage E variants
-  int besta = -1, beste = -1;
-  if (zop_bucket(h->N)) {
-    float ta[2];
-    for (int v = 0; v < 2; ++v) {
+  int besta = h->N <= kTcMaxN || zop_bucket(h->N) == 0 ? -1 : 1, beste = -1;
+  {
+    // -1: the tensor-core kernel where it applies, else by size
+    float ta = 0;
+    for (int v : {-1, 0, 1}) {
+      if (v == 1 && !zop_bucket(h->N)) continue;
+      if (v == -1 && h->N > kTcMaxN) continue;
       h->tune_a = v;
-      ta[v] = timeit([&] { launch_stageA<T>(h, ts, 1); });
+      const float t = timeit([&] { launch_stageA<T>(h, ts, 1); });
+      if (ta == 0 || t < ta) {
+        ta = t;
+        besta = v;
+      }
     }
-    besta = ta[1] <= ta[0] ? 1 : 0;
   }
   {
-    // 0 tiled (any N), 1 register-column (N in a register bucket), 2 tiled
-    // with bulk-copied input tiles (N in a register bucket)
+    // 0 tiled (any N), 1 register-column (N in a register bucket), 2 tensor
+    // cores (N <= 40)
     float bt = 0;
-    for (int v = 0; v < 4; ++v) {
-      if ((v == 1 && !zop_bucket(h->N)) || (v == 2 && !stageE_b_fits<T>(h)) || (v == 3 && !stageE_b_fits<T>(h, true)))
-        continue;
+    for (int v = 0; v < 3; ++v) {
+      if ((v == 1 && !zop_bucket(h->N)) || (v == 2 && h->N > kTcMaxN)) continue;
       h->tune_e = v;
-      const float t = timeit([&] { launch_stageE<T>(h, ts); });
+      const float t = timeit([&] { launch_stageE<T>(h, ts, v == 2 && h->use_bi); });
       if (beste < 0 || t < bt) {
         bt = t;
         beste = v;
@@ -1863,7 +1857,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
         if (v == 2 && h->N > kTcMaxN) continue;
         if (v == 3 && (role == 3 || (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32 > kSys2MaxThreads)) continue;
         h->sys_role[role] = v;
-        const float t = timeit([&] { launch_solve_bi<T>(h, ts, role, cpen, kstart); });
+        const float t = timeit([&] { launch_solve_bi<T>(h, ts, role, cpen, kstart, v == 2 && stageE_is_t(h), false); });
         if (v == 0 || t < best) {
           best = t;
           bestv = v;
@@ -1886,7 +1880,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
   }
   if (choice) {
     choice[0] = h->tune_ytx;
-    choice[1] = h->tune_a;
+    choice[1] = h->tune_a < 0 && zop_bucket(h->N) ? 1 : h->tune_a;  // the tensor-core kernel's columns sit in registers too
     choice[2] = h->tune_e;
     choice[3] = h->sys_role[3] >= 0 ? h->sys_role[3] : h->use_sys;
   }
@@ -2090,6 +2084,7 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
   } else {
     cudaGetDevice(&h->dev);
   }
+  cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->dev);
   h->nx = d.nx;
   h->ny = d.ny;
   h->N = d.nzloc;
@@ -2175,7 +2170,6 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
        up(h, &h->dxw, xw) || up(h, &h->dyw, yw) || up(h, &h->dcf, cf) || up(h, &h->dzg, zg) || up(h, &h->dzh, zh) ||
        up(h, &h->dwg, h->tab.wg) || up(h, &h->dal, h->tab.alpol) || up(h, &h->dsig, h->tab.sigma) ||
        up(h, &h->dmeang, mg);
-  if (!r) r = build_stageE_ops(h);
   r |= dalloc(h, &h->dwnl, h->plane * 2) || dalloc(h, &h->dwvr, h->plane * 2) || dalloc(h, &h->dred, std::max<size_t>(64, 4 * (size_t)h->nz)) ||
        dalloc(h, &h->dcnt, 8) || dalloc(h, &h->dflag, 4) || dalloc(h, &h->derr, 2) ||
        cudaHostAlloc((void**)&h->herr, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
@@ -2234,7 +2228,6 @@ int iw_destroy(iw_handle* h) {
   for (double* p : {h->ddzinv, h->dpart, h->dDt, h->dD2t, h->dLt, h->dD, h->dD2, h->dL, h->dh, h->dxw, h->dyw, h->dcf, h->dzg, h->dzh, h->dwg, h->dal, h->dsig,
                     h->dmeang, h->dwnl, h->dwvr, h->dred})
     cudaFree(p);
-  cudaFree(h->deops);
   cudaFree(h->dcnt);
   cudaFree(h->dflag);
   cudaFree(h->derr);
@@ -2385,7 +2378,7 @@ int iw_set_launch(iw_handle* h, int which, int value) {
       if (value < -1 || value > (which == IW_LAUNCH_STAGE_E ? 3 : 1))
         return set_err(IW_ERR_CONFIG, "stage variant: -1, 0, 1 (or 2, 3 for stage E)");
       if (value == 1 && !zop_bucket(h->N)) return set_err(IW_ERR_CONFIG, "register-column stages need N <= 33");
-      if (value >= 2 && !(h->mixed ? stageE_b_fits<float>(h, value == 3) : stageE_b_fits<double>(h, value == 3)))
+      if (value >= 2 && (!zop_bucket(h->N) || h->plane * (h->mixed ? 4 : 8) % 16 != 0))
         return set_err(IW_ERR_CONFIG, "bulk-staged stage E needs N <= 33 and whole 16-byte planes");
       (which == IW_LAUNCH_STAGE_A ? h->tune_a : h->tune_e) = value;
       return IW_OK;

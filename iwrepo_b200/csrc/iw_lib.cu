@@ -71,10 +71,17 @@ __device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
 
+// (re, im) pair of one complex value stored as two T
 template <typename T>
-__device__ __forceinline__ T ld(const T* p) {
-  return __ldg(p);
-}
+struct Pair;
+template <>
+struct Pair<float> {
+  typedef float2 t;
+};
+template <>
+struct Pair<double> {
+  typedef double2 t;
+};
 
 // ===========================================================================
 // K_A: round-trip projection + w(1,1,:)=0 + z derivatives.
@@ -724,11 +731,6 @@ struct EArgs {
   T* F[4];      // out: filtered u*
   double* wnl;  // (nxpp,ny,2)
   int filter;
-  // k_stageE_b: its zero-padded operators as one table built once on the
-  // host ([NM][NP] doubles of L - I, then [NM][NP] T of D, the size rounded
-  // up to 16 bytes); null: every CTA builds them from D and the filter
-  const void* ops;
-  unsigned ops_bytes;
 };
 
 template <typename T>
@@ -802,226 +804,13 @@ __device__ __forceinline__ void stageE_tile(const Geo& g, const EArgs<T>& a, con
   }
 }
 
-// Tiled K_E with its input tiles staged by bulk asynchronous copies and the
-// z operators unrolled at a compile-time size NM >= N (the zero-padded
-// bucket of the register-column kernels).  The CTA tiling is stageE_tile's
-// (32 x points of one (y, subdomain), 8 warps) and so are the sums, in the
-// same order (every rounding written out, so it agrees to rounding).  The
-// seven input tiles (Z, B, S_n, S_{n-1}, F1, F_n, F_{n-1}) are requested at
-// once, one cp.async.bulk per row completing on an mbarrier (Z on its own,
-// so that D Z starts while the rest lands).  Warp w computes all of its
-// output rows k1 = w + 8 r at once, so each column value feeds every row and
-// each pair of operator entries is one 8-byte broadcast; with NM known every
-// shared-memory address is a base plus an immediate.  A row of 32 points is
-// copied from the 16-byte boundary at or below its first point (FP32 rows of
-// an nxpp = 2 (mod 4) field start 8 bytes into a unit); the copy may run up to
-// 15 bytes past the field's end, inside the 16 bytes every field buffer is
-// allocated with beyond its end.  The launch requires nxpp*ny*sizeof(T) to be
-// a multiple of 16, so that every row of a CTA has the same offset.
-// z operators of the register-column kernels and of k_stageE_b<.., true>: kernel
-// parameters, i.e. served from the constant bank
+// z operators of the register-column kernels: kernel parameters, i.e. served
+// from the constant bank
 template <typename T, int NM>
 struct ZOp {
   T D[NM * NM];       // D[k1*NM + k2], zero outside N x N
   double L[NM * NM];  // precombined Legendre filter minus the identity, same layout (FP64, see k_stageE)
 };
-constexpr int kEBArr = 7;
-template <typename T>
-__host__ __device__ inline int eb_rs() {  // tile row stride (elements): 32 points and room for the offset
-  return kTX + 16 / (int)sizeof(T);
-}
-__host__ __device__ constexpr int eb_np(int NM) { return (NM + 1) & ~1; }  // operator row stride: pairs stay aligned
-template <typename T>
-__host__ inline size_t eb_smem(int N, int NM, bool cb = false) {
-  return 16 + ((size_t)NM + (size_t)(kEBArr - 1) * N) * eb_rs<T>() * sizeof(T) +
-         (cb ? 0 : (size_t)NM * eb_np(NM) * sizeof(double) + (size_t)NM * eb_np(NM) * sizeof(T)) +
-         (size_t)NM * kTX * sizeof(T);
-}
-// two consecutive operator entries (an 8-byte broadcast load for FP32)
-__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
-  const float2 v = *(const float2*)p;
-  a = v.x;
-  b = v.y;
-}
-__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b) {
-  a = p[0];
-  b = p[1];
-}
-
-// CB: D and L - I from the kernel parameter op (the constant bank; a warp's
-// rows are warp-uniform, so every operator entry is a uniform load) instead of
-// shared memory; the same sums in the same order.
-template <typename T, int NM, bool CB = false>
-__global__ void __launch_bounds__(kTX* kTW) k_stageE_b(Geo g, EArgs<T> a, Coefs c, int* __restrict__ err,
-                                                       const __grid_constant__ ZOp<T, NM> op) {
-  constexpr int NP = eb_np(NM), RB = (NM + kTW - 1) / kTW;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int N = g.N, RS = eb_rs<T>();
-  uint64_t* bar = (uint64_t*)smraw;  // [0]: Z, [1]: the other six tiles
-  T* tiles = (T*)(smraw + 16);       // Z: [NM][RS], then arrays 1..6: [N][RS] each
-  double* sL = (double*)(tiles + ((size_t)NM + (size_t)(kEBArr - 1) * N) * RS);  // [NM][NP]: L - I (not CB)
-  T* sD = (T*)(sL + (CB ? 0 : NM * NP));                                          // [NM][NP] (not CB)
-  T* tf = sD + (CB ? 0 : NM * NP);                                                // [NM][kTX]: F* tile
-  const int q = blockIdx.z;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int i0 = blockIdx.x * kTX, i = i0 + lane;
-  const int j = blockIdx.y % g.ny, ks = blockIdx.y / g.ny;
-  const int nval = min(kTX, g.nxpp - i0);
-  const bool pre = !CB && a.ops != nullptr;
-  if (tid == 0) {
-    mbar_init(&bar[0], (uint32_t)N + (pre ? 1u : 0u));
-    mbar_init(&bar[1], (uint32_t)((kEBArr - 1) * N));
-  }
-  __syncthreads();
-  if (pre && tid == (int)blockDim.x - 1) {  // the operators, with the Z tile (the copy may run 15 bytes into tf)
-    mbar_expect_tx(&bar[0], a.ops_bytes);
-    bulk_g2s(sL, a.ops, a.ops_bytes, &bar[0]);
-  }
-  for (int t = tid; t < kEBArr * N; t += blockDim.x) {
-    const int arr = t / N, k = t - arr * N;
-    const T* base = arr == 0 ? a.Z[q]
-                    : arr == 1 ? a.B[q]
-                    : arr == 2 ? a.Snold[q]
-                    : arr == 3 ? a.Snm_w[q]
-                    : arr == 4 ? a.F1[q]
-                    : arr == 5 ? a.Fn[q]
-                               : a.Fnm_w[q];
-    const uintptr_t ga = (uintptr_t)(base + fidx<T>(g, i0, j, ks * N + k));
-    const uint32_t off = (uint32_t)(ga & 15u);
-    const uint32_t bytes = (off + (uint32_t)nval * (uint32_t)sizeof(T) + 15u) & ~15u;
-    uint64_t* b = &bar[arr == 0 ? 0 : 1];
-    T* dst = tiles + (arr == 0 ? (size_t)k : (size_t)NM + (size_t)(arr - 1) * N + k) * RS;
-    mbar_expect_tx(b, bytes);
-    bulk_g2s(dst, (const void*)(ga - off), bytes, b);
-  }
-  // operators zero-padded to NM x NM (unless copied above), the padding rows of
-  // the Z and F* tiles zero
-  if (!pre && !CB) {
-    for (int t = tid; t < NM * NP; t += blockDim.x) {
-      const int r = t / NP, cc = t - r * NP;
-      const bool in = r < N && cc < N;
-      sD[t] = in ? (T)g.D[r * N + cc] : (T)0;
-      sL[t] = in ? g.Lfil[r * N + cc] - (r == cc ? 1.0 : 0.0) : 0.0;
-    }
-  }
-  for (int t = N * RS + tid; t < NM * RS; t += blockDim.x) tiles[t] = (T)0;
-  for (int t = N * kTX + tid; t < NM * kTX; t += blockDim.x) tf[t] = (T)0;
-  // element offset of this CTA's first point inside each copied row (the
-  // same for every row: the planes are whole 16-byte units)
-  const int eo = (int)((((size_t)i0 + (size_t)g.nxpp * ((size_t)j + (size_t)g.ny * (size_t)(ks * N))) * sizeof(T)) &
-                       15u) /
-                 (int)sizeof(T);
-  const bool ok0 = mbar_wait(&bar[0], 0, 2000000000ull);
-  __syncthreads();  // the operator tables and padding are in place
-  const bool act = i < g.nxpp;
-  const T fac = (T)g.hfac[ks];
-  const T f1 = (T)c.fac1, f2 = (T)c.fac2, f3 = (T)c.fac3;
-  // D Z for this warp's rows; lanes past the field's end compute on stale
-  // tile entries and store nothing
-  T dz[RB];
-#pragma unroll
-  for (int r = 0; r < RB; ++r) dz[r] = 0;
-  const T* zc = tiles + eo + lane;  // this lane's column of the Z tile
-  const T* dw = sD + w * NP;        // row w of D; row w + 8 r is dw + 8 r NP
-#pragma unroll
-  for (int k2 = 0; k2 < NM; k2 += 2) {
-    const T z0 = zc[k2 * RS];
-    const T z1 = k2 + 1 < NM ? zc[(k2 + 1) * RS] : (T)0;
-#pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      if (r < RB - 1 || w + kTW * r < NM) {
-        T d0, d1;
-        if constexpr (CB) {
-          const T* od = op.D + (w + kTW * r) * NM + k2;
-          if (k2 + 1 < NM) {
-            d0 = od[0];
-            d1 = od[1];
-            dz[r] = fma_t(d1, z1, fma_t(d0, z0, dz[r]));
-          } else {
-            dz[r] = fma_t(od[0], z0, dz[r]);
-          }
-        } else if (k2 + 1 < NM) {
-          ld_pair(dw + r * kTW * NP + k2, d0, d1);
-          dz[r] = fma_t(d1, z1, fma_t(d0, z0, dz[r]));
-        } else {
-          dz[r] = fma_t(dw[r * kTW * NP + k2], z0, dz[r]);
-        }
-      }
-    }
-  }
-  const bool ok1 = mbar_wait(&bar[1], 0, 2000000000ull);
-  if (__syncthreads_or(!(ok0 && ok1))) {  // a copy never completed: report, let the copies finish, leave
-    if (tid == 0) err[1] = 1;
-    mbar_wait(&bar[0], 0, 2000000000ull);
-    mbar_wait(&bar[1], 0, 2000000000ull);
-    return;
-  }
-#pragma unroll
-  for (int r = 0; r < RB; ++r) {
-    const int k1 = w + kTW * r;
-    if (k1 >= N) break;
-    T fsv = 0;
-    if (act) {
-      const int kk = ks * N + k1;
-      const size_t p = fidx<T>(g, i, j, kk);
-      const size_t e = (size_t)NM * RS + (size_t)k1 * RS + eo + lane;  // array 1 (B), row k1
-      const size_t AS = (size_t)N * RS;
-      const T sn = tiles[e + 1 * AS];
-      const T snm = tiles[e + 2 * AS];
-      T F2;
-      if (i < 2) {
-        const T va = tiles[e + 3 * AS];
-        const T vb = a.F1[q][fidx<T>(g, i, (g.ny - j) % g.ny, kk)];
-        F2 = i == 0 ? (T)0.5 * (va + vb) : (T)0.5 * (va - vb);
-      } else if (i >= g.nx) {
-        F2 = i == g.nx ? tiles[e + 3 * AS] * (T)g.scaley : (T)0;
-      } else {
-        F2 = tiles[e + 3 * AS];
-      }
-      const T fn = tiles[e + 4 * AS];
-      const T fnm = tiles[e + 5 * AS];
-      T S;
-      stageE_point<T>(c, fac, f1, f2, f3, tiles[e], dz[r], sn, snm, F2, fn, fnm, S, fsv);
-      if (q == 2 && ((kk == 0) || (kk == g.nz - 1))) {
-        const int side = kk == 0 ? 0 : 1;
-        a.wnl[(size_t)i + (size_t)g.nxpp * ((size_t)j + (size_t)g.ny * side)] = stageE_wall<T>(f1, f2, f3, S, sn, snm);
-      }
-      a.Snm_w[q][p] = S;
-      a.Fnm_w[q][p] = F2;
-    }
-    tf[k1 * kTX + lane] = fsv;
-  }
-  __syncthreads();
-  if (!act) return;
-  if (!a.filter) {
-#pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      const int k1 = w + kTW * r;
-      if (k1 < N) a.F[q][fidx<T>(g, i, j, ks * N + k1)] = tf[k1 * kTX + lane];
-    }
-    return;
-  }
-  const double cfm1 = g.cfour[(size_t)j * g.nxhp + (i >> 1)] - 1.0;
-  // (L - I) F* in FP64 for all of this warp's rows at once, sums in k2 order
-  double s2[RB];
-#pragma unroll
-  for (int r = 0; r < RB; ++r) s2[r] = 0.0;
-  const double* lw = sL + w * NP;
-#pragma unroll
-  for (int k2 = 0; k2 < NM; ++k2) {
-    const double f = (double)tf[k2 * kTX + lane];
-#pragma unroll
-    for (int r = 0; r < RB; ++r)
-      if (r < RB - 1 || w + kTW * r < NM)
-        s2[r] = __fma_rn(CB ? op.L[(w + kTW * r) * NM + k2] : lw[r * kTW * NP + k2], f, s2[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < RB; ++r) {
-    const int k1 = w + kTW * r;
-    if (k1 < N) a.F[q][fidx<T>(g, i, j, ks * N + k1)] = (T)stageE_filtered((double)tf[k1 * kTX + lane], s2[r], cfm1);
-  }
-}
-
 // The tiled K_E kernels.  FP32 fields: at most 32 registers so that 8 CTAs
 // fit on an SM (the kernel waits on global loads, more resident warps pay);
 // FP64 fields: the compiler's own allocation.
@@ -1193,70 +982,65 @@ __global__ void __launch_bounds__(128) k_stageE_r(Geo g, EArgs<T> a, Coefs c, co
 
 // rotational viscous term at the walls (solver.f:318-394, rotvisc 1210-1253):
 // wviscrot = -nu * (fac1 rot(n) + fac2 rot(n-1) + fac3 rot(n-2)),
-// rot = (kx^2+ky^2) w + i kx du/dz + i ky dv/dz at k0.
+// rot = (kx^2+ky^2) w + i kx du/dz + i ky dv/dz at k0.  A CTA takes 32 columns of
+// one y index and wall; its six warps form du/dz and dv/dz of the three levels,
+// each the chain of N multiply-adds, and the first warp puts them together.
 template <typename T>
-__global__ void k_wviscrot(Geo g, const T* __restrict__ u1, const T* __restrict__ v1, const T* __restrict__ w1,
-                           const T* __restrict__ un, const T* __restrict__ vn, const T* __restrict__ wn,
-                           const T* __restrict__ unm, const T* __restrict__ vnm, const T* __restrict__ wnm, Coefs c,
-                           double xnu, double* __restrict__ wvr) {
-  long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  long total = (long)g.nxhp * g.ny * 2;
-  if (gid >= total) return;
-  int ii = gid % g.nxhp;
-  long r = gid / g.nxhp;
-  int j = r % g.ny;
-  int side = r / g.ny;
-  const int N = g.N;
-  int ks = side == 0 ? 0 : g.ns - 1;
-  int k0 = side == 0 ? 0 : N - 1;
-  double fac = g.hfac[ks];
-  double xw = g.xw[ii], yw = g.yw[j];
-  double rr = 0, ri = 0;
-  for (int l = 0; l < 3; ++l) {
-    const T* U = l == 0 ? u1 : l == 1 ? un : unm;
-    const T* V = l == 0 ? v1 : l == 1 ? vn : vnm;
-    const T* W = l == 0 ? w1 : l == 1 ? wn : wnm;
-    double dur = 0, dui = 0, dvr = 0, dvi = 0;
-    for (int k2 = 0; k2 < N; ++k2) {
-      int kk = ks * N + k2;
-      double d = g.D[k0 * N + k2];
-      double ur, ui, vr, vi;
-      if (l == 0) {
-        ur = proj_val<T>(g, U, 2 * ii, j, kk);
-        ui = proj_val<T>(g, U, 2 * ii + 1, j, kk);
-        vr = proj_val<T>(g, V, 2 * ii, j, kk);
-        vi = proj_val<T>(g, V, 2 * ii + 1, j, kk);
-      } else {
-        ur = U[fidx<T>(g, 2 * ii, j, kk)];
-        ui = U[fidx<T>(g, 2 * ii + 1, j, kk)];
-        vr = V[fidx<T>(g, 2 * ii, j, kk)];
-        vi = V[fidx<T>(g, 2 * ii + 1, j, kk)];
+__global__ void __launch_bounds__(192) k_wviscrot(Geo g, const T* __restrict__ u1, const T* __restrict__ v1,
+                                                  const T* __restrict__ w1, const T* __restrict__ un,
+                                                  const T* __restrict__ vn, const T* __restrict__ wn,
+                                                  const T* __restrict__ unm, const T* __restrict__ vnm,
+                                                  const T* __restrict__ wnm, Coefs c, double xnu,
+                                                  double* __restrict__ wvr) {
+  __shared__ double sd[6][2][32];
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5, l = wq >> 1;
+  const int ii = blockIdx.x * 32 + lane, j = blockIdx.y, side = blockIdx.z;
+  const bool act = ii < g.nxhp;
+  const int N = g.N, ks = side == 0 ? 0 : g.ns - 1, k0 = side == 0 ? 0 : N - 1;
+  const double fac = g.hfac[ks];
+  // level n goes through the projection; only the kx = 0 and Nyquist columns change
+  const bool special = l == 0 && (ii == 0 || ii == g.nxh);
+  const T* F = (wq & 1) ? (l == 0 ? v1 : l == 1 ? vn : vnm) : (l == 0 ? u1 : l == 1 ? un : unm);
+  double dr = 0, di = 0;
+  if (act) {
+    const double* D = g.D + (size_t)k0 * N;
+    if (special) {
+      for (int k2 = 0; k2 < N; ++k2) {
+        dr += D[k2] * (double)proj_val<T>(g, F, 2 * ii, j, ks * N + k2);
+        di += D[k2] * (double)proj_val<T>(g, F, 2 * ii + 1, j, ks * N + k2);
       }
-      dur += d * ur;
-      dui += d * ui;
-      dvr += d * vr;
-      dvi += d * vi;
-    }
-    dur *= fac;
-    dui *= fac;
-    dvr *= fac;
-    dvi *= fac;
-    int kk0 = ks * N + k0;
-    double wr, wi;
-    if (l == 0) {
-      wr = proj_val<T>(g, W, 2 * ii, j, kk0);
-      wi = proj_val<T>(g, W, 2 * ii + 1, j, kk0);
     } else {
-      wr = W[fidx<T>(g, 2 * ii, j, kk0)];
-      wi = W[fidx<T>(g, 2 * ii + 1, j, kk0)];
+      typedef typename Pair<T>::t P2;
+      const T* p = F + fidx<T>(g, 2 * ii, j, ks * N);
+#pragma unroll 8
+      for (int k2 = 0; k2 < N; ++k2) {
+        const P2 v = *(const P2*)(p + (size_t)k2 * g.plane);
+        dr += D[k2] * (double)v.x;
+        di += D[k2] * (double)v.y;
+      }
     }
-    double re = xw * xw * wr + yw * yw * wr - xw * dui - yw * dvi;
-    double im = xw * xw * wi + yw * yw * wi + xw * dur + yw * dvr;
-    double f = l == 0 ? c.fac1 : l == 1 ? c.fac2 : c.fac3;
+  }
+  sd[wq][0][lane] = dr * fac;
+  sd[wq][1][lane] = di * fac;
+  __syncthreads();
+  if (wq != 0 || !act) return;
+  const double xw = g.xw[ii], yw = g.yw[j];
+  const int kk0 = ks * N + k0;
+  double rr = 0, ri = 0;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const T* W = m == 0 ? w1 : m == 1 ? wn : wnm;
+    const double wr = m == 0 ? (double)proj_val<T>(g, W, 2 * ii, j, kk0) : (double)W[fidx<T>(g, 2 * ii, j, kk0)];
+    const double wi = m == 0 ? (double)proj_val<T>(g, W, 2 * ii + 1, j, kk0) : (double)W[fidx<T>(g, 2 * ii + 1, j, kk0)];
+    const double dur = sd[2 * m][0][lane], dui = sd[2 * m][1][lane], dvr = sd[2 * m + 1][0][lane],
+                 dvi = sd[2 * m + 1][1][lane];
+    const double re = xw * xw * wr + yw * yw * wr - xw * dui - yw * dvi;
+    const double im = xw * xw * wi + yw * yw * wi + xw * dur + yw * dvr;
+    const double f = m == 0 ? c.fac1 : m == 1 ? c.fac2 : c.fac3;
     rr += f * re;
     ri += f * im;
   }
-  size_t base = (size_t)g.nxpp * ((size_t)j + (size_t)g.ny * side) + 2 * ii;
+  const size_t base = (size_t)g.nxpp * ((size_t)j + (size_t)g.ny * side) + 2 * ii;
   wvr[base] = -(xnu * rr);
   wvr[base + 1] = -(xnu * ri);
 }
@@ -2094,19 +1878,6 @@ __global__ void k_press_g(Geo g, SolveTabs tb, const Task* __restrict__ tasks, i
 // ===========================================================================
 constexpr int kSolveThreads = 128;
 
-// (re, im) pair of one complex value stored as two T
-template <typename T>
-struct Pair;
-template <>
-struct Pair<float> {
-  typedef float2 t;
-};
-template <>
-struct Pair<double> {
-  typedef double2 t;
-};
-
-
 // dst = (accum ? dst : 0) + A^-1 src for R right-hand sides of length n.
 // rz, zz: R*m doubles of shared scratch.  Ends synchronised.
 template <int R>
@@ -2250,8 +2021,8 @@ __device__ void legen_filter_cta(const Geo& g, const double* __restrict__ Lt, co
 // refine: one FP64 residual sweep x += A^-1 (b - A x).
 template <typename T, int R>
 __global__ void __launch_bounds__(kSolveThreads) k_solve_cta(
-    Geo g, BlockInv bi, SolveTabs tb, const Task* __restrict__ tasks, T* __restrict__ F0, T* __restrict__ F1,
-    T* __restrict__ F2, double rdiv, int role, int cpen, int meanu, int refine, const double* __restrict__ Dt,
+    Geo g, BlockInv bi, SolveTabs tb, const Task* __restrict__ tasks, T* F0, T* F1, T* F2, const T* S0, const T* S1,
+    int cols, double rdiv, int role, int cpen, int meanu, int refine, const double* __restrict__ Dt,
     const double* __restrict__ D2t, const double* __restrict__ Lt, const double* __restrict__ zh,
     const double* __restrict__ wnl, const double* __restrict__ wvr, int kstart) {
   extern __shared__ __align__(16) double sm[];
@@ -2277,6 +2048,11 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_cta(
     cii[tid] = c < 0 ? -1 : c % g.nxhp;
   }
   __syncthreads();
+  // offset of row k of column slot ci in the sources (cols: scratch fields of
+  // whole columns, [column][k] complex; the pressure also writes there)
+  auto at = [&](int ci, int k) -> size_t {
+    return cols ? ((size_t)(cj[ci] * g.nxhp + cii[ci]) * n + k) * 2 : fidx<T>(g, 2 * cii[ci], cj[ci], k);
+  };
   if (role == 3) {
     // one 8-byte (re, im) load per field and column, all in flight at once
     typedef typename Pair<T>::t P2;
@@ -2285,7 +2061,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_cta(
       for (int ci = 0; ci < R / 2; ++ci) {
         P2 u2 = {0, 0}, v2 = {0, 0}, w2 = {0, 0};
         if (cj[ci] >= 0) {
-          const size_t p = fidx<T>(g, 2 * cii[ci], cj[ci], k);
+          const size_t p = at(ci, k);
           u2 = *(const P2*)(F0 + p);
           v2 = *(const P2*)(F1 + p);
           w2 = *(const P2*)(F2 + p);
@@ -2366,8 +2142,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_cta(
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const int ci = r / per, rr = r - ci * per;
-          const T* F = (role == 0 && rr >= 2) ? F1 : F0;
-          v[r] = cj[ci] >= 0 ? (double)F[fidx<T>(g, 2 * cii[ci] + (rr & 1), cj[ci], k)] : 0.0;
+          const T* F = (role == 0 && rr >= 2) ? S1 : S0;
+          v[r] = cj[ci] >= 0 ? (double)F[at(ci, k) + (rr & 1)] : 0.0;
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) b[(size_t)r * n + k] = -(-(v[r] / rdiv) * eps);
@@ -2404,7 +2180,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_cta(
       for (int ci = 0; ci < R / 2; ++ci) {
         if (cj[ci] < 0) continue;
         const int j = cj[ci], ii = cii[ci];
-        const size_t pr = fidx<T>(g, 2 * ii, j, k), pi = pr + 1;
+        const size_t pr = at(ci, k), pi = pr + 1;
         if (k < kstart) {
           F0[pr] = 0;
           F0[pi] = 0;
@@ -2969,11 +2745,11 @@ __global__ void __launch_bounds__(kSys2MaxThreads, 2) k_solve_sys2(
 constexpr int kTcMaxN = 40;
 // Operator columns in shared memory are AP = 4 (mod 8) doubles apart: the 4
 // columns x 8 rows of a B fragment then fall in two shared-memory wavefronts.
-__host__ __device__ inline int tc_ap(int N) {
-  int a = N;
-  while (a % 8 != 4) ++a;
-  return a;
-}
+// They are padded to a multiple of 4 columns with zeros, so that no fragment
+// needs a bounds check.
+__host__ __device__ constexpr int tc_nt(int N) { return N <= 16 ? 2 : (N + 7) / 8; }
+__host__ __device__ constexpr int tc_ap(int N) { return ((N + 3) & ~7) + 4; }
+__host__ __device__ constexpr int tc_nc(int N) { return (N + 3) & ~3; }
 // Staged right-hand sides: [tile][row][8] values of T; of FP64 rows the halves
 // swap places on every other pair of rows, so that an A fragment (4 rows x 8)
 // has no bank conflicts (FP32 fragments are 32 consecutive words as they are).
@@ -2990,12 +2766,12 @@ __host__ __device__ inline TcSmem tc_smem(int n, int N, int ns, int nb, bool pre
   TcSmem o;
   const size_t m = 2 * (size_t)(ns - 1), ap = tc_ap(N), D = sizeof(double), R = press ? 8 : 16;
   o.a = 0;
-  o.l = o.a + (size_t)nb * N * ap * D;
+  o.l = o.a + (size_t)nb * tc_nc(N) * ap * D;
   o.m = o.l + m * N * D;
   o.rz = o.m + m * m * D;
   o.zz = o.rz + m * R * D;
   o.d = o.zz + m * R * D;
-  o.raw = o.d + (press ? (size_t)N * ap * D : 0);
+  o.raw = o.d + (press ? (size_t)tc_nc(N) * ap * D : 0);
   o.total = o.raw + (press ? 3 : 2) * (size_t)n * 8 * sizeof(T) + 16 * D;  // (room for a fragment past the last column)
   return o;
 }
@@ -3015,10 +2791,10 @@ __device__ __forceinline__ double div_by(double v, double d, double y) {
   q = __fma_rn(__fma_rn(-q, d, v), y, q);
   return __fma_rn(__fma_rn(-q, d, v), y, q);
 }
-// acc[i][nt][h] += sum_c op[c ap + 8 nt + 2 t + h] b_i(c) for right-hand side g of NI
-// tiles: a(i, kt) gives b at row 4 kt + t (0 past N).  Rows past N read what follows
-// the column in shared memory; their sums are not used.  LEFT: also lacc[i]:
-// <l, b> for the left vector l of lane column g (null: 0).
+// acc[i][nt][h] = sum_c op[c AP + 8 nt + 2 t + h] b_i(c) for right-hand side g of NI
+// tiles: a(i, kt) gives b at row 4 kt + t (0 past N).  Rows past N read the padding of
+// the column; their sums are not used.  LEFT: also lacc[i]: <l, b> for the left
+// vector l of lane column g (null: 0).
 template <int NT, int NI, bool LEFT, typename A>
 __device__ __forceinline__ void tc_product(const double* op, int ap, int N, int g, int t, A&& a, double (&acc)[NI][NT][2],
                                            const double* l, double (&lacc)[NI][2]) {
@@ -3028,11 +2804,10 @@ __device__ __forceinline__ void tc_product(const double* op, int ap, int N, int 
     for (int nt = 0; nt < NT; ++nt) acc[i][nt][0] = acc[i][nt][1] = 0.0;
     lacc[i][0] = lacc[i][1] = 0.0;
   }
+  const double* o = op + t * ap + g;
 #pragma unroll
-  for (int kt = 0; kt < 2 * NT; ++kt)
+  for (int kt = 0; kt < 2 * NT; ++kt, o += 4 * ap)
     if (4 * kt < N) {  // the same for the whole warp
-      const int c = min(4 * kt + t, N - 1);
-      const double* o = op + (size_t)c * ap + g;
       double b[NI];
 #pragma unroll
       for (int i = 0; i < NI; ++i) b[i] = a(i, kt);
@@ -3043,7 +2818,7 @@ __device__ __forceinline__ void tc_product(const double* op, int ap, int N, int 
         for (int i = 0; i < NI; ++i) dmma884(acc[i][nt][0], acc[i][nt][1], b[i], ov);
       }
       if (LEFT) {
-        const double lv = l ? l[c] : 0.0;
+        const double lv = l ? l[4 * kt + t] : 0.0;
 #pragma unroll
         for (int i = 0; i < NI; ++i) dmma884(lacc[i][0], lacc[i][1], b[i], lv);
       }
@@ -3053,18 +2828,18 @@ __device__ __forceinline__ void tc_product(const double* op, int ap, int N, int 
 template <int NT>
 __device__ __forceinline__ void tc_rank2(const double* op, int ap, int N, int g, int t, double z0, double z1,
                                          double (&acc)[NT][2]) {
-  const double* o = op + (t == 1 ? (size_t)(N - 1) * ap : 0) + g;
+  const double* o = op + (t == 1 ? (N - 1) * ap : 0) + g;
   const double b = t == 0 ? -z0 : t == 1 ? -z1 : 0.0;
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) dmma884(acc[nt][0], acc[nt][1], b, o[8 * nt]);
 }
 // Accumulators v[nt][h] (row 8 nt + 2 t + h of lane (g, t)) as the A operand of the next
 // product: row 4 kt + t
-template <int NT>
-__device__ __forceinline__ double tc_next(const double (&v)[NT][2], int kt, int g, int t) {
+template <int NT, typename V>
+__device__ __forceinline__ double tc_next(const V (&v)[NT][2], int kt, int g, int t) {
   const int src = 4 * g + 2 * (kt & 1) + (t >> 1);
-  const double a = __shfl_sync(0xffffffffu, v[kt >> 1][0], src), b = __shfl_sync(0xffffffffu, v[kt >> 1][1], src);
-  return (t & 1) ? b : a;
+  const V a = __shfl_sync(0xffffffffu, v[kt >> 1][0], src), b = __shfl_sync(0xffffffffu, v[kt >> 1][1], src);
+  return (double)((t & 1) ? b : a);
 }
 // Lanes of an even and an odd right-hand side (re, im of one column) swap values
 // so that each holds one complex value: row 8 nt + 2 t of the even lane, the next row of
@@ -3093,14 +2868,54 @@ __device__ __forceinline__ void tc_interface(const double* sM, const double* srz
   }
   __syncthreads();
 }
-// the system's inverse blocks (columns AP apart), left vectors and interface matrix
+// nb column-major N x N operators into AP-strided columns, each block followed by zero
+// columns up to a multiple of 4; a warp takes every nw-th column
+__device__ __forceinline__ void tc_columns(double* dst, const double* src, int nb, int N) {
+  const int AP = tc_ap(N), NC = tc_nc(N), lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int b = 0; b < nb; ++b, dst += NC * AP, src += N * N) {
+    const double* s = src + w * N + lane;
+    double* d = dst + w * AP + lane;
+    for (int c = w; c < NC; c += nw, s += nw * N, d += nw * AP) {
+      if (c >= N) {
+        if (lane < AP) *d = 0.0;
+        if (lane + 32 < AP) d[32] = 0.0;
+      } else {
+        if (lane < N) cp_async_8(d, s);
+        if (lane + 32 < N) cp_async_8(d + 32, s + 32);
+      }
+    }
+  }
+}
+// the system's inverse blocks, left vectors and interface matrix
 __device__ __forceinline__ void tc_tables(const double* ag, const double* lg, const double* mg, int nb, int N, int m,
-                                          int ap, double* sA, double* sL, double* sM) {
-  const int lane = threadIdx.x & 31;
-  for (int c = threadIdx.x >> 5; c < nb * N; c += blockDim.x >> 5)
-    for (int r = lane; r < N; r += 32) cp_async_8(sA + (size_t)c * ap + r, ag + (size_t)c * N + r);
+                                          double* sA, double* sL, double* sM) {
+  tc_columns(sA, ag, nb, N);
   for (int q = threadIdx.x; q < m * N; q += blockDim.x) cp_async_8(sL + q, lg + q);
   for (int q = threadIdx.x; q < m * m; q += blockDim.x) cp_async_8(sM + q, mg + q);
+}
+
+// A warp's gather of NS column slots (lane i < NS holds slot i's column, -1: none)
+// from scratch fields of whole columns, [column][k] complex: consecutive lanes
+// read consecutive rows of one column.
+template <typename T, int NS, typename S, typename D>
+__device__ __forceinline__ void tc_gather_cols(int c, int N, int lane, S&& src, D&& dst) {
+  typedef typename Pair<T>::t P2;
+  int slot = lane / N, r = lane - slot * N;
+  for (int b = 0; b < NS * N; b += 32) {
+    const int cs = __shfl_sync(0xffffffffu, c, min(slot, NS - 1));
+    if (slot < NS) {
+      P2* d = dst(slot, r);
+      if (cs >= 0)
+        cp_async_c<P2>(d, src(slot, r, cs));
+      else
+        *d = P2{0, 0};
+    }
+    r += 32;
+    while (r >= N) {
+      r -= N;
+      ++slot;
+    }
+  }
 }
 
 // The u/v, w and rho solves do not depend on one another: one launch takes up
@@ -3115,16 +2930,17 @@ struct TcJob {
   int zero00;    // the (0,0) column has no system and becomes 0 (w)
   int meanu;     // damp the (0,0) column of F0
   double rdiv, irdiv;
-  T *F0, *F1;
+  T *F0, *F1;           // results
+  const T *S0, *S1;     // right-hand sides: the same fields, or with cols scratch fields of whole columns
 };
 template <typename T>
 struct TcJobs {
   TcJob<T> j[3];
-  int n, nb;
+  int n, nb, cols;
   int bmap[IW_MAX_SUBD];
 };
 template <typename T, int NT>
-__global__ void __maxnreg__(80) k_solve_tc(Geo g, const __grid_constant__ TcJobs<T> jobs,
+__global__ void __maxnreg__(NT <= 2 ? 56 : NT == 3 ? 64 : 80) k_solve_tc(Geo g, const __grid_constant__ TcJobs<T> jobs,
                                                   const int* __restrict__ col_order,
                                                   const double* __restrict__ meang) {
   typedef typename Pair<T>::t P2;
@@ -3151,20 +2967,26 @@ __global__ void __maxnreg__(80) k_solve_tc(Geo g, const __grid_constant__ TcJobs
     // complex slot sl of the 8 (2 tiles of 4): column sl (w, rho) or u, v of column sl / 2
     const int sl = lane & 7, ci = uv ? sl >> 1 : sl;
     const int c = ci < count ? col_order[tk.first + ci] : -1;
-    const int cj = c / g.nxhp;
-    const T* src = ((uv && (sl & 1)) ? J.F1 : J.F0) + (c < 0 ? 0 : fidx<T>(g, 2 * (c - cj * g.nxhp), cj, ks * N));
-    T* dst = raw + (sl >> 2) * ts;
-    const int p = 2 * (sl & 3);
-    for (int r = lane >> 3; r < N; r += 4) {
-      P2* d = (P2*)(dst + tc_pos<T>(r, p));
-      if (c >= 0)
-        cp_async_c<P2>(d, (const P2*)(src + (size_t)r * g.plane));
-      else
-        *d = P2{0, 0};
+    if (jobs.cols) {
+      tc_gather_cols<T, 8>(c, N, lane, [&](int slot, int r, int cs) -> const P2* {
+        return (const P2*)(((uv && (slot & 1)) ? J.S1 : J.S0) + ((size_t)cs * n + ks * N + r) * 2);
+      }, [&](int slot, int r) { return (P2*)(raw + (slot >> 2) * ts + tc_pos<T>(r, 2 * (slot & 3))); });
+    } else {
+      const int cj = c / g.nxhp;
+      const T* src = ((uv && (sl & 1)) ? J.S1 : J.S0) + (c < 0 ? 0 : fidx<T>(g, 2 * (c - cj * g.nxhp), cj, ks * N));
+      T* dst = raw + (sl >> 2) * ts;
+      const int p = 2 * (sl & 3);
+      for (int r = lane >> 3; r < N; r += 4) {
+        P2* d = (P2*)(dst + tc_pos<T>(r, p));
+        if (c >= 0)
+          cp_async_c<P2>(d, (const P2*)(src + (size_t)r * g.plane));
+        else
+          *d = P2{0, 0};
+      }
     }
   }
-  tc_tables(J.ainv + (size_t)s * nb * N * N, J.lvec + (size_t)s * m * N, J.minv + (size_t)s * m * m, nb, N, m, AP, sA, sL,
-            sM);
+  tc_tables(J.ainv + (size_t)s * nb * N * N, J.lvec + (size_t)s * m * N, J.minv + (size_t)s * m * m, nb, N, m, sA, sL,
+                sM);
   if (J.zero00 && (int)blockIdx.x == J.first)  // (0,0) column: element 0 of every plane
     for (int k = tid; k < n; k += blockDim.x) *(P2*)(J.F0 + (size_t)k * g.plane) = P2{0, 0};
   const double eps = J.sys[s].eps, rdiv = J.rdiv, irdiv = J.irdiv;
@@ -3173,10 +2995,13 @@ __global__ void __maxnreg__(80) k_solve_tc(Geo g, const __grid_constant__ TcJobs
   const bool lo = ks >= 1, hi = ks <= ns - 2;  // neighbours below and above
   // left vectors: c_{ks+1} on this block (lane column 0), d_{ks-1} (lane column 1)
   const double* l = lg == 0 ? (hi ? sL + (size_t)ks * N : nullptr) : lg == 1 && lo ? sL + (size_t)(ns - 2 + ks) * N : nullptr;
-  const double* op = sA + (size_t)jobs.bmap[ks] * N * AP;
+  const double* op = sA + (size_t)jobs.bmap[ks] * tc_nc(N) * AP;
+  // right-hand side at row 4 kt + t: its place in the tile differs from that of row t by a constant of kt
+  const T* rl[2] = {raw + tc_pos<T>(lt, lg), raw + ts + tc_pos<T>(lt, lg)};
   auto rhs = [&](int i, int kt) -> double {
-    const int r = 4 * kt + lt;
-    return r < N ? __dmul_rn(div_by((double)raw[i * ts + tc_pos<T>(r, lg)], rdiv, irdiv), eps) : 0.0;
+    double v = 0.0;
+    if ((NT > 2 && kt < 2 * NT - 2) || 4 * kt + lt < N) v = __dmul_rn(div_by((double)rl[i][32 * kt], rdiv, irdiv), eps);
+    return v;
   };
   auto body = [&](auto ni) {
     constexpr int NI = decltype(ni)::value;
@@ -3225,18 +3050,18 @@ __global__ void __maxnreg__(80) k_solve_tc(Geo g, const __grid_constant__ TcJobs
 // Pressure and projection (calcuvwt.f:87-229, 826-901), 4 columns (8 right-hand
 // sides) per CTA; blockIdx.y takes the task's other columns.
 template <typename T, int NT>
-__global__ void __maxnreg__(80) k_press_tc(Geo g, const __grid_constant__ BlockInv bi,
+__global__ void __maxnreg__(NT <= 4 ? 64 : 80) k_press_tc(Geo g, const __grid_constant__ BlockInv bi,
                                                   const Task* __restrict__ tasks, const int* __restrict__ col_order,
                                                   T* __restrict__ U, T* __restrict__ V, T* __restrict__ W,
                                                   const double* __restrict__ Dt, const double* __restrict__ wnl,
-                                                  const double* __restrict__ wvr, int kstart) {
+                                                  const double* __restrict__ wvr, int kstart, int cols) {
   typedef typename Pair<T>::t P2;
   constexpr int R = 8;
   extern __shared__ __align__(16) unsigned char smraw[];
   const Task tk = tasks[blockIdx.x];
   const int count = min(tk.count - 4 * (int)blockIdx.y, 4);
   if (count <= 0) return;
-  const int* cols = col_order + tk.first + 4 * blockIdx.y;
+  const int* order = col_order + tk.first + 4 * blockIdx.y;
   const int n = g.nz, N = g.N, ns = g.ns, m = 2 * (ns - 1), nb = bi.nb, s = tk.sys;
   const int tid = threadIdx.x, lane = tid & 31, ks = tid >> 5, lg = lane >> 2, lt = lane & 3;
   const int AP = tc_ap(N);
@@ -3251,27 +3076,32 @@ __global__ void __maxnreg__(80) k_press_tc(Geo g, const __grid_constant__ BlockI
   const size_t ts = (size_t)n * 8;
   {
     const int ci = lane & 3;
-    const int c = ci < count ? cols[ci] : -1;
+    const int c = ci < count ? order[ci] : -1;
     const int cj = c / g.nxhp;
     const size_t cb = c < 0 ? 0 : fidx<T>(g, 2 * (c - cj * g.nxhp), cj, ks * N);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
-      const T* src = (f == 0 ? U : f == 1 ? V : W) + cb;
-      for (int r = lane >> 2; r < N; r += 8) {
-        P2* d = (P2*)(raw + f * ts + tc_pos<T>(r, 2 * ci));
-        if (c >= 0)
-          cp_async_c<P2>(d, (const P2*)(src + (size_t)r * g.plane));
-        else
-          *d = P2{0, 0};
+      const T* src = f == 0 ? U : f == 1 ? V : W;
+      if (cols) {
+        tc_gather_cols<T, 4>(c, N, lane, [&](int, int r, int cs) -> const P2* {
+          return (const P2*)(src + ((size_t)cs * n + ks * N + r) * 2);
+        }, [&](int slot, int r) { return (P2*)(raw + f * ts + tc_pos<T>(r, 2 * slot)); });
+      } else {
+        for (int r = lane >> 2; r < N; r += 8) {
+          P2* d = (P2*)(raw + f * ts + tc_pos<T>(r, 2 * ci));
+          if (c >= 0)
+            cp_async_c<P2>(d, (const P2*)(src + cb + (size_t)r * g.plane));
+          else
+            *d = P2{0, 0};
+        }
       }
     }
   }
-  for (int c = ks; c < N; c += ns)
-    for (int r = lane; r < N; r += 32) cp_async_8(sD + (size_t)c * AP + r, Dt + (size_t)c * N + r);
-  tc_tables((const double*)bi.ainv + (size_t)s * nb * N * N, bi.lvec + (size_t)s * m * N, bi.minv + (size_t)s * m * m, nb, N,
-            m, AP, sA, sL, sM);
+  tc_columns(sD, Dt, 1, N);
+  tc_tables((const double*)bi.ainv + (size_t)s * nb * N * N, bi.lvec + (size_t)s * m * N, bi.minv + (size_t)s * m * m, nb,
+                N, m, sA, sL, sM);
   const double eps = bi.sys[s].eps, dt = g.dt, fac = g.hfac[ks];
-  const int c = (lg >> 1) < count ? cols[lg >> 1] : -1;
+  const int c = (lg >> 1) < count ? order[lg >> 1] : -1;
   const bool cok = c >= 0;
   const int cj = cok ? c / g.nxhp : 0, cii = cok ? c - cj * g.nxhp : 0;
   const double xw = g.xw[cii], yw = g.yw[cj];
@@ -3279,12 +3109,14 @@ __global__ void __maxnreg__(80) k_press_tc(Geo g, const __grid_constant__ BlockI
   __syncthreads();
   const bool lo = ks >= 1, hi = ks <= ns - 2, im = lg & 1;
   const double* l = lg == 0 ? (hi ? sL + (size_t)ks * N : nullptr) : lg == 1 && lo ? sL + (size_t)(ns - 2 + ks) * N : nullptr;
-  const double* op = sA + (size_t)bi.bmap[ks] * N * AP;
+  const double* op = sA + (size_t)bi.bmap[ks] * tc_nc(N) * AP;
   const T *ru = raw, *rv = raw + ts, *rw = raw + 2 * ts;
   double acc[1][NT][2], bv[NT][2], lacc[1][2];
+  const T* wl = rw + tc_pos<T>(lt, lg);
   tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) {
-    const int r = 4 * kt + lt;
-    return r < N ? (double)rw[tc_pos<T>(r, lg)] : 0.0;
+    double v = 0.0;
+    if ((NT > 2 && kt < 2 * NT - 2) || 4 * kt + lt < N) v = (double)wl[32 * kt];
+    return v;
   }, acc, nullptr, lacc);
   // b = -((i kx u* + i ky v* + (2/h) D w*) / dt) eps and the Neumann data at the walls
   const double idt = __drcp_rn(dt);
@@ -3326,7 +3158,8 @@ __global__ void __maxnreg__(80) k_press_tc(Geo g, const __grid_constant__ BlockI
     for (int h = 0; h < 2; ++h) bv[nt][h] = 8 * nt + 2 * lt + h < N ? acc[0][nt][h] : 0.0;
   tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) { return tc_next<NT>(bv, kt, lg, lt); }, acc, nullptr, lacc);
   const double dtx = __dmul_rn(dt, xw), dty = __dmul_rn(dt, yw);
-  const size_t cb = fidx<T>(g, 2 * cii, cj, ks * N);
+  const size_t cb = cols ? ((size_t)max(c, 0) * n + ks * N) * 2 : fidx<T>(g, 2 * cii, cj, ks * N);
+  const size_t rs = cols ? 2 : g.plane;
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
     T u[2], v[2], w[2];
@@ -3342,10 +3175,274 @@ __global__ void __maxnreg__(80) k_press_tc(Geo g, const __grid_constant__ BlockI
     const P2 zu = tc_pair<T>(u[0], u[1], lg), zv = tc_pair<T>(v[0], v[1], lg), zw = tc_pair<T>(w[0], w[1], lg);
     const int ro = 8 * nt + 2 * lt + (lg & 1);
     if (cok && ro < N) {
-      const size_t p = cb + (size_t)ro * g.plane;
+      const size_t p = cb + (size_t)ro * rs;
       *(P2*)(U + p) = zu;
       *(P2*)(V + p) = zv;
       *(P2*)(W + p) = zw;
+    }
+  }
+}
+
+// ===========================================================================
+// z-column stages on the FP64 tensor cores (N <= 40), for either storage type.
+// A warp owns 8 consecutive points of the flattened (x, y) plane of one field and
+// subdomain, i.e. one row tile of the products X^T = F^T Op^T of k_solve_tc: lane
+// (g, t) holds point g, the operand rows 4 kt + t and the result rows 8 nt + 2 t + h.
+// D and L - I sit in shared memory once per persistent CTA; warps work on their own,
+// without CTA-wide barriers, and walk the tiles in the order of memory, so that the
+// SMs stay on the same few hundred pages (z-planes are a megabyte and more apart).  The
+// products run in FP64 whatever the storage type, with one rounding of each result to
+// it (FP64 fields: the FMA chain, i.e. the bits, of the tiled kernels).
+// ===========================================================================
+__device__ __forceinline__ void z_ops(double* op, const double* __restrict__ rowmajor, int N, int ap, bool minus1) {
+  for (int q = threadIdx.x; q < tc_nc(N) * ap; q += blockDim.x) {
+    const int c = q / ap, r = q - c * ap;
+    op[q] = r < N && c < N ? rowmajor[r * N + c] - (minus1 && r == c ? 1.0 : 0.0) : 0.0;
+  }
+}
+// A warp's walk over the tiles: first point t0 of the plane and (subdomain, field) row
+struct ZWalk {
+  unsigned t0, row, step, plane8;
+  __device__ __forceinline__ ZWalk(unsigned plane) {
+    plane8 = (plane + 7) & ~7u;
+    step = ((gridDim.x * blockDim.x) >> 5) * 8;
+    t0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 8;
+    row = t0 / plane8;
+    t0 -= row * plane8;
+  }
+  __device__ __forceinline__ void next() {
+    t0 += step;
+    while (t0 >= plane8) {
+      t0 -= plane8;
+      ++row;
+    }
+  }
+};
+// K_A: projection, w mean = 0, z derivative.  The N x 8 operand goes from global
+// memory straight to registers.
+template <typename T, int NT>
+__global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict__ F0, const T* __restrict__ F1_,
+                                                     const T* __restrict__ F2_, const T* __restrict__ F3_,
+                                                     T* __restrict__ O0, T* __restrict__ O1, T* __restrict__ O2,
+                                                     T* __restrict__ O3, T* __restrict__ Z0, T* __restrict__ Z1,
+                                                     T* __restrict__ Z2, T* __restrict__ Z3, int proj,
+                                                     int* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double* sD = (double*)smraw;
+  const int N = g.N, AP = tc_ap(N), lane = threadIdx.x & 31, lg = lane >> 2, lt = lane & 3;
+  z_ops(sD, g.D, N, AP, false);
+  __syncthreads();
+  const unsigned pl = (unsigned)g.plane, nxpp = (unsigned)g.nxpp, rows = 4 * g.ns;
+  const size_t pl4 = (size_t)4 * pl, pl8 = (size_t)8 * pl;
+  const unsigned nx = (unsigned)g.nx;
+  for (ZWalk w(pl); w.row < rows; w.next()) {
+    const int q = w.row & 3, ks = w.row >> 2;
+    const unsigned tt = w.t0 + lg, j = tt / nxpp, i = tt - j * nxpp;
+    const size_t k0 = (size_t)(ks * N) * pl;
+    const T* F = (q == 0 ? F0 : q == 1 ? F1_ : q == 2 ? F2_ : F3_) + k0;
+    T* O = (q == 0 ? O0 : q == 1 ? O1 : q == 2 ? O2 : O3) + k0;
+    T* Z = (q == 0 ? Z0 : q == 1 ? Z1 : q == 2 ? Z2 : Z3) + k0;
+    const double fac = g.hfac[ks];
+    // the projection changes the kx = 0 and Nyquist columns
+    const bool special = (proj && (i < 2 || i >= nx)) || (q == 2 && tt < 2);
+    auto tile = [&](auto plain_) {
+      constexpr bool PLAIN = decltype(plain_)::value;  // a whole tile of points the projection leaves alone
+      const bool act = PLAIN || tt < pl;
+      auto in = [&](int r, int last) { return ((NT > 2 && last < 8 * (NT - 1)) || r < N) && act; };  // rows <= last < N need no test
+      T x[2 * NT];
+      const T* f = F + tt + (size_t)lt * pl;
+#pragma unroll
+      for (int kt = 0; kt < 2 * NT; ++kt, f += pl4) {
+        x[kt] = (T)0;
+        if (in(4 * kt + lt, 4 * kt + 3)) x[kt] = *f;
+      }
+      bool bad = false;
+#pragma unroll
+      for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
+      if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
+      if (!PLAIN && special) {
+        const bool wzero = q == 2 && tt < 2;
+#pragma unroll
+        for (int kt = 0; kt < 2 * NT; ++kt) {
+          const int r = 4 * kt + lt;
+          if (act && r < N) x[kt] = wzero ? (T)0 : proj_val<T>(g, F, i, j, r);
+        }
+      }
+      T* o = O + tt + (size_t)lt * pl;
+#pragma unroll
+      for (int kt = 0; kt < 2 * NT; ++kt, o += pl4)
+        if (in(4 * kt + lt, 4 * kt + 3)) *o = x[kt];
+      double acc[1][NT][2], none[1][2];
+      tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) { return (double)x[kt]; }, acc, nullptr, none);
+      T* z = Z + tt + (size_t)(2 * lt) * pl;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt, z += pl8)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (in(8 * nt + 2 * lt + h, 8 * nt + 7)) z[h * (size_t)pl] = (T)__dmul_rn(acc[0][nt][h], fac);
+    };
+    if (__any_sync(0xffffffffu, special || tt >= pl))
+      tile(std::false_type());
+    else
+      tile(std::true_type());
+  }
+}
+
+// K_E.  Each warp stages its 7 x N rows of 8 points by cp.async; the next tile's copies
+// go out as soon as the inputs are consumed, before the filter product and the
+// stores.  cols: the filtered u* goes to a scratch field as whole columns, [column][k] complex,
+// where the solves read it without strided accesses (a.F then is that scratch).
+constexpr int kZArr = 7;  // Z, B, S_n, S_{n-1}, F1, F_n, F_{n-1}
+// Staged place of row r, in rows [place][array][8 points]: rows of one parity take
+// consecutive places, so the rows 2 t of a read in the layout of the results fall in
+// different banks (of FP64 rows the halves also swap on every other pair of places).
+__host__ __device__ __forceinline__ int ze_place(int r) { return (r & ~7) | ((r & 1) << 2) | ((r >> 1) & 3); }
+template <typename T>
+__device__ __forceinline__ int ze_pos(int r, int arr, int u) {
+  const int sl = ze_place(r);
+  return (sl * kZArr + arr) * 8 + (sizeof(T) == 8 ? u ^ (((sl >> 1) & 1) << 2) : u);
+}
+template <typename T>
+__host__ __device__ inline size_t ze_buf(int N) {  // bytes of one warp's tiles
+  int top = 0;
+  for (int r = N & ~7; r < N; ++r) top = ze_place(r) > top ? ze_place(r) : top;
+  return (size_t)((N & 7) ? top + 1 : N) * kZArr * 8 * sizeof(T);
+}
+template <typename T, int NT>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 640 : 512) k_stageE_t(Geo g, const __grid_constant__ EArgs<T> a, Coefs c,
+                                                                        int cols, int v16) {
+  typedef typename Pair<T>::t P2;
+  constexpr int EC = 16 / (int)sizeof(T), CH = 8 / EC;  // points per 16-byte copy, copies per row
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int N = g.N, AP = tc_ap(N), lane = threadIdx.x & 31, lg = lane >> 2, lt = lane & 3;
+  double* sD = (double*)smraw;
+  double* sL = sD + tc_nc(N) * AP;
+  T* buf = (T*)((unsigned char*)(sL + tc_nc(N) * AP + 8) + (size_t)(threadIdx.x >> 5) * ze_buf<T>(N));
+  z_ops(sD, g.D, N, AP, false);
+  z_ops(sL, g.Lfil, N, AP, true);
+  __syncthreads();
+  const unsigned pl = (unsigned)g.plane, nxpp = (unsigned)g.nxpp, rows = 4 * g.ns;
+  const size_t pl8 = (size_t)8 * pl;
+  auto stage = [&](const ZWalk& w) {
+    const int q = w.row & 3;
+    const size_t o0 = (size_t)((int)(w.row >> 2) * N) * pl + w.t0;
+#pragma unroll
+    for (int arr = 0; arr < kZArr; ++arr) {
+      const T* src = (arr == 0   ? a.Z[q]
+                      : arr == 1 ? a.B[q]
+                      : arr == 2 ? a.Snold[q]
+                      : arr == 3 ? a.Snm_w[q]
+                      : arr == 4 ? a.F1[q]
+                      : arr == 5 ? a.Fn[q]
+                                 : a.Fnm_w[q]) + o0;
+      if (sizeof(T) == 8 || v16) {
+        const int e = (lane % CH) * EC, rl = lane / CH;
+        if (w.t0 + e < pl) {
+          const T* s = src + e + (size_t)rl * pl;
+          T* d = buf + ze_pos<T>(rl, arr, e);  // rows 8 apart: places 8 apart
+#pragma unroll
+          for (int m = 0; m < NT * CH / 4; ++m, s += (32 / CH) * (size_t)pl)
+            if (m * (32 / CH) + rl < N) cp_async_c<double2>((double2*)(d + m * (32 / CH) * kZArr * 8), (const double2*)s);
+          if ((NT * CH) % 4 != 0) {
+            const int m = NT * CH / 4;
+            if (m * (32 / CH) + rl < N) cp_async_c<double2>((double2*)(d + m * (32 / CH) * kZArr * 8), (const double2*)s);
+          }
+        }
+      } else {  // rows of odd planes start 8 bytes into a unit
+        const int e = (lane & 3) * 2;
+        if (w.t0 + e < pl) {
+          const T* s = src + e + (size_t)(lane >> 2) * pl;
+          for (int r = lane >> 2; r < N; r += 8, s += pl8)
+            cp_async_c<float2>((float2*)(buf + ze_pos<T>(r, arr, e)), (const float2*)s);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const T f1 = (T)c.fac1, f2 = (T)c.fac2, f3 = (T)c.fac3;
+  const T* eb = buf + ze_pos<T>(2 * lt, 1, lg);  // B at row 2 t
+  const T* zl = buf + (4 * (lt & 1) + (lt >> 1)) * kZArr * 8;
+  const T* const zb[2] = {zl + lg, zl + (sizeof(T) == 8 ? lg ^ 4 : lg)};  // Z at rows 4 kt + t, kt even, odd
+  ZWalk w(pl);
+  if (w.row < rows) stage(w);
+  while (w.row < rows) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+    const int q = w.row & 3, ks = w.row >> 2;
+    const unsigned tt = w.t0 + lg;
+    const bool act = tt < pl;
+    const unsigned j = tt / nxpp, i = tt - j * nxpp;
+    const bool special = act && (i < 2 || i >= (unsigned)g.nx);  // columns that the projection changes
+    const bool wq = q == 2 && (ks == 0 || ks == g.ns - 1);       // this subdomain holds a wall row of w
+    const size_t o0 = (size_t)(ks * N) * pl + tt, o2 = o0 + (size_t)(2 * lt) * pl;
+    double acc[1][NT][2], none[1][2];
+    T fs[NT][2];
+    tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) {
+      T z = (T)0;  // rows past N are not staged
+      if ((NT > 2 && kt < 2 * NT - 2) || 4 * kt + lt < N) z = zb[kt & 1][(8 * (kt >> 1) + 2 * (kt & 1)) * kZArr * 8];
+      return (double)z;
+    }, acc, nullptr, none);
+    const double fac = g.hfac[ks];
+    auto points = [&](auto plain_) {
+      constexpr bool PLAIN = decltype(plain_)::value;  // a whole tile without wall rows and special columns
+      T *sw = a.Snm_w[q] + o2, *fw = a.Fnm_w[q] + o2;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt, sw += pl8, fw += pl8)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 8 * nt + 2 * lt + h;
+          fs[nt][h] = (T)0;
+          if ((NT > 2 && nt < NT - 1) || r < N) {  // (needs no test but in the last tile)
+            const T* e = eb + (8 * nt + 4 * h) * kZArr * 8;
+            const T sn = e[8], snm = e[16];
+            T F2 = e[24];
+            if (!PLAIN && special) {
+              if (i < 2) {
+                const T vb = a.F1[q][fidx<T>(g, i, (g.ny - (int)j) % g.ny, ks * N + r)];
+                F2 = i == 0 ? (T)0.5 * (F2 + vb) : (T)0.5 * (F2 - vb);
+              } else {
+                F2 = i == (unsigned)g.nx ? F2 * (T)g.scaley : (T)0;
+              }
+            }
+            const T S = (T)__fma_rn(acc[0][nt][h], fac, (double)e[0]);
+            const T se = fma_t(f3, snm, fma_t(f2, sn, mul_t(f1, S)));
+            fs[nt][h] = bdf_combine_rn<T>(c, se, F2, e[32], e[40]);
+            if (!PLAIN && wq && act && ((ks == 0 && r == 0) || (ks == g.ns - 1 && r == N - 1)))
+              a.wnl[tt + (ks == 0 && r == 0 ? 0 : g.plane)] = stageE_wall<T>(f1, f2, f3, S, sn, snm);
+            if (PLAIN || act) {
+              sw[h * (size_t)pl] = S;
+              fw[h * (size_t)pl] = F2;
+            }
+          }
+        }
+    };
+    if (__any_sync(0xffffffffu, special || !act) || wq)
+      points(std::false_type());
+    else
+      points(std::true_type());
+    __syncwarp();
+    w.next();
+    if (w.row < rows) stage(w);
+    if (a.filter)  // (L - I) F* in FP64
+      tc_product<NT, 1, false>(sL, AP, N, lg, lt, [&](int, int kt) { return tc_next<NT>(fs, kt, lg, lt); }, acc, nullptr, none);
+    const double cfm1 = act && a.filter ? g.cfour[j * (unsigned)g.nxhp + (i >> 1)] - 1.0 : 0.0;
+    T* dst = cols ? a.F[q] + (size_t)(tt >> 1) * (2 * g.nz) + 2 * (ks * N + 2 * lt + (lg & 1)) : a.F[q] + o2;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      T o[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        o[h] = a.filter ? (T)stageE_filtered((double)fs[nt][h], acc[0][nt][h], cfm1) : fs[nt][h];
+      const bool whole = NT > 2 && nt < NT - 1;
+      if (cols) {
+        const P2 p = tc_pair<T>(o[0], o[1], lg);
+        if (act && (whole || 8 * nt + 2 * lt + (lg & 1) < N)) *(P2*)(dst + 16 * nt) = p;
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (act && (whole || 8 * nt + 2 * lt + h < N)) dst[h * (size_t)pl] = o[h];
+        dst += pl8;
+      }
     }
   }
 }
