@@ -121,13 +121,10 @@ int factor_dense_or_params(iw_handle* h, const double* pen6, double eps, int bot
   fa.sys = dsd;
   fa.pen = dpen;
   fa.ab = dab;
-  fa.ipiv = dip;
-  fa.info = dinfo;
   fa.nsys = 1;
   fa.D = h->dD;
   fa.D2 = h->dD2;
   fa.zh = h->dzh;
-  fa.assemble = 1;
   if (dense) {
     // band_lu.f:19-34 packing done on the host
     std::vector<double> ab((size_t)ldab * n, 0.0);
@@ -135,9 +132,9 @@ int factor_dense_or_params(iw_handle* h, const double* pen6, double eps, int bot
       for (int i = std::max(1, j - N); i <= std::min(n, j + N); ++i)
         ab[(size_t)(2 * N + i - j) + (size_t)ldab * (j - 1)] = dense[(size_t)(i - 1) + (size_t)n * (j - 1)];
     CK(scopy(h, dab, ab.data(), ab.size() * sizeof(double), cudaMemcpyHostToDevice));
-    fa.assemble = 0;
   }
-  k_factor<<<1, 32, 0, h->st>>>(geo(h), fa);
+  if (!dense) k_assemble_band<<<1, 32, 0, h->st>>>(geo(h), fa);
+  launch_band_lu(h->st, 1, n, N, dab, dip, dinfo);
   int info = 0;
   CK(scopy(h, &info, dinfo, sizeof info, cudaMemcpyDeviceToHost));
   cudaFree(dsd);
@@ -730,19 +727,9 @@ int iw_bandlu_solve_noalloc(const double* ain_dev, double* x_dev, int nzloc, int
   g.nz = n;
   g.N = nzloc;
   g.ns = nsubd;
-  FactorArgs fa;
-  memset(&fa, 0, sizeof fa);
-  fa.sys = sd;
-  fa.pen = base;  // not read without assembly
-  fa.ab = ab;
-  fa.ipiv = ipiv;
-  fa.info = info;
-  fa.nsys = 1;
-  fa.assemble = 0;
-  fa.factor = 1;
   cudaStream_t st = (cudaStream_t)stream;
   k_pack_band<<<64, 256, 0, st>>>(ain_dev, n, nzloc, ldab, ab, sd, info);
-  k_factor<<<1, 32, 0, st>>>(g, fa);
+  launch_band_lu(st, 1, n, nzloc, ab, ipiv, info);
   k_solve_one<<<1, 32, (size_t)nrhs * n * sizeof(double), st>>>(g, ab, ipiv, x_dev, nrhs);
   CK(cudaGetLastError());
   return IW_OK;

@@ -363,6 +363,8 @@ struct iw_handle {
   // systems
   std::vector<double> akv;     // distinct kx^2+ky^2 values
   std::vector<int> col_u;      // column -> distinct index
+  std::vector<int> order;      // columns sorted by distinct index
+  double* dakv = 0;            // akv on the device
   int* dcolorder = 0;          // columns sorted by distinct index
   int nsys_kind[SYS_KINDS] = {0, 0, 0, 0};
   double* dab[SYS_KINDS] = {0, 0, 0, 0};
@@ -374,7 +376,7 @@ struct iw_handle {
   // block inverses of the viscous / diffusive systems
   struct BI {
     void* ainv = 0;
-    double *cvec = 0, *dvec = 0, *minv = 0, *pen = 0, *lvec = 0;
+    double *minv = 0, *pen = 0, *lvec = 0;
     double* ainv_raw = 0;  // unfiltered inverses of systems [0, nsys_raw) when ainv has the filter folded in
     int nsys_raw = 0;
     SysDesc* sys = 0;
@@ -572,7 +574,9 @@ static void build_distinct(iw_handle* h) {
   std::vector<int> order(h->ncol);
   for (int c = 0; c < h->ncol; ++c) order[c] = c;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->col_u[a] < h->col_u[b]; });
+  h->order = order;
   up(h, &h->dcolorder, order);
+  up(h, &h->dakv, h->akv);
 }
 
 static int kind_bcs(const iw_handle* h, int kind, int& bot, int& top) {
@@ -595,9 +599,7 @@ static int kind_bcs(const iw_handle* h, int kind, int& bot, int& top) {
 constexpr double kRefineCond = 1e5;
 
 static int build_tasks(iw_handle* h, int kind, const std::vector<int>& colsys, int G) {
-  std::vector<int> order(h->ncol);
-  for (int c = 0; c < h->ncol; ++c) order[c] = c;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->col_u[a] < h->col_u[b]; });
+  const std::vector<int>& order = h->order;
   std::vector<Task> tasks;
   int i = 0;
   while (i < h->ncol) {
@@ -618,23 +620,20 @@ static int build_tasks(iw_handle* h, int kind, const std::vector<int>& colsys, i
 // tasks of k_solve_sys: after the k_solve_cta prefix (the refined tasks and
 // the columns without a system, which sort first), runs of the sorted column
 // order that share one system, in pieces of at most 4 (u/v) or 8 columns
-static int build_sys_tasks(iw_handle* h, int kind, const std::vector<int>& colsys) {
+static int build_sys_tasks(iw_handle* h, int kind) {
   const auto& tk = h->htasks[kind];
+  const int skip = (kind == SYS_P || kind == SYS_W) && h->akv[0] == 0.0 ? 1 : 0;
   int nold = h->nrefine[kind];
   while (nold < (int)tk.size() && tk[nold].sys < 0) ++nold;
-  for (int t = nold; t < (int)tk.size(); ++t)
-    if (tk[t].sys < 0) nold = t + 1;  // a system-less task after the prefix stays with k_solve_cta
   h->nold[kind] = nold;
   const int G = kind == SYS_U ? kSysR / 4 : kSysR / 2;
-  std::vector<int> order(h->ncol);
-  for (int c = 0; c < h->ncol; ++c) order[c] = c;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->col_u[a] < h->col_u[b]; });
+  const std::vector<int>& order = h->order;
   std::vector<Task> tasks;
   int i = nold < (int)tk.size() ? tk[nold].first : h->ncol;
   while (i < h->ncol) {
-    const int s = colsys[order[i]];
+    const int s = h->col_u[order[i]] - skip;
     int jn = i;
-    while (jn < h->ncol && colsys[order[jn]] == s && jn - i < G) ++jn;
+    while (jn < h->ncol && h->col_u[order[jn]] - skip == s && jn - i < G) ++jn;
     tasks.push_back(Task{s, i, jn - i});
     i = jn;
   }
@@ -643,6 +642,13 @@ static int build_sys_tasks(iw_handle* h, int kind, const std::vector<int>& colsy
   h->ntask2[kind] = (int)tasks.size();
   if (!tasks.empty() && up(h, &h->dtasks2[kind], tasks)) return IW_ERR_NOMEM;
   return 0;
+}
+
+// SGBTF2 of nsys assembled bands (k_band_lu)
+static void launch_band_lu(cudaStream_t st, int nsys, int n, int N, double* ab, int* ipiv, int* info) {
+  const size_t sm = lu_smem(N);
+  cudaFuncSetAttribute(k_band_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_band_lu<<<nsys, kLuThreads, sm, st>>>(n, N, ab, ipiv, info);
 }
 
 // (re)build the factors of one kind for the current bdfv/dt
@@ -707,19 +713,15 @@ static int build_factors(iw_handle* h, int kind) {
   CK(cudaMemcpyAsync(h->dcolsys[kind], colsys.data(), colsys.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
   if (nsys > 0) {
     FactorArgs fa;
-    fa.assemble = 1;
-    fa.factor = 1;
     fa.sys = h->dsys[kind];
     fa.pen = h->dpen[kind];
     fa.ab = h->dab[kind];
-    fa.ipiv = h->dipiv[kind];
-    fa.info = h->dinfo[kind];
     fa.nsys = nsys;
     fa.D = h->dD;
     fa.D2 = h->dD2;
     fa.zh = h->dzh;
-    int warps = 4;
-    k_factor<<<(nsys + warps - 1) / warps, 32 * warps, 0, h->st>>>(geo(h), fa);
+    k_assemble_band<<<(nsys + 3) / 4, 128, 0, h->st>>>(geo(h), fa);
+    launch_band_lu(h->st, nsys, n, N, fa.ab, h->dipiv[kind], h->dinfo[kind]);
     CK(cudaGetLastError());
     // host copies must stay alive until the copies finish
     CK(cudaStreamSynchronize(h->st));
@@ -735,155 +737,105 @@ static int build_factors(iw_handle* h, int kind) {
   return 0;
 }
 
-// distinct systems of one kind for the current coefficients
-static void enumerate_systems(iw_handle* h, int kind, std::vector<SysDesc>& sys, std::vector<double>& pen,
-                              std::vector<int>& colsys) {
-  const int ns = h->ns, N = h->N;
-  const int nd = (int)h->akv.size();
-  int bot, top;
-  kind_bcs(h, kind, bot, top);
-  std::vector<int> dmap(nd, -1);
-  sys.clear();
-  pen.clear();
-  const double facvel = 1. / (h->p.xnu * h->p.dt), fact = 1. / (h->p.xkappa * h->p.dt);
-  for (int u = 0; u < nd; ++u) {
-    double ak = h->akv[u];
-    if ((kind == SYS_P || kind == SYS_W) && ak == 0.0) continue;
-    double eps = kind == SYS_P ? 1. / ak : kind == SYS_T ? 1. / (ak + h->c.bdfv * fact) : 1. / (ak + h->c.bdfv * facvel);
-    SysDesc sd;
-    memset(&sd, 0, sizeof sd);
-    sd.eps = eps;
-    sd.ifbcbot = bot;
-    sd.ifbctop = top;
-    std::vector<double> pp(6 * ns);
-    h_penalty(ns, N, h->p, eps, bot, top, pp.data());
-    sd.tau1_bot = pp[4 * ns + 0];
-    sd.tau2_top = pp[5 * ns + ns - 1];
-    dmap[u] = (int)sys.size();
-    sys.push_back(sd);
-    pen.insert(pen.end(), pp.begin(), pp.end());
-  }
-  colsys.resize(h->ncol);
-  for (int c = 0; c < h->ncol; ++c) colsys[c] = dmap[h->col_u[c]];
+// Tables of nsys systems (k_build_systems) for epsilon = 1 / (ak + c0)
+static int build_systems(iw_handle* h, const double* dak, int nsys, double c0, int bot, int top, bool fold, int nraw,
+                         double* ainv, double* ainv_raw, double* lvec, double* minv, double* pen, SysDesc* sys) {
+  if (nsys <= 0) return 0;
+  BuildArgs b;
+  memset(&b, 0, sizeof b);
+  b.N = h->N;
+  b.ns = h->ns;
+  b.nb = h->nb;
+  b.nsys = nsys;
+  b.nraw = nraw;
+  b.bot = bot;
+  b.top = top;
+  b.c0 = c0;
+  b.facdir = h->p.facdir;
+  b.facneumn = h->p.facneumn;
+  b.facrobin = h->p.facrobin;
+  memcpy(b.bmap, h->bmap, sizeof b.bmap);
+  memcpy(b.brep, h->brep, sizeof b.brep);
+  b.ak = dak;
+  b.D = h->dD;
+  b.D2 = h->dD2;
+  b.zh = h->dzh;
+  b.L = fold ? h->dL : nullptr;
+  b.sys = sys;
+  b.pen = pen;
+  b.ainv = ainv;
+  b.ainv_raw = ainv_raw;
+  b.lvec = lvec;
+  b.minv = minv;
+  const size_t sm = build_smem(h->N, h->ns);
+  CK(cudaFuncSetAttribute(k_build_systems, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  k_build_systems<<<nsys, 256, sm, h->st>>>(b);
+  CK(cudaGetLastError());
+  return 0;
 }
 
-// block inverses (FP32 for the mixed path, FP64 otherwise) of one kind
+// cond(I - eps (2/h)^2 D2 + penalty) <~ 1 + eps max_ks (2/h_ks)^2 |D2|_inf
+static double cond_slope(const iw_handle* h) {
+  const int N = h->N;
+  double d2n = 0;
+  for (int k1 = 0; k1 < N; ++k1) {
+    double rs = 0;
+    for (int k = 0; k < N; ++k) rs += std::fabs(h->tab.D2[(size_t)k1 * N + k]);
+    d2n = std::max(d2n, rs);
+  }
+  double hmin = 1e300;
+  for (int ks = 0; ks < h->ns; ++ks) hmin = std::min(hmin, h->p.zh[ks]);
+  return d2n * (2.0 / hmin) * (2.0 / hmin);
+}
+
+// block inverses of one kind.  The systems of a kind are the distinct kx^2+ky^2 whatever
+// dt and bdfv are, so their number, the tables' memory, the column map and the tasks
+// are made once; a change of dt or bdfv is one kernel in stream order.
 static int build_blockinv(iw_handle* h, int kind, bool fold) {
-  const int ns = h->ns, N = h->N, n = h->nz, ldab = 3 * N + 1, m = 2 * (ns - 1);
-  const size_t tib = sizeof(double);  // the solves run in FP64 in both precisions
-  std::vector<SysDesc> sys;
-  std::vector<double> pen;
-  std::vector<int> colsys;
-  enumerate_systems(h, kind, sys, pen, colsys);
-  const int nsys = (int)sys.size();
+  const int ns = h->ns, N = h->N, m = 2 * (ns - 1);
+  const int skip = (kind == SYS_P || kind == SYS_W) && h->akv[0] == 0.0 ? 1 : 0;  // no system at k = 0
+  const int nsys = (int)h->akv.size() - skip;
+  int bot, top;
+  kind_bcs(h, kind, bot, top);
+  const double facvel = 1. / (h->p.xnu * h->p.dt), fact = 1. / (h->p.xkappa * h->p.dt);
+  const double c0 = kind == SYS_P ? 0.0 : kind == SYS_T ? h->c.bdfv * fact : h->c.bdfv * facvel;
   iw_handle::BI& B = h->bi[kind];
-  if (B.nsys != nsys) {
-    cudaFree(B.ainv);
-    cudaFree(B.cvec);
-    cudaFree(B.dvec);
-    cudaFree(B.minv);
-    cudaFree(B.pen);
-    cudaFree(B.lvec);
-    cudaFree(B.ainv_raw);
-    cudaFree(B.sys);
-    cudaFree(B.colsys);
-    B = iw_handle::BI();
+  bool fresh = !B.colsys;
+  if (fresh) {
+    const size_t n1 = std::max(nsys, 1);
     char* ai = nullptr;
+    std::vector<int> colsys(h->ncol);
+    for (int c = 0; c < h->ncol; ++c) colsys[c] = h->col_u[c] - skip;
     // (+16 bytes: k_solve_sys copies whole 16-byte units)
-    if (dalloc(h, &ai, (size_t)std::max(nsys, 1) * h->nb * N * N * tib + 16) ||
-        dalloc(h, &B.cvec, (size_t)std::max(nsys, 1) * ns * N) || dalloc(h, &B.dvec, (size_t)std::max(nsys, 1) * ns * N) ||
-        dalloc(h, &B.minv, (size_t)std::max(nsys, 1) * std::max(m * m, 1)) ||
-        dalloc(h, &B.pen, (size_t)std::max(nsys, 1) * 6 * ns) || dalloc(h, &B.sys, (size_t)std::max(nsys, 1)) ||
-        dalloc(h, &B.lvec, (size_t)std::max(nsys, 1) * std::max(m, 1) * N) ||
-        dalloc(h, &B.colsys, (size_t)h->ncol))
+    if (dalloc(h, &ai, n1 * h->nb * N * N * sizeof(double) + 16) || dalloc(h, &B.minv, n1 * std::max(m * m, 1)) ||
+        dalloc(h, &B.pen, n1 * 6 * ns) || dalloc(h, &B.sys, n1) || dalloc(h, &B.lvec, n1 * std::max(m, 1) * N))
       return IW_ERR_NOMEM;
     B.ainv = ai;
     B.nsys = nsys;
+    if (build_tasks(h, kind, colsys, kind == SYS_U ? 1 : 2)) return IW_ERR_NOMEM;
+    if (up(h, &B.colsys, colsys)) return IW_ERR_NOMEM;
   }
-  if (nsys > 0) {
-    CK(scopy(h, B.sys, sys.data(), nsys * sizeof(SysDesc), cudaMemcpyHostToDevice));
-    CK(scopy(h, B.pen, pen.data(), pen.size() * sizeof(double), cudaMemcpyHostToDevice));
-  }
-  CK(scopy(h, B.colsys, colsys.data(), colsys.size() * sizeof(int), cudaMemcpyHostToDevice));
-  if (build_tasks(h, kind, colsys, kind == SYS_U ? 1 : 2)) return IW_ERR_NOMEM;
-  {
-    // cond(I - eps (2/h)^2 D2 + penalty) <~ 1 + eps max_ks (2/h_ks)^2 |D2|_inf
-    double d2n = 0;
-    for (int k1 = 0; k1 < N; ++k1) {
-      double rs = 0;
-      for (int k = 0; k < N; ++k) rs += std::fabs(h->tab.D2[(size_t)k1 * N + k]);
-      d2n = std::max(d2n, rs);
-    }
-    double hmin = 1e300;
-    for (int ks = 0; ks < ns; ++ks) hmin = std::min(hmin, h->p.zh[ks]);
-    const double rho = d2n * (2.0 / hmin) * (2.0 / hmin);
-    int last = -1;
-    const auto& tk = h->htasks[kind];
-    for (int t = 0; t < (int)tk.size(); ++t)
-      if (tk[t].sys >= 0 && 1.0 + sys[tk[t].sys].eps * rho > kRefineCond) last = t;
+  // tasks [0, last] get a residual sweep: the systems above the condition bound
+  const double rho = cond_slope(h);
+  int last = -1, nraw = 0;
+  const auto& tk = h->htasks[kind];
+  for (int t = 0; t < (int)tk.size(); ++t)
+    if (tk[t].sys >= 0 && 1.0 + 1. / (h->akv[tk[t].sys + skip] + c0) * rho > kRefineCond) last = t;
+  if (fold)
+    for (int t = 0; t <= last; ++t) nraw = std::max(nraw, tk[t].sys + 1);
+  if (fresh || h->nrefine[kind] != last + 1) {
     h->nrefine[kind] = last + 1;
-    if (build_sys_tasks(h, kind, colsys)) return IW_ERR_NOMEM;
-    int nraw = 0;
-    if (fold)
-      for (int t = 0; t <= last; ++t) nraw = std::max(nraw, tk[t].sys + 1);
+    if (build_sys_tasks(h, kind)) return IW_ERR_NOMEM;
+  }
+  if (B.nsys_raw != nraw) {
     cudaFree(B.ainv_raw);
     B.ainv_raw = nullptr;
     B.nsys_raw = nraw;
     if (nraw > 0 && dalloc(h, &B.ainv_raw, (size_t)nraw * h->nb * N * N)) return IW_ERR_NOMEM;
   }
-  // chunked: assemble -> invert blocks -> interface matrix -> store
-  const int CH = std::max(1, std::min(nsys, (int)(1200000000ull / ((size_t)ldab * n * 8 + (size_t)ns * N * N * 8 + 1))));
-  double *tab = nullptr, *tinv = nullptr, *twork = nullptr;
-  int* tinfo = nullptr;
-  CK(cudaMalloc(&tab, (size_t)CH * ldab * n * sizeof(double)));
-  CK(cudaMalloc(&tinv, (size_t)CH * ns * N * N * sizeof(double)));
-  CK(cudaMalloc(&twork, (size_t)CH * 2 * std::max(m * m, 1) * sizeof(double)));
-  CK(cudaMalloc(&tinfo, (size_t)CH * sizeof(int)));
-  Geo g = geo(h);
-  for (int s0 = 0; s0 < nsys; s0 += CH) {
-    const int cn = std::min(CH, nsys - s0);
-    FactorArgs fa;
-    memset(&fa, 0, sizeof fa);
-    fa.sys = B.sys + s0;
-    fa.pen = B.pen + (size_t)s0 * 6 * ns;
-    fa.ab = tab;
-    fa.ipiv = nullptr;
-    fa.info = tinfo;
-    fa.nsys = cn;
-    fa.D = h->dD;
-    fa.D2 = h->dD2;
-    fa.zh = h->dzh;
-    fa.assemble = 1;
-    fa.factor = 0;
-    k_factor<<<(cn + 3) / 4, 128, 0, h->st>>>(g, fa);
-    const int wpb = 2;
-    size_t sm = (size_t)wpb * N * 2 * N * sizeof(double);
-    cudaFuncSetAttribute(k_block_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_block_invert<<<(cn * ns + wpb - 1) / wpb, 32 * wpb, sm, h->st>>>(g, tab, cn, tinv, B.cvec + (size_t)s0 * ns * N,
-                                                                      B.dvec + (size_t)s0 * ns * N);
-    if (m > 0)
-      k_iface_matrix<<<(cn + 63) / 64, 64, 0, h->st>>>(g, cn, tinv, B.cvec + (size_t)s0 * ns * N,
-                                                       B.dvec + (size_t)s0 * ns * N, B.minv + (size_t)s0 * m * m, twork);
-    if (m > 0)
-      k_left_vecs<<<1184, 256, 0, h->st>>>(g, cn, tinv, B.cvec + (size_t)s0 * ns * N, B.dvec + (size_t)s0 * ns * N,
-                                         B.lvec + (size_t)s0 * m * N);
-    const size_t cnt = (size_t)cn * ns * N * N;
-    BlockRep rep;
-    memcpy(rep.r, h->brep, sizeof rep.r);
-    const int nb = h->nb;
-    if (fold && s0 < B.nsys_raw)
-      k_compact_blocks<<<2368, 256, 0, h->st>>>(N, std::min(B.nsys_raw, s0 + cn) - s0, ns, nb, rep, nullptr, tinv,
-                                                B.ainv_raw + (size_t)s0 * nb * N * N);
-    k_compact_blocks<<<2368, 256, 0, h->st>>>(N, cn, ns, nb, rep, fold ? h->dL : nullptr, tinv,
-                                              (double*)B.ainv + (size_t)s0 * nb * N * N);
-    (void)cnt;
-    CK(cudaGetLastError());
-  }
-  CK(cudaStreamSynchronize(h->st));
-  cudaFree(tab);
-  cudaFree(tinv);
-  cudaFree(twork);
-  cudaFree(tinfo);
+  if (int r = build_systems(h, h->dakv + skip, nsys, c0, bot, top, fold, nraw, (double*)B.ainv, B.ainv_raw, B.lvec, B.minv,
+                            B.pen, B.sys))
+    return r;
   h->bi_bdfv[kind] = h->c.bdfv;
   h->bi_dt[kind] = h->p.dt;
   h->bi_fold[kind] = fold;
@@ -1417,6 +1369,35 @@ static bool tc_zero00(const iw_handle* h, int role) {
          h->htasks[kind][0].first == 0 && h->htasks[kind][0].count == 1;
 }
 
+// k_solve_tc over nblk tasks of the jobs
+template <typename T>
+static void launch_jobs_tc(iw_handle* h, const TcJobs<T>& jobs, int nblk, const int* order) {
+  const Geo g = geo(h);
+  const size_t smem = tc_smem<T>(h->nz, h->N, h->ns, h->nb, false).total;
+#define IW_TC_CASE(NT)                                                                               \
+  case NT:                                                                                           \
+    cudaFuncSetAttribute(k_solve_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    k_solve_tc<T, NT><<<nblk, 32 * h->ns, smem, h->st>>>(g, jobs, order, h->dmeang);                 \
+    break;
+  switch (tc_nt(h->N)) { IW_TC_CASE(2) IW_TC_CASE(3) IW_TC_CASE(4) IW_TC_CASE(5) }
+#undef IW_TC_CASE
+}
+
+// k_helm_tc over ntask tasks
+template <typename T>
+void launch_helm_tc(iw_handle* h, const HelmTc& H, int ntask) {
+  const size_t smem = helm_smem(h->nz, h->N, h->ns, h->nb).total;
+  const Geo g = geo(h);
+  const dim3 grid((unsigned)ntask, 2);
+#define IW_HT_CASE(NT)                                                                              \
+  case NT:                                                                                          \
+    cudaFuncSetAttribute(k_helm_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    k_helm_tc<NT><<<grid, 32 * h->ns, smem, h->st>>>(g, H);                                         \
+    break;
+  switch (tc_nt(h->N)) { IW_HT_CASE(2) IW_HT_CASE(3) IW_HT_CASE(4) IW_HT_CASE(5) }
+#undef IW_HT_CASE
+}
+
 // The system-grouped tensor-core solves of the listed roles (0..2: one launch
 // for all of them; 3: the pressure).  The row tiles of 8 are fixed at compile
 // time; one warp per subdomain.
@@ -1476,14 +1457,7 @@ void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles
     j.S1 = S[1];
     nblk += h->ntask2[kind];
   }
-  if (nblk == 0) return;
-#define IW_TC_CASE(NT)                                                                                       \
-  case NT:                                                                                                   \
-    cudaFuncSetAttribute(k_solve_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
-    k_solve_tc<T, NT><<<nblk, 32 * h->ns, smem, h->st>>>(g, jobs, h->dcolorder, h->dmeang);                  \
-    break;
-  switch (nt) { IW_TC_CASE(2) IW_TC_CASE(3) IW_TC_CASE(4) IW_TC_CASE(5) }
-#undef IW_TC_CASE
+  if (nblk > 0) launch_jobs_tc<T>(h, jobs, nblk, h->dcolorder);
 }
 
 template <typename T>
@@ -1492,8 +1466,6 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   const int kind = role_kind(role);
   BlockInv bi;
   bi.ainv = h->bi[kind].ainv;
-  bi.cvec = h->bi[kind].cvec;
-  bi.dvec = h->bi[kind].dvec;
   bi.minv = h->bi[kind].minv;
   bi.pen = h->bi[kind].pen;
   bi.sys = h->bi[kind].sys;
@@ -1606,8 +1578,10 @@ IW_INST_FFT(, double)
 IW_INST_Z(, float)
 #else
 IW_INST_Z(, double)
+template void launch_helm_tc<double>(iw_handle*, const HelmTc&, int);
 #endif
 #else
+extern template void launch_helm_tc<double>(iw_handle*, const HelmTc&, int);
 IW_INST_FFT(extern, float)
 IW_INST_FFT(extern, double)
 IW_INST_Z(extern, float)
@@ -2212,11 +2186,13 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
 }
 
 static int out_join(iw_handle* h);
+static void helm_free(iw_handle* h);
 
 int iw_destroy(iw_handle* h) {
   if (!h) return IW_OK;
   cudaSetDevice(h->dev);
   out_join(h);
+  helm_free(h);
   if (h->out_host) cudaFreeHost(h->out_host);
   if (h->anim_host) cudaFreeHost(h->anim_host);
   if (h->leg_host) cudaFreeHost(h->leg_host);
@@ -2234,12 +2210,11 @@ int iw_destroy(iw_handle* h) {
   if (h->herr) cudaFreeHost(h->herr);
   if (h->err_ev) cudaEventDestroy(h->err_ev);
   cudaFree(h->dcolorder);
+  cudaFree(h->dakv);
   for (int k = 0; k < SYS_KINDS; ++k) {
     cudaFree(h->dtasks[k]);
     cudaFree(h->dtasks2[k]);
     cudaFree(h->bi[k].ainv);
-    cudaFree(h->bi[k].cvec);
-    cudaFree(h->bi[k].dvec);
     cudaFree(h->bi[k].minv);
     cudaFree(h->bi[k].pen);
     cudaFree(h->bi[k].lvec);
@@ -2549,42 +2524,52 @@ struct HelmCache {
   SysDesc* sys = nullptr;
   double* pen = nullptr;
   int* colsys = nullptr;
+  double* lam = nullptr;  // distinct lambdas, ascending
+  // block inverses of the systems [first, nsys) that k_solve_tc takes (mode 0) and
+  // their tasks; the columns of the others stay with the band LU (list, nlist)
+  double *ainv = nullptr, *lvec = nullptr, *minv = nullptr, *pen2 = nullptr;
+  SysDesc* sys2 = nullptr;
+  Task* tasks = nullptr;
+  int ntask = 0, first = 0;
+  int *order = nullptr, *list = nullptr, nlist = 0;
 };
 static std::map<std::pair<iw_handle*, std::string>, HelmCache> g_helm;
 
 // y = A x for the penalty matrix of system s (matrix-free, FP64)
-__device__ double apply_A_row(const Geo& g, const double* __restrict__ D2, const double* __restrict__ zh, double eps,
-                              const double* __restrict__ pen, const double* x, int r) {
+// row r; x(i): element i
+template <typename X>
+__device__ __forceinline__ double apply_A_row(const Geo& g, const double* __restrict__ D2, const double* __restrict__ zh,
+                                              double eps, const double* __restrict__ pen, X&& x, int r) {
   const int N = g.N, ns = g.ns;
   const int ks = r / N, k1 = r % N, km = ks * N;
   const double *pa = pen, *pb = pen + ns, *pg = pen + 2 * ns, *pd = pen + 3 * ns, *pt1 = pen + 4 * ns,
                *pt2 = pen + 5 * ns;
   const double h2 = (2.0 / zh[ks]);
   double s2 = 0;
-  for (int k = 0; k < N; ++k) s2 += D2[k1 * N + k] * x[km + k];
-  double y = x[r] - eps * h2 * h2 * s2;
+  for (int k = 0; k < N; ++k) s2 += D2[k1 * N + k] * x(km + k);
+  double y = x(r) - eps * h2 * h2 * s2;
   if (k1 == 0) {
     double s0 = 0;
-    for (int k = 0; k < N; ++k) s0 += g.D[0 * N + k] * x[km + k];
-    y += pt1[ks] * pa[ks] * x[km] - pt1[ks] * pb[ks] * eps * h2 * s0;
+    for (int k = 0; k < N; ++k) s0 += g.D[0 * N + k] * x(km + k);
+    y += pt1[ks] * pa[ks] * x(km) - pt1[ks] * pb[ks] * eps * h2 * s0;
     if (ks > 0) {
       double hl = 2.0 / zh[ks - 1];
       double sl = 0;
-      for (int k = 0; k < N; ++k) sl += g.D[(N - 1) * N + k] * x[km - N + k];
-      y += -0.5 * pt1[ks] * pa[ks] * x[km] + 0.5 * pt1[ks] * pb[ks] * eps * h2 * s0 - 0.5 * pt1[ks] * pa[ks] * x[km - 1] +
+      for (int k = 0; k < N; ++k) sl += g.D[(N - 1) * N + k] * x(km - N + k);
+      y += -0.5 * pt1[ks] * pa[ks] * x(km) + 0.5 * pt1[ks] * pb[ks] * eps * h2 * s0 - 0.5 * pt1[ks] * pa[ks] * x(km - 1) +
            0.5 * pt1[ks] * pb[ks] * eps * hl * sl;
     }
   }
   if (k1 == N - 1) {
     double s1 = 0;
-    for (int k = 0; k < N; ++k) s1 += g.D[(N - 1) * N + k] * x[km + k];
-    y += pt2[ks] * pg[ks] * x[km + N - 1] + pt2[ks] * pd[ks] * eps * h2 * s1;
+    for (int k = 0; k < N; ++k) s1 += g.D[(N - 1) * N + k] * x(km + k);
+    y += pt2[ks] * pg[ks] * x(km + N - 1) + pt2[ks] * pd[ks] * eps * h2 * s1;
     if (ks < ns - 1) {
       double hr = 2.0 / zh[ks + 1];
       double sr = 0;
-      for (int k = 0; k < N; ++k) sr += g.D[0 * N + k] * x[km + N + k];
-      y += -0.5 * pt2[ks] * pg[ks] * x[km + N - 1] - 0.5 * pt2[ks] * pd[ks] * eps * h2 * s1 -
-           0.5 * pt2[ks] * pg[ks] * x[km + N] - 0.5 * pt2[ks] * pd[ks] * eps * hr * sr;
+      for (int k = 0; k < N; ++k) sr += g.D[0 * N + k] * x(km + N + k);
+      y += -0.5 * pt2[ks] * pg[ks] * x(km + N - 1) - 0.5 * pt2[ks] * pd[ks] * eps * h2 * s1 -
+           0.5 * pt2[ks] * pg[ks] * x(km + N) - 0.5 * pt2[ks] * pd[ks] * eps * hr * sr;
     }
   }
   return y;
@@ -2647,13 +2632,14 @@ __device__ void band_solve_warp_f(const float* __restrict__ ab, const int* __res
 }
 
 // mode 0: FP64 factors and solve; mode 1: FP32 solve + one FP64 residual
-// refinement sweep.  rhs/sol: [ncol][nz] complex (re,im).
-__global__ void k_helm(Geo g, HelmCache hc, const double* __restrict__ rhs, double* __restrict__ sol, int ncol,
-                       int mode, const double* __restrict__ D2, const double* __restrict__ zh) {
+// refinement sweep.  rhs/sol: [ncol][nz] complex (re,im); list: the columns, or all.
+static __global__ void k_helm(Geo g, HelmCache hc, const double* __restrict__ rhs, double* __restrict__ sol, int ncol,
+                              int mode, const double* __restrict__ D2, const double* __restrict__ zh,
+                              const int* __restrict__ list) {
   extern __shared__ __align__(16) double smh[];
   const int warps = blockDim.x / 32, wid = threadIdx.x / 32, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * warps + wid;
-  if (c >= ncol) return;
+  if (blockIdx.x * warps + wid >= ncol) return;
+  const int c = list ? list[blockIdx.x * warps + wid] : blockIdx.x * warps + wid;
   const int n = g.nz, N = g.N, ldab = 3 * N + 1;
   const int s = hc.colsys[c];
   double* b = smh + (size_t)wid * 6 * n;  // b (2n), x (2n), r (2n)
@@ -2682,8 +2668,8 @@ __global__ void k_helm(Geo g, HelmCache hc, const double* __restrict__ rhs, doub
   const double eps = hc.sys[s].eps;
   const double* pen = hc.pen + (size_t)s * 6 * g.ns;
   for (int k = lane; k < n; k += 32) {
-    double r0 = b[k] - apply_A_row(g, D2, zh, eps, pen, x, k);
-    double r1 = b[n + k] - apply_A_row(g, D2, zh, eps, pen, x + n, k);
+    double r0 = b[k] - apply_A_row(g, D2, zh, eps, pen, [&](int i) { return x[i]; }, k);
+    double r1 = b[n + k] - apply_A_row(g, D2, zh, eps, pen, [&](int i) { return x[n + i]; }, k);
     xf[k] = (float)r0;
     xf[n + k] = (float)r1;
   }
@@ -2693,6 +2679,87 @@ __global__ void k_helm(Geo g, HelmCache hc, const double* __restrict__ rhs, doub
     sol[((size_t)c * n + k) * 2] = x[k] + (double)xf[k];
     sol[((size_t)c * n + k) * 2 + 1] = x[n + k] + (double)xf[n + k];
   }
+}
+
+// Mode 1 with a right-hand side per lane: a warp takes 16 columns in the order of their
+// systems (real and imaginary part in neighbouring lanes) and keeps their vectors in shared
+// memory, [row][lane] FP32.  A lane runs its own band sweep: no shuffles and no
+// barriers, the factor entries of a step are independent loads that lanes of one
+// system share, and the updates of a step are independent.  The arithmetic of every element and
+// its order are band_solve_warp_f's, so the FP32 sweeps give the same bits.  The FP64
+// residual walks block by block; a block's residual replaces its x one block later (the
+// next block's coupling row still reads it) and x waits in sol.
+__device__ __forceinline__ void band_sweep_lane(const float* __restrict__ ab, const int* __restrict__ ipiv, float* b,
+                                                int n, int N) {
+  const int ldab = 3 * N + 1, kd = 2 * N, k = 2 * N;  // b: element i at b[32 i]
+  for (int j = 0; j < n - 1; ++j) {
+    const int lm = min(N, n - 1 - j), l = __ldg(ipiv + j) - 1;
+    const float* col = ab + (size_t)ldab * j + kd;
+    float* bj = b + 32 * j;
+    const float v = bj[0], y = b[32 * l];
+    if (l != j) {
+      b[32 * l] = v;
+      bj[0] = y;
+    }
+#pragma unroll 8
+    for (int i = 1; i <= lm; ++i) bj[32 * i] = __fmaf_rn(-__ldg(col + i), y, bj[32 * i]);
+  }
+  for (int j = n - 1; j >= 0; --j) {
+    const float* col = ab + (size_t)ldab * j + k;
+    float* bj = b + 32 * j;
+    const float xj = __fdiv_rn(bj[0], __ldg(col));
+    bj[0] = xj;
+    const int m = min(k, j);
+#pragma unroll 8
+    for (int i = 1; i <= m; ++i) bj[-32 * i] = __fmaf_rn(-xj, __ldg(col - i), bj[-32 * i]);
+  }
+}
+static size_t helm32_smem(int n, int N) { return (size_t)(n + 2 * N) * 32 * sizeof(float); }
+static __global__ void __launch_bounds__(32) k_helm32(Geo g, HelmCache hc, const double* __restrict__ rhs,
+                                                      double* __restrict__ sol, int ncol, const double* __restrict__ D2,
+                                                      const double* __restrict__ zh, const int* __restrict__ order) {
+  extern __shared__ __align__(16) float smf[];
+  const int n = g.nz, N = g.N, ldab = 3 * N + 1, lane = threadIdx.x;
+  const int at = blockIdx.x * 16 + (lane >> 1);
+  if (at >= ncol) return;
+  const int c = order[at], s = hc.colsys[c];
+  const double* rc = rhs + (size_t)c * n * 2 + (lane & 1);
+  double* xc = sol + (size_t)c * n * 2 + (lane & 1);
+  float* b = smf + lane;
+  float* tmp = smf + (size_t)n * 32 + lane;  // two blocks of residuals
+  const float* ab = hc.ab32 + (size_t)s * ldab * n;
+  const int* ip = hc.ipiv + (size_t)s * n;
+#pragma unroll 8
+  for (int k = 0; k < n; ++k) b[32 * k] = (float)rc[2 * k];
+  band_sweep_lane(ab, ip, b, n, N);
+  const double eps = hc.sys[s].eps;
+  const double* pen = hc.pen + (size_t)s * 6 * g.ns;
+  auto x = [&](int i) { return (double)b[32 * i]; };
+  for (int ks = 0; ks < g.ns; ++ks) {
+    float* t = tmp + (ks & 1) * N * 32;
+    for (int k1 = 0; k1 < N; ++k1) {
+      const int r = ks * N + k1;
+      t[32 * k1] = (float)(rc[2 * r] - apply_A_row(g, D2, zh, eps, pen, x, r));
+    }
+    if (ks > 0) {  // block ks - 1 is read no more
+      const float* p = tmp + ((ks - 1) & 1) * N * 32;
+      for (int k1 = 0; k1 < N; ++k1) {
+        const int r = (ks - 1) * N + k1;
+        const double x1 = x(r);
+        b[32 * r] = p[32 * k1];
+        xc[2 * r] = x1;
+      }
+    }
+  }
+  const float* p = tmp + ((g.ns - 1) & 1) * N * 32;
+  for (int k1 = 0; k1 < N; ++k1) {
+    const int r = (g.ns - 1) * N + k1;
+    const double x1 = x(r);
+    b[32 * r] = p[32 * k1];
+    xc[2 * r] = x1;
+  }
+  band_sweep_lane(ab, ip, b, n, N);
+  for (int k = 0; k < n; ++k) xc[2 * k] += (double)b[32 * k];
 }
 
 static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, int top, const double* rhs,
@@ -2717,8 +2784,57 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     s.erase(std::unique(s.begin(), s.end()), s.end());
     HelmCache hc;
     hc.nsys = (int)s.size();
+    std::vector<int> cs(ncol), order(ncol);
+    for (int c = 0; c < ncol; ++c) {
+      cs[c] = (int)(std::lower_bound(s.begin(), s.end(), lam[c]) - s.begin());
+      order[c] = c;
+    }
+    // Block inverses (system-grouped, on the tensor cores) for the systems whose estimated condition
+    // needs no residual sweep, as in the time step; the others keep the pivoted band LU.
+    const bool tc = h->ns <= 16 && N <= kTcMaxN && n <= kSysMaxRows &&
+                    helm_smem(n, N, ns, h->nb).total <= 200 * 1024;
+    const double rho = cond_slope(h);
+    hc.first = hc.nsys;
+    if (tc)
+      while (hc.first > 0 && s[hc.first - 1] > 0 && 1.0 + rho / s[hc.first - 1] <= kRefineCond) --hc.first;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cs[a] < cs[b]; });
+    std::vector<Task> tasks;
+    std::vector<int> list;
+    for (int i = 0; i < ncol;) {
+      const int u = cs[order[i]];
+      int j = i;
+      while (j < ncol && cs[order[j]] == u && j - i < kSysR / 2) ++j;
+      if (u < hc.first)
+        list.insert(list.end(), order.begin() + i, order.begin() + j);
+      else
+        tasks.push_back(Task{u - hc.first, i, j - i});
+      i = j;
+    }
+    hc.ntask = (int)tasks.size();
+    hc.nlist = (int)list.size();
+    if (up(h, &hc.lam, s) || up(h, &hc.colsys, cs)) return IW_ERR_NOMEM;
+    if (up(h, &hc.order, order) || (hc.ntask > 0 && up(h, &hc.tasks, tasks))) return IW_ERR_NOMEM;
+    if (hc.nlist > 0 && up(h, &hc.list, list)) return IW_ERR_NOMEM;
+    it = g_helm.emplace(key, hc).first;
+  }
+  HelmCache& hc = it->second;
+  // k_solve_tc copies whole complex values: 16-byte aligned columns
+  const bool tc = mode == 0 && hc.ntask > 0 && (((uintptr_t)rhs | (uintptr_t)sol) & 15) == 0;
+  const int nt = hc.nsys - hc.first, m = 2 * (ns - 1);
+  if (tc && !hc.ainv) {
+    double* ainv = nullptr;
+    if (dalloc(h, &ainv, (size_t)nt * h->nb * N * N) || dalloc(h, &hc.lvec, (size_t)nt * std::max(m, 1) * N) ||
+        dalloc(h, &hc.minv, (size_t)nt * std::max(m * m, 1)) || dalloc(h, &hc.pen2, (size_t)nt * 6 * ns) ||
+        dalloc(h, &hc.sys2, (size_t)nt))
+      return IW_ERR_NOMEM;
+    if (int r = build_systems(h, hc.lam + hc.first, nt, 0.0, bot, top, false, 0, ainv, nullptr, hc.lvec, hc.minv, hc.pen2, hc.sys2))
+      return r;
+    hc.ainv = ainv;
+  }
+  if ((!tc || hc.nlist > 0) && !hc.ab) {  // band LU factors
     std::vector<SysDesc> sys(hc.nsys);
-    std::vector<double> pen((size_t)hc.nsys * 6 * ns);
+    std::vector<double> pen((size_t)hc.nsys * 6 * ns), s(hc.nsys);
+    CK(scopy(h, s.data(), hc.lam, s.size() * sizeof(double), cudaMemcpyDeviceToHost));
     for (int u = 0; u < hc.nsys; ++u) {
       memset(&sys[u], 0, sizeof(SysDesc));
       sys[u].eps = 1. / s[u];
@@ -2728,36 +2844,76 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
       sys[u].tau1_bot = pen[(size_t)u * 6 * ns + 4 * ns];
       sys[u].tau2_top = pen[(size_t)u * 6 * ns + 5 * ns + ns - 1];
     }
-    std::vector<int> cs(ncol);
-    for (int c = 0; c < ncol; ++c) cs[c] = (int)(std::lower_bound(s.begin(), s.end(), lam[c]) - s.begin());
-    if (dalloc(h, &hc.ab, (size_t)hc.nsys * ldab * n) || dalloc(h, &hc.ab32, (size_t)hc.nsys * ldab * n) ||
+    double* ab = nullptr;
+    if (dalloc(h, &ab, (size_t)hc.nsys * ldab * n) || dalloc(h, &hc.ab32, (size_t)hc.nsys * ldab * n) ||
         dalloc(h, &hc.ipiv, (size_t)hc.nsys * n) || dalloc(h, &hc.info, (size_t)hc.nsys) ||
-        up(h, &hc.sys, sys) || up(h, &hc.pen, pen) || up(h, &hc.colsys, cs))
+        up(h, &hc.sys, sys) || up(h, &hc.pen, pen))
       return IW_ERR_NOMEM;
+    hc.ab = ab;
     FactorArgs fa;
     fa.sys = hc.sys;
     fa.pen = hc.pen;
     fa.ab = hc.ab;
-    fa.ipiv = hc.ipiv;
-    fa.info = hc.info;
     fa.nsys = hc.nsys;
     fa.D = h->dD;
     fa.D2 = h->dD2;
     fa.zh = h->dzh;
-    fa.assemble = 1;
-    k_factor<<<(hc.nsys + 3) / 4, 128, 0, h->st>>>(geo(h), fa);
+    k_assemble_band<<<(hc.nsys + 3) / 4, 128, 0, h->st>>>(geo(h), fa);
+    launch_band_lu(h->st, hc.nsys, n, N, hc.ab, hc.ipiv, hc.info);
     size_t tot = (size_t)hc.nsys * ldab * n;
     k_convert<double, float><<<2048, 256, 0, h->st>>>(hc.ab, hc.ab32, tot);
-    CK(cudaStreamSynchronize(h->st));
-    it = g_helm.emplace(key, hc).first;
+    CK(cudaGetLastError());
   }
-  const HelmCache& hc = it->second;
-  const int warps = 4;
-  size_t smem = (size_t)warps * 6 * n * sizeof(double);
-  cudaFuncSetAttribute(k_helm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_helm<<<(ncol + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), hc, rhs, sol, ncol, mode, h->dD2, h->dzh);
-  CK(cudaGetLastError());
+  if (tc) {
+    HelmTc H;
+    memset(&H, 0, sizeof H);
+    H.ainv = hc.ainv;
+    H.lvec = hc.lvec;
+    H.minv = hc.minv;
+    H.pen = hc.pen2;
+    H.sys = hc.sys2;
+    H.D = h->dD;
+    H.D2t = h->dD2t;
+    H.zh = h->dzh;
+    H.tasks = hc.tasks;
+    H.order = hc.order;
+    H.rhs = rhs;
+    H.sol = sol;
+    H.nb = h->nb;
+    memcpy(H.bmap, h->bmap, sizeof H.bmap);
+    launch_helm_tc<double>(h, H, hc.ntask);
+    CK(cudaGetLastError());
+  }
+  const int nc = tc ? hc.nlist : ncol;
+  const size_t sm32 = helm32_smem(n, N);
+  if (mode != 0 && sm32 <= 200 * 1024 && rhs != sol) {
+    cudaFuncSetAttribute(k_helm32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
+    k_helm32<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), hc, rhs, sol, ncol, h->dD2, h->dzh, hc.order);
+    CK(cudaGetLastError());
+  } else if (nc > 0) {
+    const int warps = 4;
+    size_t smem = (size_t)warps * 6 * n * sizeof(double);
+    cudaFuncSetAttribute(k_helm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), hc, rhs, sol, nc, mode, h->dD2, h->dzh,
+                                                                  tc ? hc.list : nullptr);
+    CK(cudaGetLastError());
+  }
   return 0;
+}
+
+// the isolated-solve tables of a handle that goes away
+static void helm_free(iw_handle* h) {
+  for (auto it = g_helm.begin(); it != g_helm.end();) {
+    if (it->first.first != h) {
+      ++it;
+      continue;
+    }
+    HelmCache& c = it->second;
+    for (void* p : {(void*)c.ab, (void*)c.ab32, (void*)c.ipiv, (void*)c.info, (void*)c.sys, (void*)c.pen, (void*)c.colsys,
+                    (void*)c.lam, (void*)c.pen2, (void*)c.sys2, (void*)c.ainv, (void*)c.lvec, (void*)c.minv, (void*)c.tasks, (void*)c.order, (void*)c.list})
+      cudaFree(p);
+    it = g_helm.erase(it);
+  }
 }
 
 #include "iw_abi.inl"

@@ -25,7 +25,7 @@
 // dumps, Legendre spectra (k_speclegen) and the TKE budget (k_row_dot,
 // k_sub_rowmean), written by a host thread from pinned buffers.
 // The penalty systems (penalty.f + band_lu.f) are assembled on the device
-// (k_factor) when epsilon changes (steps 1-3 and a dt change), one per distinct
+// (k_build_systems, k_assemble_band) when epsilon changes (steps 1-3 and a dt change), one per distinct
 // kx^2+ky^2 and system type, then factored (band LU) or turned into block
 // inverses of their distinct subdomain blocks.
 #include <cuda_runtime.h>
@@ -1047,9 +1047,9 @@ __global__ void __launch_bounds__(192) k_wviscrot(Geo g, const T* __restrict__ u
 
 // ===========================================================================
 // Band factorisation (penalty.f:403-634 assembly, band_lu.f:19-34 packing,
-// bandludcmp.f:238-440 SGBTF2).  One warp per system; the arithmetic follows
-// the reference order with no fused multiply-add, so the factors equal the
-// CPU ones bit for bit.
+// bandludcmp.f:238-440 SGBTF2).  The arithmetic follows the reference order with
+// no fused multiply-add, so the factors equal the CPU ones bit for bit.  Assembly: one
+// warp per system.
 // ===========================================================================
 struct SysDesc {
   double eps;
@@ -1062,35 +1062,29 @@ struct FactorArgs {
   const SysDesc* sys = nullptr;
   const double* pen = nullptr;  // per system: 6*ns (alpha,beta,gamma,delta,tau1,tau2)
   double* ab = nullptr;         // per system: ldab*nz
-  int* ipiv = nullptr;          // per system: nz
-  int* info = nullptr;          // per system
   int nsys = 0;
   const double* D = nullptr;
   const double* D2 = nullptr;
   const double* zh = nullptr;  // ns
-  int assemble = 1;            // 0: ab already holds the packed matrix (bandlu_solve_)
-  int factor = 1;              // 0: assemble only (block-inverse systems)
 };
 
 __device__ __forceinline__ double& ABr(double* ab, int ldab, int r, int c) {
   return ab[(size_t)(r - 1) + (size_t)ldab * (size_t)(c - 1)];
 }
 
-static __global__ void k_factor(Geo g, FactorArgs fa) {
+static __global__ void k_assemble_band(Geo g, FactorArgs fa) {
   const int warps = blockDim.x / 32;
   const int s = blockIdx.x * warps + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (s >= fa.nsys) return;
   const int n = g.nz, N = g.N, ns = g.ns, kl = N, ku = N, ldab = 2 * kl + ku + 1;
   double* ab = fa.ab + (size_t)s * ldab * n;
-  int* ipiv = fa.ipiv + (size_t)s * n;
   const double eps = fa.sys[s].eps;
   const double* pen = fa.pen + (size_t)s * 6 * ns;
   const double *pa = pen, *pb = pen + ns, *pg = pen + 2 * ns, *pd = pen + 3 * ns, *pt1 = pen + 4 * ns,
                *pt2 = pen + 5 * ns;
   const double* d = fa.D;
   const double* d2 = fa.D2;
-  if (fa.assemble) {
   // zero the band
   for (size_t t = lane; t < (size_t)ldab * n; t += 32) ab[t] = 0.0;
   __syncwarp();
@@ -1158,75 +1152,116 @@ static __global__ void k_factor(Geo g, FactorArgs fa) {
     }
   }
 #undef AEL
-  }
-  if (!fa.factor) return;
-  // SGBTF2
-  const int kv = ku + kl;
-  int info = 0;
-  for (int jj = ku + 2; jj <= min(kv, n); ++jj)
-    for (int i = kv - jj + 2 + lane; i <= kl; i += 32) ABr(ab, ldab, i, jj) = 0.0;
-  __syncwarp();
-  int ju = 1;
-  for (int j = 1; j <= n; ++j) {
-    if (j + kv <= n)
-      for (int i = 1 + lane; i <= kl; i += 32) ABr(ab, ldab, i, j + kv) = 0.0;
-    __syncwarp();
-    const int km = min(kl, n - j);
-    // ISAMAX: first index of the largest |a|
-    double best = -1.0;
-    int bi = 1 << 30;
-    for (int i = 1 + lane; i <= km + 1; i += 32) {
-      double v = fabs(ABr(ab, ldab, kv + i, j));
-      if (v > best) {
-        best = v;
-        bi = i;
+}
+
+// SGBTF2 (bandludcmp.f:238-440), one CTA per system.  The columns a step touches (j .. j + kl
+// + ku) live in a ring in shared memory; the next ones arrive by cp.async eight steps
+// ahead, and a finished column goes back to global memory.  Per step the first warp finds the
+// pivot and forms the multipliers, then every thread swaps and updates its part of the
+// remaining columns: two barriers, no dependent access to global memory.  Bound by that
+// chain of about 500 cycles per column; the arithmetic of every element and its
+// order are the reference's.
+constexpr int kLuThreads = 128, kLuAhead = 8;
+__host__ __device__ inline int lu_ring(int N) { return 2 * N + 1 + kLuAhead; }
+__host__ __device__ inline size_t lu_smem(int N) {
+  return ((size_t)lu_ring(N) * (3 * N + 1) + N + 2) * sizeof(double);
+}
+static __global__ void __launch_bounds__(kLuThreads) k_band_lu(int n, int N, double* __restrict__ abs_, int* __restrict__ ipivs,
+                                                               int* __restrict__ infos) {
+  extern __shared__ __align__(16) double sml[];
+  __shared__ int sjp;
+  const int kl = N, ku = N, kv = kl + ku, ldab = 2 * kl + ku + 1, W = lu_ring(N);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double* ab = abs_ + (size_t)blockIdx.x * ldab * n;
+  int* ipiv = ipivs + (size_t)blockIdx.x * n;
+  double* ring = sml;                     // column j at ring + (j % W) ldab
+  double* lb = ring + (size_t)W * ldab;   // multipliers of the current step
+  // column c (0-based): the kl fill rows start as 0
+  auto fetch = [&](int c) {
+    if (c < n) {
+      double* d = ring + (size_t)(c % W) * ldab;
+      const double* s = ab + (size_t)c * ldab;
+      for (int r = tid; r < ldab; r += kLuThreads) {
+        if (r < kl)
+          d[r] = 0.0;
+        else
+          cp_async_c<float2>((float2*)(d + r), (const float2*)(s + r));
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) {
-        best = ob;
-        bi = oi;
-      }
-    }
-    const int jp = bi;
-    if (lane == 0) ipiv[j - 1] = jp + j - 1;
-    const double piv = ABr(ab, ldab, kv + jp, j);
-    __syncwarp();
-    if (piv != 0.0) {
-      ju = max(ju, min(j + ku + jp - 1, n));
-      if (jp != 1) {
-        for (int cc = lane; cc < ju - j + 1; cc += 32) {
-          double t1 = ABr(ab, ldab, kv + jp - cc, j + cc);
-          ABr(ab, ldab, kv + jp - cc, j + cc) = ABr(ab, ldab, kv + 1 - cc, j + cc);
-          ABr(ab, ldab, kv + 1 - cc, j + cc) = t1;
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  for (int c = 0; c <= kv; ++c) fetch(c);
+  for (int c = kv + 1; c < kv + kLuAhead; ++c) fetch(c);
+  int ju = 0, info = 0;  // last column touched so far (0-based)
+  for (int j = 0; j < n; ++j) {
+    fetch(j + kv + kLuAhead);  // its slot held column j - 1, stored before the last barrier
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kLuAhead) : "memory");  // columns <= j + kv are here
+    __syncthreads();
+    const int km = min(kl, n - 1 - j);
+    double* cj = ring + (size_t)(j % W) * ldab;
+    if (wid == 0) {
+      // ISAMAX: first index of the largest |a| in rows kv .. kv + km
+      double best = -1.0;
+      int bi = 1 << 30;
+      for (int i = lane; i <= km; i += 32) {
+        const double v = fabs(cj[kv + i]);
+        if (v > best) {
+          best = v;
+          bi = i;
         }
       }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+        }
+      }
+      if (bi > km) bi = 0;  // only NaNs: the first row, as ISAMAX
+      const double piv = cj[kv + bi], top = cj[kv];
       __syncwarp();
-      if (km > 0) {
-        const double rcp = __ddiv_rn(1.0, ABr(ab, ldab, kv + 1, j));
-        for (int i = 1 + lane; i <= km; i += 32) ABr(ab, ldab, kv + 1 + i, j) = rmul(rcp, ABr(ab, ldab, kv + 1 + i, j));
-        __syncwarp();
-        if (ju > j) {
-          for (int jj = 1 + lane; jj <= ju - j; jj += 32) {
-            double y = ABr(ab, ldab, kv + 1 - jj, j + jj);
-            if (y != 0.0) {
-              double temp = -y;
-              for (int ii = 1; ii <= km; ++ii) {
-                double& x = ABr(ab, ldab, kv + 1 + ii - jj, j + jj);
-                x = radd(x, rmul(ABr(ab, ldab, kv + 1 + ii, j), temp));
-              }
-            }
-          }
+      if (lane == 0) {
+        sjp = piv != 0.0 ? bi : -1 - bi;
+        ipiv[j] = j + bi + 1;
+      }
+      if (piv != 0.0) {
+        const double rcp = km > 0 ? __ddiv_rn(1.0, piv) : 0.0;
+        for (int i = 1 + lane; i <= km; i += 32) {
+          const double l = rmul(rcp, i == bi ? top : cj[kv + i]);
+          lb[i] = l;
+          cj[kv + i] = l;
         }
-        __syncwarp();
+        if (lane == 0) cj[kv] = piv;
+      }
+    }
+    __syncthreads();
+    const int jp = sjp;
+    if (jp >= 0) {
+      ju = max(ju, min(j + ku + jp, n - 1));
+      // a thread per column j + 1 .. ju (at most 2 N of them)
+      for (int cc = 1 + tid; cc <= ju - j; cc += kLuThreads) {
+        int sl = (j % W) + cc;
+        if (sl >= W) sl -= W;
+        double* col = ring + (size_t)sl * ldab + kv - cc;  // row i of the step at col[i]
+        const double y = col[jp];
+        if (jp != 0) {
+          col[jp] = col[0];
+          col[0] = y;
+        }
+        if (y != 0.0) {
+          const double temp = -y;
+#pragma unroll 8
+          for (int i = 1; i <= km; ++i) col[i] = radd(col[i], rmul(lb[i], temp));
+        }
       }
     } else if (info == 0) {
-      info = j;
+      info = j + 1;
     }
+    for (int r = tid; r < ldab; r += kLuThreads) ab[(size_t)j * ldab + r] = cj[r];
+    __syncthreads();
   }
-  if (lane == 0) fa.info[s] = info;
+  if (tid == 0) infos[blockIdx.x] = info;
 }
 
 // ===========================================================================
@@ -1475,8 +1510,6 @@ struct BlockInv {
   const void* ainv;
   int nb;
   int bmap[IW_MAX_SUBD];
-  const double* cvec;   // per system: ns*N (c_ks, ks>=1)
-  const double* dvec;   // per system: ns*N (d_ks, ks<=ns-2)
   const double* minv;   // per system: m*m, m = 2(ns-1), row major
   const double* pen;    // per system: 6*ns penalty parameters
   const SysDesc* sys;
@@ -1485,133 +1518,224 @@ struct BlockInv {
   const double* lvec;   // per system: m*N left vectors (see k_solve_cta)
 };
 
-// warp per (system, block): invert A_ks from the assembled band
-static __global__ void k_block_invert(Geo g, const double* __restrict__ ab, int nsys, double* __restrict__ ainv64,
-                               double* __restrict__ cvec, double* __restrict__ dvec) {
-  extern __shared__ __align__(16) double smi[];
-  const int warps = blockDim.x / 32, wid = threadIdx.x / 32, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * warps + wid;
-  const int N = g.N, ns = g.ns, n = g.nz, ldab = 3 * N + 1;
-  if (task >= nsys * ns) return;
-  const int s = task / ns, ks = task % ns, km = ks * N;
-  const double* a = ab + (size_t)s * ldab * n;
-  double* M = smi + (size_t)wid * N * 2 * N;  // row major N x 2N
-  auto AB = [&](int r, int c) -> double {     // 0-based global (r, c)
-    int br = 2 * N + r - c;                    // 0-based band row
-    if (br < 0 || br >= ldab) return 0.0;
-    return a[(size_t)br + (size_t)ldab * c];
-  };
-  for (int t = lane; t < N * 2 * N; t += 32) {
-    int r = t / (2 * N), c = t % (2 * N);
-    M[t] = c < N ? AB(km + r, km + c) : (c - N == r ? 1.0 : 0.0);
-  }
-  for (int k = lane; k < N; k += 32) {
-    cvec[((size_t)s * ns + ks) * N + k] = ks > 0 ? AB(km, km - N + k) : 0.0;
-    dvec[((size_t)s * ns + ks) * N + k] = ks < ns - 1 ? AB(km + N - 1, km + N + k) : 0.0;
-  }
-  __syncwarp();
-  for (int col = 0; col < N; ++col) {
-    // pivot: largest |M[r][col]|, r >= col
-    double best = -1.0;
-    int bi = col;
-    for (int r = col + lane; r < N; r += 32) {
-      double v = fabs(M[r * 2 * N + col]);
-      if (v > best) {
-        best = v;
-        bi = r;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) {
-        best = ob;
-        bi = oi;
-      }
-    }
-    if (bi != col)
-      for (int c = lane; c < 2 * N; c += 32) {
-        double t = M[col * 2 * N + c];
-        M[col * 2 * N + c] = M[bi * 2 * N + c];
-        M[bi * 2 * N + c] = t;
-      }
-    __syncwarp();
-    const double inv = 1.0 / M[col * 2 * N + col];
-    for (int c = lane; c < 2 * N; c += 32) M[col * 2 * N + c] *= inv;
-    __syncwarp();
-    for (int r = 0; r < N; ++r) {
-      if (r == col) continue;
-      const double f = M[r * 2 * N + col];
-      if (f != 0.0)
-        for (int c = lane; c < 2 * N; c += 32) M[r * 2 * N + c] -= f * M[col * 2 * N + c];
-    }
-    __syncwarp();
-  }
-  double* out = ainv64 + ((size_t)s * ns + ks) * N * N;
-  for (int t = lane; t < N * N; t += 32) {
-    int c = t / N, r = t % N;  // column major
-    out[t] = M[r * 2 * N + N + c];
+// ===========================================================================
+// Tables of the block-inverse solves, one CTA per system, straight from epsilon:
+// penalty parameters (penalty.f:57-157), the distinct subdomain blocks and the
+// coupling vectors (penalty.f:403-634, the operations of k_assemble_band in its
+// order), Gauss-Jordan inverses with partial pivoting, left vectors, interface
+// matrix and its inverse, the Legendre filter folded into the inverses.  Everything
+// stays in shared memory until the tables are written; no band, no workspace, nothing on
+// the host.  Bound by the serial pivot steps (two barriers each); a system's blocks
+// are few, so several CTAs per SM hide them.
+// ===========================================================================
+struct BuildArgs {
+  int N, ns, nb, nsys, nraw;  // nraw: systems that also keep their unfiltered inverses
+  int bot, top;               // boundary conditions (0 Dirichlet, 1 Neumann)
+  double c0;                  // epsilon = 1 / (ak + c0)
+  double facdir, facneumn, facrobin;
+  int bmap[IW_MAX_SUBD], brep[IW_MAX_SUBD];
+  const double *ak, *D, *D2, *zh, *L;  // L: filter to fold in, or null
+  SysDesc* sys;
+  double *pen, *ainv, *ainv_raw, *lvec, *minv;
+};
+// penalty.f:57-157 (h_param_set, with every rounding written out)
+static __device__ void d_param_set(const BuildArgs& b, int ifbc, double eps, double ybar, double& a0, double& b0,
+                                   double& t0) {
+  const double omega = __ddiv_rn(2., (double)((b.N + 1) * (b.N + 2)));
+  if (ifbc == 0) {
+    const double h = __ddiv_rn(2., ybar), fac = rmul(b.facdir, rmul(h, h));
+    a0 = 1.;
+    b0 = 0.;
+    t0 = __ddiv_rn(rmul(fac, eps), rmul(omega, omega));
+  } else if (ifbc == 1) {
+    a0 = 0.;
+    b0 = 1.;
+    t0 = __ddiv_rn(__ddiv_rn(rmul(b.facneumn, 2.), ybar), omega);
+  } else {
+    a0 = 1.;
+    b0 = 1.;
+    const double dn = __ddiv_rn(1., rmul(omega, eps));
+    const double t1 = __dsqrt_rn(radd(rmul(omega, omega), rmul(eps, omega)));
+    const double t2 = rsub(rmul(2., omega), rmul(2., t1));
+    const double facm = __ddiv_rn(1., eps) >= 1.e5 ? b.facrobin : 1.;
+    t0 = __ddiv_rn(rmul(rmul(rmul(facm, dn), radd(eps, t2)), 2.), ybar);
   }
 }
-
-// thread per system: interface matrix M (m = 2(ns-1)) and its inverse
-static __global__ void k_iface_matrix(Geo g, int nsys, const double* __restrict__ ainv64, const double* __restrict__ cvec,
-                               const double* __restrict__ dvec, double* __restrict__ minv, double* __restrict__ work) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int N = g.N, ns = g.ns, m = 2 * (ns - 1);
-  if (s >= nsys || m == 0) return;
-  double* A = work + (size_t)s * 2 * m * m;  // m x 2m
-  for (int t = 0; t < 2 * m * m; ++t) A[t] = 0.0;
-  // unknown index: sigma_ks (ks=1..ns-1) -> ks-1 ; tau_ks (ks=0..ns-2) -> ns-1+ks
-  auto inv = [&](int ks, int r, int c) { return ainv64[(((size_t)s * ns + ks) * N + c) * N + r]; };
-  for (int ks = 0; ks < ns; ++ks) {
-    if (ks + 1 <= ns - 1) {  // row for sigma_{ks+1}
-      int row = ks;          // sigma_{ks+1} index
-      const double* c = cvec + ((size_t)s * ns + ks + 1) * N;
-      double cp = 0, cq = 0;
-      for (int k = 0; k < N; ++k) {
-        cp += c[k] * inv(ks, k, 0);
-        cq += c[k] * inv(ks, k, N - 1);
+// Gauss-Jordan on the n x 2 n matrix A (right half: the identity) with the CTA's
+// threads; skip: columns left of the pivot hold zeros in the pivot row
+static __device__ void gauss_jordan(double* A, int n, int* piv, double* pinv) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, n2 = 2 * n;
+  for (int col = 0; col < n; ++col) {
+    if (w == 0) {  // the first row of the largest |A(r, col)|, r >= col
+      double best = -1.0;
+      int bi = col;
+      for (int r = col + lane; r < n; r += 32) {
+        const double v = fabs(A[r * n2 + col]);
+        if (v > best) {
+          best = v;
+          bi = r;
+        }
       }
-      A[row * 2 * m + row] += 1.0;
-      if (ks >= 1) A[row * 2 * m + (ks - 1)] += cp;
-      if (ks <= ns - 2) A[row * 2 * m + (ns - 1 + ks)] += cq;
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+        }
+      }
+      if (lane == 0) {
+        *piv = bi;
+        *pinv = __ddiv_rn(1.0, A[bi * n2 + col]);
+      }
     }
-    if (ks - 1 >= 0) {  // row for tau_{ks-1}
-      int row = ns - 1 + ks - 1;
-      const double* d = dvec + ((size_t)s * ns + ks - 1) * N;
-      double dp = 0, dq = 0;
-      for (int k = 0; k < N; ++k) {
-        dp += d[k] * inv(ks, k, 0);
-        dq += d[k] * inv(ks, k, N - 1);
-      }
-      A[row * 2 * m + row] += 1.0;
-      if (ks >= 1) A[row * 2 * m + (ks - 1)] += dp;
-      if (ks <= ns - 2) A[row * 2 * m + (ns - 1 + ks)] += dq;
+    __syncthreads();
+    const int bi = *piv;
+    const double iv = *pinv;
+    for (int c = col + threadIdx.x; c < n2; c += blockDim.x) {
+      const double p = A[bi * n2 + c];
+      if (bi != col) A[bi * n2 + c] = A[col * n2 + c];
+      A[col * n2 + c] = rmul(p, iv);
     }
+    __syncthreads();
+    for (int r = w; r < n; r += nw) {
+      if (r == col) continue;
+      const double f = A[r * n2 + col];
+      __syncwarp();
+      if (f != 0.0)
+        for (int c = col + lane; c < n2; c += 32) A[r * n2 + c] = __fma_rn(-f, A[col * n2 + c], A[r * n2 + c]);
+    }
+    __syncthreads();
   }
-  for (int r = 0; r < m; ++r) A[r * 2 * m + m + r] = 1.0;
-  for (int col = 0; col < m; ++col) {
-    int bi = col;
-    for (int r = col + 1; r < m; ++r)
-      if (fabs(A[r * 2 * m + col]) > fabs(A[bi * 2 * m + col])) bi = r;
-    if (bi != col)
-      for (int c = 0; c < 2 * m; ++c) {
-        double t = A[col * 2 * m + c];
-        A[col * 2 * m + c] = A[bi * 2 * m + c];
-        A[bi * 2 * m + c] = t;
-      }
-    double iv = 1.0 / A[col * 2 * m + col];
-    for (int c = 0; c < 2 * m; ++c) A[col * 2 * m + c] *= iv;
-    for (int r = 0; r < m; ++r)
-      if (r != col) {
-        double f = A[r * 2 * m + col];
-        if (f != 0.0)
-          for (int c = 0; c < 2 * m; ++c) A[r * 2 * m + c] -= f * A[col * 2 * m + c];
-      }
+}
+__host__ __device__ inline size_t build_smem(int N, int ns) {
+  const size_t m = 2 * (size_t)(ns - 1);
+  return ((size_t)N * 2 * N + 2 * (size_t)ns * N + 2 * m + m * 2 * m + 6 * (size_t)ns + 4) * sizeof(double);
+}
+static __global__ void __launch_bounds__(256) k_build_systems(const __grid_constant__ BuildArgs b) {
+  extern __shared__ __align__(16) double smb[];
+  __shared__ int piv;
+  __shared__ double pinv;
+  const int N = b.N, ns = b.ns, m = 2 * (ns - 1), s = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
+  double* M = smb;                // N x 2 N
+  double* cv = M + N * 2 * N;     // c_ks (row 0 of block ks against block ks - 1)
+  double* dv = cv + ns * N;       // d_ks (row N - 1 of block ks against block ks + 1)
+  double* ends = dv + ns * N;     // first and last entry of every left vector
+  double* A = ends + 2 * m;       // interface matrix, m x 2 m
+  double* pen = A + m * 2 * m;
+  double *pa = pen, *pb = pen + ns, *pg = pen + 2 * ns, *pd = pen + 3 * ns, *pt1 = pen + 4 * ns, *pt2 = pen + 5 * ns;
+  const double eps = __ddiv_rn(1., radd(b.ak[s], b.c0));
+  for (int ks = tid; ks < ns; ks += nthr) {
+    d_param_set(b, ks == 0 ? b.bot : 2, eps, b.zh[ks], pa[ks], pb[ks], pt1[ks]);
+    d_param_set(b, ks == ns - 1 ? b.top : 2, eps, b.zh[ks], pg[ks], pd[ks], pt2[ks]);
   }
-  for (int r = 0; r < m; ++r)
-    for (int c = 0; c < m; ++c) minv[(size_t)s * m * m + r * m + c] = A[r * 2 * m + m + c];
+  __syncthreads();
+  for (int q = tid; q < 6 * ns; q += nthr) b.pen[(size_t)s * 6 * ns + q] = pen[q];
+  if (tid == 0) {
+    SysDesc sd;
+    sd.eps = eps;
+    sd.tau1_bot = pt1[0];
+    sd.tau2_top = pt2[ns - 1];
+    sd.ifbcbot = b.bot;
+    sd.ifbctop = b.top;
+    sd.pad[0] = sd.pad[1] = 0;
+    b.sys[s] = sd;
+  }
+  for (int q = tid; q < ns * N; q += nthr) {
+    const int ks = q / N, k = q - ks * N;
+    double c = 0.0, d = 0.0;
+    if (ks > 0) {
+      if (k == N - 1) c = -rmul(rmul(0.5, pt1[ks]), pa[ks]);
+      c = radd(c, rmul(__ddiv_rn(rmul(rmul(rmul(rmul(0.5, pt1[ks]), pb[ks]), eps), 2.0), b.zh[ks - 1]), b.D[(N - 1) * N + k]));
+    }
+    if (ks < ns - 1) {
+      if (k == 0) d = rsub(0.0, rmul(rmul(0.5, pt2[ks]), pg[ks]));
+      d = radd(d, rmul(-__ddiv_rn(rmul(rmul(rmul(rmul(0.5, pt2[ks]), pd[ks]), eps), 2.0), b.zh[ks + 1]), b.D[k]));
+    }
+    cv[q] = c;
+    dv[q] = d;
+  }
+  __syncthreads();
+  for (int blk = 0; blk < b.nb; ++blk) {
+    const int ks = b.brep[blk];
+    const double ybar = b.zh[ks], h = __ddiv_rn(2.0, ybar), eh = rmul(eps, rmul(h, h));
+    const bool lo = ns > 1 && ks != 0, hi = ns > 1 && ks != ns - 1;
+    const double t1b = rmul(rmul(rmul(pt1[ks], pb[ks]), eps), 2.0), t2d = rmul(rmul(rmul(pt2[ks], pd[ks]), eps), 2.0);
+    const double cf1 = -__ddiv_rn(t1b, ybar), cf2 = __ddiv_rn(t2d, ybar);
+    const double cl = __ddiv_rn(rmul(rmul(rmul(rmul(0.5, pt1[ks]), pb[ks]), eps), 2.0), ybar);
+    const double ch = -__ddiv_rn(rmul(rmul(rmul(rmul(0.5, pt2[ks]), pd[ks]), eps), 2.0), ybar);
+    for (int q = tid; q < N * 2 * N; q += nthr) {
+      const int r = q / (2 * N), c = q - r * 2 * N;
+      double v = 0.0;
+      if (c >= N) {
+        v = c - N == r ? 1.0 : 0.0;
+      } else {
+        v = -rmul(eh, b.D2[r * N + c]);
+        if (r == c) v = radd(v, 1.0);
+        if (r == 0) {
+          if (c == 0) v = radd(v, rmul(pt1[ks], pa[ks]));
+          v = radd(v, rmul(cf1, b.D[c]));
+          if (lo) {
+            if (c == 0) v = rsub(v, rmul(rmul(0.5, pt1[ks]), pa[ks]));
+            v = radd(v, rmul(cl, b.D[c]));
+          }
+        }
+        if (r == N - 1) {
+          if (c == N - 1) v = radd(v, rmul(pt2[ks], pg[ks]));
+          v = radd(v, rmul(cf2, b.D[(N - 1) * N + c]));
+          if (hi) {
+            if (c == N - 1) v = rsub(v, rmul(rmul(0.5, pt2[ks]), pg[ks]));
+            v = radd(v, rmul(ch, b.D[(N - 1) * N + c]));
+          }
+        }
+      }
+      M[q] = v;
+    }
+    __syncthreads();
+    gauss_jordan(M, N, &piv, &pinv);
+    // the inverse is M(r, N + c): tables column major
+    double* out = b.ainv + ((size_t)s * b.nb + blk) * N * N;
+    double* raw = s < b.nraw ? b.ainv_raw + ((size_t)s * b.nb + blk) * N * N : nullptr;
+    for (int q = tid; q < N * N; q += nthr) {
+      const int c = q / N, r = q - c * N;
+      const double v = M[r * 2 * N + N + c];
+      if (raw) raw[q] = v;
+      if (b.L) {
+        const double* lr = b.L + (size_t)r * N;
+        double a = 0.0;
+        for (int j = 0; j < N; ++j) a = __fma_rn(lr[j], M[j * 2 * N + N + c], a);
+        out[q] = a;
+      } else {
+        out[q] = v;
+      }
+    }
+    // left vectors of the subdomains with this block: c_{ks+1} (e = ks) and d_{ks-1} (e = ns - 2 + ks)
+    for (int q = tid; q < m * N; q += nthr) {
+      const int e = q / N, c = q - e * N;
+      const int kb = e < ns - 1 ? e : e - (ns - 1) + 1;
+      if (b.bmap[kb] != blk) continue;
+      const double* v = e < ns - 1 ? cv + (e + 1) * N : dv + (kb - 1) * N;
+      double a = 0.0;
+      for (int k = 0; k < N; ++k) a = __fma_rn(M[k * 2 * N + N + c], v[k], a);
+      b.lvec[((size_t)s * m + e) * N + c] = a;
+      if (c == 0) ends[2 * e] = a;
+      if (c == N - 1) ends[2 * e + 1] = a;
+    }
+    __syncthreads();
+  }
+  if (m == 0) return;
+  // unknowns: sigma_ks (ks = 1 .. ns-1) -> ks - 1, tau_ks (ks = 0 .. ns-2) -> ns - 1 + ks
+  for (int q = tid; q < m * 2 * m; q += nthr) A[q] = (q % (2 * m)) - m == q / (2 * m) ? 1.0 : 0.0;
+  __syncthreads();
+  for (int row = tid; row < m; row += nthr) {
+    const int ks = row < ns - 1 ? row : row - (ns - 1) + 1;  // the block the row's coupling vector acts on
+    A[row * 2 * m + row] += 1.0;
+    if (ks >= 1) A[row * 2 * m + (ks - 1)] += ends[2 * row];
+    if (ks <= ns - 2) A[row * 2 * m + (ns - 1 + ks)] += ends[2 * row + 1];
+  }
+  __syncthreads();
+  gauss_jordan(A, m, &piv, &pinv);
+  for (int q = tid; q < m * m; q += nthr) b.minv[(size_t)s * m * m + q] = A[(q / m) * 2 * m + m + q % m];
 }
 
 // ===========================================================================
@@ -3183,6 +3307,162 @@ __global__ void __maxnreg__(NT <= 4 ? 64 : 80) k_press_tc(Geo g, const __grid_co
   }
 }
 
+// Isolated solves (iw_helm_solve_batched, mode 0) with the products of k_solve_tc and one
+// FP64 residual sweep, x += A^-1 (b - A x): the penalty rows of A are large, and the sweep
+// brings the residual of the block-inverse form to that of the pivoted band LU.
+// Right-hand sides and solutions are whole columns, [column][k] complex; 4 columns (8
+// right-hand sides) per CTA, blockIdx.y takes the task's other columns.  x, A x and the
+// residual stay in accumulator registers; the CTA exchanges four numbers per block and
+// right-hand side (the boundary values and derivatives) for the coupling rows.
+// 33024 columns of 8 x 25 points: 8.8 ms with the band LU (a warp per column, bound by the
+// latency of its serial sweep).
+struct HelmTc {
+  const double *ainv, *lvec, *minv, *pen, *D, *D2t, *zh;
+  const SysDesc* sys;
+  const Task* tasks;
+  const int* order;
+  const double* rhs;
+  double* sol;
+  int nb;
+  int bmap[IW_MAX_SUBD];
+};
+struct HelmSmem {  // byte offsets
+  size_t a, l, m, rz, zz, d2, dr, ex, raw, total;
+};
+__host__ __device__ inline HelmSmem helm_smem(int n, int N, int ns, int nb) {
+  HelmSmem o;
+  const size_t m = 2 * (size_t)(ns - 1), ap = tc_ap(N), D = sizeof(double);
+  o.a = 0;
+  o.l = o.a + (size_t)nb * tc_nc(N) * ap * D;
+  o.m = o.l + m * N * D;
+  o.rz = o.m + m * m * D;
+  o.zz = o.rz + m * 8 * D;
+  o.d2 = o.zz + m * 8 * D;
+  o.dr = o.d2 + (size_t)tc_nc(N) * ap * D;
+  o.ex = o.dr + 2 * (size_t)tc_nc(N) * D;
+  o.raw = o.ex + (size_t)ns * 4 * 8 * D;
+  o.total = o.raw + (size_t)n * 8 * D + 16 * D;
+  return o;
+}
+template <int NT>
+__global__ void __maxnreg__(NT <= 3 ? 64 : 80) k_helm_tc(Geo g, const __grid_constant__ HelmTc H) {
+  constexpr int R = 8;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const Task tk = H.tasks[blockIdx.x];
+  const int count = min(tk.count - 4 * (int)blockIdx.y, 4);
+  if (count <= 0) return;
+  const int* order = H.order + tk.first + 4 * blockIdx.y;
+  const int n = g.nz, N = g.N, ns = g.ns, m = 2 * (ns - 1), s = tk.sys;
+  const int tid = threadIdx.x, lane = tid & 31, ks = tid >> 5, lg = lane >> 2, lt = lane & 3;
+  const int AP = tc_ap(N);
+  const HelmSmem L = helm_smem(n, N, ns, H.nb);
+  double* sA = (double*)(smraw + L.a);
+  double* sL = (double*)(smraw + L.l);
+  double* sM = (double*)(smraw + L.m);
+  double* srz = (double*)(smraw + L.rz);
+  double* szz = (double*)(smraw + L.zz);
+  double* sD2 = (double*)(smraw + L.d2);
+  double* sDr = (double*)(smraw + L.dr);  // rows 0 and N - 1 of D
+  double* ex = (double*)(smraw + L.ex);   // [block][x_0, x_{N-1}, (D x)_0, (D x)_{N-1}][R]
+  double* raw = (double*)(smraw + L.raw) + (size_t)ks * N * 8;
+  {
+    const int ci = lane & 3;
+    const int c = ci < count ? order[ci] : -1;
+    tc_gather_cols<double, 4>(c, N, lane, [&](int, int r, int cs) {
+      return (const double2*)(H.rhs + ((size_t)cs * n + ks * N + r) * 2);
+    }, [&](int slot, int r) { return (double2*)(raw + tc_pos<double>(r, 2 * slot)); });
+  }
+  tc_columns(sD2, H.D2t, 1, N);
+  tc_tables(H.ainv + (size_t)s * H.nb * N * N, H.lvec + (size_t)s * m * N, H.minv + (size_t)s * m * m, H.nb, N, m, sA, sL, sM);
+  for (int q = tid; q < 2 * tc_nc(N); q += blockDim.x) {
+    const int c = q % tc_nc(N), row = q / tc_nc(N);
+    sDr[q] = c < N ? H.D[(row ? N - 1 : 0) * N + c] : 0.0;
+  }
+  const double eps = H.sys[s].eps;
+  cp_async_wait_all();
+  __syncthreads();
+  const bool lo = ks >= 1, hi = ks <= ns - 2;
+  const double* l = lg == 0 ? (hi ? sL + (size_t)ks * N : nullptr) : lg == 1 && lo ? sL + (size_t)(ns - 2 + ks) * N : nullptr;
+  const double* op = sA + (size_t)H.bmap[ks] * tc_nc(N) * AP;
+  double acc[1][NT][2], lacc[1][2], xv[NT][2], rv[NT][2];
+  auto solve = [&](auto&& rhs) {  // acc = A^-1 rhs
+    tc_product<NT, 1, true>(op, AP, N, lg, lt, rhs, acc, l, lacc);
+    if (m > 0) {
+      if (lt == 0) {
+        if (hi) srz[(size_t)ks * R + lg] = lacc[0][0];
+        if (lo) srz[(size_t)(ns - 2 + ks) * R + lg] = lacc[0][1];
+      }
+      tc_interface<R>(sM, srz, szz, m, R);
+      tc_rank2<NT>(op, AP, N, lg, lt, lo ? szz[(size_t)(ks - 1) * R + lg] : 0.0,
+                   hi ? szz[(size_t)(ns - 1 + ks) * R + lg] : 0.0, acc[0]);
+    }
+  };
+  const double* bl = raw + tc_pos<double>(lt, lg);
+  solve([&](int, int kt) {
+    double v = 0.0;
+    if ((NT > 2 && kt < 2 * NT - 2) || 4 * kt + lt < N) v = bl[32 * kt];
+    return v;
+  });
+  double* e = ex + (size_t)ks * 4 * R;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 8 * nt + 2 * lt + h;
+      xv[nt][h] = r < N ? acc[0][nt][h] : 0.0;
+      if (r == 0) e[lg] = xv[nt][h];
+      if (r == N - 1) e[R + lg] = xv[nt][h];
+    }
+  // D2 x and the derivatives at both ends of the block
+  const double* dl = lg == 0 ? sDr : lg == 1 ? sDr + tc_nc(N) : nullptr;
+  tc_product<NT, 1, true>(sD2, AP, N, lg, lt, [&](int, int kt) { return tc_next<NT>(xv, kt, lg, lt); }, acc, dl, lacc);
+  if (lt == 0) {
+    e[2 * R + lg] = lacc[0][0];
+    e[3 * R + lg] = lacc[0][1];
+  }
+  __syncthreads();
+  const double* pen = H.pen + (size_t)s * 6 * ns;
+  const double h2 = 2.0 / H.zh[ks], ee = eps * (h2 * h2);
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 8 * nt + 2 * lt + h;
+      rv[nt][h] = 0.0;
+      if (r < N) {
+        double v = xv[nt][h] - ee * acc[0][nt][h];
+        if (r == 0) {
+          const double pa = pen[ks], pb = pen[ns + ks], t1 = pen[4 * ns + ks], s0 = e[2 * R + lg];
+          v += t1 * pa * xv[nt][h] - t1 * pb * eps * h2 * s0;
+          if (lo) {
+            const double* el = e - 4 * R;
+            v += -0.5 * t1 * pa * xv[nt][h] + 0.5 * t1 * pb * eps * h2 * s0 - 0.5 * t1 * pa * el[R + lg] +
+                 0.5 * t1 * pb * eps * (2.0 / H.zh[ks - 1]) * el[3 * R + lg];
+          }
+        }
+        if (r == N - 1) {
+          const double pg = pen[2 * ns + ks], pd = pen[3 * ns + ks], t2 = pen[5 * ns + ks], s1 = e[3 * R + lg];
+          v += t2 * pg * xv[nt][h] + t2 * pd * eps * h2 * s1;
+          if (hi) {
+            const double* eh = e + 4 * R;
+            v += -0.5 * t2 * pg * xv[nt][h] - 0.5 * t2 * pd * eps * h2 * s1 - 0.5 * t2 * pg * eh[lg] -
+                 0.5 * t2 * pd * eps * (2.0 / H.zh[ks + 1]) * eh[2 * R + lg];
+          }
+        }
+        rv[nt][h] = raw[tc_pos<double>(r, lg)] - v;
+      }
+    }
+  solve([&](int, int kt) { return tc_next<NT>(rv, kt, lg, lt); });
+  const int c = (lg >> 1) < count ? order[lg >> 1] : -1;
+  double* dst = H.sol + ((size_t)max(c, 0) * n + ks * N) * 2;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    const double2 o = tc_pair<double>(xv[nt][0] + acc[0][nt][0], xv[nt][1] + acc[0][nt][1], lg);
+    const int ro = 8 * nt + 2 * lt + (lg & 1);
+    if (c >= 0 && ro < N) *(double2*)(dst + 2 * (size_t)ro) = o;
+  }
+}
+
 // ===========================================================================
 // z-column stages on the FP64 tensor cores (N <= 40), for either storage type.
 // A warp owns 8 consecutive points of the flattened (x, y) plane of one field and
@@ -3444,59 +3724,6 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 640 : 512) k_stageE_t(Geo g, 
         dst += pl8;
       }
     }
-  }
-}
-
-// Distinct blocks of each system into compact storage: out[s][b] = in[s][rep[b]],
-// with the Legendre filter folded in when L is given (out = L in, per column).
-struct BlockRep {
-  int r[IW_MAX_SUBD];
-};
-static __global__ void k_compact_blocks(int N, int nsys, int ns, int nb, BlockRep rep, const double* __restrict__ L,
-                                 const double* __restrict__ in, double* __restrict__ out) {
-  const size_t nn = (size_t)N * N, tot = (size_t)nsys * nb * nn;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < tot; q += (size_t)gridDim.x * blockDim.x) {
-    const size_t e = q % nn;
-    const size_t sb = q / nn;
-    const int b = (int)(sb % nb);
-    const size_t s = sb / nb;
-    const double* src = in + (s * ns + rep.r[b]) * nn;
-    if (!L) {
-      out[q] = src[e];
-    } else {
-      const int kk = (int)(e % N);
-      const double* col = src + (e - kk);
-      const double* lr = L + (size_t)kk * N;
-      double acc = 0.0;
-      for (int j = 0; j < N; ++j) acc += lr[j] * col[j];
-      out[q] = acc;
-    }
-  }
-}
-
-// lvec[s][e][c] = sum_k A_blk^-1[k][c] v_e[k]: v_e = c_{e+1} on block e (e < ns-1),
-// d_t on block t+1 (e = ns-1+t).  One thread per (system, e, c).
-static __global__ void k_left_vecs(Geo g, int nsys, const double* __restrict__ ainv, const double* __restrict__ cvec,
-                            const double* __restrict__ dvec, double* __restrict__ lvec) {
-  const int N = g.N, ns = g.ns, m = 2 * (ns - 1);
-  const size_t tot = (size_t)nsys * m * N;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < tot; q += (size_t)gridDim.x * blockDim.x) {
-    const int c = (int)(q % N);
-    const int e = (int)((q / N) % m);
-    const size_t s = q / ((size_t)N * m);
-    int blk;
-    const double* v;
-    if (e < ns - 1) {
-      blk = e;
-      v = cvec + (s * ns + e + 1) * N;
-    } else {
-      blk = e - (ns - 1) + 1;
-      v = dvec + (s * ns + blk - 1) * N;
-    }
-    const double* ai = ainv + (s * ns + blk) * (size_t)N * N + (size_t)c * N;
-    double acc = 0.0;
-    for (int k = 0; k < N; ++k) acc += ai[k] * v[k];
-    lvec[q] = acc;
   }
 }
 
