@@ -477,111 +477,134 @@ int iw_init_mode1(iw_handle* h, double A, double anoise, uint64_t seed) {
 
 }  // extern "C"
 
+// z derivatives of src[0..3] into dst[0..3]
+template <typename T>
+static void launch_dz4(iw_handle* h, FieldSet<T>& fs, T* const* src, T* const* dst) {
+  if (h->N <= kTcMaxN) {
+    FieldSet<T> v = fs;
+    for (int q = 0; q < 4; ++q) {
+      v.F[q] = src[q];
+      v.Z4[q] = dst[q];
+    }
+    const int keep = h->tune_a;
+    h->tune_a = -1;
+    launch_stageA<T>(h, v, -1);
+    h->tune_a = keep;
+    return;
+  }
+  for (int q = 0; q < 4; ++q)
+    k_dz_field<T><<<(unsigned)((h->ntot + 255) / 256), 256, 0, h->st>>>(geo(h), src[q], dst[q]);
+}
+
+// Runs k_xrow_stats over n entries whose rows are in a.src and brings the partials
+// to the host: nblk blocks per entry, kStatSlots values each, in h->hstat.  more:
+// queues further copies before the one wait.
+template <typename T, typename M>
+static int stats_to_host(iw_handle* h, FieldSet<T>& fs, StatRows<T>& a, int n, int* nblk, M&& more) {
+  const double dx = h->p.xlen / h->nx, dy = h->p.ylen / h->ny;
+  a.cflh[0] = h->p.dt / dx;
+  a.cflh[1] = h->p.dt / dy;
+  a.rg = -(h->p.rho0 * h->p.brunt * h->p.brunt) / h->p.grav;
+  a.zlim = 0.2 * h->p.zlen;
+  a.dzinv = h->ddzinv;
+  const int lines = h->ny * h->nz, most = std::min<int>((int)(kPartDoubles / (n * kStatSlots)), 12 * h->nsm / n);
+  *nblk = std::max(1, std::min(most, (lines + kStatThreads / 32 - 1) / (kStatThreads / 32)));
+  if (!h->hstat) CK(cudaHostAlloc((void**)&h->hstat, (kPartDoubles + 4) * sizeof(double), cudaHostAllocDefault));
+  launch_xstats<T>(h, fs, a, n, *nblk);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(h->hstat, h->dpart, (size_t)n * *nblk * kStatSlots * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  const int r = more();
+  if (r) return r;
+  CK(cudaStreamSynchronize(h->st));
+  return 0;
+}
+
 template <typename T>
 static int diag_impl(iw_handle* h, FieldSet<T>& fs, iw_diag_out* out) {
-  Geo g = geo(h);
-  T* dst = fs.Y12[0];
-  T* tmp = fs.Y12[1];
-  // KE: u,v,w ; eps: 9 gradients.  Per-block slots (296 for KE, 296 for
-  // eps) in the second half of dpart, added in order on the host.
-  double* rp = h->dpart + (size_t)4 * 296 * 5;
-  CK(cudaMemsetAsync(rp, 0, 2 * 296 * sizeof(double), h->st));
+  // (kx, y) rows of u, v, w, rho, the y derivatives and the z derivatives of u, v, w
+  // (scratch: Z4, Y12); the x derivatives are the first three rows times i kx
+  launch_dz4<T>(h, fs, fs.F, fs.Z4);
+  YJobs<T> jb;
+  memset(&jb, 0, sizeof jb);
+  for (int q = 0; q < 4; ++q) jb.j[q] = YJob<T>{fs.F[q], nullptr, fs.Y12[q], 0};
   for (int q = 0; q < 3; ++q) {
-    phys_of<T>(h, fs, fs.F[q], dst, tmp, 0);
-    k_reduce_sq<T><<<296, 256, 0, h->st>>>(g, dst, 1, rp);
-    for (int op = 1; op <= 3; ++op) {
-      phys_of<T>(h, fs, fs.F[q], dst, tmp, op);
-      k_reduce_sq<T><<<296, 256, 0, h->st>>>(g, dst, 1, rp + 296);
+    jb.j[4 + q] = YJob<T>{fs.F[q], nullptr, fs.Y12[4 + q], 1};
+    jb.j[7 + q] = YJob<T>{fs.Z4[q], nullptr, fs.Y12[7 + q], 0};
+  }
+  launch_y<T>(h, fs, jb, 10, h->nz, false);
+  StatRows<T> a;
+  memset(&a, 0, sizeof a);
+  for (int e = 0; e < 13; ++e) {
+    a.src[e] = fs.Y12[e < 10 ? e : e - 10];
+    a.q[e] = e < 4 ? e : -1;
+    a.kx[e] = e >= 10;
+  }
+  int nblk = 0;
+  int* ints = nullptr;  // counts[4], flag, error words[2]
+  const int r = stats_to_host<T>(h, fs, a, 13, &nblk, [&]() -> int {
+    ints = (int*)(h->hstat + kPartDoubles);
+    CK(cudaMemcpyAsync(ints, h->dcnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaMemsetAsync(h->dflag, 0, sizeof(int), h->st));
+    k_nonfinite<T><<<dim3(296, 4), 256, 0, h->st>>>(fs.F[0], fs.F[1], fs.F[2], fs.F[3], h->ntot, h->dflag);
+    CK(cudaMemcpyAsync(ints + 4, h->dflag, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaMemcpyAsync(ints + 5, h->derr, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->st));
+    return 0;
+  });
+  if (r) return r;
+  double red[2] = {0, 0}, mm[4][2], cf[4] = {0, 0, 0, 0}, s2 = 0, cnt = 0;
+  for (int e = 0; e < 13; ++e)
+    for (int b = 0; b < nblk; ++b) {
+      const double* o = h->hstat + ((size_t)e * nblk + b) * kStatSlots;
+      if (e != 3) red[e < 4 ? 0 : 1] += o[0];
+      if (e > 3) continue;
+      mm[e][0] = b == 0 ? o[1] : std::min(mm[e][0], o[1]);
+      mm[e][1] = b == 0 ? o[2] : std::max(mm[e][1], o[2]);
+      cf[e] = std::max(cf[e], o[3]);
+      s2 += o[4];
+      cnt += o[5];
     }
-  }
-  double red[2] = {0, 0};
-  // maxcalc statistics on the physical fields
-  {
-    const double dx = h->p.xlen / h->nx, dy = h->p.ylen / h->ny;
-    const double rg = -(h->p.rho0 * h->p.brunt * h->p.brunt) / h->p.grav;
-    for (int q = 0; q < 4; ++q) {
-      phys_of<T>(h, fs, fs.F[q], dst, tmp, 0);
-      const double cflh = q == 0 ? h->p.dt / dx : q == 1 ? h->p.dt / dy : 0.0;
-      k_phys_stats<T><<<296, 256, 0, h->st>>>(g, dst, q, h->dzg, h->ddzinv, cflh, rg, 0.2 * h->p.zlen,
-                                              h->dpart + (size_t)q * 296 * 5);
-    }
-  }
-  std::vector<double> part((size_t)4 * 296 * 5 + 2 * 296);
-  CK(cudaMemcpyAsync(part.data(), h->dpart, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  for (int b = 0; b < 296; ++b) {
-    red[0] += part[(size_t)4 * 296 * 5 + b];
-    red[1] += part[(size_t)4 * 296 * 5 + 296 + b];
-  }
   memset(out, 0, sizeof *out);
-  {
-    double mm[4][2], cf[4] = {0, 0, 0, 0}, s2 = 0, cnt = 0;
-    for (int q = 0; q < 4; ++q) {
-      mm[q][0] = part[(size_t)q * 296 * 5];
-      mm[q][1] = part[(size_t)q * 296 * 5 + 1];
-      for (int b = 0; b < 296; ++b) {
-        const double* o = part.data() + ((size_t)q * 296 + b) * 5;
-        mm[q][0] = std::min(mm[q][0], o[0]);
-        mm[q][1] = std::max(mm[q][1], o[1]);
-        cf[q] = std::max(cf[q], o[2]);
-        if (q == 2) {
-          s2 += o[3];
-          cnt += o[4];
-        }
-      }
-    }
-    out->umin = mm[0][0];
-    out->umax = mm[0][1];
-    out->vmin = mm[1][0];
-    out->vmax = mm[1][1];
-    out->wmin = mm[2][0];
-    out->wmax = mm[2][1];
-    out->tmin = mm[3][0];
-    out->tmax = mm[3][1];
-    out->cflx = cf[0];
-    out->cfly = cf[1];
-    out->cflz = cf[2];
-    out->wrms_bottom = cnt > 0 ? std::sqrt(s2 / cnt) : 0.0;
-  }
+  out->umin = mm[0][0];
+  out->umax = mm[0][1];
+  out->vmin = mm[1][0];
+  out->vmax = mm[1][1];
+  out->wmin = mm[2][0];
+  out->wmax = mm[2][1];
+  out->tmin = mm[3][0];
+  out->tmax = mm[3][1];
+  out->cflx = cf[0];
+  out->cfly = cf[1];
+  out->cflz = cf[2];
+  out->wrms_bottom = cnt > 0 ? std::sqrt(s2 / cnt) : 0.0;
   out->ke = 0.5 * red[0];
   out->eps = h->p.xnu * red[1];
   out->t = h->t;
   out->dt = h->p.dt;
   out->istep = h->istep;
-  int cnt[4] = {0, 0, 0, 0};
-  CK(scopy(h, cnt, h->dcnt, sizeof cnt, cudaMemcpyDeviceToHost));
-  for (int q = 0; q < 4; ++q) out->interface_avg_count[q] = cnt[q];
-  // non-finite check of the state
-  CK(cudaMemsetAsync(h->dflag, 0, sizeof(int), h->st));
-  for (int q = 0; q < 4; ++q) k_nonfinite<T><<<296, 256, 0, h->st>>>(fs.F[q], h->ntot, h->dflag);
-  int flag = 0;
-  CK(cudaMemcpyAsync(&flag, h->dflag, sizeof flag, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  if (flag) return set_err(IW_ERR_NONFINITE, "non-finite value in the state");
-  return sync_errors(h);
+  for (int q = 0; q < 4; ++q) out->interface_avg_count[q] = ints[q];
+  if (ints[4]) return set_err(IW_ERR_NONFINITE, "non-finite value in the state");
+  return err_code(ints + 5);
 }
 
 // CFL numbers of the state for the adaptive rule: maxcalc's cflxmax and
 // cflzmax (various.f:780-870), from the same per-block partials as iw_diag.
 template <typename T>
 static int step_cfl(iw_handle* h, FieldSet<T>& fs, double* cflx, double* cflz) {
-  Geo g = geo(h);
-  T* dst = fs.Y12[0];
-  T* tmp = fs.Y12[1];
-  const double dx = h->p.xlen / h->nx, rg = -(h->p.rho0 * h->p.brunt * h->p.brunt) / h->p.grav;
-  for (int q = 0; q <= 2; q += 2) {
-    phys_of<T>(h, fs, fs.F[q], dst, tmp, 0);
-    k_phys_stats<T><<<296, 256, 0, h->st>>>(g, dst, q, h->dzg, h->ddzinv, q == 0 ? h->p.dt / dx : 0.0, rg,
-                                            0.2 * h->p.zlen, h->dpart + (size_t)q * 296 * 5);
+  YJobs<T> jb;
+  memset(&jb, 0, sizeof jb);
+  StatRows<T> a;
+  memset(&a, 0, sizeof a);
+  for (int e = 0; e < 2; ++e) {
+    jb.j[e] = YJob<T>{fs.F[2 * e], nullptr, fs.Y12[e], 0};
+    a.src[e] = fs.Y12[e];
+    a.q[e] = 2 * e;
   }
-  std::vector<double> part((size_t)3 * 296 * 5);
-  CK(cudaMemcpyAsync(part.data(), h->dpart, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
+  launch_y<T>(h, fs, jb, 2, h->nz, false);
+  int nblk = 0;
+  if (int r = stats_to_host<T>(h, fs, a, 2, &nblk, [] { return 0; })) return r;
   double cf[2] = {0, 0};
-  for (int b = 0; b < 296; ++b) {
-    cf[0] = std::max(cf[0], part[(size_t)b * 5 + 2]);
-    cf[1] = std::max(cf[1], part[((size_t)2 * 296 + b) * 5 + 2]);
-  }
+  for (int e = 0; e < 2; ++e)
+    for (int b = 0; b < nblk; ++b) cf[e] = std::max(cf[e], h->hstat[((size_t)e * nblk + b) * kStatSlots + 3]);
   *cflx = cf[0];
   *cflz = cf[1];
   return IW_OK;

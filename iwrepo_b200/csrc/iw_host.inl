@@ -355,6 +355,7 @@ struct iw_handle {
   int* dflag = 0;
   int* derr = 0;  // device error words: [0] non-finite state, [1] a bounded device wait gave up
   int* herr = 0;  // pinned host copy of derr, written after each eager step or graph run
+  double* hstat = 0;  // pinned: k_xrow_stats' partials and four ints behind them
   cudaEvent_t err_ev = 0;
   bool err_ev_live = false;
   FftPlan plx, ply;
@@ -457,6 +458,7 @@ static void prof_flush(iw_handle* h) {
 }
 
 static iw_handle* g_bound = nullptr;
+constexpr size_t kPartDoubles = 6400;  // per-block partials of k_xrow_stats
 
 // Every host<->device copy goes through the handle's (non-blocking) stream
 // and waits for it: a plain cudaMemcpy from pageable memory may return before
@@ -1065,6 +1067,11 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
 template <typename T>
 void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int nplanes, bool four) {
   typedef typename cplx_t<T>::type C;
+  if (h->ny == 1) {
+    const size_t nc = h->plane * (size_t)nplanes / 2;
+    k_y1<T><<<dim3((unsigned)((nc + 255) / 256), (unsigned)njobs), 256, 0, h->st>>>(jobs, nc);
+    return;
+  }
   const int tx = ytx<T>(h, four);
   const int ntile = (h->nxhp + tx - 1) / tx;
   dim3 grid(ntile, nplanes, njobs);
@@ -1182,6 +1189,33 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
 #undef IW_XCASE
     }
   xrow_done:;
+  }
+}
+
+// k_xrow_stats over n entries, nblk CTAs each
+template <typename T>
+void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, int nblk) {
+  typedef typename cplx_t<T>::type C;
+  const int M = h->nx / 2;
+  const size_t smem = (size_t)(kStatThreads / 32) * 2 * xstride(M) * sizeof(C);
+  const dim3 grid((unsigned)nblk, (unsigned)n);
+  const Geo g = geo(h);
+  const bool p2 = (M & (M - 1)) == 0;
+  switch (fft_dpt(M) * (p2 ? 1 : -1)) {
+#define IW_SCASE(D, P)                                                                                       \
+  case (P ? D : -D):                                                                                         \
+    cudaFuncSetAttribute(k_xrow_stats<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+    k_xrow_stats<T, D, P><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);        \
+    break;
+    IW_SCASE(4, true)
+    IW_SCASE(8, true)
+    IW_SCASE(16, true)
+    IW_SCASE(32, true)
+    IW_SCASE(4, false)
+    IW_SCASE(8, false)
+    IW_SCASE(16, false)
+    IW_SCASE(32, false)
+#undef IW_SCASE
   }
 }
 
@@ -1563,7 +1597,8 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
 // (iw_inst.cu, once per storage type and group), all at the same time.
 #define IW_INST_FFT(X, T)                                                       \
   X template void launch_y<T>(iw_handle*, FieldSet<T>&, YJobs<T>&, int, int, bool); \
-  X template void launch_xrow<T>(iw_handle*, FieldSet<T>&);
+  X template void launch_xrow<T>(iw_handle*, FieldSet<T>&);                    \
+  X template void launch_xstats<T>(iw_handle*, FieldSet<T>&, const StatRows<T>&, int, int);
 #define IW_INST_Z(X, T)                                                             \
   X template void launch_stageA<T>(iw_handle*, FieldSet<T>&, int);                  \
   X template void launch_stageE<T>(iw_handle*, FieldSet<T>&, int);                  \
@@ -1786,29 +1821,16 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
     h->tune_xthr = bestx;
   }
   // stage A and stage E variants
-  int besta = h->N <= kTcMaxN || zop_bucket(h->N) == 0 ? -1 : 1, beste = -1;
-  {
-    // -1: the tensor-core kernel where it applies, else by size
-    float ta = 0;
-    for (int v : {-1, 0, 1}) {
-      if (v == 1 && !zop_bucket(h->N)) continue;
-      if (v == -1 && h->N > kTcMaxN) continue;
-      h->tune_a = v;
-      const float t = timeit([&] { launch_stageA<T>(h, ts, 1); });
-      if (ta == 0 || t < ta) {
-        ta = t;
-        besta = v;
-      }
-    }
-  }
-  {
-    // 0 tiled (any N), 1 register-column (N in a register bucket), 2 tensor
-    // cores (N <= 40)
+  // Where the tensor-core kernels apply (N <= 40) they were the fastest at every size measured (64^2 x (4 x 17) to
+  // 512^2 x (12 x 33), both precisions) and are kept; the older variants round differently in mixed precision, so a
+  // tuned run keeps the bits of an untuned one.  Larger N: tiled or, within the register buckets, register-column.
+  int besta = -1, beste = h->N <= kTcMaxN ? 2 : -1;
+  if (h->N > kTcMaxN) {
     float bt = 0;
-    for (int v = 0; v < 3; ++v) {
-      if ((v == 1 && !zop_bucket(h->N)) || (v == 2 && h->N > kTcMaxN)) continue;
+    for (int v = 0; v < 2; ++v) {
+      if (v == 1 && !zop_bucket(h->N)) continue;
       h->tune_e = v;
-      const float t = timeit([&] { launch_stageE<T>(h, ts, v == 2 && h->use_bi); });
+      const float t = timeit([&] { launch_stageE<T>(h, ts, 0); });
       if (beste < 0 || t < bt) {
         bt = t;
         beste = v;
@@ -1823,15 +1845,22 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
       h->use_bi) {
     const int cpen = (h->p.ispecfilterexp == 1) && ((h->istep + 1) % h->p.nspecfilterexp == 0);
     const int kstart = h->p.bc_variant == IW_BC_NOSLIP ? 1 : 0;
-    // each solve role (pressure, u/v, w, rho) keeps its own fastest variant
+    // each solve role (pressure, u/v, w, rho) keeps its own fastest variant; with all four on the
+    // tensor cores stage E hands them whole columns, which no mixture matched
+    bool all_tc = stageE_is_t(h);
+    for (int role = 0; role < 4; ++role) {
+      h->sys_role[role] = 2;
+      all_tc = all_tc && solve_variant<T>(h, role, cpen) == 2;
+    }
     for (int role : {3, 0, 1, 2}) {
+      if (all_tc) continue;
       float best = 0;
       int bestv = 1;
       for (int v = 0; v < 4; ++v) {
         if (v == 2 && h->N > kTcMaxN) continue;
         if (v == 3 && (role == 3 || (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32 > kSys2MaxThreads)) continue;
         h->sys_role[role] = v;
-        const float t = timeit([&] { launch_solve_bi<T>(h, ts, role, cpen, kstart, v == 2 && stageE_is_t(h), false); });
+        const float t = timeit([&] { launch_solve_bi<T>(h, ts, role, cpen, kstart, 0, false); });
         if (v == 0 || t < best) {
           best = t;
           bestv = v;
@@ -2138,7 +2167,7 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
         const double zm = kg - 1 >= 1 ? zf[kg - 1] : zgl[nz - 1];
         dzi[k] = 1.0 / (zf[kg] - zm);
       }
-    r |= up(h, &h->ddzinv, dzi) || dalloc(h, &h->dpart, (size_t)4 * 296 * 5 + 2 * 296);
+    r |= up(h, &h->ddzinv, dzi) || dalloc(h, &h->dpart, kPartDoubles);
   }
   r |= up(h, &h->dD, h->tab.D) || up(h, &h->dD2, h->tab.D2) || up(h, &h->dL, h->tab.Lfil) || up(h, &h->dh, hf) ||
        up(h, &h->dxw, xw) || up(h, &h->dyw, yw) || up(h, &h->dcf, cf) || up(h, &h->dzg, zg) || up(h, &h->dzh, zh) ||
@@ -2208,6 +2237,7 @@ int iw_destroy(iw_handle* h) {
   cudaFree(h->dflag);
   cudaFree(h->derr);
   if (h->herr) cudaFreeHost(h->herr);
+  if (h->hstat) cudaFreeHost(h->hstat);
   if (h->err_ev) cudaEventDestroy(h->err_ev);
   cudaFree(h->dcolorder);
   cudaFree(h->dakv);

@@ -21,7 +21,7 @@
 //        the averaging change comes back; every plane gets the spectral effect
 //        of the round trip.
 // Around the step (iw_restart.inl, iw_output.inl, iw_postp.inl): the adaptive
-// time step's CFL numbers (k_phys_stats), restart files, field and animation
+// time step's CFL numbers (k_xrow_stats), restart files, field and animation
 // dumps, Legendre spectra (k_speclegen) and the TKE budget (k_row_dot,
 // k_sub_rowmean), written by a host thread from pinned buffers.
 // The penalty systems (penalty.f + band_lu.f) are assembled on the device
@@ -219,6 +219,15 @@ template <typename T>
 struct YJobs {
   YJob<T> j[16];
 };
+
+// ny = 1: every transform is the identity (ky = 0, scale 1)
+template <typename T>
+__global__ void __launch_bounds__(256) k_y1(YJobs<T> jobs, size_t nc) {
+  typedef typename cplx_t<T>::type C;
+  const YJob<T> jb = jobs.j[blockIdx.y];
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < nc && (jb.mode == 1 || jb.src != jb.dst)) ((C*)jb.dst)[e] = jb.mode == 1 ? cmk<C>(0, 0) : ((const C*)jb.src)[e];
+}
 
 // slots per padded y column: >= fpadlen(ny) and = 2 (mod 16), so that the
 // TX columns of a tile sit in different banks
@@ -3498,8 +3507,9 @@ struct ZWalk {
     }
   }
 };
-// K_A: projection, w mean = 0, z derivative.  The N x 8 operand goes from global
-// memory straight to registers.
+// K_A: projection, w mean = 0, z derivative (proj < 0: the derivative alone, nothing
+// is written to O).  The N x 8 operand goes from global memory straight to
+// registers.
 template <typename T, int NT>
 __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict__ F0, const T* __restrict__ F1_,
                                                      const T* __restrict__ F2_, const T* __restrict__ F3_,
@@ -3524,7 +3534,7 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
     T* Z = (q == 0 ? Z0 : q == 1 ? Z1 : q == 2 ? Z2 : Z3) + k0;
     const double fac = g.hfac[ks];
     // the projection changes the kx = 0 and Nyquist columns
-    const bool special = (proj && (i < 2 || i >= nx)) || (q == 2 && tt < 2);
+    const bool special = (proj > 0 && (i < 2 || i >= nx)) || (proj >= 0 && q == 2 && tt < 2);
     auto tile = [&](auto plain_) {
       constexpr bool PLAIN = decltype(plain_)::value;  // a whole tile of points the projection leaves alone
       const bool act = PLAIN || tt < pl;
@@ -3536,10 +3546,12 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
         x[kt] = (T)0;
         if (in(4 * kt + lt, 4 * kt + 3)) x[kt] = *f;
       }
-      bool bad = false;
+      if (proj >= 0) {
+        bool bad = false;
 #pragma unroll
-      for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
-      if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
+        for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
+        if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
+      }
       if (!PLAIN && special) {
         const bool wzero = q == 2 && tt < 2;
 #pragma unroll
@@ -3548,10 +3560,12 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
           if (act && r < N) x[kt] = wzero ? (T)0 : proj_val<T>(g, F, i, j, r);
         }
       }
-      T* o = O + tt + (size_t)lt * pl;
+      if (proj >= 0) {
+        T* o = O + tt + (size_t)lt * pl;
 #pragma unroll
-      for (int kt = 0; kt < 2 * NT; ++kt, o += pl4)
-        if (in(4 * kt + lt, 4 * kt + 3)) *o = x[kt];
+        for (int kt = 0; kt < 2 * NT; ++kt, o += pl4)
+          if (in(4 * kt + lt, 4 * kt + 3)) *o = x[kt];
+      }
       double acc[1][NT][2], none[1][2];
       tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) { return (double)x[kt]; }, acc, nullptr, none);
       T* z = Z + tt + (size_t)(2 * lt) * pl;
@@ -3919,97 +3933,116 @@ __global__ void k_filter_field(Geo g, T* F, int ifourier, int ilegen) {
   }
 }
 
-// reductions for diagnostics: physical-space sums over i<nx, k>=1
-// Deterministic: a fixed grid and stride, fixed-order warp and block sums,
-// and each block adds its sum to its own slot part[blockIdx.x]; the host adds
-// the slots in order.  Repeated calls on the same state give the same bits.
+// Statistics of physical fields straight from their (kx, y) rows: a warp transforms a
+// row of one list entry back in its own two buffers in shared memory (the next row's
+// copy is in flight meanwhile) and adds the values up in registers; no physical
+// field is written.  Entries: a field (KE sum over levels k >= 1, and maxcalc's extrema,
+// CFL maximum (x, y: |f| dt/dx; z: |w| dt/dz with the reference's merged-interface
+// spacing, dzinv; extrema start from 0, or 1 for rho, whose background 1 + rhograd z is
+// added) and, for w, the sum of squares and count below zlim, various.f:665-987), or a derivative (sum of squares over k >= 1).  grid.y: the entry; a
+// fixed grid and order, so repeated calls give the same bits.
+// part[(entry gridDim.x + block) 6 + {sum, min, max, cfl, sum w^2, count}].
+// 256^2 x (8 x 25) mixed, iw_diag: 4.8 ms with a transform, a derivative and a reduction
+// kernel per field and derivative (16 transforms written and read back).
+constexpr int kStatThreads = 128, kStatSlots = 6, kStatMax = 13;
 template <typename T>
-__global__ void k_reduce_sq(Geo g, const T* __restrict__ a, int kmin, double* part) {
-  __shared__ double ws[32];
-  double s = 0;
-  long total = (long)g.nx * g.ny * (g.nz - kmin);
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-    int i = t % g.nx;
-    long r = t / g.nx;
-    int j = r % g.ny;
-    int k = kmin + r / g.ny;
-    double x = (double)a[fidx<T>(g, i, j, k)];
-    s += x * x;
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b += ws[w];
-    part[blockIdx.x] += b;
-  }
-}
-
-// maxcalc statistics of one physical field (various.f:665-987 without the
-// adaptive step): extrema starting from the reference's initial values (0, or
-// 1 for rho whose background 1 + rhograd z is added), the CFL maximum
-// (x, y: |f| dt/dx; z: |w| dt/dz with the reference's merged-interface
-// spacing, dzinv), and for w the sum of squares and count below zlim.
-// Per-block partials: part[5*block + {min, max, cfl, sum w^2, count}].
-template <typename T>
-__global__ void k_phys_stats(Geo g, const T* __restrict__ a, int q, const double* __restrict__ zg,
-                             const double* __restrict__ dzinv, double cflh, double rg, double zlim, double* part) {
-  double mn = q == 3 ? 1.0 : 0.0, mx = 0.0, cf = 0.0, s2 = 0.0, cnt = 0.0;
-  const long total = (long)g.nx * g.ny * g.nz;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long r = t / g.nx;
-    const int j = (int)(r % g.ny), k = (int)(r / g.ny);
-    double x = (double)a[fidx<T>(g, i, j, k)];
-    if (q == 0 || q == 1) cf = fmax(cf, fabs(x) * cflh);
-    if (q == 2) {
-      cf = fmax(cf, fabs(x) * g.dt * dzinv[k]);
-      if (zg[k] < zlim) {
-        s2 += x * x;
-        cnt += 1.0;
+struct StatRows {
+  const T* src[kStatMax];
+  int q[kStatMax];   // field 0..3 whose statistics are wanted, -1: a derivative
+  int kx[kStatMax];  // multiply by i kx first
+  double cflh[2], rg, zlim;
+  const double* dzinv;
+};
+template <typename T, int DPT, bool POW2>
+__global__ void __launch_bounds__(kStatThreads) k_xrow_stats(Geo g, const __grid_constant__ StatRows<T> a, FftPlan pl,
+                                                            const typename cplx_t<T>::type* __restrict__ Wm,
+                                                            const typename cplx_t<T>::type* __restrict__ Wn,
+                                                            double* __restrict__ part) {
+  typedef typename cplx_t<T>::type C;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double sh[kStatThreads / 32][kStatSlots];
+  const int M = g.nx / 2, RS = xstride(M), lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kStatThreads / 32;
+  const int ent = blockIdx.y, q = a.q[ent], lines = g.ny * g.nz, step = gridDim.x * nw;
+  const bool mulkx = a.kx[ent] != 0;
+  const T kxs = (T)g.xw[1];
+  C* buf = (C*)smraw + (size_t)wid * 2 * RS;
+  const C* src = (const C*)a.src[ent];
+  auto fetch = [&](int line, C* d) {
+    if (line < lines)
+      for (int kk = lane; kk <= M; kk += 32) cp_async_c<C>(d + fpad(kk), src + (size_t)line * (M + 1) + kk);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  double sum = 0.0, mn = q == 3 ? 1.0 : 0.0, mx = 0.0, cf = 0.0, s2 = 0.0, cnt = 0.0;
+  int line = blockIdx.x * nw + wid;
+  fetch(line, buf);
+  for (int p = 0; line < lines; line += step, p ^= 1) {
+    C* row = buf + p * RS;
+    fetch(line + step, buf + (p ^ 1) * RS);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncwarp();
+    for (int kk = lane; kk <= M / 2; kk += 32) xprep_pair<C, T>(row, kk, M, Wn, mulkx, kxs);
+    __syncwarp();
+    fft_warp<C, DPT, POW2>(row, pl, Wm, true, lane);
+    const int k = line / g.ny;
+    const double dzi = q == 2 ? a.dzinv[k] : 0.0, bg = q == 3 ? 1.0 + a.rg * g.zg[k] : 0.0;
+    const bool low = q == 2 && g.zg[k] < a.zlim;
+    double ls = 0.0;
+    for (int i = lane; i < M; i += 32) {
+      const C v = row[fpad(i)];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        double x = (double)(h ? v.y : v.x);
+        ls += x * x;
+        if (q >= 0) {
+          if (q < 2) cf = fmax(cf, fabs(x) * a.cflh[q]);
+          if (q == 2) cf = fmax(cf, fabs(x) * g.dt * dzi);
+          if (q == 3) x += bg;
+          mn = fmin(mn, x);
+          mx = fmax(mx, x);
+        }
       }
     }
-    if (q == 3) x += 1.0 + rg * zg[k];
-    mn = fmin(mn, x);
-    mx = fmax(mx, x);
+    if (low) s2 += ls;
+    if (k >= 1) sum += ls;
+    if (low && lane == 0) cnt += (double)g.nx;
+    __syncwarp();
   }
   for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
     mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
     mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     cf = fmax(cf, __shfl_xor_sync(0xffffffffu, cf, o));
     s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   }
-  __shared__ double sh[32][5];
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    sh[w][0] = mn;
-    sh[w][1] = mx;
-    sh[w][2] = cf;
-    sh[w][3] = s2;
-    sh[w][4] = cnt;
+  if (lane == 0) {
+    const double v[kStatSlots] = {sum, mn, mx, cf, s2, cnt};
+    for (int e = 0; e < kStatSlots; ++e) sh[wid][e] = v[e];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int v = 1; v < nw; ++v) {
-      mn = fmin(mn, sh[v][0]);
-      mx = fmax(mx, sh[v][1]);
-      cf = fmax(cf, sh[v][2]);
-      s2 += sh[v][3];
-      cnt += sh[v][4];
+    for (int w = 1; w < nw; ++w) {
+      sum += sh[w][0];
+      mn = fmin(mn, sh[w][1]);
+      mx = fmax(mx, sh[w][2]);
+      cf = fmax(cf, sh[w][3]);
+      s2 += sh[w][4];
+      cnt += sh[w][5];
     }
-    double* o = part + 5 * (size_t)blockIdx.x;
-    o[0] = mn;
-    o[1] = mx;
-    o[2] = cf;
-    o[3] = s2;
-    o[4] = cnt;
+    double* o = part + ((size_t)ent * gridDim.x + blockIdx.x) * kStatSlots;
+    o[0] = sum;
+    o[1] = mn;
+    o[2] = mx;
+    o[3] = cf;
+    o[4] = s2;
+    o[5] = cnt;
   }
 }
 
 template <typename T>
-__global__ void k_nonfinite(const T* __restrict__ a, size_t n, int* flag) {
+__global__ void k_nonfinite(const T* __restrict__ a0, const T* __restrict__ a1, const T* __restrict__ a2,
+                            const T* __restrict__ a3, size_t n, int* flag) {
+  const T* a = blockIdx.y == 0 ? a0 : blockIdx.y == 1 ? a1 : blockIdx.y == 2 ? a2 : a3;
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
     if (!isfinite((double)a[t])) {
       atomicExch(flag, 1);
