@@ -85,13 +85,15 @@ double g_setup_eps = -1.0;
 
 // one penalty system for eps and BCs, assembled, factored (1 warp), and
 // used to solve for nr right-hand sides b[r*nz + k] (device).
-__global__ void k_solve_one(Geo g, const double* ab, const int* ipiv, double* b, int nr) {
+__global__ void k_solve_one(Geo g, const double* ab, const int* ipiv, double* b) {  // a warp per right-hand side
   extern __shared__ double sb[];
-  const int n = g.nz;
-  for (int t = threadIdx.x; t < nr * n; t += 32) sb[t] = b[t];
+  const int n = g.nz, lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  double* x = sb + (size_t)r * n;
+  b += (size_t)r * n;
+  for (int t = lane; t < n; t += 32) x[t] = b[t];
   __syncwarp();
-  band_solve_warp(ab, ipiv, sb, nr, n, g.N, g.N, threadIdx.x);
-  for (int t = threadIdx.x; t < nr * n; t += 32) b[t] = sb[t];
+  band_solve_warp(ab, ipiv, x, 1, n, g.N, g.N, lane);
+  for (int t = lane; t < n; t += 32) b[t] = x[t];
 }
 
 __global__ void k_legen_one(Geo g, const double* wg, const double* alpol, const double* sigma, double* b, int N) {
@@ -133,7 +135,7 @@ int factor_dense_or_params(iw_handle* h, const double* pen6, double eps, int bot
         ab[(size_t)(2 * N + i - j) + (size_t)ldab * (j - 1)] = dense[(size_t)(i - 1) + (size_t)n * (j - 1)];
     CK(scopy(h, dab, ab.data(), ab.size() * sizeof(double), cudaMemcpyHostToDevice));
   }
-  if (!dense) k_assemble_band<<<1, 32, 0, h->st>>>(geo(h), fa);
+  if (!dense) k_assemble_band<<<1, 256, 0, h->st>>>(geo(h), fa);
   launch_band_lu(h->st, 1, n, N, dab, dip, dinfo);
   int info = 0;
   CK(scopy(h, &info, dinfo, sizeof info, cudaMemcpyDeviceToHost));
@@ -319,7 +321,7 @@ void penalty_main_(const double* epsilon, const int* ifuncreal, const double* bc
   if (factor_dense_or_params(h, pen.data(), eps, *ifbcbot, *ifbctop, nullptr, &dab, &dip)) return;
   DBuf db(2 * (size_t)n);
   scopy(h, db.p, b.data(), b.size() * sizeof(double), cudaMemcpyHostToDevice);
-  k_solve_one<<<1, 32, 2 * n * sizeof(double), h->st>>>(geo(h), dab, dip, db.p, 2);
+  k_solve_one<<<1, 64, 2 * n * sizeof(double), h->st>>>(geo(h), dab, dip, db.p);
   cudaStreamSynchronize(h->st);
   scopy(h, b.data(), db.p, b.size() * sizeof(double), cudaMemcpyDeviceToHost);
   for (int k = 0; k < n; ++k) {
@@ -346,7 +348,7 @@ void bandlu_solve_(const double* ain, double* xr, double* xi, const int* ifuncre
   }
   DBuf db(2 * (size_t)n);
   scopy(h, db.p, b.data(), b.size() * sizeof(double), cudaMemcpyHostToDevice);
-  k_solve_one<<<1, 32, 2 * n * sizeof(double), h->st>>>(geo(h), dab, dip, db.p, nr);
+  k_solve_one<<<1, 32 * nr, (size_t)nr * n * sizeof(double), h->st>>>(geo(h), dab, dip, db.p);
   cudaStreamSynchronize(h->st);
   scopy(h, b.data(), db.p, b.size() * sizeof(double), cudaMemcpyDeviceToHost);
   for (int k = 0; k < n; ++k) {
@@ -478,20 +480,19 @@ int iw_init_mode1(iw_handle* h, double A, double anoise, uint64_t seed) {
 }  // extern "C"
 
 // z derivatives of src[0..3] into dst[0..3]
+// (flag: set when a source value is not finite)
 template <typename T>
-static void launch_dz4(iw_handle* h, FieldSet<T>& fs, T* const* src, T* const* dst) {
+static void launch_dz4(iw_handle* h, FieldSet<T>& fs, T* const* src, T* const* dst, int* flag) {
   if (h->N <= kTcMaxN) {
     FieldSet<T> v = fs;
     for (int q = 0; q < 4; ++q) {
       v.F[q] = src[q];
       v.Z4[q] = dst[q];
     }
-    const int keep = h->tune_a;
-    h->tune_a = -1;
-    launch_stageA<T>(h, v, -1);
-    h->tune_a = keep;
+    launch_stageA<T>(h, v, -1, flag);
     return;
   }
+  k_nonfinite<T><<<dim3(296, 4), 256, 0, h->st>>>(src[0], src[1], src[2], src[3], h->ntot, flag);
   for (int q = 0; q < 4; ++q)
     k_dz_field<T><<<(unsigned)((h->ntot + 255) / 256), 256, 0, h->st>>>(geo(h), src[q], dst[q]);
 }
@@ -523,7 +524,8 @@ template <typename T>
 static int diag_impl(iw_handle* h, FieldSet<T>& fs, iw_diag_out* out) {
   // (kx, y) rows of u, v, w, rho, the y derivatives and the z derivatives of u, v, w
   // (scratch: Z4, Y12); the x derivatives are the first three rows times i kx
-  launch_dz4<T>(h, fs, fs.F, fs.Z4);
+  CK(cudaMemsetAsync(h->dflag, 0, sizeof(int), h->st));
+  launch_dz4<T>(h, fs, fs.F, fs.Z4, h->dflag);
   YJobs<T> jb;
   memset(&jb, 0, sizeof jb);
   for (int q = 0; q < 4; ++q) jb.j[q] = YJob<T>{fs.F[q], nullptr, fs.Y12[q], 0};
@@ -544,8 +546,6 @@ static int diag_impl(iw_handle* h, FieldSet<T>& fs, iw_diag_out* out) {
   const int r = stats_to_host<T>(h, fs, a, 13, &nblk, [&]() -> int {
     ints = (int*)(h->hstat + kPartDoubles);
     CK(cudaMemcpyAsync(ints, h->dcnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaMemsetAsync(h->dflag, 0, sizeof(int), h->st));
-    k_nonfinite<T><<<dim3(296, 4), 256, 0, h->st>>>(fs.F[0], fs.F[1], fs.F[2], fs.F[3], h->ntot, h->dflag);
     CK(cudaMemcpyAsync(ints + 4, h->dflag, sizeof(int), cudaMemcpyDeviceToHost, h->st));
     CK(cudaMemcpyAsync(ints + 5, h->derr, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->st));
     return 0;
@@ -753,7 +753,7 @@ int iw_bandlu_solve_noalloc(const double* ain_dev, double* x_dev, int nzloc, int
   cudaStream_t st = (cudaStream_t)stream;
   k_pack_band<<<64, 256, 0, st>>>(ain_dev, n, nzloc, ldab, ab, sd, info);
   launch_band_lu(st, 1, n, nzloc, ab, ipiv, info);
-  k_solve_one<<<1, 32, (size_t)nrhs * n * sizeof(double), st>>>(g, ab, ipiv, x_dev, nrhs);
+  k_solve_one<<<1, 32 * nrhs, (size_t)nrhs * n * sizeof(double), st>>>(g, ab, ipiv, x_dev);
   CK(cudaGetLastError());
   return IW_OK;
 }

@@ -722,7 +722,7 @@ static int build_factors(iw_handle* h, int kind) {
     fa.D = h->dD;
     fa.D2 = h->dD2;
     fa.zh = h->dzh;
-    k_assemble_band<<<(nsys + 3) / 4, 128, 0, h->st>>>(geo(h), fa);
+    k_assemble_band<<<nsys, 128, 0, h->st>>>(geo(h), fa);
     launch_band_lu(h->st, nsys, n, N, fa.ab, h->dipiv[kind], h->dinfo[kind]);
     CK(cudaGetLastError());
     // host copies must stay alive until the copies finish
@@ -771,7 +771,7 @@ static int build_systems(iw_handle* h, const double* dak, int nsys, double c0, i
   b.minv = minv;
   const size_t sm = build_smem(h->N, h->ns);
   CK(cudaFuncSetAttribute(k_build_systems, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  k_build_systems<<<nsys, 256, sm, h->st>>>(b);
+  k_build_systems<<<nsys, 64 * kBuildGroups, sm, h->st>>>(b);
   CK(cudaGetLastError());
   return 0;
 }
@@ -922,15 +922,16 @@ static void launch_stageA_r(iw_handle* h, FieldSet<T>& fs, int proj) {
 }
 
 template <typename T>
-void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj) {
-  if (h->tune_a < 0 && h->N <= kTcMaxN) {  // tensor-core kernel
+void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj, int* err) {
+  // tensor-core kernel (proj < 0, the derivative alone, exists only there)
+  if ((h->tune_a < 0 || proj < 0) && h->N <= kTcMaxN) {
     const size_t sm = ((size_t)tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);
     const int blocks = z_grid(h, 16, 2);
 #define IW_ATCASE(NT)                                                                                                   \
   case NT:                                                                                                              \
     k_stageA_t<T, NT><<<blocks, 512, sm, h->st>>>(geo(h), fs.F[0], fs.F[1], fs.F[2], fs.F[3], fs.F1[0], fs.F1[1],       \
                                                   fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], fs.Z4[3], proj,     \
-                                                  h->derr);                                                             \
+                                                  err);                                                             \
     return;
     switch (tc_nt(h->N)) { IW_ATCASE(2) IW_ATCASE(3) IW_ATCASE(4) IW_ATCASE(5) }
 #undef IW_ATCASE
@@ -1201,6 +1202,20 @@ void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, i
   const dim3 grid((unsigned)nblk, (unsigned)n);
   const Geo g = geo(h);
   const bool p2 = (M & (M - 1)) == 0;
+  switch (p2 && M >= 32 && M <= 512 ? M : 0) {  // compile-time plans for power-of-two lengths
+#define IW_SCT(MC, D)                                                                                            \
+  case MC:                                                                                                       \
+    cudaFuncSetAttribute(k_xrow_stats<T, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+    k_xrow_stats<T, D, true, MC><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);     \
+    return;
+    IW_SCT(32, 4)
+    IW_SCT(64, 4)
+    IW_SCT(128, 4)
+    IW_SCT(256, 8)
+    IW_SCT(512, 16)
+#undef IW_SCT
+    default: break;
+  }
   switch (fft_dpt(M) * (p2 ? 1 : -1)) {
 #define IW_SCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
@@ -1227,7 +1242,7 @@ static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj, int cols = 0) {
   const int M = h->nx / 2;
   mark(h, -1);
   // K_A
-  launch_stageA<T>(h, fs, proj);
+  launch_stageA<T>(h, fs, proj, h->derr);
   mark(h, 0);
   if (h->anim_pending) {  // the dump sees the fields convec sees: projected, mean w removed
     h->anim_pending = false;
@@ -1600,7 +1615,7 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   X template void launch_xrow<T>(iw_handle*, FieldSet<T>&);                    \
   X template void launch_xstats<T>(iw_handle*, FieldSet<T>&, const StatRows<T>&, int, int);
 #define IW_INST_Z(X, T)                                                             \
-  X template void launch_stageA<T>(iw_handle*, FieldSet<T>&, int);                  \
+  X template void launch_stageA<T>(iw_handle*, FieldSet<T>&, int, int*);            \
   X template void launch_stageE<T>(iw_handle*, FieldSet<T>&, int);                  \
   X template void launch_solve_tc<T>(iw_handle*, FieldSet<T>&, const int*, int, int, int); \
   X template void launch_solve_bi<T>(iw_handle*, FieldSet<T>&, int, int, int, int, bool);
@@ -2719,32 +2734,91 @@ static __global__ void k_helm(Geo g, HelmCache hc, const double* __restrict__ rh
 // its order are band_solve_warp_f's, so the FP32 sweeps give the same bits.  The FP64
 // residual walks block by block; a block's residual replaces its x one block later (the
 // next block's coupling row still reads it) and x waits in sol.
+// NB >= N: the entries of the next step's factor column are loaded while the current
+// one is applied (registers; NB = 0: no prefetch, any N).
+template <int NB>
 __device__ __forceinline__ void band_sweep_lane(const float* __restrict__ ab, const int* __restrict__ ipiv, float* b,
                                                 int n, int N) {
-  const int ldab = 3 * N + 1, kd = 2 * N, k = 2 * N;  // b: element i at b[32 i]
-  for (int j = 0; j < n - 1; ++j) {
-    const int lm = min(N, n - 1 - j), l = __ldg(ipiv + j) - 1;
-    const float* col = ab + (size_t)ldab * j + kd;
-    float* bj = b + 32 * j;
-    const float v = bj[0], y = b[32 * l];
-    if (l != j) {
-      b[32 * l] = v;
-      bj[0] = y;
+  const int ldab = 3 * N + 1, k = 2 * N;  // b: element i at b[32 i]
+  if constexpr (NB == 0) {
+    for (int j = 0; j < n - 1; ++j) {
+      const int lm = min(N, n - 1 - j), l = __ldg(ipiv + j) - 1;
+      const float* col = ab + (size_t)ldab * j + k;
+      float* bj = b + 32 * j;
+      const float v = bj[0], y = b[32 * l];
+      if (l != j) {
+        b[32 * l] = v;
+        bj[0] = y;
+      }
+#pragma unroll 8
+      for (int i = 1; i <= lm; ++i) bj[32 * i] = __fmaf_rn(-__ldg(col + i), y, bj[32 * i]);
     }
+    for (int j = n - 1; j >= 0; --j) {
+      const float* col = ab + (size_t)ldab * j + k;
+      float* bj = b + 32 * j;
+      const float xj = __fdiv_rn(bj[0], __ldg(col));
+      bj[0] = xj;
+      const int m = min(k, j);
 #pragma unroll 8
-    for (int i = 1; i <= lm; ++i) bj[32 * i] = __fmaf_rn(-__ldg(col + i), y, bj[32 * i]);
-  }
-  for (int j = n - 1; j >= 0; --j) {
-    const float* col = ab + (size_t)ldab * j + k;
-    float* bj = b + 32 * j;
-    const float xj = __fdiv_rn(bj[0], __ldg(col));
-    bj[0] = xj;
-    const int m = min(k, j);
-#pragma unroll 8
-    for (int i = 1; i <= m; ++i) bj[-32 * i] = __fmaf_rn(-xj, __ldg(col - i), bj[-32 * i]);
+      for (int i = 1; i <= m; ++i) bj[-32 * i] = __fmaf_rn(-xj, __ldg(col - i), bj[-32 * i]);
+    }
+  } else {
+    float m[NB], mn[NB];
+    int l = __ldg(ipiv) - 1, ln = 0;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) m[i] = i < min(N, n - 1) ? __ldg(ab + k + 1 + i) : 0.f;
+    for (int j = 0; j < n - 1; ++j) {
+      const int lm = min(N, n - 1 - j);
+      if (j + 1 < n - 1) {
+        const float* cn = ab + (size_t)ldab * (j + 1) + k + 1;
+        const int lmn = min(N, n - 2 - j);
+        ln = __ldg(ipiv + j + 1) - 1;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) mn[i] = i < lmn ? __ldg(cn + i) : 0.f;
+      }
+      float* bj = b + 32 * j;
+      const float v = bj[0], y = b[32 * l];
+      if (l != j) {
+        b[32 * l] = v;
+        bj[0] = y;
+      }
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (i < lm) bj[32 * (i + 1)] = __fmaf_rn(-m[i], y, bj[32 * (i + 1)]);
+      l = ln;
+#pragma unroll
+      for (int i = 0; i < NB; ++i) m[i] = mn[i];
+    }
+    float v[2 * NB], vn[2 * NB], dg, dgn = 0.f;
+    {
+      const float* col = ab + (size_t)ldab * (n - 1) + k;
+      dg = __ldg(col);
+#pragma unroll
+      for (int i = 0; i < 2 * NB; ++i) v[i] = i < min(k, n - 1) ? __ldg(col - 1 - i) : 0.f;
+    }
+    for (int j = n - 1; j >= 0; --j) {
+      if (j > 0) {
+        const float* col = ab + (size_t)ldab * (j - 1) + k;
+        const int mm = min(k, j - 1);
+        dgn = __ldg(col);
+#pragma unroll
+        for (int i = 0; i < 2 * NB; ++i) vn[i] = i < mm ? __ldg(col - 1 - i) : 0.f;
+      }
+      float* bj = b + 32 * j;
+      const float xj = __fdiv_rn(bj[0], dg);
+      bj[0] = xj;
+      const int mj = min(k, j);
+#pragma unroll
+      for (int i = 0; i < 2 * NB; ++i)
+        if (i < mj) bj[-32 * (i + 1)] = __fmaf_rn(-xj, v[i], bj[-32 * (i + 1)]);
+      dg = dgn;
+#pragma unroll
+      for (int i = 0; i < 2 * NB; ++i) v[i] = vn[i];
+    }
   }
 }
 static size_t helm32_smem(int n, int N) { return (size_t)(n + 2 * N) * 32 * sizeof(float); }
+template <int NB>
 static __global__ void __launch_bounds__(32) k_helm32(Geo g, HelmCache hc, const double* __restrict__ rhs,
                                                       double* __restrict__ sol, int ncol, const double* __restrict__ D2,
                                                       const double* __restrict__ zh, const int* __restrict__ order) {
@@ -2761,7 +2835,7 @@ static __global__ void __launch_bounds__(32) k_helm32(Geo g, HelmCache hc, const
   const int* ip = hc.ipiv + (size_t)s * n;
 #pragma unroll 8
   for (int k = 0; k < n; ++k) b[32 * k] = (float)rc[2 * k];
-  band_sweep_lane(ab, ip, b, n, N);
+  band_sweep_lane<NB>(ab, ip, b, n, N);
   const double eps = hc.sys[s].eps;
   const double* pen = hc.pen + (size_t)s * 6 * g.ns;
   auto x = [&](int i) { return (double)b[32 * i]; };
@@ -2788,7 +2862,7 @@ static __global__ void __launch_bounds__(32) k_helm32(Geo g, HelmCache hc, const
     b[32 * r] = p[32 * k1];
     xc[2 * r] = x1;
   }
-  band_sweep_lane(ab, ip, b, n, N);
+  band_sweep_lane<NB>(ab, ip, b, n, N);
   for (int k = 0; k < n; ++k) xc[2 * k] += (double)b[32 * k];
 }
 
@@ -2888,7 +2962,7 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     fa.D = h->dD;
     fa.D2 = h->dD2;
     fa.zh = h->dzh;
-    k_assemble_band<<<(hc.nsys + 3) / 4, 128, 0, h->st>>>(geo(h), fa);
+    k_assemble_band<<<hc.nsys, 128, 0, h->st>>>(geo(h), fa);
     launch_band_lu(h->st, hc.nsys, n, N, hc.ab, hc.ipiv, hc.info);
     size_t tot = (size_t)hc.nsys * ldab * n;
     k_convert<double, float><<<2048, 256, 0, h->st>>>(hc.ab, hc.ab32, tot);
@@ -2917,8 +2991,10 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
   const int nc = tc ? hc.nlist : ncol;
   const size_t sm32 = helm32_smem(n, N);
   if (mode != 0 && sm32 <= 200 * 1024 && rhs != sol) {
-    cudaFuncSetAttribute(k_helm32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
-    k_helm32<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), hc, rhs, sol, ncol, h->dD2, h->dzh, hc.order);
+    // (the prefetch of the next factor column costs 6 NB registers; beyond 33 it spills)
+    auto* kern = N <= 9 ? k_helm32<9> : N <= 17 ? k_helm32<17> : N <= 25 ? k_helm32<25> : N <= 33 ? k_helm32<33> : k_helm32<0>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
+    kern<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), hc, rhs, sol, ncol, h->dD2, h->dzh, hc.order);
     CK(cudaGetLastError());
   } else if (nc > 0) {
     const int warps = 4;

@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(192) k_wviscrot(Geo g, const T* __restrict__ u
 // Band factorisation (penalty.f:403-634 assembly, band_lu.f:19-34 packing,
 // bandludcmp.f:238-440 SGBTF2).  The arithmetic follows the reference order with
 // no fused multiply-add, so the factors equal the CPU ones bit for bit.  Assembly: one
-// warp per system.
+// CTA per system, a warp per subdomain.
 // ===========================================================================
 struct SysDesc {
   double eps;
@@ -1082,10 +1082,7 @@ __device__ __forceinline__ double& ABr(double* ab, int ldab, int r, int c) {
 }
 
 static __global__ void k_assemble_band(Geo g, FactorArgs fa) {
-  const int warps = blockDim.x / 32;
-  const int s = blockIdx.x * warps + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (s >= fa.nsys) return;
+  const int s = blockIdx.x, lane = threadIdx.x & 31;
   const int n = g.nz, N = g.N, ns = g.ns, kl = N, ku = N, ldab = 2 * kl + ku + 1;
   double* ab = fa.ab + (size_t)s * ldab * n;
   const double eps = fa.sys[s].eps;
@@ -1095,11 +1092,11 @@ static __global__ void k_assemble_band(Geo g, FactorArgs fa) {
   const double* d = fa.D;
   const double* d2 = fa.D2;
   // zero the band
-  for (size_t t = lane; t < (size_t)ldab * n; t += 32) ab[t] = 0.0;
-  __syncwarp();
+  for (size_t t = threadIdx.x; t < (size_t)ldab * n; t += blockDim.x) ab[t] = 0.0;
+  __syncthreads();
   // A(r,c) 0-based -> band row kl+ku+1+r-c (1-based), column c+1
 #define AEL(r, c) ABr(ab, ldab, kl + ku + 1 + (r) - (c), (c) + 1)
-  for (int ks = 0; ks < ns; ++ks) {
+  for (int ks = threadIdx.x >> 5; ks < ns; ks += blockDim.x >> 5) {  // a warp per subdomain: its own rows
     const double ybar = fa.zh[ks];
     const double ybarl = ks > 0 ? fa.zh[ks - 1] : 0.0;
     const double ybarr = ks < ns - 1 ? fa.zh[ks + 1] : 0.0;
@@ -1165,30 +1162,65 @@ static __global__ void k_assemble_band(Geo g, FactorArgs fa) {
 
 // SGBTF2 (bandludcmp.f:238-440), one CTA per system.  The columns a step touches (j .. j + kl
 // + ku) live in a ring in shared memory; the next ones arrive by cp.async eight steps
-// ahead, and a finished column goes back to global memory.  Per step the first warp finds the
-// pivot and forms the multipliers, then every thread swaps and updates its part of the
-// remaining columns: two barriers, no dependent access to global memory.  Bound by that
-// chain of about 500 cycles per column; the arithmetic of every element and its
-// order are the reference's.
-constexpr int kLuThreads = 128, kLuAhead = 8;
-__host__ __device__ inline int lu_ring(int N) { return 2 * N + 1 + kLuAhead; }
+// ahead, and a finished column goes back to global memory.  In a step, lanes take the rows and
+// warps the columns of the update; warp 0 updates column j + 1 first, finds its pivot and
+// forms the next multipliers while the other warps finish, so a step is one barrier and
+// no dependent access to global memory.  Bound by warp 0's chain (update, maximum over lanes,
+// reciprocal).  The arithmetic of every element and its order are the reference's.
+constexpr int kLuThreads = 256, kLuAhead = 8;
+__host__ __device__ inline int lu_ring(int N) { return 2 * N + 2 + kLuAhead; }
 __host__ __device__ inline size_t lu_smem(int N) {
-  return ((size_t)lu_ring(N) * (3 * N + 1) + N + 2) * sizeof(double);
+  return ((size_t)lu_ring(N) * (3 * N + 1) + 2 * (N + 2)) * sizeof(double);
+}
+// Pivot and multipliers of column j (cj, updated by the steps before) by one warp: the
+// first row of the largest |a|, rows kv .. kv + km; the multipliers go to lb[1 .. km]
+// and the column.  Returns the pivot's row, or -1 - row for a zero pivot.
+static __device__ __forceinline__ int lu_pivot(double* cj, double* lb, int kv, int km, int lane) {
+  double best = -1.0;
+  int bi = 1 << 30;
+  for (int i = lane; i <= km; i += 32) {
+    const double v = fabs(cj[kv + i]);
+    if (v > best) {
+      best = v;
+      bi = i;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (ob > best || (ob == best && oi < bi)) {
+      best = ob;
+      bi = oi;
+    }
+  }
+  if (bi > km) bi = 0;  // only NaNs
+  const double piv = cj[kv + bi], top = cj[kv];
+  __syncwarp();
+  if (piv == 0.0) return -1 - bi;
+  const double rcp = km > 0 ? __ddiv_rn(1.0, piv) : 0.0;
+  for (int i = 1 + lane; i <= km; i += 32) {
+    const double l = rmul(rcp, i == bi ? top : cj[kv + i]);
+    lb[i] = l;
+    cj[kv + i] = l;
+  }
+  if (lane == 0) cj[kv] = piv;
+  __syncwarp();
+  return bi;
 }
 static __global__ void __launch_bounds__(kLuThreads) k_band_lu(int n, int N, double* __restrict__ abs_, int* __restrict__ ipivs,
                                                                int* __restrict__ infos) {
   extern __shared__ __align__(16) double sml[];
-  __shared__ int sjp;
+  __shared__ int sjp[2];
   const int kl = N, ku = N, kv = kl + ku, ldab = 2 * kl + ku + 1, W = lu_ring(N);
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = kLuThreads >> 5;
   double* ab = abs_ + (size_t)blockIdx.x * ldab * n;
   int* ipiv = ipivs + (size_t)blockIdx.x * n;
-  double* ring = sml;                     // column j at ring + (j % W) ldab
-  double* lb = ring + (size_t)W * ldab;   // multipliers of the current step
+  double* ring = sml;                    // column j at ring + (j % W) ldab
+  double* lbs = ring + (size_t)W * ldab;  // multipliers of steps of either parity
   // column c (0-based): the kl fill rows start as 0
-  auto fetch = [&](int c) {
+  auto fetch = [&](int c, int slot) {
     if (c < n) {
-      double* d = ring + (size_t)(c % W) * ldab;
+      double* d = ring + (size_t)slot * ldab;
       const double* s = ab + (size_t)c * ldab;
       for (int r = tid; r < ldab; r += kLuThreads) {
         if (r < kl)
@@ -1199,76 +1231,59 @@ static __global__ void __launch_bounds__(kLuThreads) k_band_lu(int n, int N, dou
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  for (int c = 0; c <= kv; ++c) fetch(c);
-  for (int c = kv + 1; c < kv + kLuAhead; ++c) fetch(c);
-  int ju = 0, info = 0;  // last column touched so far (0-based)
-  for (int j = 0; j < n; ++j) {
-    fetch(j + kv + kLuAhead);  // its slot held column j - 1, stored before the last barrier
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kLuAhead) : "memory");  // columns <= j + kv are here
-    __syncthreads();
-    const int km = min(kl, n - 1 - j);
-    double* cj = ring + (size_t)(j % W) * ldab;
-    if (wid == 0) {
-      // ISAMAX: first index of the largest |a| in rows kv .. kv + km
-      double best = -1.0;
-      int bi = 1 << 30;
-      for (int i = lane; i <= km; i += 32) {
-        const double v = fabs(cj[kv + i]);
-        if (v > best) {
-          best = v;
-          bi = i;
-        }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (bi > km) bi = 0;  // only NaNs: the first row, as ISAMAX
-      const double piv = cj[kv + bi], top = cj[kv];
-      __syncwarp();
-      if (lane == 0) {
-        sjp = piv != 0.0 ? bi : -1 - bi;
-        ipiv[j] = j + bi + 1;
-      }
-      if (piv != 0.0) {
-        const double rcp = km > 0 ? __ddiv_rn(1.0, piv) : 0.0;
-        for (int i = 1 + lane; i <= km; i += 32) {
-          const double l = rmul(rcp, i == bi ? top : cj[kv + i]);
-          lb[i] = l;
-          cj[kv + i] = l;
-        }
-        if (lane == 0) cj[kv] = piv;
-      }
+  for (int c = 0; c < kv + 1 + kLuAhead; ++c) fetch(c, c);
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(kLuAhead) : "memory");  // columns <= kv
+  __syncthreads();
+  if (wid == 0) {
+    const int p = lu_pivot(ring, lbs, kv, min(kl, n - 1), lane);
+    if (lane == 0) {
+      sjp[0] = p;
+      ipiv[0] = (p >= 0 ? p : -1 - p) + 1;
     }
-    __syncthreads();
-    const int jp = sjp;
+  }
+  int ju = 0, info = 0, sj = 0;  // last column touched so far (0-based), slot of column j
+  int sf = kv + 1 + kLuAhead;    // slot of column j + kv + 1 + kLuAhead: held column j - 1
+  if (sf >= W) sf -= W;
+  for (int j = 0; j < n; ++j) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kLuAhead - 1) : "memory");  // columns <= j + kv + 1
+    __syncthreads();  // step j - 1 and the pivot of column j are done
+    fetch(j + kv + 1 + kLuAhead, sf);
+    const int km = min(kl, n - 1 - j), jp = sjp[j & 1];
+    const double* lb = lbs + (j & 1) * (N + 2);
+    const double* cj = ring + (size_t)sj * ldab;
     if (jp >= 0) {
       ju = max(ju, min(j + ku + jp, n - 1));
-      // a thread per column j + 1 .. ju (at most 2 N of them)
-      for (int cc = 1 + tid; cc <= ju - j; cc += kLuThreads) {
-        int sl = (j % W) + cc;
+      // rows i = 1 + lane (and 33 + lane) of columns j + 1 .. ju; warp 0 takes column j + 1 alone
+      const int i0 = 1 + lane, i1 = 33 + lane;
+      const double l0 = i0 <= km ? lb[i0] : 0.0, l1 = i1 <= km ? lb[i1] : 0.0;
+      for (int cc = wid == 0 ? 1 : 1 + wid; cc <= ju - j; cc += wid == 0 ? 1 << 20 : nw - 1) {
+        int sl = sj + cc;
         if (sl >= W) sl -= W;
         double* col = ring + (size_t)sl * ldab + kv - cc;  // row i of the step at col[i]
-        const double y = col[jp];
-        if (jp != 0) {
-          col[jp] = col[0];
-          col[0] = y;
-        }
-        if (y != 0.0) {
-          const double temp = -y;
-#pragma unroll 8
-          for (int i = 1; i <= km; ++i) col[i] = radd(col[i], rmul(lb[i], temp));
-        }
+        const double y = col[jp], t0 = col[0];
+        const double x0 = i0 <= km ? (i0 == jp ? t0 : col[i0]) : 0.0, x1 = i1 <= km ? (i1 == jp ? t0 : col[i1]) : 0.0;
+        __syncwarp();
+        const double temp = -y;
+        if (i0 <= km) col[i0] = y != 0.0 ? radd(x0, rmul(l0, temp)) : x0;
+        if (i1 <= km) col[i1] = y != 0.0 ? radd(x1, rmul(l1, temp)) : x1;
+        if (lane == 0) col[0] = y;
+        __syncwarp();
       }
     } else if (info == 0) {
       info = j + 1;
     }
+    if (wid == 0 && j + 1 < n) {
+      int sn = sj + 1;
+      if (sn >= W) sn -= W;
+      const int p = lu_pivot(ring + (size_t)sn * ldab, lbs + ((j + 1) & 1) * (N + 2), kv, min(kl, n - 2 - j), lane);
+      if (lane == 0) {
+        sjp[(j + 1) & 1] = p;
+        ipiv[j + 1] = j + 1 + (p >= 0 ? p : -1 - p) + 1;
+      }
+    }
     for (int r = tid; r < ldab; r += kLuThreads) ab[(size_t)j * ldab + r] = cj[r];
-    __syncthreads();
+    if (++sj >= W) sj -= W;
+    if (++sf >= W) sf -= W;
   }
   if (tid == 0) infos[blockIdx.x] = info;
 }
@@ -1570,10 +1585,11 @@ static __device__ void d_param_set(const BuildArgs& b, int ifbc, double eps, dou
     t0 = __ddiv_rn(rmul(rmul(rmul(facm, dn), radd(eps, t2)), 2.), ybar);
   }
 }
-// Gauss-Jordan on the n x 2 n matrix A (right half: the identity) with the CTA's
-// threads; skip: columns left of the pivot hold zeros in the pivot row
-static __device__ void gauss_jordan(double* A, int n, int* piv, double* pinv) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, n2 = 2 * n;
+// Gauss-Jordan on the n x 2 n matrix A (right half: the identity) by nthr threads that
+// meet at barrier bar; columns left of the pivot hold zeros in the pivot row and are skipped
+static __device__ void gauss_jordan(double* A, int n, int* piv, double* pinv, int tid, int nthr, int bar) {
+  const int lane = tid & 31, w = tid >> 5, nw = nthr >> 5, n2 = 2 * n;
+  auto sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nthr) : "memory"); };
   for (int col = 0; col < n; ++col) {
     if (w == 0) {  // the first row of the largest |A(r, col)|, r >= col
       double best = -1.0;
@@ -1598,15 +1614,15 @@ static __device__ void gauss_jordan(double* A, int n, int* piv, double* pinv) {
         *pinv = __ddiv_rn(1.0, A[bi * n2 + col]);
       }
     }
-    __syncthreads();
+    sync();
     const int bi = *piv;
     const double iv = *pinv;
-    for (int c = col + threadIdx.x; c < n2; c += blockDim.x) {
+    for (int c = col + tid; c < n2; c += nthr) {
       const double p = A[bi * n2 + c];
       if (bi != col) A[bi * n2 + c] = A[col * n2 + c];
       A[col * n2 + c] = rmul(p, iv);
     }
-    __syncthreads();
+    sync();
     for (int r = w; r < n; r += nw) {
       if (r == col) continue;
       const double f = A[r * n2 + col];
@@ -1614,20 +1630,22 @@ static __device__ void gauss_jordan(double* A, int n, int* piv, double* pinv) {
       if (f != 0.0)
         for (int c = col + lane; c < n2; c += 32) A[r * n2 + c] = __fma_rn(-f, A[col * n2 + c], A[r * n2 + c]);
     }
-    __syncthreads();
+    sync();
   }
 }
+constexpr int kBuildGroups = 3;  // blocks inverted at the same time, two warps each
 __host__ __device__ inline size_t build_smem(int N, int ns) {
   const size_t m = 2 * (size_t)(ns - 1);
-  return ((size_t)N * 2 * N + 2 * (size_t)ns * N + 2 * m + m * 2 * m + 6 * (size_t)ns + 4) * sizeof(double);
+  return ((size_t)kBuildGroups * N * 2 * N + 2 * (size_t)ns * N + 2 * m + m * 2 * m + 6 * (size_t)ns + 4) * sizeof(double);
 }
-static __global__ void __launch_bounds__(256) k_build_systems(const __grid_constant__ BuildArgs b) {
+static __global__ void __launch_bounds__(64 * kBuildGroups) k_build_systems(const __grid_constant__ BuildArgs b) {
   extern __shared__ __align__(16) double smb[];
-  __shared__ int piv;
-  __shared__ double pinv;
+  __shared__ int piv[kBuildGroups];
+  __shared__ double pinv[kBuildGroups];
   const int N = b.N, ns = b.ns, m = 2 * (ns - 1), s = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
-  double* M = smb;                // N x 2 N
-  double* cv = M + N * 2 * N;     // c_ks (row 0 of block ks against block ks - 1)
+  const int gr = tid >> 6, gt = tid & 63;  // group of two warps and the thread in it
+  double* M = smb + gr * N * 2 * N;        // N x 2 N
+  double* cv = smb + kBuildGroups * N * 2 * N;  // c_ks (row 0 of block ks against block ks - 1)
   double* dv = cv + ns * N;       // d_ks (row N - 1 of block ks against block ks + 1)
   double* ends = dv + ns * N;     // first and last entry of every left vector
   double* A = ends + 2 * m;       // interface matrix, m x 2 m
@@ -1665,7 +1683,7 @@ static __global__ void __launch_bounds__(256) k_build_systems(const __grid_const
     dv[q] = d;
   }
   __syncthreads();
-  for (int blk = 0; blk < b.nb; ++blk) {
+  for (int blk = gr; blk < b.nb; blk += kBuildGroups) {
     const int ks = b.brep[blk];
     const double ybar = b.zh[ks], h = __ddiv_rn(2.0, ybar), eh = rmul(eps, rmul(h, h));
     const bool lo = ns > 1 && ks != 0, hi = ns > 1 && ks != ns - 1;
@@ -1673,7 +1691,7 @@ static __global__ void __launch_bounds__(256) k_build_systems(const __grid_const
     const double cf1 = -__ddiv_rn(t1b, ybar), cf2 = __ddiv_rn(t2d, ybar);
     const double cl = __ddiv_rn(rmul(rmul(rmul(rmul(0.5, pt1[ks]), pb[ks]), eps), 2.0), ybar);
     const double ch = -__ddiv_rn(rmul(rmul(rmul(rmul(0.5, pt2[ks]), pd[ks]), eps), 2.0), ybar);
-    for (int q = tid; q < N * 2 * N; q += nthr) {
+    for (int q = gt; q < N * 2 * N; q += 64) {
       const int r = q / (2 * N), c = q - r * 2 * N;
       double v = 0.0;
       if (c >= N) {
@@ -1700,12 +1718,12 @@ static __global__ void __launch_bounds__(256) k_build_systems(const __grid_const
       }
       M[q] = v;
     }
-    __syncthreads();
-    gauss_jordan(M, N, &piv, &pinv);
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + gr) : "memory");
+    gauss_jordan(M, N, piv + gr, pinv + gr, gt, 64, 1 + gr);
     // the inverse is M(r, N + c): tables column major
     double* out = b.ainv + ((size_t)s * b.nb + blk) * N * N;
     double* raw = s < b.nraw ? b.ainv_raw + ((size_t)s * b.nb + blk) * N * N : nullptr;
-    for (int q = tid; q < N * N; q += nthr) {
+    for (int q = gt; q < N * N; q += 64) {
       const int c = q / N, r = q - c * N;
       const double v = M[r * 2 * N + N + c];
       if (raw) raw[q] = v;
@@ -1719,7 +1737,7 @@ static __global__ void __launch_bounds__(256) k_build_systems(const __grid_const
       }
     }
     // left vectors of the subdomains with this block: c_{ks+1} (e = ks) and d_{ks-1} (e = ns - 2 + ks)
-    for (int q = tid; q < m * N; q += nthr) {
+    for (int q = gt; q < m * N; q += 64) {
       const int e = q / N, c = q - e * N;
       const int kb = e < ns - 1 ? e : e - (ns - 1) + 1;
       if (b.bmap[kb] != blk) continue;
@@ -1730,8 +1748,9 @@ static __global__ void __launch_bounds__(256) k_build_systems(const __grid_const
       if (c == 0) ends[2 * e] = a;
       if (c == N - 1) ends[2 * e + 1] = a;
     }
-    __syncthreads();
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + gr) : "memory");
   }
+  __syncthreads();
   if (m == 0) return;
   // unknowns: sigma_ks (ks = 1 .. ns-1) -> ks - 1, tau_ks (ks = 0 .. ns-2) -> ns - 1 + ks
   for (int q = tid; q < m * 2 * m; q += nthr) A[q] = (q % (2 * m)) - m == q / (2 * m) ? 1.0 : 0.0;
@@ -1743,7 +1762,7 @@ static __global__ void __launch_bounds__(256) k_build_systems(const __grid_const
     if (ks <= ns - 2) A[row * 2 * m + (ns - 1 + ks)] += ends[2 * row + 1];
   }
   __syncthreads();
-  gauss_jordan(A, m, &piv, &pinv);
+  gauss_jordan(A, m, piv, pinv, tid, nthr, 0);
   for (int q = tid; q < m * m; q += nthr) b.minv[(size_t)s * m * m + q] = A[(q / m) * 2 * m + m + q % m];
 }
 
@@ -3546,12 +3565,10 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
         x[kt] = (T)0;
         if (in(4 * kt + lt, 4 * kt + 3)) x[kt] = *f;
       }
-      if (proj >= 0) {
-        bool bad = false;
+      bool bad = false;
 #pragma unroll
-        for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
-        if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
-      }
+      for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
+      if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
       if (!PLAIN && special) {
         const bool wzero = q == 2 && tt < 2;
 #pragma unroll
@@ -3953,7 +3970,7 @@ struct StatRows {
   double cflh[2], rg, zlim;
   const double* dzinv;
 };
-template <typename T, int DPT, bool POW2>
+template <typename T, int DPT, bool POW2, int MC = 0>
 __global__ void __launch_bounds__(kStatThreads) k_xrow_stats(Geo g, const __grid_constant__ StatRows<T> a, FftPlan pl,
                                                             const typename cplx_t<T>::type* __restrict__ Wm,
                                                             const typename cplx_t<T>::type* __restrict__ Wn,
@@ -3961,7 +3978,8 @@ __global__ void __launch_bounds__(kStatThreads) k_xrow_stats(Geo g, const __grid
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double sh[kStatThreads / 32][kStatSlots];
-  const int M = g.nx / 2, RS = xstride(M), lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kStatThreads / 32;
+  const int M = MC > 0 ? MC : g.nx / 2, RS = xstride(M);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kStatThreads / 32;
   const int ent = blockIdx.y, q = a.q[ent], lines = g.ny * g.nz, step = gridDim.x * nw;
   const bool mulkx = a.kx[ent] != 0;
   const T kxs = (T)g.xw[1];
@@ -3982,7 +4000,10 @@ __global__ void __launch_bounds__(kStatThreads) k_xrow_stats(Geo g, const __grid
     __syncwarp();
     for (int kk = lane; kk <= M / 2; kk += 32) xprep_pair<C, T>(row, kk, M, Wn, mulkx, kxs);
     __syncwarp();
-    fft_warp<C, DPT, POW2>(row, pl, Wm, true, lane);
+    if constexpr (MC > 0)
+      fft_warp_ct<C, MC>(row, Wm, true, lane);
+    else
+      fft_warp<C, DPT, POW2>(row, pl, Wm, true, lane);
     const int k = line / g.ny;
     const double dzi = q == 2 ? a.dzinv[k] : 0.0, bg = q == 3 ? 1.0 + a.rg * g.zg[k] : 0.0;
     const bool low = q == 2 && g.zg[k] < a.zlim;
