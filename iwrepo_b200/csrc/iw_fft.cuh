@@ -1,8 +1,7 @@
 // Shared-memory FFT building blocks for sm_100a.
 //
 // Complex FFTs of length M (M = 2^a 3^b 5^c) are done as Stockham autosort
-// passes (radix 8, 4, 2, 3, 5; the power-of-two radices are
-// in-register DFTs) on data held in shared memory; a thread block
+// passes (radix 8, 6, 5, 4, 3, 2, in-register DFTs) on data held in shared memory; a thread block
 // works on a batch of independent transforms at once, one butterfly per
 // thread per pass.  Real transforms of length N = 2M use the half-length
 // complex transform plus the usual even/odd split.  Twiddles come from tables
@@ -76,6 +75,8 @@ struct FftPlan {
   int ns[12];       // accumulated size before the pass
   int nbsh[12];     // log2(M/R) if a power of two, else -1
   int nssh[12];     // log2(ns) if a power of two, else -1
+  float inb[12];    // 1 / (M/R), 1 / ns: (int)((q + 0.5f) * inv) is q / n for the small q here
+  float ins[12];
 };
 
 // v * w with w = c - i s (forward) or c + i s (inverse)
@@ -85,7 +86,7 @@ __device__ __forceinline__ C crot(C v, decltype(C().x) c, decltype(C().x) s, boo
   return cmk<C>(v.x * c - v.y * t, v.x * t + v.y * c);
 }
 
-// In-register DFT of v[0..R-1] (natural order in and out) for R = 2, 4, 8.
+// In-register DFT of v[0..R-1] (natural order in and out) for R = 2, 3, 4, 5, 6, 8.
 // R = 8 is split 2x4 (n = a + 2b, k = c + 4d); h = cos(pi/4).
 template <typename C>
 __device__ __forceinline__ void dft4(C& a0, C& a1, C& a2, C& a3, bool inv) {
@@ -97,6 +98,18 @@ __device__ __forceinline__ void dft4(C& a0, C& a1, C& a2, C& a3, bool inv) {
   a3 = csub(t1, t3);
 }
 
+// R = 3: o1, o2 = v0 - t/2 -+ i (sqrt(3)/2) (v1 - v2), t = v1 + v2
+template <typename C>
+__device__ __forceinline__ void dft3(C& a0, C& a1, C& a2, bool inv) {
+  typedef decltype(C().x) T;
+  const T h = (T)0.86602540378443864676;  // sin(2 pi / 3)
+  const C t = cadd(a1, a2), d = csub(a1, a2);
+  const C m = cmk<C>(a0.x - (T)0.5 * t.x, a0.y - (T)0.5 * t.y);
+  const C s = cmul_mi(cmk<C>(h * d.x, h * d.y), inv);
+  a0 = cadd(a0, t);
+  a1 = cadd(m, s);
+  a2 = csub(m, s);
+}
 template <typename C, int R>
 __device__ __forceinline__ void dft_reg(C* v, bool inv) {
   typedef decltype(C().x) T;
@@ -105,8 +118,37 @@ __device__ __forceinline__ void dft_reg(C* v, bool inv) {
     C t = v[0];
     v[0] = cadd(t, v[1]);
     v[1] = csub(t, v[1]);
+  } else if (R == 3) {
+    dft3(v[0], v[1], v[2], inv);
   } else if (R == 4) {
     dft4(v[0], v[1], v[2], v[3], inv);
+  } else if (R == 5) {
+    // cosines and sines of 2 pi / 5 and 4 pi / 5
+    const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
+    const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
+    const C t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]), d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
+    const C m1 = cmk<C>(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
+    const C m2 = cmk<C>(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
+    const C n1 = cmul_mi(cmk<C>(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y), inv);
+    const C n2 = cmul_mi(cmk<C>(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y), inv);
+    v[0] = cadd(v[0], cadd(t1, t2));
+    v[1] = cadd(m1, n1);
+    v[4] = csub(m1, n1);
+    v[2] = cadd(m2, n2);
+    v[3] = csub(m2, n2);
+  } else if (R == 6) {
+    // even and odd halves of three, joined with the sixth roots 1, (1 -+ i sqrt(3))/2, (-1 -+ i sqrt(3))/2
+    const T g = (T)0.86602540378443864676;
+    dft3(v[0], v[2], v[4], inv);
+    dft3(v[1], v[3], v[5], inv);
+    const C o1 = crot(v[3], (T)0.5, g, inv), o2 = crot(v[5], (T)-0.5, g, inv);
+    const C e0 = v[0], e1 = v[2], e2 = v[4], o0 = v[1];
+    v[0] = cadd(e0, o0);
+    v[1] = cadd(e1, o1);
+    v[2] = cadd(e2, o2);
+    v[3] = csub(e0, o0);
+    v[4] = csub(e1, o1);
+    v[5] = csub(e2, o2);
   } else if (R == 8) {
     // a in {0,1}: DFT4 over v[a + 2b]
     dft4(v[0], v[2], v[4], v[6], inv);
@@ -153,25 +195,7 @@ __device__ __forceinline__ void fft_pass_r(const C* __restrict__ src, C* __restr
         v[r] = cmul(v[r], tw);
       }
     }
-    if (R == 3 || R == 5) {
-      const int q0 = M / R;
-      C o[R];
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        C acc = v[0];
-#pragma unroll
-        for (int p = 1; p < R; ++p) {
-          C tw = W[((p * q) % R) * q0];
-          if (inv) tw.y = -tw.y;
-          acc = cadd(acc, cmul(v[p], tw));
-        }
-        o[q] = acc;
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = o[r];
-    } else {
-      dft_reg<C, R>(v, inv);
-    }
+    dft_reg<C, R>(v, inv);
     const int base = jq * Ns * R + jm;
 #pragma unroll
     for (int r = 0; r < R; ++r) d[base + r * Ns] = v[r];
@@ -191,6 +215,7 @@ __device__ C* fft_run(C* a, C* b, const FftPlan& pl, int nbatch, const C* W, boo
       case 4: fft_pass_r<C, 4>(src, dst, pl.M, Ns, nbatch, W, inv, tid, nthr, bs, ss); break;
       case 2: fft_pass_r<C, 2>(src, dst, pl.M, Ns, nbatch, W, inv, tid, nthr, bs, ss); break;
       case 3: fft_pass_r<C, 3>(src, dst, pl.M, Ns, nbatch, W, inv, tid, nthr, bs, ss); break;
+      case 6: fft_pass_r<C, 6>(src, dst, pl.M, Ns, nbatch, W, inv, tid, nthr, bs, ss); break;
       default: fft_pass_r<C, 5>(src, dst, pl.M, Ns, nbatch, W, inv, tid, nthr, bs, ss); break;
     }
     __syncthreads();
@@ -203,8 +228,8 @@ __device__ C* fft_run(C* a, C* b, const FftPlan& pl, int nbatch, const C* W, boo
 
 
 // ---------------------------------------------------------------------------
-// Warp-synchronous in-place transforms.  One warp owns one transform of length
-// M held in shared memory with one pad slot after every 16 values (index
+// Warp-synchronous in-place transforms.  One warp owns a transform of length M, or
+// several short ones at once, held in shared memory with one pad slot after every 16 values (index
 // fpad(i)), which keeps the strided Stockham stores free of bank conflicts.
 // Every pass loads all of its butterflies into registers, then stores them:
 // no second buffer and no CTA-wide barrier.  DPT >= M/32 values per lane.
@@ -213,22 +238,24 @@ __host__ __device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }
 // slots needed for L padded values
 __host__ __device__ __forceinline__ int fpadlen(int L) { return L > 0 ? fpad(L - 1) + 1 : 0; }
 
-template <typename C, int R, int NB>
-__device__ __forceinline__ void fft_pass_w(C* row, int M, int Ns, const C* __restrict__ W, bool inv, int lane,
-                                           int nssh) {
+// One pass over the butterflies of G rows (RS values apart) at once: short rows share
+// the warp's lanes.  G M / R <= 32 IT.
+template <typename C, int R, int IT>
+__device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns, float inb, float ins,
+                                           const C* __restrict__ W, bool inv, int lane) {
   const int nb = M / R;
-  const int step = M / (Ns * R);
-  C v[NB][R];
+  const int step = M / (Ns * R), items = G * nb;
+  C v[IT][R];
 #pragma unroll
-  for (int q = 0; q < NB; ++q) {
-    const int j = lane + 32 * q;
-    if (j < nb) {
-      const int jq = nssh >= 0 ? (j >> nssh) : (j / Ns);
-      const int jm = j - jq * Ns;
+  for (int q = 0; q < IT; ++q) {
+    const int it = lane + 32 * q;
+    if (it < items) {
+      const int g = (int)(((float)it + 0.5f) * inb), j = it - g * nb;
+      const C* row = base + g * RS;
 #pragma unroll
       for (int r = 0; r < R; ++r) v[q][r] = row[fpad(j + r * nb)];
       if (Ns > 1) {
-        const int e = jm * step;
+        const int jm = j - (int)(((float)j + 0.5f) * ins) * Ns, e = jm * step;
 #pragma unroll
         for (int r = 1; r < R; ++r) {
           C tw = W[r * e];
@@ -236,69 +263,61 @@ __device__ __forceinline__ void fft_pass_w(C* row, int M, int Ns, const C* __res
           v[q][r] = cmul(v[q][r], tw);
         }
       }
-      if (R == 3 || R == 5) {
-        const int q0 = M / R;
-        C o[R];
-#pragma unroll
-        for (int qq = 0; qq < R; ++qq) {
-          C acc = v[q][0];
-#pragma unroll
-          for (int p = 1; p < R; ++p) {
-            C tw = W[((p * qq) % R) * q0];
-            if (inv) tw.y = -tw.y;
-            acc = cadd(acc, cmul(v[q][p], tw));
-          }
-          o[qq] = acc;
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[q][r] = o[r];
-      } else {
-        dft_reg<C, R>(v[q], inv);
-      }
+      dft_reg<C, R>(v[q], inv);
     }
   }
   __syncwarp();
 #pragma unroll
-  for (int q = 0; q < NB; ++q) {
-    const int j = lane + 32 * q;
-    if (j < nb) {
-      const int jq = nssh >= 0 ? (j >> nssh) : (j / Ns);
-      const int jm = j - jq * Ns;
-      const int base = jq * Ns * R + jm;
+  for (int q = 0; q < IT; ++q) {
+    const int it = lane + 32 * q;
+    if (it < items) {
+      const int g = (int)(((float)it + 0.5f) * inb), j = it - g * nb;
+      const int jq = (int)(((float)j + 0.5f) * ins), jm = j - jq * Ns;
+      C* row = base + g * RS;
+      const int b0 = jq * Ns * R + jm;
 #pragma unroll
-      for (int r = 0; r < R; ++r) row[fpad(base + r * Ns)] = v[q][r];
+      for (int r = 0; r < R; ++r) row[fpad(b0 + r * Ns)] = v[q][r];
     }
   }
   __syncwarp();
 }
 
-// In-place transform of one padded row by one warp (all lanes call it).
-// POW2: the length is a power of two, so only radix 8, 4, 2 passes are
+// rows of length M that one warp transforms at a time with DPT values per lane
+__host__ __device__ constexpr int fft_rows_of(int M, int DPT) { return 32 * DPT / M > 1 ? 32 * DPT / M : 1; }
+
+// In-place transform of G <= fft_rows_of(M, DPT) padded rows by one warp (all lanes
+// call it).  POW2: the length is a power of two, so only radix 8, 4, 2 passes are
 // compiled (every compiled radix raises the register count of the kernel).
 template <typename C, int DPT, bool POW2>
-__device__ __forceinline__ void fft_warp(C* row, const FftPlan& pl, const C* __restrict__ W, bool inv, int lane) {
+__device__ __forceinline__ void fft_warp(C* base, int RS, int G, const FftPlan& pl, const C* __restrict__ W, bool inv,
+                                         int lane) {
   for (int p = 0; p < pl.npass; ++p) {
-    const int Ns = pl.ns[p], ss = pl.nssh[p];
+    const int Ns = pl.ns[p];
+    const float ib = pl.inb[p], is = pl.ins[p];
     switch (pl.rad[p]) {
-      case 8: fft_pass_w<C, 8, (DPT + 7) / 8>(row, pl.M, Ns, W, inv, lane, ss); break;
-      case 4: fft_pass_w<C, 4, (DPT + 3) / 4>(row, pl.M, Ns, W, inv, lane, ss); break;
-      case 2: fft_pass_w<C, 2, (DPT + 1) / 2>(row, pl.M, Ns, W, inv, lane, ss); break;
+      case 8: fft_pass_w<C, 8, (DPT + 7) / 8>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
+      case 4: fft_pass_w<C, 4, (DPT + 3) / 4>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
+      case 2: fft_pass_w<C, 2, (DPT + 1) / 2>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
       default:
         if (!POW2) {
           if (pl.rad[p] == 3)
-            fft_pass_w<C, 3, (DPT + 2) / 3>(row, pl.M, Ns, W, inv, lane, ss);
+            fft_pass_w<C, 3, (DPT + 2) / 3>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+          else if (pl.rad[p] == 6)
+            fft_pass_w<C, 6, (DPT + 5) / 6>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
           else
-            fft_pass_w<C, 5, (DPT + 4) / 5>(row, pl.M, Ns, W, inv, lane, ss);
+            fft_pass_w<C, 5, (DPT + 4) / 5>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
         }
         break;
     }
   }
 }
 
-// minimum resident CTAs of 256 threads for a warp-transform kernel
-template <typename T, int DPT>
+// minimum resident CTAs of 256 threads for a warp-transform kernel (the mixed-radix
+// kernels hold every radix and get more registers)
+template <typename T, int DPT, bool POW2 = true>
 struct FftOcc {
-  static constexpr int v = sizeof(T) == 4 ? (DPT <= 8 ? 4 : DPT <= 16 ? 2 : 1) : (DPT <= 4 ? 4 : DPT <= 8 ? 2 : 1);
+  static constexpr int v0 = sizeof(T) == 4 ? (DPT <= 8 ? 4 : DPT <= 16 ? 2 : 1) : (DPT <= 4 ? 4 : DPT <= 8 ? 2 : 1);
+  static constexpr int v = POW2 || v0 < 4 ? v0 : 3;
 };
 
 
@@ -315,16 +334,25 @@ struct CtPlan {
   __host__ __device__ static constexpr int bits(int q) { return a / np + (q < a % np ? 1 : 0); }
 };
 
+// values per lane of the compile-time transforms: short rows share the warp
+template <int M>
+struct CtRows {
+  static constexpr int DPT = M <= 256 ? 8 : M / 32;
+  static constexpr int G = fft_rows_of(M, DPT);
+};
 template <typename C, int M, int R, int NS>
-__device__ __forceinline__ void fft_pass_ct(C* row, const C* __restrict__ W, bool inv, int lane) {
+__device__ __forceinline__ void fft_pass_ct(C* base, int RS, int G, const C* __restrict__ W, bool inv, int lane) {
   constexpr int nb = M / R;
   constexpr int step = M / (NS * R);
-  constexpr int NB = (nb + 31) / 32;
+  constexpr int NB = (CtRows<M>::G * nb + 31) / 32;
+  const int items = CtRows<M>::G > 1 ? G * nb : nb;
   C v[NB][R];
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
-    const int j = lane + 32 * q;
-    if (nb % 32 == 0 || j < nb) {
+    const int it = lane + 32 * q;
+    if ((CtRows<M>::G == 1 && nb % 32 == 0) || it < items) {
+      const int g = CtRows<M>::G > 1 ? it / nb : 0, j = CtRows<M>::G > 1 ? it % nb : it;
+      const C* row = base + g * RS;
       const int jm = j & (NS - 1);
 #pragma unroll
       for (int r = 0; r < R; ++r) v[q][r] = row[fpad(j + r * nb)];
@@ -343,40 +371,33 @@ __device__ __forceinline__ void fft_pass_ct(C* row, const C* __restrict__ W, boo
   __syncwarp();
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
-    const int j = lane + 32 * q;
-    if (nb % 32 == 0 || j < nb) {
+    const int it = lane + 32 * q;
+    if ((CtRows<M>::G == 1 && nb % 32 == 0) || it < items) {
+      const int g = CtRows<M>::G > 1 ? it / nb : 0, j = CtRows<M>::G > 1 ? it % nb : it;
+      C* row = base + g * RS;
       const int jq = j / NS, jm = j & (NS - 1);
-      const int base = jq * NS * R + jm;
+      const int b0 = jq * NS * R + jm;
 #pragma unroll
-      for (int r = 0; r < R; ++r) row[fpad(base + r * NS)] = v[q][r];
+      for (int r = 0; r < R; ++r) row[fpad(b0 + r * NS)] = v[q][r];
     }
   }
   __syncwarp();
 }
 
-template <typename C, int M, int P, int NS>
-__device__ __forceinline__ void fft_passes_ct(C* row, const C* __restrict__ W, bool inv, int lane) {
-  if constexpr (P < CtPlan<M>::np) {
-    constexpr int R = 1 << CtPlan<M>::bits(P);
-    fft_pass_ct<C, M, R, NS>(row, W, inv, lane);
-    fft_passes_ct<C, M, P + 1, NS * R>(row, W, inv, lane);
-  }
-}
-
-// Passes P .. PEND-1 only (the first or last pass run elsewhere).
+// Passes P .. PEND-1 (the first or last pass may run elsewhere) of G <= CtRows<M>::G rows.
 template <typename C, int M, int P, int PEND, int NS>
-__device__ __forceinline__ void fft_passes_ct_to(C* row, const C* __restrict__ W, bool inv, int lane) {
+__device__ __forceinline__ void fft_passes_ct(C* base, int RS, int G, const C* __restrict__ W, bool inv, int lane) {
   if constexpr (P < PEND) {
     constexpr int R = 1 << CtPlan<M>::bits(P);
-    fft_pass_ct<C, M, R, NS>(row, W, inv, lane);
-    fft_passes_ct_to<C, M, P + 1, PEND, NS * R>(row, W, inv, lane);
+    fft_pass_ct<C, M, R, NS>(base, RS, G, W, inv, lane);
+    fft_passes_ct<C, M, P + 1, PEND, NS * R>(base, RS, G, W, inv, lane);
   }
 }
 
-// In-place transform of one padded row of power-of-two length M by one warp.
+// In-place transform of G <= CtRows<M>::G padded rows of power-of-two length M by one warp.
 template <typename C, int M>
-__device__ __forceinline__ void fft_warp_ct(C* row, const C* __restrict__ W, bool inv, int lane) {
-  fft_passes_ct<C, M, 0, 1>(row, W, inv, lane);
+__device__ __forceinline__ void fft_warp_ct(C* base, int RS, int G, const C* __restrict__ W, bool inv, int lane) {
+  fft_passes_ct<C, M, 0, CtPlan<M>::np, 1>(base, RS, G, W, inv, lane);
 }
 
 }  // namespace iw

@@ -238,32 +238,36 @@ FftPlan make_plan(int M) {
     p.ns[p.npass] = ns;
     p.nbsh[p.npass] = lg2(M / r);
     p.nssh[p.npass] = lg2(ns);
+    p.inb[p.npass] = 1.0f / (float)(M / r);
+    p.ins[p.npass] = 1.0f / (float)ns;
     ns *= r;
     p.npass++;
   };
   // powers of two: ceil(a/3) passes of radix <= 8, bits spread evenly
   // (512 -> 8*8*8, 256 -> 8*8*4); larger radices cost more registers than
-  // they save in passes
-  int a2 = 0;
-  while (m % 2 == 0) {
-    m /= 2;
-    ++a2;
-  }
-  if (a2 > 0) {
-    const int np = (a2 + 2) / 3;
-    for (int q = 0; q < np; ++q) {
-      const int bits = a2 / np + (q < a2 % np ? 1 : 0);
-      push(1 << bits);
+  // they save in passes.  Mixed lengths: the fewest passes over 8, 6, 5, 4, 3, 2,
+  // and of those the smallest sum of radices (96 -> 6*4*4, 120 -> 6*5*4).
+  int a2 = 0, a3 = 0, a5 = 0;
+  while (m % 2 == 0) m /= 2, ++a2;
+  while (m % 3 == 0) m /= 3, ++a3;
+  while (m % 5 == 0) m /= 5, ++a5;
+  int best6 = 0, bestn = 1 << 30, bests = 0;
+  for (int n6 = 0; n6 <= std::min(a2, a3); ++n6) {
+    const int b2 = a2 - n6, n = n6 + (b2 + 2) / 3 + (a3 - n6);
+    int sum = 6 * n6 + 3 * (a3 - n6);
+    for (int q = 0, np = (b2 + 2) / 3; q < np; ++q) sum += 1 << (b2 / np + (q < b2 % np ? 1 : 0));
+    if (n < bestn || (n == bestn && sum < bests)) {
+      best6 = n6;
+      bestn = n;
+      bests = sum;
     }
   }
-  while (m % 3 == 0) {
-    push(3);
-    m /= 3;
-  }
-  while (m % 5 == 0) {
-    push(5);
-    m /= 5;
-  }
+  for (int q = 0; q < best6; ++q) push(6);
+  a2 -= best6;
+  a3 -= best6;
+  for (int q = 0, np = (a2 + 2) / 3; q < np; ++q) push(1 << (a2 / np + (q < a2 % np ? 1 : 0)));
+  for (int q = 0; q < a3; ++q) push(3);
+  for (int q = 0; q < a5; ++q) push(5);
   if (m != 1) p.npass = -1;
   return p;
 }
@@ -409,7 +413,7 @@ struct iw_handle {
   int bmap[IW_MAX_SUBD] = {};
   // launch choices set by iw_autotune (0 / -1: built-in heuristic)
   int tune_ytx = 0;  // y-tile width
-  int tune_xthr = 0;  // threads per x-row CTA: 0 or 256, or 128
+  int tune_xthr = 0;  // threads per x-row CTA: 256 or 128, 0: by length
   int tune_a = -1;   // stage A: 1 register-column, 0 tiled
   int tune_e = -1;   // stage E: 1 register-column, 0 tiled, 2 tiled with bulk-copied tiles
   int brep[IW_MAX_SUBD] = {};
@@ -1016,13 +1020,14 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
 // values per lane of a warp transform of length M
 static int fft_dpt(int M) {
   const int d = (M + 31) / 32;
-  return d <= 4 ? 4 : d <= 8 ? 8 : d <= 16 ? 16 : 32;
+  return d <= 8 ? 8 : d <= 16 ? 16 : 32;
 }
 
 template <typename T>
 static int ytx(const iw_handle* h, bool two) {  // y-FFT tile width
   const size_t cs = 2 * sizeof(T);
   int tx = h->tune_ytx > 0 ? h->tune_ytx : 8;
+  if (tx == 8 && h->ny <= 128) tx = 16;  // two short columns per warp
   while (tx > 1 && (two ? 2 : 1) * (size_t)tx * ystride(h->ny) * cs > 110 * 1024) tx /= 2;
   return tx;
 }
@@ -1032,15 +1037,26 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
                         const typename cplx_t<T>::type* Wy) {
   Geo g = geo(h);
   const bool p2 = (h->ny & (h->ny - 1)) == 0;
-  if constexpr (TX == 8) {  // compile-time plans for the common power-of-two lengths
+  if constexpr (TX == 16) {  // compile-time plans for the common power-of-two lengths
     switch (p2 ? h->ny : 0) {
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
     cudaFuncSetAttribute(k_yfft<T, TX, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     k_yfft<T, TX, D, true, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     return;
-      IW_YCT(64, 4)
-      IW_YCT(128, 4)
+      IW_YCT(64, 8)
+      IW_YCT(128, 8)
+#undef IW_YCT
+      default: break;
+    }
+  }
+  if constexpr (TX == 8) {
+    switch (p2 ? h->ny : 0) {
+#define IW_YCT(MC, D)                                                                                        \
+  case MC:                                                                                                   \
+    cudaFuncSetAttribute(k_yfft<T, TX, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    k_yfft<T, TX, D, true, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+    return;
       IW_YCT(256, 8)
       IW_YCT(512, 16)
 #undef IW_YCT
@@ -1053,16 +1069,20 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
     cudaFuncSetAttribute(k_yfft<T, TX, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
     k_yfft<T, TX, D, P><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                          \
     break;
-    IW_YCASE(4, true)
     IW_YCASE(8, true)
-    IW_YCASE(16, true)
-    IW_YCASE(32, true)
-    IW_YCASE(4, false)
     IW_YCASE(8, false)
-    IW_YCASE(16, false)
-    IW_YCASE(32, false)
-#undef IW_YCASE
+    default: break;
   }
+  if constexpr (TX < 16) {  // (16 columns only for ny <= 128)
+    switch (fft_dpt(h->ny) * (p2 ? 1 : -1)) {
+      IW_YCASE(16, true)
+      IW_YCASE(32, true)
+      IW_YCASE(16, false)
+      IW_YCASE(32, false)
+      default: break;
+    }
+  }
+#undef IW_YCASE
 }
 
 template <typename T>
@@ -1078,6 +1098,7 @@ void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int npla
   dim3 grid(ntile, nplanes, njobs);
   const size_t smem = (four ? 2 : 1) * (size_t)tx * ystride(h->ny) * sizeof(C);
   switch (tx) {
+    case 16: launch_y_tx<T, 16>(h, jobs, grid, smem, nplanes, fs.Wy); break;
     case 8: launch_y_tx<T, 8>(h, jobs, grid, smem, nplanes, fs.Wy); break;
     case 4: launch_y_tx<T, 4>(h, jobs, grid, smem, nplanes, fs.Wy); break;
     case 2: launch_y_tx<T, 2>(h, jobs, grid, smem, nplanes, fs.Wy); break;
@@ -1124,7 +1145,8 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
   typedef typename cplx_t<T>::type C;
   Geo g = geo(h);
   const int M = h->nx / 2;
-  const int xthr = h->tune_xthr == 128 ? 128 : 256;
+  // short rows: fewer warps, each with several rows (rows of 32..128 values fill a warp only together)
+  const int xthr = h->tune_xthr > 0 ? h->tune_xthr : M <= 128 ? 128 : 256;
   {
     NLArgs<T> a;
     memset(&a, 0, sizeof a);
@@ -1165,9 +1187,9 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
     cudaFuncSetAttribute(k_xrow_nl<T, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     k_xrow_nl<T, D, true, MC><<<grid, xthr, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn);                     \
     goto xrow_done;
-      IW_XCT(32, 4)
-      IW_XCT(64, 4)
-      IW_XCT(128, 4)
+      IW_XCT(32, 8)
+      IW_XCT(64, 8)
+      IW_XCT(128, 8)
       IW_XCT(256, 8)
       IW_XCT(512, 16)
 #undef IW_XCT
@@ -1179,12 +1201,10 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
     cudaFuncSetAttribute(k_xrow_nl<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
     k_xrow_nl<T, D, P><<<grid, xthr, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn);                        \
     break;
-      IW_XCASE(4, true)
-      IW_XCASE(8, true)
+        IW_XCASE(8, true)
       IW_XCASE(16, true)
       IW_XCASE(32, true)
-      IW_XCASE(4, false)
-      IW_XCASE(8, false)
+        IW_XCASE(8, false)
       IW_XCASE(16, false)
       IW_XCASE(32, false)
 #undef IW_XCASE
@@ -1208,9 +1228,9 @@ void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, i
     cudaFuncSetAttribute(k_xrow_stats<T, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
     k_xrow_stats<T, D, true, MC><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);     \
     return;
-    IW_SCT(32, 4)
-    IW_SCT(64, 4)
-    IW_SCT(128, 4)
+    IW_SCT(32, 8)
+    IW_SCT(64, 8)
+    IW_SCT(128, 8)
     IW_SCT(256, 8)
     IW_SCT(512, 16)
 #undef IW_SCT
@@ -1222,11 +1242,9 @@ void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, i
     cudaFuncSetAttribute(k_xrow_stats<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
     k_xrow_stats<T, D, P><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);        \
     break;
-    IW_SCASE(4, true)
     IW_SCASE(8, true)
     IW_SCASE(16, true)
     IW_SCASE(32, true)
-    IW_SCASE(4, false)
     IW_SCASE(8, false)
     IW_SCASE(16, false)
     IW_SCASE(32, false)
@@ -2439,7 +2457,7 @@ int iw_get_launch(iw_handle* h, int which, int* value) {
     case IW_LAUNCH_SOLVE_W: *value = h->sys_role[1]; return IW_OK;
     case IW_LAUNCH_SOLVE_RHO: *value = h->sys_role[2]; return IW_OK;
     case IW_LAUNCH_SOLVE_PRESSURE: *value = h->sys_role[3]; return IW_OK;
-    case IW_LAUNCH_XROW_THREADS: *value = h->tune_xthr == 128 ? 128 : 256; return IW_OK;
+    case IW_LAUNCH_XROW_THREADS: *value = h->tune_xthr > 0 ? h->tune_xthr : h->nx <= 256 ? 128 : 256; return IW_OK;
     default: return set_err(IW_ERR_CONFIG, "unknown launch choice");
   }
 }

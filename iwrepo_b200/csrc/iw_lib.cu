@@ -237,7 +237,7 @@ __host__ __device__ __forceinline__ int ystride(int ny) {
 }
 
 template <typename T, int TX, int DPT, bool POW2, int MC = 0>
-__global__ void __launch_bounds__(256, (FftOcc<T, DPT>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
+__global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
                                               const typename cplx_t<T>::type* __restrict__ Wy) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -360,18 +360,24 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT>::v)) k_yfft(Geo g, YJobs<
   }
   // the x-Nyquist column (ii = nxh) is not transformed
   const int nb = ny > 1 ? max(0, min(TX, g.nxh - ii0)) : 0;
-  const int nrow = two ? 2 * nb : nb;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int r = threadIdx.x >> 5; r < nrow; r += nw) {
-    C* row = r < nb ? A + r * RSY : A2 + (r - nb) * RSY;
-    if constexpr (fuseL)  // the first pass ran at load, the last runs at the store
-      fft_passes_ct_to<C, (MC > 0 ? MC : 2), 1, NPS - 1, R0>(row, Wy, !fwd, lane);
-    else if constexpr (fuse1)
-      fft_passes_ct<C, (MC > 0 ? MC : 2), 1, R0>(row, Wy, !fwd, lane);  // the first pass ran at load
-    else if constexpr (MC > 0)
-      fft_warp_ct<C, MC>(row, Wy, !fwd, lane);
-    else
-      fft_warp<C, DPT, POW2>(row, pl, Wy, !fwd, lane);
+  const int gmax = MC > 0 ? CtRows<(MC > 0 ? MC : 2)>::G : fft_rows_of(ny, DPT);  // columns a warp takes at a time
+  const int gb = gmax > 1 ? max(1, min(gmax, ((two ? 2 : 1) * nb + nw - 1) / nw)) : 1;
+  const int ng = gb > 1 ? (nb + gb - 1) / gb : nb;  // groups of gb columns
+  {
+    for (int q = threadIdx.x >> 5; q < (two ? 2 : 1) * ng; q += nw) {
+      const int r = (q < ng ? q : q - ng) * gb;
+      C* row = (q < ng ? A : A2) + r * RSY;
+      const int G = min(gb, nb - r);
+      if constexpr (fuseL)  // the first pass ran at load, the last runs at the store
+        fft_passes_ct<C, (MC > 0 ? MC : 2), 1, NPS - 1, R0>(row, RSY, G, Wy, !fwd, lane);
+      else if constexpr (fuse1)
+        fft_passes_ct<C, (MC > 0 ? MC : 2), 1, NPS, R0>(row, RSY, G, Wy, !fwd, lane);  // the first pass ran at load
+      else if constexpr (MC > 0)
+        fft_warp_ct<C, MC>(row, RSY, G, Wy, !fwd, lane);
+      else
+        fft_warp<C, DPT, POW2>(row, RSY, G, pl, Wy, !fwd, lane);
+    }
   }
   __syncthreads();
   const T sc = fwd ? (T)g.scaley : (T)1;
@@ -541,7 +547,7 @@ __host__ __device__ __forceinline__ int xstride(int M) { return fpadlen(M + 1); 
 // K_C: CTA per (j,k) row; 20 padded rows of M+1 values in shared memory; each
 // warp transforms whole rows in place.
 template <typename T, int DPT, bool POW2, int MC = 0>
-__global__ void __launch_bounds__(256, (FftOcc<T, DPT>::v)) k_xrow_nl(Geo g, NLArgs<T> a, FftPlan pl,
+__global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo g, NLArgs<T> a, FftPlan pl,
                                                  const typename cplx_t<T>::type* __restrict__ Wm,
                                                  const typename cplx_t<T>::type* __restrict__ Wn) {
   typedef typename cplx_t<T>::type C;
@@ -591,11 +597,15 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT>::v)) k_xrow_nl(Geo g, NLA
     }
   }
   __syncthreads();
-  for (int r = wid; r < nrow; r += nw) {
-    if constexpr (MC > 0)
-      fft_warp_ct<C, MC>(buf + r * RS, Wm, true, lane);
-    else
-      fft_warp<C, DPT, POW2>(buf + r * RS, pl, Wm, true, lane);
+  const int gmax = MC > 0 ? CtRows<(MC > 0 ? MC : 2)>::G : fft_rows_of(M, DPT);  // rows a warp takes at a time
+  {
+    const int gb = min(gmax, (nrow + nw - 1) / nw);
+    for (int r = wid * gb; r < nrow; r += nw * gb) {
+      if constexpr (MC > 0)
+        fft_warp_ct<C, MC>(buf + r * RS, RS, min(gb, nrow - r), Wm, true, lane);
+      else
+        fft_warp<C, DPT, POW2>(buf + r * RS, RS, min(gb, nrow - r), pl, Wm, true, lane);
+    }
   }
   __syncthreads();
   // physical value i of row r
@@ -651,11 +661,14 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT>::v)) k_xrow_nl(Geo g, NLA
     P(12, i) = -(w * t);
   }
   __syncthreads();
-  for (int r = wid; r < 13; r += nw) {
-    if constexpr (MC > 0)
-      fft_warp_ct<C, MC>(buf + r * RS, Wm, false, lane);
-    else
-      fft_warp<C, DPT, POW2>(buf + r * RS, pl, Wm, false, lane);
+  {
+    const int gb = min(gmax, (13 + nw - 1) / nw);
+    for (int r = wid * gb; r < 13; r += nw * gb) {
+      if constexpr (MC > 0)
+        fft_warp_ct<C, MC>(buf + r * RS, RS, min(gb, 13 - r), Wm, false, lane);
+      else
+        fft_warp<C, DPT, POW2>(buf + r * RS, RS, min(gb, 13 - r), pl, Wm, false, lane);
+    }
   }
   __syncthreads();
   const T invN = (T)1 / (T)nx;
@@ -4001,9 +4014,9 @@ __global__ void __launch_bounds__(kStatThreads) k_xrow_stats(Geo g, const __grid
     for (int kk = lane; kk <= M / 2; kk += 32) xprep_pair<C, T>(row, kk, M, Wn, mulkx, kxs);
     __syncwarp();
     if constexpr (MC > 0)
-      fft_warp_ct<C, MC>(row, Wm, true, lane);
+      fft_warp_ct<C, MC>(row, RS, 1, Wm, true, lane);
     else
-      fft_warp<C, DPT, POW2>(row, pl, Wm, true, lane);
+      fft_warp<C, DPT, POW2>(row, RS, 1, pl, Wm, true, lane);
     const int k = line / g.ny;
     const double dzi = q == 2 ? a.dzinv[k] : 0.0, bg = q == 3 ? 1.0 + a.rg * g.zg[k] : 0.0;
     const bool low = q == 2 && g.zg[k] < a.zlim;
