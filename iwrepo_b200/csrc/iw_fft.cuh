@@ -38,6 +38,21 @@ template <typename C>
 __device__ __forceinline__ C csub(C a, C b) {
   return cmk<C>(a.x - b.x, a.y - b.y);
 }
+// two FP32 additions in one instruction (each rounded as ever)
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  float2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
 template <typename C>
 __device__ __forceinline__ C cmul(C a, C b) {
   return cmk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -86,7 +101,8 @@ __device__ __forceinline__ C crot(C v, decltype(C().x) c, decltype(C().x) s, boo
   return cmk<C>(v.x * c - v.y * t, v.x * t + v.y * c);
 }
 
-// In-register DFT of v[0..R-1] (natural order in and out) for R = 2, 3, 4, 5, 6, 8.
+// In-register DFT of v[0..R-1] (natural order in and out) for R = 2, 3, 4, 5, 6, 8,
+// 10, 16.
 // R = 8 is split 2x4 (n = a + 2b, k = c + 4d); h = cos(pi/4).
 template <typename C>
 __device__ __forceinline__ void dft4(C& a0, C& a1, C& a2, C& a3, bool inv) {
@@ -110,6 +126,23 @@ __device__ __forceinline__ void dft3(C& a0, C& a1, C& a2, bool inv) {
   a1 = cadd(m, s);
   a2 = csub(m, s);
 }
+template <typename C>
+__device__ __forceinline__ void dft5(C& a0, C& a1, C& a2, C& a3, C& a4, bool inv) {
+  typedef decltype(C().x) T;
+  // cosines and sines of 2 pi / 5 and 4 pi / 5
+  const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
+  const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
+  const C t1 = cadd(a1, a4), t2 = cadd(a2, a3), d1 = csub(a1, a4), d2 = csub(a2, a3);
+  const C m1 = cmk<C>(a0.x + c1 * t1.x + c2 * t2.x, a0.y + c1 * t1.y + c2 * t2.y);
+  const C m2 = cmk<C>(a0.x + c2 * t1.x + c1 * t2.x, a0.y + c2 * t1.y + c1 * t2.y);
+  const C n1 = cmul_mi(cmk<C>(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y), inv);
+  const C n2 = cmul_mi(cmk<C>(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y), inv);
+  a0 = cadd(a0, cadd(t1, t2));
+  a1 = cadd(m1, n1);
+  a4 = csub(m1, n1);
+  a2 = cadd(m2, n2);
+  a3 = csub(m2, n2);
+}
 template <typename C, int R>
 __device__ __forceinline__ void dft_reg(C* v, bool inv) {
   typedef decltype(C().x) T;
@@ -123,19 +156,7 @@ __device__ __forceinline__ void dft_reg(C* v, bool inv) {
   } else if (R == 4) {
     dft4(v[0], v[1], v[2], v[3], inv);
   } else if (R == 5) {
-    // cosines and sines of 2 pi / 5 and 4 pi / 5
-    const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
-    const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
-    const C t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]), d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
-    const C m1 = cmk<C>(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    const C m2 = cmk<C>(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    const C n1 = cmul_mi(cmk<C>(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y), inv);
-    const C n2 = cmul_mi(cmk<C>(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y), inv);
-    v[0] = cadd(v[0], cadd(t1, t2));
-    v[1] = cadd(m1, n1);
-    v[4] = csub(m1, n1);
-    v[2] = cadd(m2, n2);
-    v[3] = csub(m2, n2);
+    dft5(v[0], v[1], v[2], v[3], v[4], inv);
   } else if (R == 6) {
     // even and odd halves of three, joined with the sixth roots 1, (1 -+ i sqrt(3))/2, (-1 -+ i sqrt(3))/2
     const T g = (T)0.86602540378443864676;
@@ -165,6 +186,43 @@ __device__ __forceinline__ void dft_reg(C* v, bool inv) {
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = o[i];
+  } else if (R == 10) {
+    // even and odd halves of five, joined with the tenth roots
+    const T c1 = (T)0.80901699437494742410, s1 = (T)0.58778525229247312917;
+    const T c2 = (T)0.30901699437494742410, s2 = (T)0.95105651629515357212;
+    dft5(v[0], v[2], v[4], v[6], v[8], inv);
+    dft5(v[1], v[3], v[5], v[7], v[9], inv);
+    C o[5] = {v[1], crot(v[3], c1, s1, inv), crot(v[5], c2, s2, inv), crot(v[7], -c2, s2, inv),
+              crot(v[9], -c1, s1, inv)};
+    C e[5] = {v[0], v[2], v[4], v[6], v[8]};
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      v[c] = cadd(e[c], o[c]);
+      v[c + 5] = csub(e[c], o[c]);
+    }
+  } else if (R == 16) {
+    // a in 0..3: DFT4 over v[a + 4 b], twiddles w16^(a c), DFT4 over a
+    const T c1 = (T)0.92387953251128675613, s1 = (T)0.38268343236508977173;  // pi / 8
+#pragma unroll
+    for (int a = 0; a < 4; ++a) dft4(v[a], v[a + 4], v[a + 8], v[a + 12], inv);
+    v[5] = crot(v[5], c1, s1, inv);
+    v[6] = crot(v[6], h, h, inv);
+    v[7] = crot(v[7], s1, c1, inv);
+    v[9] = crot(v[9], h, h, inv);
+    v[10] = cmul_mi(v[10], inv);
+    v[11] = crot(v[11], -h, h, inv);
+    v[13] = crot(v[13], s1, c1, inv);
+    v[14] = crot(v[14], -h, h, inv);
+    v[15] = crot(v[15], -c1, -s1, inv);
+    C o[16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      dft4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3], inv);
+#pragma unroll
+      for (int d = 0; d < 4; ++d) o[c + 4 * d] = v[4 * c + d];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = o[i];
   }
 }
 

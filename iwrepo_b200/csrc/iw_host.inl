@@ -918,15 +918,16 @@ static int z_grid(const iw_handle* h, int W, int occ) {
 }
 
 template <typename T, int NM>
-static void launch_stageA_r(iw_handle* h, FieldSet<T>& fs, int proj) {
+static void launch_stageA_r(iw_handle* h, FieldSet<T>& fs, int proj, T* z3) {
   dim3 grid((unsigned)((h->plane + 127) / 128), (unsigned)h->ns, 4);
   k_stageA_r<T, NM><<<grid, 128, 0, h->st>>>(geo(h), make_zop<T, NM>(h), fs.F[0], fs.F[1], fs.F[2], fs.F[3], fs.F1[0],
-                                             fs.F1[1], fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], fs.Z4[3], proj,
+                                             fs.F1[1], fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], z3, proj,
                                              h->derr);
 }
 
 template <typename T>
 void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj, int* err) {
+  T* z3 = proj < 0 ? fs.Z4[3] : nullptr;  // no step uses d rho / dz (rho is advected in flux form)
   // tensor-core kernel (proj < 0, the derivative alone, exists only there)
   if ((h->tune_a < 0 || proj < 0) && h->N <= kTcMaxN) {
     const size_t sm = ((size_t)tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);
@@ -934,25 +935,25 @@ void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj, int* err) {
 #define IW_ATCASE(NT)                                                                                                   \
   case NT:                                                                                                              \
     k_stageA_t<T, NT><<<blocks, 512, sm, h->st>>>(geo(h), fs.F[0], fs.F[1], fs.F[2], fs.F[3], fs.F1[0], fs.F1[1],       \
-                                                  fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], fs.Z4[3], proj,     \
+                                                  fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], z3, proj,     \
                                                   err);                                                             \
     return;
     switch (tc_nt(h->N)) { IW_ATCASE(2) IW_ATCASE(3) IW_ATCASE(4) IW_ATCASE(5) }
 #undef IW_ATCASE
   }
   switch (h->tune_a == 0 ? 0 : zop_bucket(h->N)) {
-    case 9: launch_stageA_r<T, 9>(h, fs, proj); return;
-    case 17: launch_stageA_r<T, 17>(h, fs, proj); return;
-    case 21: launch_stageA_r<T, 21>(h, fs, proj); return;
-    case 25: launch_stageA_r<T, 25>(h, fs, proj); return;
-    case 29: launch_stageA_r<T, 29>(h, fs, proj); return;
-    case 33: launch_stageA_r<T, 33>(h, fs, proj); return;
+    case 9: launch_stageA_r<T, 9>(h, fs, proj, z3); return;
+    case 17: launch_stageA_r<T, 17>(h, fs, proj, z3); return;
+    case 21: launch_stageA_r<T, 21>(h, fs, proj, z3); return;
+    case 25: launch_stageA_r<T, 25>(h, fs, proj, z3); return;
+    case 29: launch_stageA_r<T, 29>(h, fs, proj, z3); return;
+    case 33: launch_stageA_r<T, 33>(h, fs, proj, z3); return;
     default: break;
   }
   dim3 grid((unsigned)((h->nxpp + kTX - 1) / kTX), (unsigned)(h->ny * h->ns), 4);
   size_t smem = (size_t)(h->N * h->N + h->N * kTX) * sizeof(T);
   k_stageA<T><<<grid, kTX * kTW, smem, h->st>>>(geo(h), fs.F[0], fs.F[1], fs.F[2], fs.F[3], fs.F1[0], fs.F1[1],
-                                                fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], fs.Z4[3], proj,
+                                                fs.F1[2], fs.F1[3], fs.Z4[0], fs.Z4[1], fs.Z4[2], z3, proj,
                                                 h->derr);
 }
 
@@ -1138,8 +1139,36 @@ static int legspec_dump(iw_handle* h, FieldSet<T>& fs);
 template <typename T>
 static int postp_step(iw_handle* h, FieldSet<T>& fs);
 
-// K_C: x rows (k_xrow_nl), one CTA per (y, z) row with 256 threads, or 128
-// when the autotuner measured that faster (tune_xthr)
+// K_C for the lengths of k_xrow_reg; false for any other
+template <typename T>
+static bool launch_xrow_reg(iw_handle* h, FieldSet<T>& fs, const NLArgs<T>& a) {
+  switch (h->nx / 2) {
+#define IW_XREG(R0, NB)                                                                                          \
+  case R0 * NB: {                                                                                                \
+    typedef XReg<T, R0, NB> X;                                                                                   \
+    cudaFuncSetAttribute(k_xrow_reg<T, R0, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X::smem);     \
+    k_xrow_reg<T, R0, NB><<<dim3((h->ny + X::YR - 1) / X::YR, h->nz), X::threads, X::smem, h->st>>>(geo(h), a, fs.Wm, \
+                                                                                                    fs.Wn);      \
+    return true;                                                                                                 \
+  }
+    IW_XREG(2, 8)
+    IW_XREG(4, 8)
+    IW_XREG(6, 8)
+    IW_XREG(8, 8)
+    IW_XREG(10, 8)
+    IW_XREG(6, 16)
+    IW_XREG(8, 16)
+    IW_XREG(10, 16)
+    IW_XREG(6, 32)
+    IW_XREG(8, 32)
+    IW_XREG(10, 32)
+#undef IW_XREG
+    default: return false;
+  }
+}
+
+// K_C: x rows; of the other lengths one CTA per (y, z) row (k_xrow_nl) with 256 threads, or
+// 128 (short rows, or when the autotuner measured that faster, tune_xthr)
 template <typename T>
 void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
   typedef typename cplx_t<T>::type C;
@@ -1150,11 +1179,7 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
   {
     NLArgs<T> a;
     memset(&a, 0, sizeof a);
-    for (int q = 0; q < 4; ++q) {
-      a.in[q] = fs.Y12[q];       // u v w t
-      a.in[4 + q] = fs.Y12[4 + q];  // dy
-      a.in[8 + q] = fs.Y12[8 + q];  // dz
-    }
+    for (int q = 0; q < 10; ++q) a.in[q] = fs.Y12[q];  // u v w t | dy u v w | dz u v w
     for (int q = 0; q < 11; ++q) a.out[q] = fs.X11[q];
     const double bz = h->p.brunt;
     const double rg = -(h->p.rho0 * (bz * bz) / h->p.grav);
@@ -1178,19 +1203,16 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
       a.f_amp_r = (xa * um) * (-(1 / om)) * bz * bz * (h->p.rho0 / h->p.grav) * (um / zdim) * ph;
     }
     a.dx = (pi2_of(h) / (pi2_of(h) / h->p.xlen)) / h->nx;
-    const size_t smem = 20 * (size_t)xstride(M) * sizeof(C);
+    if (launch_xrow_reg<T>(h, fs, a)) return;
+    const size_t smem = 17 * (size_t)xstride(M) * sizeof(C);
     dim3 grid(h->ny, h->nz);
     const bool p2 = (M & (M - 1)) == 0;
-    switch (p2 && M >= 32 && M <= 512 ? M : 0) {  // compile-time plans for power-of-two lengths
+    switch (M) {  // compile-time plan
 #define IW_XCT(MC, D)                                                                                       \
   case MC:                                                                                                  \
     cudaFuncSetAttribute(k_xrow_nl<T, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     k_xrow_nl<T, D, true, MC><<<grid, xthr, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn);                     \
     goto xrow_done;
-      IW_XCT(32, 8)
-      IW_XCT(64, 8)
-      IW_XCT(128, 8)
-      IW_XCT(256, 8)
       IW_XCT(512, 16)
 #undef IW_XCT
       default: break;
@@ -1267,16 +1289,16 @@ static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj, int cols = 0) {
     int r = anim_dump<T>(h, fs);
     if (r) return r;
   }
-  // K_B: y-inverse of 12 arrays
+  // K_B: y-inverse of 10 arrays (rho is advected in flux form: none of its derivatives are needed)
   {
     YJobs<T> jb;
     memset(&jb, 0, sizeof jb);
-    for (int q = 0; q < 4; ++q) {
-      jb.j[q] = YJob<T>{fs.F1[q], nullptr, fs.Y12[q], 0};
+    for (int q = 0; q < 4; ++q) jb.j[q] = YJob<T>{fs.F1[q], nullptr, fs.Y12[q], 0};
+    for (int q = 0; q < 3; ++q) {
       jb.j[4 + q] = YJob<T>{fs.F1[q], nullptr, fs.Y12[4 + q], 1};
-      jb.j[8 + q] = YJob<T>{fs.Z4[q], nullptr, fs.Y12[8 + q], 0};
+      jb.j[7 + q] = YJob<T>{fs.Z4[q], nullptr, fs.Y12[7 + q], 0};
     }
-    launch_y<T>(h, fs, jb, 12, h->nz, false);
+    launch_y<T>(h, fs, jb, 10, h->nz, false);
   }
   mark(h, 1);
   // K_C
@@ -1818,7 +1840,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
     return ms;
   };
   const int save[4] = {h->tune_ytx, h->tune_a, h->tune_e, h->use_sys};
-  // y tiles: the 12-job inverse and the 4-job forward-with-fold launches
+  // y tiles: the 10-job inverse and the 4-job forward-with-fold launches
   float best = 1e30f;
   int besttx = 8;
   for (int tx : {8, 4, 2}) {
@@ -1828,9 +1850,9 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
       YJobs<T> ji, jf;
       memset(&ji, 0, sizeof ji);
       memset(&jf, 0, sizeof jf);
-      for (int q = 0; q < 11; ++q) ji.j[q] = YJob<T>{fs.Y12[q], nullptr, fs.X11[q], q < 4 ? 0 : 1};
+      for (int q = 0; q < 10; ++q) ji.j[q] = YJob<T>{fs.Y12[q], nullptr, fs.X11[q], q < 7 ? 0 : 1};
       for (int q = 0; q < 4; ++q) jf.j[q] = YJob<T>{fs.X11[q], fs.X11[4 + q], fs.B8[4 + q], 3};
-      launch_y<T>(h, ts, ji, 11, h->nz, false);
+      launch_y<T>(h, ts, ji, 10, h->nz, false);
       launch_y<T>(h, ts, jf, 4, h->nz, true);
     });
     if (ms < best) {

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kTX* kTW) k_stageA(Geo g, const T* __restrict_
     tile[k * kTX + lane] = x;
   }
   __syncthreads();
-  if (!act) return;
+  if (!act || Z == nullptr) return;
   const T fac = (T)g.hfac[ks];
   for (int k1 = w; k1 < N; k1 += kTW) {
     const T* dr = sD + k1 * N;
@@ -487,7 +487,7 @@ __device__ __forceinline__ C xfwd_post(const C* Z, int k, int M, const C* __rest
 // Parameters of the fused NL row kernel.
 template <typename T>
 struct NLArgs {
-  const T* in[12];  // (kx,y): u v w t | dy u v w t | dz u v w t
+  const T* in[10];  // (kx,y): u v w t | dy u v w | dz u v w
   T* out[11];       // (kx,y): Au Av Aw At | uv vv vw vt | uw ww wt
   double coef_buoy; // N^2 / rhograd
   double rg;        // rhograd
@@ -544,7 +544,7 @@ __device__ __forceinline__ C xfwd_post_p(const C* row, int k, int M, const C* __
 // slots per padded x row (M+1 half-complex values)
 __host__ __device__ __forceinline__ int xstride(int M) { return fpadlen(M + 1); }
 
-// K_C: CTA per (j,k) row; 20 padded rows of M+1 values in shared memory; each
+// K_C: CTA per (j,k) row; 17 padded rows of M+1 values in shared memory; each
 // warp transforms whole rows in place.
 template <typename T, int DPT, bool POW2, int MC = 0>
 __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo g, NLArgs<T> a, FftPlan pl,
@@ -561,22 +561,22 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
   const bool nb_lo = (kl == 0 && k > 0);
   const bool nb_hi = (kl == N - 1 && k < g.nz - 1);
   const int knb = nb_lo ? k - 1 : k + 1;
-  const int nrow = 16 + ((nb_lo || nb_hi) ? 4 : 0);
+  const int nrow = 13 + ((nb_lo || nb_hi) ? 4 : 0);
   const T kxs = (T)g.xw[1];
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
-  // rows 0..3 u v w t, 4..7 dx, 8..11 dy, 12..15 dz, 16..19 neighbour u v w t:
+  // rows 0..3 u v w t, 4..6 dx of u v w, 7..9 dy, 10..12 dz, 13..16 neighbour u v w t:
   // half-complex rows (M+1 values), all copies in flight at once
   // Element offsets of this (j, k) row and of the neighbour's, once per CTA.
   // A thread keeps its kk and walks the rows (fixed strides, no index
   // arithmetic per copy); kk = M, the last value of a row, goes to thread r.
   const size_t roff = fidx<T>(g, 0, j, k), roffn = fidx<T>(g, 0, j, knb);
   auto rsrc = [&](int r) -> const C* {
-    return (const C*)((r < 4 ? a.in[r] : r < 16 ? a.in[r - 4] : a.in[r - 16]) + (r < 16 ? roff : roffn));
+    return (const C*)((r < 4 ? a.in[r] : r < 7 ? a.in[r - 4] : r < 13 ? a.in[r - 3] : a.in[r - 13]) + (r < 13 ? roff : roffn));
   };
   for (int kk = tid; kk < M; kk += nthr) {
     C* d = buf + fpad(kk);
 #pragma unroll
-    for (int r = 0; r < 20; ++r)
+    for (int r = 0; r < 17; ++r)
       if (r < nrow) cp_async_c<C>(d + r * RS, rsrc(r) + kk);
   }
   if (tid < nrow) cp_async_c<C>(buf + tid * RS + fpad(M), rsrc(tid) + M);
@@ -588,12 +588,12 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
     // a thread keeps its pair kk < M/2 and steps over rows by nthr/(M/2);
     // the middle pair kk = M/2 goes to thread r
     const int kk = tid % H2, rs = nthr / H2;
-    for (int r = tid / H2; r < nrow; r += rs) xprep_pair<C, T>(buf + r * RS, kk, M, Wn, r >= 4 && r < 8, kxs);
-    if (tid < nrow) xprep_pair<C, T>(buf + tid * RS, H2, M, Wn, tid >= 4 && tid < 8, kxs);
+    for (int r = tid / H2; r < nrow; r += rs) xprep_pair<C, T>(buf + r * RS, kk, M, Wn, r >= 4 && r < 7, kxs);
+    if (tid < nrow) xprep_pair<C, T>(buf + tid * RS, H2, M, Wn, tid >= 4 && tid < 7, kxs);
   } else {
     for (int q = tid; q < nrow * nh; q += nthr) {
       const int r = q / nh, kk = q - r * nh;
-      xprep_pair<C, T>(buf + r * RS, kk, M, Wn, r >= 4 && r < 8, kxs);
+      xprep_pair<C, T>(buf + r * RS, kk, M, Wn, r >= 4 && r < 7, kxs);
     }
   }
   __syncthreads();
@@ -615,25 +615,25 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
   for (int i = tid; i < nx; i += nthr) {
     const T u = P(0, i), v = P(1, i), w = P(2, i), t = P(3, i);
     const T ux = P(4, i), vx = P(5, i), wx = P(6, i);
-    const T uy = P(8, i), vy = P(9, i), wy = P(10, i);
-    const T uz = P(12, i), vz = P(13, i), wz = P(14, i);
+    const T uy = P(7, i), vy = P(8, i), wy = P(9, i);
+    const T uz = P(10, i), vz = P(11, i), wz = P(12, i);
     T qu = (T)-0.5 * (u * ux + v * uy + w * uz);
     T qv = (T)-0.5 * (u * vx + v * vy + w * vz);
     T qw = (T)-0.5 * (u * wx + v * wy + w * wz) + (T)a.coef_buoy * t;
     T qt = -(w * (T)a.rg);
     if (nb_lo && w > (T)0) {  // bottom point of subdomain ks: inflow from below
       const T tau = (T)a.tau_pen[ks], al = w;
-      qu -= tau * (al * u - al * P(16, i));
-      qv -= tau * (al * v - al * P(17, i));
-      qw -= tau * (al * w - al * P(18, i));
-      qt -= tau * (al * t - al * P(19, i));
+      qu -= tau * (al * u - al * P(13, i));
+      qv -= tau * (al * v - al * P(14, i));
+      qw -= tau * (al * w - al * P(15, i));
+      qt -= tau * (al * t - al * P(16, i));
     }
     if (nb_hi && w < (T)0) {
       const T tau = (T)a.tau_pen[ks], ga = -w;
-      qu -= tau * (ga * u - ga * P(16, i));
-      qv -= tau * (ga * v - ga * P(17, i));
-      qw -= tau * (ga * w - ga * P(18, i));
-      qt -= tau * (ga * t - ga * P(19, i));
+      qu -= tau * (ga * u - ga * P(13, i));
+      qv -= tau * (ga * v - ga * P(14, i));
+      qw -= tau * (ga * w - ga * P(15, i));
+      qt -= tau * (ga * t - ga * P(16, i));
     }
     if (a.forcing == IW_PADDLE_ALL_LEVELS || (a.forcing == IW_PADDLE_ABOVE_BOTTOM && k > 0)) {
       double xx = (double)i * a.dx, zz = g.zg[k];
@@ -691,6 +691,327 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
     for (int o = 0; o < 11; ++o) *((C*)(a.out[o] + roff) + kk) = outv(o, kk);
   }
   if (tid < 11) *((C*)(a.out[tid] + roff) + M) = outv(tid, M);
+}
+
+// K_C for complex lengths M = R0 NB with R0 in {2, 4, 6, 8, 10} and NB in {8, 16, 32}, i.e.
+// the plan R0 * (NB / 2) * 2: each value passes through shared memory four times per
+// transform pair of passes less than in k_xrow_nl, which is bound by that traffic.
+//   1. A lane loads the spectrum of butterflies it and NB - it of a row's first pass
+//      (their R0 values each are each other's mirror images k, M - k), so the pre-pass of the
+//      real transform and the radix-R0 pass run in registers; a warp holds 64 / NB rows.
+//   2. The middle pass (radix NB / 2) in place, still within the warp.
+//   3. The last inverse pass (radix 2), the products and the first forward pass in
+//      registers: a thread owns values p and p + M/2 of all 13 rows.
+//   4. The forward middle pass, then the last pass (radix R0) of butterflies it and NB - it
+//      with the post-pass of the real transform, the i kx fold of the advective form and the
+//      stores, in registers.  The fold needs rows Q_q and u q at once: they sit in the two
+//      halves of a warp.
+// Lane it = 0 has the two butterflies 0 and NB / 2, which are their own mirror images: its
+// pairs are regrouped with selects, the middle value k = M/2 is one extra value E.
+// Measured (x rows of one step, against k_xrow_nl on the same 13 + 4 rows): XROWFIG
+// Place of value i of a row: padded (FP32), or exchanged within groups of 8 (FP64, whose 16-byte
+// values meet in 8 banks: strides 2, 8 and 16 then fall in different ones, and no space is lost).
+template <typename C>
+__device__ __forceinline__ int xpos(int i) {
+  return sizeof(C) == 16 ? i ^ ((i >> 3) & 7) : fpad(i);
+}
+template <typename T, int R0, int NB>
+struct XReg {
+  static constexpr int M = R0 * NB, RM = NB / 2, I = NB / 2, G = 32 / I, YR = G / 2;
+  static constexpr int threads = 16 * R0;  // = YR M / 2
+  static constexpr int RS = sizeof(T) == 8 ? M : M + (M - 1) / 16;
+  static constexpr size_t smem = (size_t)17 * YR * RS * 2 * sizeof(T);
+  static constexpr int ctas = (sizeof(T) == 4 ? 512 : R0 < 6 ? 256 : 384) / threads;
+};
+
+// Radix-R pass (output stride NS before it) over the first lim of the G rows at base, all
+// lanes of a warp.
+template <typename C, int M, int R, int NS, int G, bool INV>
+__device__ __forceinline__ void xreg_pass(C* base, int RS, int lim, const C* __restrict__ W, int lane) {
+  constexpr int nb = M / R, RPI = 32 / nb, NIT = G / RPI;  // rows at a time, rounds
+  constexpr int CV = sizeof(C) == 8 ? 16 : 8, CH = CV / R < 1 ? 1 : CV / R < NIT ? CV / R : NIT;
+  constexpr int step = M / (NS * R);
+  static_assert(nb <= 32 && G % RPI == 0 && NIT % CH == 0, "rows do not divide");
+  const int g = lane / nb, j = lane % nb, jq = j / NS, jm = j % NS;
+  if (RPI * nb < 32 && g >= RPI) lim = 0;  // idle lanes
+  C* row = base + g * RS;
+#pragma unroll 1
+  for (int c = 0; c < NIT; c += CH, row += CH * RPI * RS) {
+    C v[CH][R];
+    if (g + c * RPI < lim) {
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (q == 0 || g + (c + q) * RPI < lim) v[q][r] = row[q * RPI * RS + xpos<C>(j + r * nb)];
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        C tw = W[r * jm * step];
+        if (INV) tw.y = -tw.y;
+#pragma unroll
+        for (int q = 0; q < CH; ++q) v[q][r] = cmul(v[q][r], tw);
+      }
+#pragma unroll
+      for (int q = 0; q < CH; ++q) dft_reg<C, R>(v[q], INV);
+    }
+    __syncwarp();
+    if (g + c * RPI < lim) {
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (q == 0 || g + (c + q) * RPI < lim) row[q * RPI * RS + xpos<C>(jq * NS * R + jm + r * NS)] = v[q][r];
+    }
+  }
+  __syncwarp();
+}
+
+template <typename T, int R0, int NB>
+__global__ void __launch_bounds__(XReg<T, R0, NB>::threads, (XReg<T, R0, NB>::ctas))
+    k_xrow_reg(Geo g, const __grid_constant__ NLArgs<T> a, const typename cplx_t<T>::type* __restrict__ Wm,
+               const typename cplx_t<T>::type* __restrict__ Wn) {
+  typedef typename cplx_t<T>::type C;
+  typedef XReg<T, R0, NB> X;
+  constexpr int M = X::M, I = X::I, G = X::G, YR = X::YR, RS = X::RS, RM = X::RM, H = R0 / 2, M2 = M / 2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* buf = (C*)smraw;
+  const int j0 = blockIdx.x * YR, k = blockIdx.y;
+  const int kl = k % g.N, ks = k / g.N;
+  const bool nb_lo = (kl == 0 && k > 0);
+  const bool nb_hi = (kl == g.N - 1 && k < g.nz - 1);
+  const int knb = nb_lo ? k - 1 : k + 1;
+  const T kxs = (T)g.xw[1];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr int nw = X::threads / 32;
+  const int gr = lane / I;
+  // rows (r, y): 0..3 u v w t, 4..6 dx of u v w, 7..9 dy, 10..12 dz, 13..16 neighbour u v w t
+  const int nrow = (13 + ((nb_lo || nb_hi) ? 4 : 0)) * YR;
+#pragma unroll 1
+  for (int g0 = wid * G; g0 < nrow; g0 += nw * G) {
+    int it = lane % I;
+    if (R0 >= 6) asm volatile("" : "+r"(it));  // what depends on it is not kept in registers across the rounds
+    const bool self = it == 0;
+    const int jb = self ? NB / 2 : NB - it;
+    // pair q of a lane: k = kq(q) and M - k
+    const int khi = self ? NB / 2 - NB * H : it;
+    auto kq = [&](int q) { return (q < H ? it : khi) + NB * q; };
+    const T fit = (T)it, fkhi = (T)khi;
+    auto fkq = [&](int q) { return (q < H ? fit : fkhi) + (T)(NB * q); };
+    const int row = g0 + gr, r = row / YR, jy = j0 + row % YR;
+    const bool act = row < nrow && jy < g.ny;
+    const bool dx = r >= 4 && r < 7;
+    C P[R0], Q[R0], E = cmk<C>(0, 0);
+    if (act) {
+      const T* f = a.in[r < 4 ? r : r < 7 ? r - 4 : r < 13 ? r - 3 : r - 13];
+      const C* src = (const C*)(f + fidx<T>(g, 0, jy, r < 13 ? k : knb));
+#pragma unroll
+      for (int q = 0; q < R0; ++q) {
+        P[q] = src[kq(q)];
+        Q[q] = src[M - kq(q)];
+      }
+      if (self) E = src[M2];
+    } else {
+#pragma unroll
+      for (int q = 0; q < R0; ++q) P[q] = Q[q] = cmk<C>(0, 0);
+    }
+#pragma unroll
+    for (int q = 0; q < R0; ++q) {
+      if (dx) {
+        const T ka = kxs * fkq(q), kb = kxs * ((T)M - fkq(q));
+        P[q] = cmk<C>(-(ka * P[q].y), ka * P[q].x);
+        Q[q] = cmk<C>(-(kb * Q[q].y), kb * Q[q].x);
+      }
+      if (q == 0 && self) P[0].y = Q[0].y = 0;
+      // Z_k = s + i t, Z_{M-k} = conj(s) + i conj(t); s = X_k + conj X_{M-k}, t = conj(W_k) (X_k - conj X_{M-k})
+      const C s = cadd(P[q], cconj(Q[q])), d = csub(P[q], cconj(Q[q]));
+      const C t = cmul(cconj(Wn[kq(q)]), d);
+      P[q] = cmk<C>(s.x - t.y, s.y + t.x);
+      Q[q] = cmk<C>(s.x + t.y, t.x - s.y);
+    }
+    if (dx) {
+      const T ke = kxs * (T)M2;
+      E = cmk<C>(-(ke * E.y), ke * E.x);
+    }
+    E = cmk<C>((T)2 * E.x, (T)-2 * E.y);  // k = M/2: 2 conj(X)
+    C va[R0], vb[R0];
+#pragma unroll
+    for (int q = 0; q < R0; ++q) {
+      va[q] = q < H ? P[q] : self ? (q == H ? E : Q[R0 - q]) : P[q];
+      vb[q] = self ? (q < H ? P[q + H] : Q[R0 - 1 - q + H]) : Q[R0 - 1 - q];
+    }
+    dft_reg<C, R0>(va, true);
+    dft_reg<C, R0>(vb, true);
+    C* rw = buf + (row < nrow ? row : 0) * RS;
+    if (row < nrow) {
+#pragma unroll
+      for (int q = 0; q < R0; ++q) {
+        rw[xpos<C>(it * R0 + q)] = va[q];
+        rw[xpos<C>(jb * R0 + q)] = vb[q];
+      }
+    }
+    __syncwarp();
+    xreg_pass<C, M, RM, R0, G, true>(buf + g0 * RS, RS, nrow - g0, Wm, lane);
+  }
+  __syncthreads();
+  const int p = tid % M2, yr = tid / M2;
+  // values 2p, 2p+1 (c = 0, 1 of element 0) and 2p+M, 2p+M+1 (element 1) of row r
+  const C *c0 = buf + yr * RS + xpos<C>(p), *c1 = buf + yr * RS + xpos<C>(p + M2);
+  C tw = Wm[p];
+  tw.y = -tw.y;
+  struct V {
+    C e[2];
+  };
+  auto get = [&](int r) {
+    V o;
+    o.e[0] = c0[r * YR * RS];
+    o.e[1] = cmul(c1[r * YR * RS], tw);
+    dft_reg<C, 2>(o.e, true);
+    return o;
+  };
+  auto put = [&](int r, V o) {
+    dft_reg<C, 2>(o.e, false);
+    C* d = buf + (r * YR + yr) * RS;
+    d[xpos<C>(2 * p)] = o.e[0];
+    d[xpos<C>(2 * p + 1)] = o.e[1];
+  };
+#define IW_V(o, expr)                                            \
+  _Pragma("unroll") for (int e = 0; e < 2; ++e) {                \
+    { T& o_ = o.e[e].x; const int c = 0; (void)c; o_ = (expr); } \
+    { T& o_ = o.e[e].y; const int c = 1; (void)c; o_ = (expr); } \
+  }
+#define IW_C(v) (c == 0 ? v.e[e].x : v.e[e].y)
+  V u = get(0), v = get(1), w = get(2), t = get(3);
+  V qu, qv, qw, qt;
+  {
+    const V ux = get(4), vx = get(5), wx = get(6);
+    IW_V(qu, IW_C(u) * IW_C(ux))
+    IW_V(qv, IW_C(u) * IW_C(vx))
+    IW_V(qw, IW_C(u) * IW_C(wx))
+    const V uy = get(7), vy = get(8), wy = get(9);
+    IW_V(qu, IW_C(qu) + IW_C(v) * IW_C(uy))
+    IW_V(qv, IW_C(qv) + IW_C(v) * IW_C(vy))
+    IW_V(qw, IW_C(qw) + IW_C(v) * IW_C(wy))
+    const V uz = get(10), vz = get(11), wz = get(12);
+    IW_V(qu, (T)-0.5 * (IW_C(qu) + IW_C(w) * IW_C(uz)))
+    IW_V(qv, (T)-0.5 * (IW_C(qv) + IW_C(w) * IW_C(vz)))
+    IW_V(qw, (T)-0.5 * (IW_C(qw) + IW_C(w) * IW_C(wz)) + (T)a.coef_buoy * IW_C(t))
+    IW_V(qt, -(IW_C(w) * (T)a.rg))
+  }
+  // upwind interface penalty (solver.f:700-839): inflow from below at the bottom point of
+  // subdomain ks, from above at its top point
+  if (nb_lo || nb_hi) {
+    const T tau = (T)a.tau_pen[ks];
+    V al;
+    IW_V(al, nb_lo ? (IW_C(w) > (T)0 ? IW_C(w) : (T)0) : (IW_C(w) < (T)0 ? -IW_C(w) : (T)0))
+    auto pen = [&](V& q, const V& f, int r) {
+      const V n = get(r);
+      IW_V(q, IW_C(al) != (T)0 ? IW_C(q) - tau * (IW_C(al) * IW_C(f) - IW_C(al) * IW_C(n)) : IW_C(q))
+    };
+    pen(qu, u, 13);
+    pen(qv, v, 14);
+    pen(qw, w, 15);
+    pen(qt, t, 16);
+  }
+  if (a.forcing == IW_PADDLE_ALL_LEVELS || (a.forcing == IW_PADDLE_ABOVE_BOTTOM && k > 0)) {
+    const double zz = g.zg[k], czm = cos(a.f_xm * zz), szm = sin(a.f_xm * zz);
+    double sf[2][2], cf[2][2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        sincos(a.f_xk * ((double)(2 * p + M * e + c) * a.dx) - a.f_om * a.f_t, &sf[e][c], &cf[e][c]);
+    IW_V(qu, IW_C(qu) + (T)(a.f_amp_u * czm * sf[e][c]))
+    IW_V(qw, IW_C(qw) + (T)(a.f_amp_w * szm * cf[e][c]))
+    IW_V(qt, IW_C(qt) + (T)(a.f_amp_r * szm * sf[e][c]))
+  }
+  __syncthreads();
+  // rows to transform: Qu uu Qv uv Qw uw Qt ut vv vw vt ww wt
+  {
+    V o;
+    put(0, qu);
+    put(2, qv);
+    put(4, qw);
+    put(6, qt);
+    IW_V(o, (T)-0.5 * IW_C(u) * IW_C(u)) put(1, o);
+    IW_V(o, (T)-0.5 * IW_C(u) * IW_C(v)) put(3, o);
+    IW_V(o, (T)-0.5 * IW_C(u) * IW_C(w)) put(5, o);
+    IW_V(o, -(IW_C(u) * IW_C(t))) put(7, o);
+    IW_V(o, (T)-0.5 * IW_C(v) * IW_C(v)) put(8, o);
+    IW_V(o, (T)-0.5 * IW_C(v) * IW_C(w)) put(9, o);
+    IW_V(o, -(IW_C(v) * IW_C(t))) put(10, o);
+    IW_V(o, (T)-0.5 * IW_C(w) * IW_C(w)) put(11, o);
+    IW_V(o, -(IW_C(w) * IW_C(t))) put(12, o);
+  }
+#undef IW_V
+#undef IW_C
+  __syncthreads();
+  const T hN = (T)0.5 / (T)(2 * M);
+#pragma unroll 1
+  for (int g0 = wid * G; g0 < 13 * YR; g0 += nw * G) {
+    int it = lane % I;
+    if (R0 >= 6) asm volatile("" : "+r"(it));  // what depends on it is not kept in registers across the rounds
+    const bool self = it == 0;
+    const int jb = self ? NB / 2 : NB - it;
+    // pair q of a lane: k = kq(q) and M - k
+    const int khi = self ? NB / 2 - NB * H : it;
+    auto kq = [&](int q) { return (q < H ? it : khi) + NB * q; };
+    const T fit = (T)it, fkhi = (T)khi;
+    auto fkq = [&](int q) { return (q < H ? fit : fkhi) + (T)(NB * q); };
+    xreg_pass<C, M, RM, 2, G, false>(buf + g0 * RS, RS, G, Wm, lane);  // (a last row pair may hold one unused row)
+    const int row = g0 + gr, r = row / YR, jy = j0 + row % YR;
+    const C* rw = buf + row * RS;
+    C va[R0], vb[R0];
+#pragma unroll
+    for (int q = 0; q < R0; ++q) {
+      va[q] = rw[xpos<C>(it + NB * q)];
+      vb[q] = rw[xpos<C>(jb + NB * q)];
+    }
+#pragma unroll
+    for (int q = 1; q < R0; ++q) {
+      // the twiddles of butterfly jb = NB - it are conj(W^(q it)) times the R0-th roots w^q, which
+      // shift its outputs by one place; butterfly 0 has none
+      const C tw = Wm[q * (self ? NB / 2 : it)];
+      va[q] = cmul(va[q], self ? cmk<C>(1, 0) : tw);
+      vb[q] = cmul(vb[q], cconj(tw));
+    }
+    dft_reg<C, R0>(va, false);
+    dft_reg<C, R0>(vb, false);
+    {
+      const C v0 = vb[0];
+#pragma unroll
+      for (int q = 0; q + 1 < R0; ++q) vb[q] = vb[q + 1];
+      vb[R0 - 1] = v0;
+    }
+    // X_k = e + W_k o, X_{M-k} = conj(e - W_k o); e = (Z_k + conj Z_{M-k}) / 2N,
+    // o = (Z_k - conj Z_{M-k}) / 2iN (k = 0: Z_M = Z_0; k = M/2: conj Z)
+    const bool fold = g0 < 8 * YR;  // r = 0..7: A_q = X(Q_q) + i kx X(u q)
+    const bool odd = lane >= 16;    // the row u q of a pair
+    const int dst = fold ? (odd ? (r == 3 ? 4 : r == 5 ? 8 : -1) : r >> 1)
+                         : r == 8 ? 5 : r == 9 ? 6 : r == 10 ? 7 : r == 11 ? 9 : r == 12 ? 10 : -1;
+    const bool act = dst >= 0 && jy < g.ny;
+    C* out = act ? (C*)(a.out[dst] + fidx<T>(g, 0, jy, k)) : nullptr;
+    auto emit = [&](C x, int kk, T fk, bool on) {
+      if (fold) {
+        C y;
+        y.x = __shfl_down_sync(0xffffffffu, x.x, 16);
+        y.y = __shfl_down_sync(0xffffffffu, x.y, 16);
+        const T kx = kxs * fk;
+        if (!odd) x = cmk<C>(x.x - kx * y.y, x.y + kx * y.x);
+      }
+      if (on && act) out[kk] = x;
+    };
+#pragma unroll
+    for (int q = 0; q < R0; ++q) {
+      const C A = q < H ? va[q] : self ? vb[q - H] : va[q];
+      const C B = cconj(self ? (q == 0 ? va[0] : q < H ? va[R0 - q] : vb[R0 - 1 - q + H]) : vb[R0 - 1 - q]);
+      const C e = cmk<C>(hN * (A.x + B.x), hN * (A.y + B.y));
+      const C o = cmul(Wn[kq(q)], cmk<C>(hN * (A.y - B.y), -(hN * (A.x - B.x))));
+      emit(cadd(e, o), kq(q), fkq(q), true);
+      emit(cconj(csub(e, o)), M - kq(q), (T)M - fkq(q), true);
+    }
+    emit(cmk<C>((T)2 * hN * va[H].x, (T)-2 * hN * va[H].y), M2, (T)M2, self);
+    __syncwarp();
+  }
 }
 
 // ===========================================================================
@@ -904,6 +1225,7 @@ __global__ void __launch_bounds__(128) k_stageA_r(Geo g, const __grid_constant__
     }
   }
   if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
+  if (Z == nullptr) return;
   const T fac = (T)g.hfac[ks];
 #pragma unroll
   for (int k1 = 0; k1 < NM; ++k1) {
@@ -3563,7 +3885,7 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
     const size_t k0 = (size_t)(ks * N) * pl;
     const T* F = (q == 0 ? F0 : q == 1 ? F1_ : q == 2 ? F2_ : F3_) + k0;
     T* O = (q == 0 ? O0 : q == 1 ? O1 : q == 2 ? O2 : O3) + k0;
-    T* Z = (q == 0 ? Z0 : q == 1 ? Z1 : q == 2 ? Z2 : Z3) + k0;
+    T* Z = q == 0 ? Z0 : q == 1 ? Z1 : q == 2 ? Z2 : Z3;
     const double fac = g.hfac[ks];
     // the projection changes the kx = 0 and Nyquist columns
     const bool special = (proj > 0 && (i < 2 || i >= nx)) || (proj >= 0 && q == 2 && tt < 2);
@@ -3596,9 +3918,10 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
         for (int kt = 0; kt < 2 * NT; ++kt, o += pl4)
           if (in(4 * kt + lt, 4 * kt + 3)) *o = x[kt];
       }
+      if (Z == nullptr) return;
       double acc[1][NT][2], none[1][2];
       tc_product<NT, 1, false>(sD, AP, N, lg, lt, [&](int, int kt) { return (double)x[kt]; }, acc, nullptr, none);
-      T* z = Z + tt + (size_t)(2 * lt) * pl;
+      T* z = Z + k0 + tt + (size_t)(2 * lt) * pl;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt, z += pl8)
 #pragma unroll
