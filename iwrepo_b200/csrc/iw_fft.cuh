@@ -293,12 +293,19 @@ __device__ C* fft_run(C* a, C* b, const FftPlan& pl, int nbatch, const C* W, boo
 // no second buffer and no CTA-wide barrier.  DPT >= M/32 values per lane.
 // ---------------------------------------------------------------------------
 __host__ __device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }
+// Place of value i under layout L: 0 is fpad; 2 pads by two, so that values 64 apart lie half the
+// banks apart; 1 also exchanges neighbours in the second half of each 16, so that two values 8 apart
+// differ in parity (with an even column stride: neither those nor adjacent rows of 8 columns collide).
+template <int L>
+__host__ __device__ __forceinline__ int flay(int i) {
+  return L == 0 ? fpad(i) : (L == 1 ? i ^ ((i >> 3) & 1) : i) + 2 * (i >> 4);
+}
 // slots needed for L padded values
 __host__ __device__ __forceinline__ int fpadlen(int L) { return L > 0 ? fpad(L - 1) + 1 : 0; }
 
 // One pass over the butterflies of G rows (RS values apart) at once: short rows share
 // the warp's lanes.  G M / R <= 32 IT.
-template <typename C, int R, int IT>
+template <typename C, int R, int IT, int L>
 __device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns, float inb, float ins,
                                            const C* __restrict__ W, bool inv, int lane) {
   const int nb = M / R;
@@ -311,7 +318,7 @@ __device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns
       const int g = (int)(((float)it + 0.5f) * inb), j = it - g * nb;
       const C* row = base + g * RS;
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[q][r] = row[fpad(j + r * nb)];
+      for (int r = 0; r < R; ++r) v[q][r] = row[flay<L>(j + r * nb)];
       if (Ns > 1) {
         const int jm = j - (int)(((float)j + 0.5f) * ins) * Ns, e = jm * step;
 #pragma unroll
@@ -334,7 +341,7 @@ __device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns
       C* row = base + g * RS;
       const int b0 = jq * Ns * R + jm;
 #pragma unroll
-      for (int r = 0; r < R; ++r) row[fpad(b0 + r * Ns)] = v[q][r];
+      for (int r = 0; r < R; ++r) row[flay<L>(b0 + r * Ns)] = v[q][r];
     }
   }
   __syncwarp();
@@ -346,24 +353,24 @@ __host__ __device__ constexpr int fft_rows_of(int M, int DPT) { return 32 * DPT 
 // In-place transform of G <= fft_rows_of(M, DPT) padded rows by one warp (all lanes
 // call it).  POW2: the length is a power of two, so only radix 8, 4, 2 passes are
 // compiled (every compiled radix raises the register count of the kernel).
-template <typename C, int DPT, bool POW2>
+template <typename C, int DPT, bool POW2, int L = 0>
 __device__ __forceinline__ void fft_warp(C* base, int RS, int G, const FftPlan& pl, const C* __restrict__ W, bool inv,
                                          int lane) {
   for (int p = 0; p < pl.npass; ++p) {
     const int Ns = pl.ns[p];
     const float ib = pl.inb[p], is = pl.ins[p];
     switch (pl.rad[p]) {
-      case 8: fft_pass_w<C, 8, (DPT + 7) / 8>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
-      case 4: fft_pass_w<C, 4, (DPT + 3) / 4>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
-      case 2: fft_pass_w<C, 2, (DPT + 1) / 2>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
+      case 8: fft_pass_w<C, 8, (DPT + 7) / 8, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
+      case 4: fft_pass_w<C, 4, (DPT + 3) / 4, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
+      case 2: fft_pass_w<C, 2, (DPT + 1) / 2, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
       default:
         if (!POW2) {
           if (pl.rad[p] == 3)
-            fft_pass_w<C, 3, (DPT + 2) / 3>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+            fft_pass_w<C, 3, (DPT + 2) / 3, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
           else if (pl.rad[p] == 6)
-            fft_pass_w<C, 6, (DPT + 5) / 6>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+            fft_pass_w<C, 6, (DPT + 5) / 6, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
           else
-            fft_pass_w<C, 5, (DPT + 4) / 5>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+            fft_pass_w<C, 5, (DPT + 4) / 5, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
         }
         break;
     }
@@ -398,7 +405,7 @@ struct CtRows {
   static constexpr int DPT = M <= 256 ? 8 : M / 32;
   static constexpr int G = fft_rows_of(M, DPT);
 };
-template <typename C, int M, int R, int NS>
+template <typename C, int M, int R, int NS, int L>
 __device__ __forceinline__ void fft_pass_ct(C* base, int RS, int G, const C* __restrict__ W, bool inv, int lane) {
   constexpr int nb = M / R;
   constexpr int step = M / (NS * R);
@@ -413,7 +420,7 @@ __device__ __forceinline__ void fft_pass_ct(C* base, int RS, int G, const C* __r
       const C* row = base + g * RS;
       const int jm = j & (NS - 1);
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[q][r] = row[fpad(j + r * nb)];
+      for (int r = 0; r < R; ++r) v[q][r] = row[flay<L>(j + r * nb)];
       if (NS > 1) {
         const int e = jm * step;
 #pragma unroll
@@ -436,26 +443,26 @@ __device__ __forceinline__ void fft_pass_ct(C* base, int RS, int G, const C* __r
       const int jq = j / NS, jm = j & (NS - 1);
       const int b0 = jq * NS * R + jm;
 #pragma unroll
-      for (int r = 0; r < R; ++r) row[fpad(b0 + r * NS)] = v[q][r];
+      for (int r = 0; r < R; ++r) row[flay<L>(b0 + r * NS)] = v[q][r];
     }
   }
   __syncwarp();
 }
 
 // Passes P .. PEND-1 (the first or last pass may run elsewhere) of G <= CtRows<M>::G rows.
-template <typename C, int M, int P, int PEND, int NS>
+template <typename C, int M, int P, int PEND, int NS, int L = 0>
 __device__ __forceinline__ void fft_passes_ct(C* base, int RS, int G, const C* __restrict__ W, bool inv, int lane) {
   if constexpr (P < PEND) {
     constexpr int R = 1 << CtPlan<M>::bits(P);
-    fft_pass_ct<C, M, R, NS>(base, RS, G, W, inv, lane);
-    fft_passes_ct<C, M, P + 1, PEND, NS * R>(base, RS, G, W, inv, lane);
+    fft_pass_ct<C, M, R, NS, L>(base, RS, G, W, inv, lane);
+    fft_passes_ct<C, M, P + 1, PEND, NS * R, L>(base, RS, G, W, inv, lane);
   }
 }
 
 // In-place transform of G <= CtRows<M>::G padded rows of power-of-two length M by one warp.
-template <typename C, int M>
+template <typename C, int M, int L = 0>
 __device__ __forceinline__ void fft_warp_ct(C* base, int RS, int G, const C* __restrict__ W, bool inv, int lane) {
-  fft_passes_ct<C, M, 0, CtPlan<M>::np, 1>(base, RS, G, W, inv, lane);
+  fft_passes_ct<C, M, 0, CtPlan<M>::np, 1, L>(base, RS, G, W, inv, lane);
 }
 
 }  // namespace iw

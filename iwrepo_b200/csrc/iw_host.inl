@@ -1025,11 +1025,15 @@ static int fft_dpt(int M) {
 }
 
 template <typename T>
+static int ystride_of(int ny, int tx) {
+  return tx == 16 ? YLay<T, 16>::stride(ny) : tx == 8 ? YLay<T, 8>::stride(ny) : ystride(ny);
+}
+template <typename T>
 static int ytx(const iw_handle* h, bool two) {  // y-FFT tile width
   const size_t cs = 2 * sizeof(T);
   int tx = h->tune_ytx > 0 ? h->tune_ytx : 8;
   if (tx == 8 && h->ny <= 128) tx = 16;  // two short columns per warp
-  while (tx > 1 && (two ? 2 : 1) * (size_t)tx * ystride(h->ny) * cs > 110 * 1024) tx /= 2;
+  while (tx > 1 && (two ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * cs > 110 * 1024) tx /= 2;
   return tx;
 }
 
@@ -1097,7 +1101,7 @@ void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int npla
   const int tx = ytx<T>(h, four);
   const int ntile = (h->nxhp + tx - 1) / tx;
   dim3 grid(ntile, nplanes, njobs);
-  const size_t smem = (four ? 2 : 1) * (size_t)tx * ystride(h->ny) * sizeof(C);
+  const size_t smem = (four ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * sizeof(C);
   switch (tx) {
     case 16: launch_y_tx<T, 16>(h, jobs, grid, smem, nplanes, fs.Wy); break;
     case 8: launch_y_tx<T, 8>(h, jobs, grid, smem, nplanes, fs.Wy); break;

@@ -236,13 +236,29 @@ __host__ __device__ __forceinline__ int ystride(int ny) {
   return s + ((2 - s) % 16 + 16) % 16;
 }
 
+// Layout of a tile of TX columns: 16 FP32 values or 8 FP64 values meet per access, so 8 columns of
+// FP32 meet with two rows each (layout 1, stride 2 mod 16), every other wide tile with one (odd
+// stride).  Against layout 0 and stride 2 throughout: YLAYFIG
+template <typename T, int TX>
+struct YLay {
+  static constexpr int L = TX < 8 || sizeof(T) == 8 ? 0 : TX == 8 ? 1 : 2;
+  static constexpr int JP = L == 0 ? 1 : 2;  // pad slots per 16 rows
+  __host__ __device__ static int stride(int ny) {
+    if (TX < 8) return ystride(ny);
+    const int s = flay<L == 0 ? 0 : 2>((ny - 1) | 1) + 1, want = sizeof(T) == 4 && TX == 8 ? 2 : 1;
+    return s + ((want - s) % 16 + 16) % 16;
+  }
+};
+
 template <typename T, int TX, int DPT, bool POW2, int MC = 0>
 __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
                                               const typename cplx_t<T>::type* __restrict__ Wy) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ny = MC > 0 ? MC : g.ny;  // a constant with a compile-time plan
-  const int RSY = ystride(ny);
+  typedef YLay<T, TX> Y;
+  constexpr int YL = Y::L;
+  const int RSY = Y::stride(ny);
   C* A = (C*)smraw;
   C* A2 = A + (size_t)TX * RSY;
   const YJob<T> jb = jobs.j[blockIdx.z];
@@ -251,7 +267,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
   const bool fwd = jb.mode >= 2;
   const bool two = jb.mode == 3;
   (void)nplanes;
-  // load: column ii0+b, row j -> A[b*RSY + fpad(j)] (all copies in flight at once).
+  // load: column ii0+b, row j -> A[b*RSY + flay<YL>(j)] (all copies in flight at once).
   // With 256 threads and TX | 256 a thread keeps its column b and steps j by
   // JS = 256/TX, so both addresses advance by fixed strides.
   constexpr int JS = 256 / TX;
@@ -308,16 +324,16 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
           dft_reg<C, R0>(w, !fwd);
           const int b0 = (tj + JS * mb) * R0;
 #pragma unroll
-          for (int r = 0; r < R0; ++r) row[fpad(b0 + r)] = w[r];
+          for (int r = 0; r < R0; ++r) row[flay<YL>(b0 + r)] = w[r];
         }
       } else {
 #pragma unroll
-        for (int it = 0; it < NIT; ++it) row[fpad(tj) + it * (JS + JS / 16)] = v[it];
+        for (int it = 0; it < NIT; ++it) row[flay<YL>(tj) + it * (JS + Y::JP * (JS / 16))] = v[it];
       }
     }
   } else if (mulky) {
     const size_t g0 = fidx<T>(g, 2 * iit, tj, k);
-    C* d = A + tb * RSY + fpad(tj);
+    C* d = A + tb * RSY + flay<YL>(tj);
     const C* s1 = (const C*)(jb.src + g0);
     C v[kyload ? MC / JS : 1];
 #pragma unroll
@@ -326,11 +342,11 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
 #pragma unroll
     for (int it = 0; it < (kyload ? MC / JS : 1); ++it) {
       const T ky = (T)g.yw[tj + it * JS];
-      d[it * (JS + JS / 16)] = cmk<C>(-(ky * v[it].y), ky * v[it].x);
+      d[it * (JS + Y::JP * (JS / 16))] = cmk<C>(-(ky * v[it].y), ky * v[it].x);
     }
   } else {
     const size_t g0 = fidx<T>(g, 2 * iit, tj, k);
-    C* d = A + tb * RSY + fpad(tj);
+    C* d = A + tb * RSY + flay<YL>(tj);
     const C* s1 = (const C*)(jb.src + g0);
     const C* s2 = two ? (const C*)(jb.src2 + g0) : s1;
     for (int j = tj; j < ny; j += JS) {
@@ -341,7 +357,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
         *d = cmk<C>(0, 0);
         if (two) d[TX * RSY] = cmk<C>(0, 0);
       }
-      d += JS + JS / 16;
+      d += JS + Y::JP * (JS / 16);
       s1 = (const C*)((const T*)s1 + gstep);
       s2 = (const C*)((const T*)s2 + gstep);
     }
@@ -352,7 +368,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
     for (int t = threadIdx.x; t < TX * ny; t += blockDim.x) {
       const int b = t % TX, j = t / TX;
       const T ky = (T)g.yw[j];
-      C* d = A + b * RSY + fpad(j);
+      C* d = A + b * RSY + flay<YL>(j);
       const C v = *d;
       *d = cmk<C>(-(ky * v.y), ky * v.x);
     }
@@ -370,13 +386,13 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
       C* row = (q < ng ? A : A2) + r * RSY;
       const int G = min(gb, nb - r);
       if constexpr (fuseL)  // the first pass ran at load, the last runs at the store
-        fft_passes_ct<C, (MC > 0 ? MC : 2), 1, NPS - 1, R0>(row, RSY, G, Wy, !fwd, lane);
+        fft_passes_ct<C, (MC > 0 ? MC : 2), 1, NPS - 1, R0, YL>(row, RSY, G, Wy, !fwd, lane);
       else if constexpr (fuse1)
-        fft_passes_ct<C, (MC > 0 ? MC : 2), 1, NPS, R0>(row, RSY, G, Wy, !fwd, lane);  // the first pass ran at load
+        fft_passes_ct<C, (MC > 0 ? MC : 2), 1, NPS, R0, YL>(row, RSY, G, Wy, !fwd, lane);  // the first pass ran at load
       else if constexpr (MC > 0)
-        fft_warp_ct<C, MC>(row, RSY, G, Wy, !fwd, lane);
+        fft_warp_ct<C, MC, YL>(row, RSY, G, Wy, !fwd, lane);
       else
-        fft_warp<C, DPT, POW2>(row, RSY, G, pl, Wy, !fwd, lane);
+        fft_warp<C, DPT, POW2, YL>(row, RSY, G, pl, Wy, !fwd, lane);
     }
   }
   __syncthreads();
@@ -394,8 +410,8 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
       C va[RL], vb[RL];
 #pragma unroll
       for (int r = 0; r < RL; ++r) {
-        va[r] = ra[fpad(j + r * NSL)];
-        if (two) vb[r] = rb[fpad(j + r * NSL)];
+        va[r] = ra[flay<YL>(j + r * NSL)];
+        if (two) vb[r] = rb[flay<YL>(j + r * NSL)];
       }
       if (tr) {
 #pragma unroll
@@ -423,7 +439,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
     return;
   }
   if (colok) {
-    const C* d = A + tb * RSY + fpad(tj);
+    const C* d = A + tb * RSY + flay<YL>(tj);
     C* o1 = (C*)(jb.dst + fidx<T>(g, 2 * iit, tj, k));
     for (int j = tj; j < ny; j += JS) {
       const C v = *d;
@@ -435,7 +451,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
         o = cmk<C>(o.x - ky * w2.y, o.y + ky * w2.x);
       }
       *o1 = o;
-      d += JS + JS / 16;
+      d += JS + Y::JP * (JS / 16);
       o1 = (C*)((T*)o1 + gstep);
     }
   }
