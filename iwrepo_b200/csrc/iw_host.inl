@@ -1037,7 +1037,7 @@ static int ytx(const iw_handle* h, bool two) {  // y-FFT tile width
   return tx;
 }
 
-template <typename T, int TX>
+template <typename T, int TX, bool TWO>
 static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, int nplanes,
                         const typename cplx_t<T>::type* Wy) {
   Geo g = geo(h);
@@ -1046,8 +1046,8 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
     switch (p2 ? h->ny : 0) {
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
-    cudaFuncSetAttribute(k_yfft<T, TX, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    k_yfft<T, TX, D, true, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+    cudaFuncSetAttribute(k_yfft<T, TX, D, true, TWO, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     return;
       IW_YCT(64, 8)
       IW_YCT(128, 8)
@@ -1059,8 +1059,8 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
     switch (p2 ? h->ny : 0) {
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
-    cudaFuncSetAttribute(k_yfft<T, TX, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    k_yfft<T, TX, D, true, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+    cudaFuncSetAttribute(k_yfft<T, TX, D, true, TWO, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     return;
       IW_YCT(256, 8)
       IW_YCT(512, 16)
@@ -1071,8 +1071,8 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
   switch (fft_dpt(h->ny) * (p2 ? 1 : -1)) {
 #define IW_YCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
-    cudaFuncSetAttribute(k_yfft<T, TX, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-    k_yfft<T, TX, D, P><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                          \
+    cudaFuncSetAttribute(k_yfft<T, TX, D, P, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
+    k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                          \
     break;
     IW_YCASE(8, true)
     IW_YCASE(8, false)
@@ -1102,12 +1102,16 @@ void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int npla
   const int ntile = (h->nxhp + tx - 1) / tx;
   dim3 grid(ntile, nplanes, njobs);
   const size_t smem = (four ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * sizeof(C);
-  switch (tx) {
-    case 16: launch_y_tx<T, 16>(h, jobs, grid, smem, nplanes, fs.Wy); break;
-    case 8: launch_y_tx<T, 8>(h, jobs, grid, smem, nplanes, fs.Wy); break;
-    case 4: launch_y_tx<T, 4>(h, jobs, grid, smem, nplanes, fs.Wy); break;
-    case 2: launch_y_tx<T, 2>(h, jobs, grid, smem, nplanes, fs.Wy); break;
-    default: launch_y_tx<T, 1>(h, jobs, grid, smem, nplanes, fs.Wy); break;
+  switch (four ? -tx : tx) {
+#define IW_YTX(TX)                                                                        \
+  case TX: launch_y_tx<T, TX, false>(h, jobs, grid, smem, nplanes, fs.Wy); break;         \
+  case -TX: launch_y_tx<T, TX, true>(h, jobs, grid, smem, nplanes, fs.Wy); break;
+    IW_YTX(16)
+    IW_YTX(8)
+    IW_YTX(4)
+    IW_YTX(2)
+    IW_YTX(1)
+#undef IW_YTX
   }
 }
 

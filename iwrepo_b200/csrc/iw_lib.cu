@@ -238,7 +238,8 @@ __host__ __device__ __forceinline__ int ystride(int ny) {
 
 // Layout of a tile of TX columns: 16 FP32 values or 8 FP64 values meet per access, so 8 columns of
 // FP32 meet with two rows each (layout 1, stride 2 mod 16), every other wide tile with one (odd
-// stride).  Against layout 0 and stride 2 throughout: YLAYFIG
+// stride).  Against layout 0 and stride 2 throughoutthe y
+// transforms of 256^2 x 200 FP64 take 605 + 626 there and 561 + 579 us here.
 template <typename T, int TX>
 struct YLay {
   static constexpr int L = TX < 8 || sizeof(T) == 8 ? 0 : TX == 8 ? 1 : 2;
@@ -250,8 +251,17 @@ struct YLay {
   }
 };
 
-template <typename T, int TX, int DPT, bool POW2, int MC = 0>
-__global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
+// CTAs per SM: a single transform of a long column of the compile-time plans gains from a third CTA
+// (80 registers: 512^2 x 396 FP32 inverse 2.43 -> 2.13 ms, 256^2 x 200 FP64 561 -> 499 us); two
+// transforms (mode 3) lose by it (2.69 -> 2.94 ms, 580 -> 643 us with the other four).
+template <typename T, int DPT, bool POW2, int MC, bool TWO>
+struct YOcc {
+  static constexpr int v = !TWO && MC > 0 && MC * (int)sizeof(T) >= 2048 && MC <= 512 && FftOcc<T, DPT, POW2>::v == 2
+                               ? 3
+                               : FftOcc<T, DPT, POW2>::v;
+};
+template <typename T, int TX, int DPT, bool POW2, bool TWO, int MC = 0>
+__global__ void __launch_bounds__(256, (YOcc<T, DPT, POW2, MC, TWO>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
                                               const typename cplx_t<T>::type* __restrict__ Wy) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -265,7 +275,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_yfft(Geo g, 
   const int k = blockIdx.y;
   const int ii0 = blockIdx.x * TX;
   const bool fwd = jb.mode >= 2;
-  const bool two = jb.mode == 3;
+  constexpr bool two = TWO;  // mode 3
   (void)nplanes;
   // load: column ii0+b, row j -> A[b*RSY + flay<YL>(j)] (all copies in flight at once).
   // With 256 threads and TX | 256 a thread keeps its column b and steps j by
