@@ -412,6 +412,8 @@ struct iw_handle {
   int nb = 0;
   int bmap[IW_MAX_SUBD] = {};
   // launch choices set by iw_autotune (0 / -1: built-in heuristic)
+  cudaStream_t st2 = nullptr;  // side branch of a step (side_fork)
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int tune_ytx = 0;  // y-tile width
   int tune_xthr = 0;  // threads per x-row CTA: 256 or 128, 0: by length
   int tune_a = -1;   // stage A: 1 register-column, 0 tiled
@@ -439,6 +441,26 @@ struct iw_handle {
 
 // phases: 0 stageA, 1 yinv, 2 xrow, 3 yfwd, 4 wviscrot, 5 stageE, 6 press,
 // 7 visc_uv, 8 visc_w, 9 visc_t, 10 iface, 11 factor
+// Work beside the handle's stream: what is launched on the stream that side_fork returns is ordered
+// after all work before it and, from side_join on, before all work after it (in a capture, a
+// branch of the graph).  One stream while the phases are timed.
+static cudaStream_t side_fork(iw_handle* h) {
+  if (h->prof) return h->st;
+  cudaEventRecord(h->ev_fork, h->st);
+  cudaStreamWaitEvent(h->st2, h->ev_fork, 0);
+  return h->st2;
+}
+static void side_join(iw_handle* h) {
+  if (h->prof) return;
+  cudaEventRecord(h->ev_join, h->st2);
+  cudaStreamWaitEvent(h->st, h->ev_join, 0);
+}
+static void side_free(iw_handle* h) {  // the streams and their events
+  if (h->ev_fork) cudaEventDestroy(h->ev_fork);
+  if (h->ev_join) cudaEventDestroy(h->ev_join);
+  if (h->st2) cudaStreamDestroy(h->st2);
+  if (h->st) cudaStreamDestroy(h->st);
+}
 static void mark(iw_handle* h, int phase) {
   if (!h->prof || h->nev >= 32) return;
   cudaEventRecord(h->ev[h->nev], h->st);
@@ -1068,26 +1090,23 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
       default: break;
     }
   }
-  switch (fft_dpt(h->ny) * (p2 ? 1 : -1)) {
+  // narrow tiles serve long columns and the autotuner: one kernel for every radix
+  switch (fft_dpt(h->ny) * (p2 && TX >= 8 ? 1 : -1)) {
 #define IW_YCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
-    cudaFuncSetAttribute(k_yfft<T, TX, D, P, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-    k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                          \
+    if constexpr ((TX < 16 || D == 8) && (TX >= 8 || !P)) { /* 16 columns only for ny <= 128 */              \
+      cudaFuncSetAttribute(k_yfft<T, TX, D, P, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+    }                                                                                                        \
     break;
     IW_YCASE(8, true)
+    IW_YCASE(16, true)
+    IW_YCASE(32, true)
     IW_YCASE(8, false)
-    default: break;
-  }
-  if constexpr (TX < 16) {  // (16 columns only for ny <= 128)
-    switch (fft_dpt(h->ny) * (p2 ? 1 : -1)) {
-      IW_YCASE(16, true)
-      IW_YCASE(32, true)
-      IW_YCASE(16, false)
-      IW_YCASE(32, false)
-      default: break;
-    }
-  }
+    IW_YCASE(16, false)
+    IW_YCASE(32, false)
 #undef IW_YCASE
+  }
 }
 
 template <typename T>
@@ -1297,6 +1316,14 @@ static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj, int cols = 0) {
     int r = anim_dump<T>(h, fs);
     if (r) return r;
   }
+  // wall pressure BC term (before the histories rotate): a few columns' latency, beside the
+  // transforms, which it shares no output with; stage E overwrites its inputs and waits
+  auto wall_term = [&](cudaStream_t st) {
+    const dim3 wgrid((unsigned)((h->nxhp + 31) / 32), (unsigned)h->ny, 2);
+    k_wviscrot<T><<<wgrid, 192, 0, st>>>(g, fs.F1[0], fs.F1[1], fs.F1[2], fs.Fn[0], fs.Fn[1], fs.Fn[2], fs.Fnm[0],
+                                         fs.Fnm[1], fs.Fnm[2], h->c, h->p.xnu, h->dwvr);
+  };
+  if (!h->prof) wall_term(side_fork(h));
   // K_B: y-inverse of 10 arrays (rho is advected in flux form: none of its derivatives are needed)
   {
     YJobs<T> jb;
@@ -1328,13 +1355,10 @@ static int convec_impl(iw_handle* h, FieldSet<T>& fs, int proj, int cols = 0) {
     launch_y<T>(h, fs, jz, 4, h->nz, false);
   }
   mark(h, 3);
-  // wall pressure BC term (before the histories rotate)
-  {
-    const dim3 wgrid((unsigned)((h->nxhp + 31) / 32), (unsigned)h->ny, 2);
-    k_wviscrot<T><<<wgrid, 192, 0, h->st>>>(g, fs.F1[0], fs.F1[1], fs.F1[2], fs.Fn[0],
-                                                                      fs.Fn[1], fs.Fn[2], fs.Fnm[0], fs.Fnm[1],
-                                                                      fs.Fnm[2], h->c, h->p.xnu, h->dwvr);
-  }
+  if (h->prof)  // a phase of its own
+    wall_term(h->st);
+  else
+    side_join(h);
   mark(h, 4);
   // K_E
   launch_stageE<T>(h, fs, cols);
@@ -1600,7 +1624,13 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   const bool tc = us == 2;
   int nend = us ? std::max(h->nold[kind], nref) : nt;
   if (tc && tc_zero00(h, role) && h->ntask2[kind] > 0) nend = 0;
-  if (tc && !tc_done) launch_solve_tc<T>(h, fs, &role, 1, kstart, cols);
+  // the refined columns (a few long chains) beside the others, which they share nothing with
+  const bool beside = tc && !tc_done && nend > 0;
+  const cudaStream_t st = beside ? side_fork(h) : h->st;
+  auto main_part = [&]() {
+    if (tc && !tc_done) launch_solve_tc<T>(h, fs, &role, 1, kstart, cols);
+  };
+  if (!beside || h->prof) main_part();
   if (us && !tc && h->ntask2[kind] > 0) {
     const size_t smsys = sys_smem(h->nz, h->N, h->ns, h->nb, role == 3).total * sizeof(double);
     const int nthr = (h->nz + 31) / 32 * 32, nthr2 = (h->ns * ((h->N + 1) / 2) + 31) / 32 * 32;
@@ -1650,9 +1680,13 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
       else
         cp = 0;
     }
-    k_solve_cta<T, R><<<cnt, kSolveThreads, sm, h->st>>>(geo(h), b2, solve_tabs(h, kind), h->dtasks[kind] + t0, F0, F1,
+    k_solve_cta<T, R><<<cnt, kSolveThreads, sm, st>>>(geo(h), b2, solve_tabs(h, kind), h->dtasks[kind] + t0, F0, F1,
                                                           F2, S[role == 0 || role == 3 ? 0 : role + 1], S[1], cols, rd, role, cp, meanu, part == 0 ? 1 : 0, h->dDt, h->dD2t,
                                                           h->dLt, h->dzh, h->dwnl, h->dwvr, kstart);
+  }
+  if (beside && !h->prof) {
+    main_part();
+    side_join(h);
   }
 }
 
@@ -2168,7 +2202,11 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
   h->use_bi = prm->solver == 0 && d.nsubd <= 16;
   h->plx = make_plan(h->nx / 2);
   h->ply = make_plan(h->ny);
-  if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) {
+  if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&h->st2, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+    side_free(h);
     delete h;
     return set_err(IW_ERR_CUDA, "stream");
   }
@@ -2321,7 +2359,7 @@ int iw_destroy(iw_handle* h) {
     cudaFree(h->dpen[k]);
     cudaFree(h->dcolsys[k]);
   }
-  if (h->st) cudaStreamDestroy(h->st);
+  side_free(h);
   if (g_bound == h) g_bound = nullptr;
   delete h;
   return IW_OK;

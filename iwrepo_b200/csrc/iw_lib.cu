@@ -238,8 +238,8 @@ __host__ __device__ __forceinline__ int ystride(int ny) {
 
 // Layout of a tile of TX columns: 16 FP32 values or 8 FP64 values meet per access, so 8 columns of
 // FP32 meet with two rows each (layout 1, stride 2 mod 16), every other wide tile with one (odd
-// stride).  Against layout 0 and stride 2 throughoutthe y
-// transforms of 256^2 x 200 FP64 take 605 + 626 there and 561 + 579 us here.
+// stride).  With layout 0 and stride 2 throughout the y
+// transforms of 256^2 x 200 FP64 took 605 + 626 us, they take 561 + 579.
 template <typename T, int TX>
 struct YLay {
   static constexpr int L = TX < 8 || sizeof(T) == 8 ? 0 : TX == 8 ? 1 : 2;
