@@ -53,9 +53,12 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) {
       : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
   return d;
 }
+// a b + c, written out so that a product's rounding does not depend on what the compiler does around it
+__device__ __forceinline__ float cfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double cfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 template <typename C>
 __device__ __forceinline__ C cmul(C a, C b) {
-  return cmk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return cmk<C>(cfma(a.x, b.x, -(a.y * b.y)), cfma(a.x, b.y, a.y * b.x));
 }
 template <typename C>
 __device__ __forceinline__ C cconj(C a) {
@@ -98,7 +101,7 @@ struct FftPlan {
 template <typename C>
 __device__ __forceinline__ C crot(C v, decltype(C().x) c, decltype(C().x) s, bool inv) {
   const decltype(C().x) t = inv ? s : -s;
-  return cmk<C>(v.x * c - v.y * t, v.x * t + v.y * c);
+  return cmk<C>(cfma(v.x, c, -(v.y * t)), cfma(v.x, t, v.y * c));
 }
 
 // In-register DFT of v[0..R-1] (natural order in and out) for R = 2, 3, 4, 5, 6, 8,
@@ -135,8 +138,8 @@ __device__ __forceinline__ void dft5(C& a0, C& a1, C& a2, C& a3, C& a4, bool inv
   const C t1 = cadd(a1, a4), t2 = cadd(a2, a3), d1 = csub(a1, a4), d2 = csub(a2, a3);
   const C m1 = cmk<C>(a0.x + c1 * t1.x + c2 * t2.x, a0.y + c1 * t1.y + c2 * t2.y);
   const C m2 = cmk<C>(a0.x + c2 * t1.x + c1 * t2.x, a0.y + c2 * t1.y + c1 * t2.y);
-  const C n1 = cmul_mi(cmk<C>(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y), inv);
-  const C n2 = cmul_mi(cmk<C>(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y), inv);
+  const C n1 = cmul_mi(cmk<C>(cfma(s1, d1.x, s2 * d2.x), cfma(s1, d1.y, s2 * d2.y)), inv);
+  const C n2 = cmul_mi(cmk<C>(cfma(s2, d1.x, -(s1 * d2.x)), cfma(s2, d1.y, -(s1 * d2.y))), inv);
   a0 = cadd(a0, cadd(t1, t2));
   a1 = cadd(m1, n1);
   a4 = csub(m1, n1);
@@ -303,46 +306,63 @@ __host__ __device__ __forceinline__ int flay(int i) {
 // slots needed for L padded values
 __host__ __device__ __forceinline__ int fpadlen(int L) { return L > 0 ? fpad(L - 1) + 1 : 0; }
 
-// One pass over the butterflies of G rows (RS values apart) at once: short rows share
-// the warp's lanes.  G M / R <= 32 IT.
+// One pass over G rows, RS values apart: as many whole rows at a time as the warp's lanes hold
+// (M / R <= 32), or one row at a time in IT butterflies per lane (M / R <= 32 IT).  A lane keeps its
+// butterflies' indexes and twiddles over the rows.
 template <typename C, int R, int IT, int L>
 __device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns, float inb, float ins,
                                            const C* __restrict__ W, bool inv, int lane) {
-  const int nb = M / R;
-  const int step = M / (Ns * R), items = G * nb;
-  C v[IT][R];
+  const int nb = M / R, step = M / (Ns * R);
+  const int rpi = nb < 32 ? (int)(32.5f * inb) : 1;  // rows at a time
+  const int g = nb < 32 ? (int)(((float)lane + 0.5f) * inb) : 0, j0 = lane - g * nb;
+  const bool act = g < rpi;
+  // (values of idle lanes are set, or the compiler carries the registers of every radix through the
+  // loop over the passes)
+  C tw[IT][R];
+  int jq[IT], jm[IT];
 #pragma unroll
   for (int q = 0; q < IT; ++q) {
-    const int it = lane + 32 * q;
-    if (it < items) {
-      const int g = (int)(((float)it + 0.5f) * inb), j = it - g * nb;
-      const C* row = base + g * RS;
+    const int j = j0 + 32 * q;
+    jq[q] = (int)(((float)j + 0.5f) * ins);
+    jm[q] = j - jq[q] * Ns;
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[q][r] = row[flay<L>(j + r * nb)];
-      if (Ns > 1) {
-        const int jm = j - (int)(((float)j + 0.5f) * ins) * Ns, e = jm * step;
+    for (int r = 0; r < R; ++r) tw[q][r] = cmk<C>(1, 0);
+    if (Ns > 1 && (q == 0 || j < nb)) {
+      const int e = jm[q] * step;
 #pragma unroll
-        for (int r = 1; r < R; ++r) {
-          C tw = W[r * e];
-          if (inv) tw.y = -tw.y;
-          v[q][r] = cmul(v[q][r], tw);
-        }
+      for (int r = 1; r < R; ++r) {
+        tw[q][r] = W[r * e];
+        if (inv) tw[q][r].y = -tw[q][r].y;
       }
-      dft_reg<C, R>(v[q], inv);
     }
   }
-  __syncwarp();
+#pragma unroll 1
+  for (int r0 = 0; r0 < G; r0 += rpi) {
+    C* row = base + (r0 + g) * RS;
+    const bool on = act && r0 + g < G;
+    C v[IT][R];
 #pragma unroll
-  for (int q = 0; q < IT; ++q) {
-    const int it = lane + 32 * q;
-    if (it < items) {
-      const int g = (int)(((float)it + 0.5f) * inb), j = it - g * nb;
-      const int jq = (int)(((float)j + 0.5f) * ins), jm = j - jq * Ns;
-      C* row = base + g * RS;
-      const int b0 = jq * Ns * R + jm;
+    for (int q = 0; q < IT; ++q) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) row[flay<L>(b0 + r * Ns)] = v[q][r];
+      for (int r = 0; r < R; ++r) v[q][r] = cmk<C>(0, 0);
+      if (on && (q == 0 || j0 + 32 * q < nb)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[q][r] = row[flay<L>(j0 + 32 * q + r * nb)];
+        if (Ns > 1) {
+#pragma unroll
+          for (int r = 1; r < R; ++r) v[q][r] = cmul(v[q][r], tw[q][r]);
+        }
+        dft_reg<C, R>(v[q], inv);
+      }
     }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < IT; ++q)
+      if (on && (q == 0 || j0 + 32 * q < nb)) {
+        const int b0 = jq[q] * Ns * R + jm[q];
+#pragma unroll
+        for (int r = 0; r < R; ++r) row[flay<L>(b0 + r * Ns)] = v[q][r];
+      }
   }
   __syncwarp();
 }
@@ -350,8 +370,8 @@ __device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns
 // rows of length M that one warp transforms at a time with DPT values per lane
 __host__ __device__ constexpr int fft_rows_of(int M, int DPT) { return 32 * DPT / M > 1 ? 32 * DPT / M : 1; }
 
-// In-place transform of G <= fft_rows_of(M, DPT) padded rows by one warp (all lanes
-// call it).  POW2: the length is a power of two, so only radix 8, 4, 2 passes are
+// In-place transform of G padded rows of M <= 32 DPT values by one warp (all lanes call
+// it).  POW2: the length is a power of two, so only radix 8, 4, 2 passes are
 // compiled (every compiled radix raises the register count of the kernel).
 template <typename C, int DPT, bool POW2, int L = 0>
 __device__ __forceinline__ void fft_warp(C* base, int RS, int G, const FftPlan& pl, const C* __restrict__ W, bool inv,
@@ -381,8 +401,7 @@ __device__ __forceinline__ void fft_warp(C* base, int RS, int G, const FftPlan& 
 // kernels hold every radix and get more registers)
 template <typename T, int DPT, bool POW2 = true>
 struct FftOcc {
-  static constexpr int v0 = sizeof(T) == 4 ? (DPT <= 8 ? 4 : DPT <= 16 ? 2 : 1) : (DPT <= 4 ? 4 : DPT <= 8 ? 2 : 1);
-  static constexpr int v = POW2 || v0 < 4 ? v0 : 3;
+  static constexpr int v = sizeof(T) == 4 ? (DPT <= 8 ? (POW2 ? 4 : 3) : DPT <= 16 ? 2 : 1) : DPT <= 8 ? 2 : 1;
 };
 
 
@@ -415,6 +434,8 @@ __device__ __forceinline__ void fft_pass_ct(C* base, int RS, int G, const C* __r
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     const int it = lane + 32 * q;
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[q][r] = cmk<C>(0, 0);
     if ((CtRows<M>::G == 1 && nb % 32 == 0) || it < items) {
       const int g = CtRows<M>::G > 1 ? it / nb : 0, j = CtRows<M>::G > 1 ? it % nb : it;
       const C* row = base + g * RS;

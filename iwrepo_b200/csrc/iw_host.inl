@@ -1043,7 +1043,7 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
 // values per lane of a warp transform of length M
 static int fft_dpt(int M) {
   const int d = (M + 31) / 32;
-  return d <= 8 ? 8 : d <= 16 ? 16 : 32;
+  return d <= 4 ? 4 : d <= 8 ? 8 : d <= 16 ? 16 : 32;
 }
 
 template <typename T>
@@ -1094,14 +1094,16 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
   switch (fft_dpt(h->ny) * (p2 && TX >= 8 ? 1 : -1)) {
 #define IW_YCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
-    if constexpr ((TX < 16 || D == 8) && (TX >= 8 || !P)) { /* 16 columns only for ny <= 128 */              \
+    if constexpr ((TX < 16 || D == 4) && (TX >= 8 || !P)) { /* 16 columns only for ny <= 128 */              \
       cudaFuncSetAttribute(k_yfft<T, TX, D, P, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     }                                                                                                        \
     break;
+    IW_YCASE(4, true)
     IW_YCASE(8, true)
     IW_YCASE(16, true)
     IW_YCASE(32, true)
+    IW_YCASE(4, false)
     IW_YCASE(8, false)
     IW_YCASE(16, false)
     IW_YCASE(32, false)
@@ -1250,9 +1252,11 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
     cudaFuncSetAttribute(k_xrow_nl<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
     k_xrow_nl<T, D, P><<<grid, xthr, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn);                        \
     break;
+        IW_XCASE(4, true)
         IW_XCASE(8, true)
       IW_XCASE(16, true)
       IW_XCASE(32, true)
+        IW_XCASE(4, false)
         IW_XCASE(8, false)
       IW_XCASE(16, false)
       IW_XCASE(32, false)
@@ -1291,9 +1295,11 @@ void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, i
     cudaFuncSetAttribute(k_xrow_stats<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
     k_xrow_stats<T, D, P><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);        \
     break;
+    IW_SCASE(4, true)
     IW_SCASE(8, true)
     IW_SCASE(16, true)
     IW_SCASE(32, true)
+    IW_SCASE(4, false)
     IW_SCASE(8, false)
     IW_SCASE(16, false)
     IW_SCASE(32, false)

@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256, (YOcc<T, DPT, POW2, MC, TWO>::v)) k_yfft(
   // the x-Nyquist column (ii = nxh) is not transformed
   const int nb = ny > 1 ? max(0, min(TX, g.nxh - ii0)) : 0;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int gmax = MC > 0 ? CtRows<(MC > 0 ? MC : 2)>::G : fft_rows_of(ny, DPT);  // columns a warp takes at a time
+  const int gmax = MC > 0 ? CtRows<(MC > 0 ? MC : 2)>::G : nw * TX;  // columns a warp takes at a time
   const int gb = gmax > 1 ? max(1, min(gmax, ((two ? 2 : 1) * nb + nw - 1) / nw)) : 1;
   const int ng = gb > 1 ? (nb + gb - 1) / gb : nb;  // groups of gb columns
   {
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
     }
   }
   __syncthreads();
-  const int gmax = MC > 0 ? CtRows<(MC > 0 ? MC : 2)>::G : fft_rows_of(M, DPT);  // rows a warp takes at a time
+  const int gmax = MC > 0 ? CtRows<(MC > 0 ? MC : 2)>::G : 17;  // rows a warp takes at a time
   {
     const int gb = min(gmax, (nrow + nw - 1) / nw);
     for (int r = wid * gb; r < nrow; r += nw * gb) {
@@ -764,6 +764,10 @@ __device__ __forceinline__ void xreg_pass(C* base, int RS, int lim, const C* __r
 #pragma unroll 1
   for (int c = 0; c < NIT; c += CH, row += CH * RPI * RS) {
     C v[CH][R];
+#pragma unroll
+    for (int q = 0; q < CH; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[q][r] = cmk<C>(0, 0);  // (not carried from round to round)
     if (g + c * RPI < lim) {
 #pragma unroll
       for (int q = 0; q < CH; ++q)
