@@ -219,13 +219,13 @@ def run_reference(args, rank, world):
 
 # ----------------------------------------------------------------------
 PHASE_FIELDS = {  # algorithmic fields moved per launch (reads + writes of ntot-sized arrays)
-    "stageA": 12, "y_inverse": 20, "x_row_nl": 23, "y_forward": 19, "stageE": 40,
+    "stageA": 11, "y_inverse": 17, "x_row_nl": 21, "y_forward": 19, "stageE": 40,
     "pressure": 6, "solve_uv": 4, "solve_w": 2, "solve_rho": 2,
 }
 # kernels launched per step: stage A, y-inverse, x rows, 2 y-forward, wall BC,
-# stage E, pressure (2 when ill-conditioned systems get a residual sweep),
-# u/v, w, rho, interface averaging (2 gathers, 2 y transforms, rows, planes)
-LAUNCHES_PER_STEP = 18
+# stage E, pressure (2: ill-conditioned systems get a residual sweep beside it),
+# u/v with w and rho, interface averaging (2 gathers, 2 y transforms, rows, planes)
+LAUNCHES_PER_STEP = 16
 
 
 def dram_traffic(cfg, precision, phase):

@@ -301,10 +301,9 @@ int iw_run(iw_handle *h, int nsteps, int use_graph);
 int iw_autotune(iw_handle *h, int *choices);
 
 /* Not in the reference.  Sets one launch choice of iw_autotune directly. */
-#define IW_LAUNCH_YTILE 0   /* 0 (size heuristic), 2, 4 or 8 */
-#define IW_LAUNCH_STAGE_A 1 /* -1 (size heuristic), 0 tiled, 1 register-column */
-#define IW_LAUNCH_STAGE_E 2 /* as stage A, or 2: tiled, bulk-copied input tiles (N <= 33); 3: the same with
-                               its z operators in the constant bank */
+#define IW_LAUNCH_YTILE 0   /* columns per y tile: 0 (by size), 2, 4 or 8 (8 is 16 where ny <= 128) */
+#define IW_LAUNCH_STAGE_A 1 /* -1 (FP64 tensor cores, nzloc <= 40), 0 tiled, 1 register-column */
+#define IW_LAUNCH_STAGE_E 2 /* as stage A; 2 and 3 are the FP64 tensor cores too */
 #define IW_LAUNCH_SOLVE 3   /* 2 system-grouped on the FP64 tensor cores (default; 1 where it does not apply),
                                1 system-grouped on the FP64 pipes, 0 per task, 3 system-grouped with two rows
                                per thread (u/v, w, rho; the pressure takes 1).  All give the same bits. */
@@ -313,7 +312,8 @@ int iw_autotune(iw_handle *h, int *choices);
 #define IW_LAUNCH_SOLVE_W 5
 #define IW_LAUNCH_SOLVE_RHO 6
 #define IW_LAUNCH_SOLVE_PRESSURE 7
-#define IW_LAUNCH_XROW_THREADS 8 /* threads per x-row CTA: 256 (0 = default) or 128 */
+#define IW_LAUNCH_XROW_THREADS 8 /* threads per x-row CTA: 256 or 128 (0: by length); lengths nx/2 = R0 NB with
+                                    R0 2, 4, 6, 8, 10 and NB 8, 16, 32 have a kernel with its own number */
 int iw_set_launch(iw_handle *h, int which, int value);
 
 /* Not in the reference.  Reads one launch choice (the IW_LAUNCH_* ids), e.g.

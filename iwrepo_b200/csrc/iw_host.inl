@@ -416,8 +416,8 @@ struct iw_handle {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int tune_ytx = 0;  // y-tile width
   int tune_xthr = 0;  // threads per x-row CTA: 256 or 128, 0: by length
-  int tune_a = -1;   // stage A: 1 register-column, 0 tiled
-  int tune_e = -1;   // stage E: 1 register-column, 0 tiled, 2 tiled with bulk-copied tiles
+  int tune_a = -1;   // stage A: -1 tensor cores, 1 register-column, 0 tiled
+  int tune_e = -1;   // stage E: -1, 2, 3 tensor cores, 1 register-column, 0 tiled
   int brep[IW_MAX_SUBD] = {};
   double bi_dt[SYS_KINDS] = {-1, -1, -1, -1};
   double fac_bdfv[SYS_KINDS] = {-1, -1, -1, -1};  // bdfv the factors were built for
@@ -1054,8 +1054,8 @@ template <typename T>
 static int ytx(const iw_handle* h, bool two) {  // y-FFT tile width
   const size_t cs = 2 * sizeof(T);
   int tx = h->tune_ytx > 0 ? h->tune_ytx : 8;
-  if (tx == 8 && h->ny <= 128) tx = 16;  // two short columns per warp
-  while (tx > 1 && (two ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * cs > 110 * 1024) tx /= 2;
+  if (tx == 8 && h->ny <= 128) tx = 16;  // short columns share warps (y kernels of 64^2 x 68 FP64: 76 -> 63 us)
+  while (tx > 2 && (two ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * cs > 110 * 1024) tx /= 2;
   return tx;
 }
 
@@ -1130,8 +1130,7 @@ void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int npla
     IW_YTX(16)
     IW_YTX(8)
     IW_YTX(4)
-    IW_YTX(2)
-    IW_YTX(1)
+    IW_YTX(2)  // (two columns of ny <= 1024 always fit)
 #undef IW_YTX
   }
 }

@@ -2,21 +2,22 @@
 // Legendre multidomain penalty z) and its C ABI (include/iw_b200.h).
 //
 // One step (main.f:653-1066) on device-resident fields:
-//   K_A  k_stageA(_r)  maxcalc/convec round-trip projection, w mean = 0,
-//                      z-derivatives of u,v,w,rho                   (z columns)
-//   K_B  k_yfft        y-inverse of u,v,w,rho, dz, and i ky (.)      (planes)
-//   K_C  k_xrow_nl     x-inverse of 16 rows -> skew-symmetric products,
-//                      buoyancy, upwind interface penalty, paddle ->
-//                      x-forward with i kx folded in                 (rows)
-//   K_D  k_yfft        y-forward with i ky folded in                 (planes)
-//   K_E  k_stageE(_r)  S = B + dz(Z), SS extrapolation, BDF u*, history,
-//                      Fourier x Legendre filter (k_stageE_f32: the
-//                      tiled kernel for FP32 fields)                 (z columns)
-//        k_wviscrot    rotational viscous pressure BC                (walls)
-//   K_F  k_solve_cta   pressure Poisson (divergence, solve, filter, projection)
-//        k_solve_cta   u,v / w / rho Helmholtz solves, filters, mean mode
-//                      (block inverses; k_press_g / k_visc with the band LU
-//                      when the handle asks for the reference's LU)
+//   K_A  k_stageA_t    maxcalc/convec round-trip projection, w mean = 0, z-derivatives of
+//                      u, v, w on the FP64 tensor cores (k_stageA_r, k_stageA: FMA pipes)  (z columns)
+//   K_B  k_yfft        y-inverse of u,v,w,rho, dz(u,v,w), and i ky (u,v,w)      (planes)
+//   K_C  k_xrow_reg    x-inverse of 13 rows -> skew-symmetric products, buoyancy, upwind
+//                      interface penalty, paddle -> x-forward with i kx folded in
+//                      (k_xrow_nl: lengths it does not cover)                   (rows)
+//   K_D  k_yfft        y-forward with i ky folded in                            (planes)
+//        k_wviscrot    rotational viscous pressure BC, beside K_B..K_D          (walls)
+//   K_E  k_stageE_t    S = B + dz(Z), SS extrapolation, BDF u*, history, Fourier x Legendre
+//                      filter on the FP64 tensor cores (k_stageE_r, k_stageE_f32, k_stageE:
+//                      FMA pipes)                                               (z columns)
+//   K_F  k_press_tc    pressure Poisson (divergence, solve, filter, projection), with the
+//                      refined columns in k_solve_cta beside it
+//        k_solve_tc    u,v / w / rho Helmholtz solves, filters, mean mode, one launch
+//                      (other variants: k_solve_sys, k_solve_sys2, k_solve_cta; k_press_g /
+//                      k_visc with the band LU when the handle asks for the reference's LU)
 //   K_H  interface averaging: planes next to interfaces go to physical space,
 //        the averaging change comes back; every plane gets the spectral effect
 //        of the round trip.
@@ -734,7 +735,14 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
 //      halves of a warp.
 // Lane it = 0 has the two butterflies 0 and NB / 2, which are their own mirror images: its
 // pairs are regrouped with selects, the middle value k = M/2 is one extra value E.
-// Measured (x rows of one step, against k_xrow_nl on the same 13 + 4 rows): XROWFIG
+// Measured against k_xrow_nl (which then also carried the three rows of d rho): 512^2 x 396 FP32
+// 5.56 -> 3.39 ms, 256^2 x 200 FP64 1.96 -> 0.96 ms, 192 x 120 x 110 FP32 401 -> 123 us, 64^2 x 68 FP64
+// 83 -> 29 us.  At 512^2 it moves its 21 fields at 2.6 TB/s, bound by instruction issue (2.6 per cycle)
+// and in FP64 by the L1 data path (twiddles and rows, 62 %).
+// Threads per SM: 512 in FP32 (128 registers; with 640 a thread of R0 = 8 spills: 3.39 -> 3.94 ms),
+// 384 in FP64 (168 registers: 1.02 against 1.05 ms with 256), but 256 for R0 < 6, whose rows are so
+// short that loads in flight count (64^2: 29 against 38 us).  From R0 = 6 on the indexes and twiddles
+// of a lane are made anew in every round; kept over the rounds they cost spills (3.70 -> 4.65 ms).
 // Place of value i of a row: padded (FP32), or exchanged within groups of 8 (FP64, whose 16-byte
 // values meet in 8 banks: strides 2, 8 and 16 then fall in different ones, and no space is lost).
 template <typename C>
@@ -819,7 +827,7 @@ __global__ void __launch_bounds__(XReg<T, R0, NB>::threads, (XReg<T, R0, NB>::ct
 #pragma unroll 1
   for (int g0 = wid * G; g0 < nrow; g0 += nw * G) {
     int it = lane % I;
-    if (R0 >= 6) asm volatile("" : "+r"(it));  // what depends on it is not kept in registers across the rounds
+    if (R0 >= 6) asm volatile("" : "+r"(it));  // (not kept over the rounds)
     const bool self = it == 0;
     const int jb = self ? NB / 2 : NB - it;
     // pair q of a lane: k = kq(q) and M - k
@@ -979,7 +987,7 @@ __global__ void __launch_bounds__(XReg<T, R0, NB>::threads, (XReg<T, R0, NB>::ct
 #pragma unroll 1
   for (int g0 = wid * G; g0 < 13 * YR; g0 += nw * G) {
     int it = lane % I;
-    if (R0 >= 6) asm volatile("" : "+r"(it));  // what depends on it is not kept in registers across the rounds
+    if (R0 >= 6) asm volatile("" : "+r"(it));  // (not kept over the rounds)
     const bool self = it == 0;
     const int jb = self ? NB / 2 : NB - it;
     // pair q of a lane: k = kq(q) and M - k
