@@ -952,7 +952,7 @@ void launch_stageA(iw_handle* h, FieldSet<T>& fs, int proj, int* err) {
   T* z3 = proj < 0 ? fs.Z4[3] : nullptr;  // no step uses d rho / dz (rho is advected in flux form)
   // tensor-core kernel (proj < 0, the derivative alone, exists only there)
   if ((h->tune_a < 0 || proj < 0) && h->N <= kTcMaxN) {
-    const size_t sm = ((size_t)tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);
+    const size_t sm = (size_t)tc_op_doubles(h->N) * sizeof(double);
     const int blocks = z_grid(h, 16, 2);
 #define IW_ATCASE(NT)                                                                                                   \
   case NT:                                                                                                              \
@@ -1001,7 +1001,7 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
   if (stageE_is_t(h)) {
     if (cols)
       for (int q = 0; q < 4; ++q) a.F[q] = fs.Y12[q];
-    const size_t ops = ((size_t)2 * tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);
+    const size_t ops = ((size_t)2 * tc_nc(h->N) * tc_ap(h->N) + 8) * sizeof(double);  // (the warps' tiles follow)
     const int W = (int)std::min<size_t>(sizeof(T) == 4 ? 20 : 16, (226 * 1024 - ops) / ze_buf<T>(h->N));
     const size_t sm = ops + (size_t)W * ze_buf<T>(h->N);
     const int blocks = z_grid(h, W, 1), v16 = (h->plane * sizeof(T)) % 16 == 0;

@@ -45,6 +45,7 @@
 
 #include "../../include/iw_b200.h"
 #include "iw_fft.cuh"
+#include "iw_layout.h"
 #include "iw_kernels.cuh"
 
 using namespace iw;
@@ -3267,14 +3268,6 @@ __global__ void __launch_bounds__(kSys2MaxThreads, 2) k_solve_sys2(
 // FP64-pipe kernels (a broadcast load per multiply-add): pressure 7.97 -> 4.17 ms,
 // u/v 3.04 -> 2.49, w 2.01 -> 1.32; 256^2 x (8 x 25) FP64: pressure 1.04 -> 0.47 ms.
 // ===========================================================================
-constexpr int kTcMaxN = 40;
-// Operator columns in shared memory are AP = 4 (mod 8) doubles apart: the 4
-// columns x 8 rows of a B fragment then fall in two shared-memory wavefronts.
-// They are padded to a multiple of 4 columns with zeros, so that no fragment
-// needs a bounds check.
-__host__ __device__ constexpr int tc_nt(int N) { return N <= 16 ? 2 : (N + 7) / 8; }
-__host__ __device__ constexpr int tc_ap(int N) { return ((N + 3) & ~7) + 4; }
-__host__ __device__ constexpr int tc_nc(int N) { return (N + 3) & ~3; }
 // Staged right-hand sides: [tile][row][8] values of T; of FP64 rows the halves
 // swap places on every other pair of rows, so that an A fragment (4 rows x 8)
 // has no bank conflicts (FP32 fragments are 32 consecutive words as they are).
