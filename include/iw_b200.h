@@ -348,6 +348,9 @@ int iw_field_ptr(iw_handle *h, int f, void **dptr);
 int iw_stream(iw_handle *h, void **stream);
 /* bytes of device memory held by the handle */
 int iw_device_bytes(iw_handle *h, size_t *bytes);
+/* Not in the reference.  For tests of the error paths: the nth device allocation of this handle from
+ * now on fails with IW_ERR_NOMEM (0: none).  A step that fails so leaves the handle as it was before it. */
+int iw_fail_allocation(iw_handle *h, int nth);
 
 /* Batched vertical penalty solves (one Helmholtz system per (kx,ky)
  * column), the isolated-solve workload: lambda = kx^2+ky^2 + c, BCs by the

@@ -24,7 +24,7 @@ PI = C.POINTER(C.c_int)
 EXPORTS = [
     "iw_init", "iw_destroy", "iw_last_error", "iw_last_status", "iw_upload_state", "iw_download_state", "iw_init_mode1",
     "iw_write_restart", "iw_read_restart", "iw_write_fields", "iw_wait_fields", "iw_set_animation", "iw_set_speclegen", "iw_postp", "iw_set_postp", "iw_step", "iw_run", "iw_ensemble_run", "iw_autotune", "iw_set_launch", "iw_get_launch", "iw_step_coefs", "iw_set_coefs", "iw_diag", "iw_sync", "iw_field_ptr", "iw_stream",
-    "iw_device_bytes", "iw_helm_solve_batched", "iw_bind", "iw_profile", "iw_profile_read", "iw_mean_profiles",
+    "iw_device_bytes", "iw_fail_allocation", "iw_helm_solve_batched", "iw_bind", "iw_profile", "iw_profile_read", "iw_mean_profiles",
     "horfft_", "dpdz_", "filter_3dlegenfourier_", "filter_legenpen_", "interface_avg3d_",
     "penalty_main_", "bandlu_solve_", "iw_bandlu_solve_noalloc", "penalty_setup_", "convec_", "calcuvwt_",
     "abvar1_", "abvar2_", "abvar3_", "bdfvarv_", "bdfvar1_", "bdfvar2_", "bdfvar3_", "iw_dt_rule",
@@ -75,6 +75,7 @@ def lib():
     L.iw_field_ptr.argtypes = [vp, C.c_int, C.POINTER(vp)]
     L.iw_stream.argtypes = [vp, C.POINTER(vp)]
     L.iw_device_bytes.argtypes = [vp, C.POINTER(C.c_size_t)]
+    L.iw_fail_allocation.argtypes = [vp, C.c_int]
     L.iw_helm_solve_batched.argtypes = [vp, vp, C.c_int, C.c_int, C.c_int, vp, vp, C.c_int]
     L.iw_bandlu_solve_noalloc.argtypes = [vp, vp, C.c_int, C.c_int, C.c_int, vp]
     L.iw_bind.argtypes = [vp]

@@ -386,8 +386,12 @@ struct iw_handle {
     int nsys_raw = 0;
     SysDesc* sys = 0;
     int* colsys = 0;
-    int nsys = 0;
+    void release() {
+      for (void* p : {ainv, (void*)minv, (void*)pen, (void*)lvec, (void*)ainv_raw, (void*)sys, (void*)colsys}) cudaFree(p);
+      *this = BI();
+    }
   } bi[SYS_KINDS];
+  int fail_alloc = 0;  // iw_fail_allocation: device allocations until one is refused
   bool use_bi = true;
   // grouped solve tasks per kind (columns sharing a system, <= G per task)
   Task* dtasks[SYS_KINDS] = {0, 0, 0, 0};
@@ -498,6 +502,8 @@ static cudaError_t scopy(iw_handle* h, void* dst, const void* src, size_t bytes,
 
 template <typename T>
 static int dalloc(iw_handle* h, T** p, size_t n) {
+  *p = nullptr;
+  if (h->fail_alloc > 0 && --h->fail_alloc == 0) return set_err(IW_ERR_NOMEM, "allocation refused (iw_fail_allocation)");
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T) + 16);
   if (e != cudaSuccess) return set_err(IW_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   h->bytes += n * sizeof(T);
@@ -507,7 +513,12 @@ template <typename T>
 static int up(iw_handle* h, T** p, const std::vector<T>& v) {
   int r = dalloc(h, p, v.size());
   if (r) return r;
-  CK(scopy(h, *p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  const cudaError_t e = scopy(h, *p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(*p);
+    *p = nullptr;
+    return set_err(IW_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
+  }
   return 0;
 }
 
@@ -580,7 +591,7 @@ static void free_fields(FieldSet<T>& fs) {
 // ---------------------------------------------------------------------------
 // systems: distinct kx^2+ky^2 (the matrix of a column depends on it only)
 // ---------------------------------------------------------------------------
-static void build_distinct(iw_handle* h) {
+static int build_distinct(iw_handle* h) {
   std::vector<double> ak(h->ncol);
   for (int j = 0; j < h->ny; ++j)
     for (int ii = 0; ii < h->nxhp; ++ii) {
@@ -603,8 +614,7 @@ static void build_distinct(iw_handle* h) {
   for (int c = 0; c < h->ncol; ++c) order[c] = c;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->col_u[a] < h->col_u[b]; });
   h->order = order;
-  up(h, &h->dcolorder, order);
-  up(h, &h->dakv, h->akv);
+  return up(h, &h->dcolorder, order) || up(h, &h->dakv, h->akv);
 }
 
 static int kind_bcs(const iw_handle* h, int kind, int& bot, int& top) {
@@ -637,9 +647,10 @@ static int build_tasks(iw_handle* h, int kind, const std::vector<int>& colsys, i
     tasks.push_back(Task{s, i, jn - i});
     i = jn;
   }
+  Task* d = nullptr;
+  if (up(h, &d, tasks)) return IW_ERR_NOMEM;
   cudaFree(h->dtasks[kind]);
-  h->dtasks[kind] = nullptr;
-  if (up(h, &h->dtasks[kind], tasks)) return IW_ERR_NOMEM;
+  h->dtasks[kind] = d;
   h->ntask[kind] = (int)tasks.size();
   h->htasks[kind] = tasks;
   return 0;
@@ -647,13 +658,13 @@ static int build_tasks(iw_handle* h, int kind, const std::vector<int>& colsys, i
 
 // tasks of k_solve_sys: after the k_solve_cta prefix (the refined tasks and
 // the columns without a system, which sort first), runs of the sorted column
-// order that share one system, in pieces of at most 4 (u/v) or 8 columns
-static int build_sys_tasks(iw_handle* h, int kind) {
+// order that share one system, in pieces of at most 4 (u/v) or 8 columns.  nrefine: the
+// refined tasks; the handle takes it and the tasks over together, or neither.
+static int build_sys_tasks(iw_handle* h, int kind, int nrefine) {
   const auto& tk = h->htasks[kind];
   const int skip = (kind == SYS_P || kind == SYS_W) && h->akv[0] == 0.0 ? 1 : 0;
-  int nold = h->nrefine[kind];
+  int nold = nrefine;
   while (nold < (int)tk.size() && tk[nold].sys < 0) ++nold;
-  h->nold[kind] = nold;
   const int G = kind == SYS_U ? kSysR / 4 : kSysR / 2;
   const std::vector<int>& order = h->order;
   std::vector<Task> tasks;
@@ -665,10 +676,13 @@ static int build_sys_tasks(iw_handle* h, int kind) {
     tasks.push_back(Task{s, i, jn - i});
     i = jn;
   }
+  Task* d = nullptr;
+  if (!tasks.empty() && up(h, &d, tasks)) return IW_ERR_NOMEM;
   cudaFree(h->dtasks2[kind]);
-  h->dtasks2[kind] = nullptr;
+  h->dtasks2[kind] = d;
   h->ntask2[kind] = (int)tasks.size();
-  if (!tasks.empty() && up(h, &h->dtasks2[kind], tasks)) return IW_ERR_NOMEM;
+  h->nold[kind] = nold;
+  h->nrefine[kind] = nrefine;
   return 0;
 }
 
@@ -818,7 +832,9 @@ static double cond_slope(const iw_handle* h) {
 
 // block inverses of one kind.  The systems of a kind are the distinct kx^2+ky^2 whatever
 // dt and bdfv are, so their number, the tables' memory, the column map and the tasks
-// are made once; a change of dt or bdfv is one kernel in stream order.
+// are made once; a change of dt or bdfv is one kernel in stream order.  Where an allocation
+// fails, the handle's sizes, lists and pointers stay those of what it has, and no table counts
+// as built, so that the next step builds them.
 static int build_blockinv(iw_handle* h, int kind, bool fold) {
   const int ns = h->ns, N = h->N, m = 2 * (ns - 1);
   const int skip = (kind == SYS_P || kind == SYS_W) && h->akv[0] == 0.0 ? 1 : 0;  // no system at k = 0
@@ -828,20 +844,25 @@ static int build_blockinv(iw_handle* h, int kind, bool fold) {
   const double facvel = 1. / (h->p.xnu * h->p.dt), fact = 1. / (h->p.xkappa * h->p.dt);
   const double c0 = kind == SYS_P ? 0.0 : kind == SYS_T ? h->c.bdfv * fact : h->c.bdfv * facvel;
   iw_handle::BI& B = h->bi[kind];
-  bool fresh = !B.colsys;
-  if (fresh) {
-    const size_t n1 = std::max(nsys, 1);
+  h->bi_dt[kind] = -1;
+  if (!B.colsys) {
+    const size_t n1 = std::max(nsys, 1), had = h->bytes;
+    iw_handle::BI nb;
     char* ai = nullptr;
     std::vector<int> colsys(h->ncol);
     for (int c = 0; c < h->ncol; ++c) colsys[c] = h->col_u[c] - skip;
     // (+16 bytes: k_solve_sys copies whole 16-byte units)
-    if (dalloc(h, &ai, n1 * h->nb * N * N * sizeof(double) + 16) || dalloc(h, &B.minv, n1 * std::max(m * m, 1)) ||
-        dalloc(h, &B.pen, n1 * 6 * ns) || dalloc(h, &B.sys, n1) || dalloc(h, &B.lvec, n1 * std::max(m, 1) * N))
+    const int r = dalloc(h, &ai, n1 * h->nb * N * N * sizeof(double) + 16) || dalloc(h, &nb.minv, n1 * std::max(m * m, 1)) ||
+                  dalloc(h, &nb.pen, n1 * 6 * ns) || dalloc(h, &nb.sys, n1) || dalloc(h, &nb.lvec, n1 * std::max(m, 1) * N) ||
+                  up(h, &nb.colsys, colsys) || build_tasks(h, kind, colsys, kind == SYS_U ? 1 : 2);
+    nb.ainv = ai;
+    if (r) {
+      nb.release();
+      h->bytes = had;
       return IW_ERR_NOMEM;
-    B.ainv = ai;
-    B.nsys = nsys;
-    if (build_tasks(h, kind, colsys, kind == SYS_U ? 1 : 2)) return IW_ERR_NOMEM;
-    if (up(h, &B.colsys, colsys)) return IW_ERR_NOMEM;
+    }
+    B = nb;
+    h->nrefine[kind] = -1;  // no list of tasks yet
   }
   // tasks [0, last] get a residual sweep: the systems above the condition bound
   const double rho = cond_slope(h);
@@ -851,15 +872,13 @@ static int build_blockinv(iw_handle* h, int kind, bool fold) {
     if (tk[t].sys >= 0 && 1.0 + 1. / (h->akv[tk[t].sys + skip] + c0) * rho > kRefineCond) last = t;
   if (fold)
     for (int t = 0; t <= last; ++t) nraw = std::max(nraw, tk[t].sys + 1);
-  if (fresh || h->nrefine[kind] != last + 1) {
-    h->nrefine[kind] = last + 1;
-    if (build_sys_tasks(h, kind)) return IW_ERR_NOMEM;
-  }
+  if (h->nrefine[kind] != last + 1 && build_sys_tasks(h, kind, last + 1)) return IW_ERR_NOMEM;
   if (B.nsys_raw != nraw) {
     cudaFree(B.ainv_raw);
     B.ainv_raw = nullptr;
-    B.nsys_raw = nraw;
+    B.nsys_raw = 0;
     if (nraw > 0 && dalloc(h, &B.ainv_raw, (size_t)nraw * h->nb * N * N)) return IW_ERR_NOMEM;
+    B.nsys_raw = nraw;
   }
   if (int r = build_systems(h, h->dakv + skip, nsys, c0, bot, top, fold, nraw, (double*)B.ainv, B.ainv_raw, B.lvec, B.minv,
                             B.pen, B.sys))
@@ -1831,7 +1850,11 @@ static int full_step(iw_handle* h, FieldSet<T>& fs) {
   }
   const int cpen = (h->p.ispecfilterexp == 1) && (h->istep % h->p.nspecfilterexp == 0);
   r = ensure_factors(h, cpen);
-  if (r) return r;
+  if (r) {  // nothing of the step ran
+    h->istep -= 1;
+    if (h->ivardt == 1) h->idtstep -= 1;
+    return r;
+  }
   const int cols = step_cols<T>(h, cpen);
   convec_impl<T>(h, fs, 1, cols);
   schedule_after_convec(h);
@@ -2291,11 +2314,11 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
     cudaMemset(h->dwvr, 0, h->plane * 2 * sizeof(double));
     r = h->mixed ? alloc_fields(h, h->f32) : alloc_fields(h, h->f64);
   }
+  if (!r) r = build_distinct(h);
   if (r) {
     iw_destroy(h);
     return IW_ERR_NOMEM;
   }
-  build_distinct(h);
   // distinct subdomain blocks of the penalty systems: a block is fixed by
   // epsilon, its height and whether it has neighbours below and above
   h->nb = 0;
@@ -2350,13 +2373,7 @@ int iw_destroy(iw_handle* h) {
   for (int k = 0; k < SYS_KINDS; ++k) {
     cudaFree(h->dtasks[k]);
     cudaFree(h->dtasks2[k]);
-    cudaFree(h->bi[k].ainv);
-    cudaFree(h->bi[k].minv);
-    cudaFree(h->bi[k].pen);
-    cudaFree(h->bi[k].lvec);
-    cudaFree(h->bi[k].ainv_raw);
-    cudaFree(h->bi[k].sys);
-    cudaFree(h->bi[k].colsys);
+    h->bi[k].release();
     cudaFree(h->dab[k]);
     cudaFree(h->dipiv[k]);
     cudaFree(h->dinfo[k]);
@@ -2601,6 +2618,12 @@ int iw_field_ptr(iw_handle* h, int f, void** dptr) {
 int iw_stream(iw_handle* h, void** stream) {
   if (!h || !stream) return set_err(IW_ERR_STATE, "bad argument");
   *stream = (void*)h->st;
+  return IW_OK;
+}
+
+int iw_fail_allocation(iw_handle* h, int nth) {
+  if (!h || nth < 0) return set_err(IW_ERR_STATE, "bad argument");
+  h->fail_alloc = nth;
   return IW_OK;
 }
 
