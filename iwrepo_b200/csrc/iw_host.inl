@@ -1053,10 +1053,12 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
   }
   dim3 grid((unsigned)((h->nxpp + kTX - 1) / kTX), (unsigned)(h->ny * h->ns), 4);
   size_t smem = (size_t)h->N * h->N * sizeof(double) + (size_t)(h->N * h->N + 2 * h->N * kTX) * sizeof(T);
-  if constexpr (sizeof(T) == 4)
-    k_stageE_f32<<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c);
-  else
+  if constexpr (sizeof(T) == 4) {
+    k_stageE_f32<<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c);  // at most 39 KB
+  } else {
+    cudaFuncSetAttribute(k_stageE<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  // > 48 KB from N = 42 on
     k_stageE<T><<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c);
+  }
 }
 
 // values per lane of a warp transform of length M
@@ -2077,8 +2079,10 @@ static int capture_step(iw_handle* const* hs, int n, cudaStream_t s0, cudaGraphE
     if (ei != cudaSuccess) rc = set_err(IW_ERR_CUDA, std::string("graph instantiation failed: ") + cudaGetErrorString(ei));
   }
   if (g) cudaGraphDestroy(g);
-  if (rc != IW_OK)
+  if (rc != IW_OK) {
+    cudaGetLastError();  // reported here; the next call starts without it
     for (int i = 0; i < stepped; ++i) rotate_host(hs[i]);  // nothing ran: undo the host-side rotation
+  }
   cudaEventDestroy(fork);
   for (auto& ev : join) cudaEventDestroy(ev);
   return rc;
