@@ -3931,18 +3931,29 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
         x[kt] = (T)0;
         if (in(4 * kt + lt, 4 * kt + 3)) x[kt] = *f;
       }
+      // non-finite values are looked for after the projection, which drops the imaginary part of
+      // the x-Nyquist column (the derivative alone: in the raw values)
+      const bool pr = !PLAIN && special && proj > 0;
       bool bad = false;
+      if (!pr) {
 #pragma unroll
-      for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
-      if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
+        for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
+      }
       if (!PLAIN && special) {
         const bool wzero = q == 2 && tt < 2;
 #pragma unroll
         for (int kt = 0; kt < 2 * NT; ++kt) {
           const int r = 4 * kt + lt;
-          if (act && r < N) x[kt] = wzero ? (T)0 : proj_val<T>(g, F, i, j, r);
+          if (act && r < N) {
+            if (pr) {
+              x[kt] = proj_val<T>(g, F, i, j, r);
+              bad |= !isfinite(x[kt]);
+            }
+            if (wzero) x[kt] = (T)0;
+          }
         }
       }
+      if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
       if (proj >= 0) {
         T* o = O + tt + (size_t)lt * pl;
 #pragma unroll
