@@ -3107,16 +3107,23 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     CK(cudaGetLastError());
   }
   const int nc = tc ? hc.nlist : ncol;
-  const size_t sm32 = helm32_smem(n, N);
-  if (mode != 0 && sm32 <= 200 * 1024 && rhs != sol) {
+  const int warps = 4;
+  const size_t sm32 = helm32_smem(n, N), smem = (size_t)warps * 6 * n * sizeof(double);
+  // Mode 1 by the number of columns.  k_helm (a warp per column) is a short chain, k_helm32 (a lane per right-hand
+  // side) a two to five times longer one that the whole chip's columns share.  k_helm's columns come in waves of what is
+  // resident (two CTAs of four warps per SM, one where shared memory holds no more); from the second wave on the
+  // longer chain is the cheaper one, without its prefetch (N > 33) from the fourth.  Both give the same bits.
+  // us, k_helm / k_helm32, at 64, 1024 and 2048 columns (148 SMs: 1184 a wave): N = 9, ns = 12 165/243, 182/249, 326/257;
+  // N = 25, ns = 8 371/655, 403/672, 745/675; N = 33, ns = 12 749/1347, 808/1366, 1582/1401; at 1024, 3072 and 4096:
+  // N = 36, ns = 4 330/1034, 889/1052, 1165/1078; N = 40, ns = 8 773/2575, 2345/2689, 3560/3513.
+  const int wave = warps * h->nsm * (2 * smem <= 224 * 1024 ? 2 : 1);
+  if (mode != 0 && sm32 <= 200 * 1024 && rhs != sol && ncol > (N <= 33 ? 1 : 3) * wave) {
     // (the prefetch of the next factor column costs 6 NB registers; beyond 33 it spills)
     auto* kern = N <= 9 ? k_helm32<9> : N <= 17 ? k_helm32<17> : N <= 25 ? k_helm32<25> : N <= 33 ? k_helm32<33> : k_helm32<0>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
     kern<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), hc, rhs, sol, ncol, h->dD2, h->dzh, hc.order);
     CK(cudaGetLastError());
   } else if (nc > 0) {
-    const int warps = 4;
-    size_t smem = (size_t)warps * 6 * n * sizeof(double);
     cudaFuncSetAttribute(k_helm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), hc, rhs, sol, nc, mode, h->dD2, h->dzh,
                                                                   tc ? hc.list : nullptr);
