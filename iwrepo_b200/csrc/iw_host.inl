@@ -2678,8 +2678,8 @@ int iw_profile_read(iw_handle* h, double* ms16, long* n16) {
 // ---------------------------------------------------------------------------
 // isolated batched Helmholtz solves (one system per column, lambda given)
 // ---------------------------------------------------------------------------
+// What the kernels of the band LU read
 struct HelmCache {
-  int nsys = 0;
   double* ab = nullptr;
   float* ab32 = nullptr;
   int* ipiv = nullptr;
@@ -2687,16 +2687,27 @@ struct HelmCache {
   SysDesc* sys = nullptr;
   double* pen = nullptr;
   int* colsys = nullptr;
-  double* lam = nullptr;  // distinct lambdas, ascending
-  // block inverses of the systems [first, nsys) that k_solve_tc takes (mode 0) and
-  // their tasks; the columns of the others stay with the band LU (list, nlist)
-  double *ainv = nullptr, *lvec = nullptr, *minv = nullptr, *pen2 = nullptr;
-  SysDesc* sys2 = nullptr;
-  Task* tasks = nullptr;
-  int ntask = 0, first = 0;
-  int *order = nullptr, *list = nullptr, nlist = 0;
 };
-static std::map<std::pair<iw_handle*, std::string>, HelmCache> g_helm;
+// The tables of one set of lambdas.  Each part is made by the first call that needs it: the factors of the
+// systems [0, nlu) and their FP32 copy (lu, c.ab32), the columns by system (order), the block inverses of the
+// systems [first, nsys) with their tasks and the columns left to the band LU (tcm).  Freed with the handle.
+struct HelmEntry {
+  HelmCache c;
+  std::vector<double> lam;  // distinct lambdas, ascending
+  std::vector<int> cs;      // column -> system
+  int nsys = 0, first = 0;  // mode 0 takes the systems from first on to k_helm_tc
+  char* lu = nullptr;
+  int nlu = 0;
+  size_t lu_bytes = 0;
+  int* order = nullptr;
+  char* tcm = nullptr;
+  int ntask = 0, nlist = 0;
+  double *ainv = nullptr, *lvec = nullptr, *minv = nullptr, *pen = nullptr;
+  SysDesc* sys = nullptr;
+  Task* tasks = nullptr;
+  int* list = nullptr;
+};
+static std::map<std::pair<iw_handle*, std::string>, HelmEntry> g_helm;
 
 // y = A x for the penalty matrix of system s (matrix-free, FP64)
 // row r; x(i): element i
@@ -2984,6 +2995,134 @@ static __global__ void __launch_bounds__(32) k_helm32(Geo g, HelmCache hc, const
   for (int k = 0; k < n; ++k) xc[2 * k] += (double)b[32 * k];
 }
 
+// Pieces of one device allocation: each piece's offset, the total in `at`
+static size_t carve(size_t& at, size_t bytes) {
+  const size_t o = at;
+  at += (bytes + 255) & ~(size_t)255;
+  return o;
+}
+
+// the columns by system
+static std::vector<int> helm_order(const HelmEntry& E) {
+  std::vector<int> order(E.cs.size());
+  for (size_t c = 0; c < order.size(); ++c) order[c] = (int)c;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return E.cs[a] < E.cs[b]; });
+  return order;
+}
+
+// Band LU of the systems [0, need), and their FP32 copy for mode 1
+static int helm_lu(iw_handle* h, HelmEntry& E, int need, bool fp32, int bot, int top) {
+  const int n = h->nz, N = h->N, ldab = 3 * N + 1, ns = h->ns;
+  const size_t band = (size_t)ldab * n;
+  if (E.nlu < need) {
+    size_t at = 0;
+    const size_t osys = carve(at, need * sizeof(SysDesc)), open = carve(at, (size_t)need * 6 * ns * sizeof(double)), up_to = at;
+    const size_t oab = carve(at, need * band * sizeof(double)), opiv = carve(at, (size_t)need * n * sizeof(int)),
+                 oinfo = carve(at, need * sizeof(int));
+    std::vector<char> host(up_to, 0);
+    for (int u = 0; u < need; ++u) {
+      SysDesc& sd = ((SysDesc*)(host.data() + osys))[u];
+      double* pen = (double*)(host.data() + open) + (size_t)u * 6 * ns;
+      sd.eps = 1. / E.lam[u];
+      sd.ifbcbot = bot;
+      sd.ifbctop = top;
+      h_penalty(ns, N, h->p, sd.eps, bot, top, pen);
+      sd.tau1_bot = pen[4 * ns];
+      sd.tau2_top = pen[5 * ns + ns - 1];
+    }
+    char* m = nullptr;
+    if (dalloc(h, &m, at)) return IW_ERR_NOMEM;
+    const cudaError_t e = scopy(h, m, host.data(), up_to, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+      cudaFree(m);
+      return set_err(IW_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
+    }
+    h->bytes -= E.lu_bytes + (E.c.ab32 ? E.nlu * band * sizeof(float) : 0);
+    cudaFree(E.lu);
+    cudaFree(E.c.ab32);
+    E.lu = m;
+    E.lu_bytes = at;
+    E.nlu = need;
+    E.c.sys = (SysDesc*)(m + osys);
+    E.c.pen = (double*)(m + open);
+    E.c.ab = (double*)(m + oab);
+    E.c.ipiv = (int*)(m + opiv);
+    E.c.info = (int*)(m + oinfo);
+    E.c.ab32 = nullptr;
+    FactorArgs fa;
+    fa.sys = E.c.sys;
+    fa.pen = E.c.pen;
+    fa.ab = E.c.ab;
+    fa.nsys = need;
+    fa.D = h->dD;
+    fa.D2 = h->dD2;
+    fa.zh = h->dzh;
+    k_assemble_band<<<need, 128, 0, h->st>>>(geo(h), fa);
+    launch_band_lu(h->st, need, n, N, E.c.ab, E.c.ipiv, E.c.info);
+  }
+  if (fp32 && !E.c.ab32) {
+    if (dalloc(h, &E.c.ab32, E.nlu * band)) return IW_ERR_NOMEM;
+    k_convert<double, float><<<2048, 256, 0, h->st>>>(E.c.ab, E.c.ab32, E.nlu * band);
+  }
+  CK(cudaGetLastError());
+  return 0;
+}
+
+// Block inverses of the systems [first, nsys), their tasks and the columns of the other systems
+static int helm_blocks(iw_handle* h, HelmEntry& E, int bot, int top) {
+  if (E.tcm) return 0;
+  const int N = h->N, ns = h->ns, m = 2 * (ns - 1), nt = E.nsys - E.first, ncol = (int)E.cs.size();
+  const std::vector<int> order = helm_order(E);
+  std::vector<Task> tasks;
+  std::vector<int> list;
+  for (int i = 0; i < ncol;) {
+    const int u = E.cs[order[i]];
+    int j = i;
+    while (j < ncol && E.cs[order[j]] == u && j - i < kSysR / 2) ++j;
+    if (u < E.first)
+      list.insert(list.end(), order.begin() + i, order.begin() + j);
+    else
+      tasks.push_back(Task{u - E.first, i, j - i});
+    i = j;
+  }
+  size_t at = 0;
+  const size_t olam = carve(at, nt * sizeof(double)), otask = carve(at, tasks.size() * sizeof(Task)),
+               olist = carve(at, list.size() * sizeof(int)), up_to = at;
+  const size_t oainv = carve(at, (size_t)nt * h->nb * N * N * sizeof(double)),
+               olvec = carve(at, (size_t)nt * m * N * sizeof(double)), ominv = carve(at, (size_t)nt * m * m * sizeof(double)),
+               open = carve(at, (size_t)nt * 6 * ns * sizeof(double)), osys = carve(at, nt * sizeof(SysDesc));
+  std::vector<char> host(up_to, 0);
+  memcpy(host.data() + olam, E.lam.data() + E.first, nt * sizeof(double));
+  memcpy(host.data() + otask, tasks.data(), tasks.size() * sizeof(Task));
+  if (!list.empty()) memcpy(host.data() + olist, list.data(), list.size() * sizeof(int));
+  if (!E.order && up(h, &E.order, order)) return IW_ERR_NOMEM;
+  char* d = nullptr;
+  if (dalloc(h, &d, at)) return IW_ERR_NOMEM;
+  const cudaError_t e = scopy(h, d, host.data(), up_to, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    return set_err(IW_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
+  }
+  double* pen = (double*)(d + open);
+  SysDesc* sys = (SysDesc*)(d + osys);
+  if (int r = build_systems(h, (double*)(d + olam), nt, 0.0, bot, top, false, 0, (double*)(d + oainv), nullptr,
+                            (double*)(d + olvec), (double*)(d + ominv), pen, sys)) {
+    cudaFree(d);
+    return r;
+  }
+  E.tcm = d;
+  E.tasks = (Task*)(d + otask);
+  E.ntask = (int)tasks.size();
+  E.list = (int*)(d + olist);
+  E.nlist = (int)list.size();
+  E.ainv = (double*)(d + oainv);
+  E.lvec = (double*)(d + olvec);
+  E.minv = (double*)(d + ominv);
+  E.pen = pen;
+  E.sys = sys;
+  return 0;
+}
+
 static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, int top, const double* rhs,
                         double* sol, int mode) {
   std::vector<double> lam(ncol);
@@ -2998,115 +3137,57 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
   char kb[96];
   snprintf(kb, sizeof kb, "%d|%d|%d|%llx", ncol, bot, top, (unsigned long long)hs);
   auto key = std::make_pair(h, std::string(kb));
-  const int n = h->nz, N = h->N, ldab = 3 * N + 1, ns = h->ns;
+  const int n = h->nz, N = h->N, ns = h->ns;
   auto it = g_helm.find(key);
   if (it == g_helm.end()) {
-    std::vector<double> s = lam;
-    std::sort(s.begin(), s.end());
-    s.erase(std::unique(s.begin(), s.end()), s.end());
-    HelmCache hc;
-    hc.nsys = (int)s.size();
-    std::vector<int> cs(ncol), order(ncol);
-    for (int c = 0; c < ncol; ++c) {
-      cs[c] = (int)(std::lower_bound(s.begin(), s.end(), lam[c]) - s.begin());
-      order[c] = c;
-    }
+    HelmEntry E;
+    E.lam = lam;
+    std::sort(E.lam.begin(), E.lam.end());
+    E.lam.erase(std::unique(E.lam.begin(), E.lam.end()), E.lam.end());
+    E.nsys = (int)E.lam.size();
+    E.cs.resize(ncol);
+    for (int c = 0; c < ncol; ++c) E.cs[c] = (int)(std::lower_bound(E.lam.begin(), E.lam.end(), lam[c]) - E.lam.begin());
     // Block inverses (system-grouped, on the tensor cores) for the systems whose estimated condition
     // needs no residual sweep, as in the time step; the others keep the pivoted band LU.
     const bool tc = h->ns <= 16 && N <= kTcMaxN && n <= kSysMaxRows &&
                     helm_smem(n, N, ns, h->nb).total <= 200 * 1024;
     const double rho = cond_slope(h);
-    hc.first = hc.nsys;
+    E.first = E.nsys;
     if (tc)
-      while (hc.first > 0 && s[hc.first - 1] > 0 && 1.0 + rho / s[hc.first - 1] <= kRefineCond) --hc.first;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cs[a] < cs[b]; });
-    std::vector<Task> tasks;
-    std::vector<int> list;
-    for (int i = 0; i < ncol;) {
-      const int u = cs[order[i]];
-      int j = i;
-      while (j < ncol && cs[order[j]] == u && j - i < kSysR / 2) ++j;
-      if (u < hc.first)
-        list.insert(list.end(), order.begin() + i, order.begin() + j);
-      else
-        tasks.push_back(Task{u - hc.first, i, j - i});
-      i = j;
-    }
-    hc.ntask = (int)tasks.size();
-    hc.nlist = (int)list.size();
-    if (up(h, &hc.lam, s) || up(h, &hc.colsys, cs)) return IW_ERR_NOMEM;
-    if (up(h, &hc.order, order) || (hc.ntask > 0 && up(h, &hc.tasks, tasks))) return IW_ERR_NOMEM;
-    if (hc.nlist > 0 && up(h, &hc.list, list)) return IW_ERR_NOMEM;
-    it = g_helm.emplace(key, hc).first;
+      while (E.first > 0 && E.lam[E.first - 1] > 0 && 1.0 + rho / E.lam[E.first - 1] <= kRefineCond) --E.first;
+    if (up(h, &E.c.colsys, E.cs)) return IW_ERR_NOMEM;
+    it = g_helm.emplace(key, std::move(E)).first;
   }
-  HelmCache& hc = it->second;
-  // k_solve_tc copies whole complex values: 16-byte aligned columns
-  const bool tc = mode == 0 && hc.ntask > 0 && (((uintptr_t)rhs | (uintptr_t)sol) & 15) == 0;
-  const int nt = hc.nsys - hc.first, m = 2 * (ns - 1);
-  if (tc && !hc.ainv) {
-    double* ainv = nullptr;
-    if (dalloc(h, &ainv, (size_t)nt * h->nb * N * N) || dalloc(h, &hc.lvec, (size_t)nt * std::max(m, 1) * N) ||
-        dalloc(h, &hc.minv, (size_t)nt * std::max(m * m, 1)) || dalloc(h, &hc.pen2, (size_t)nt * 6 * ns) ||
-        dalloc(h, &hc.sys2, (size_t)nt))
-      return IW_ERR_NOMEM;
-    if (int r = build_systems(h, hc.lam + hc.first, nt, 0.0, bot, top, false, 0, ainv, nullptr, hc.lvec, hc.minv, hc.pen2, hc.sys2))
-      return r;
-    hc.ainv = ainv;
-  }
-  if ((!tc || hc.nlist > 0) && !hc.ab) {  // band LU factors
-    std::vector<SysDesc> sys(hc.nsys);
-    std::vector<double> pen((size_t)hc.nsys * 6 * ns), s(hc.nsys);
-    CK(scopy(h, s.data(), hc.lam, s.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    for (int u = 0; u < hc.nsys; ++u) {
-      memset(&sys[u], 0, sizeof(SysDesc));
-      sys[u].eps = 1. / s[u];
-      sys[u].ifbcbot = bot;
-      sys[u].ifbctop = top;
-      h_penalty(ns, N, h->p, sys[u].eps, bot, top, pen.data() + (size_t)u * 6 * ns);
-      sys[u].tau1_bot = pen[(size_t)u * 6 * ns + 4 * ns];
-      sys[u].tau2_top = pen[(size_t)u * 6 * ns + 5 * ns + ns - 1];
-    }
-    double* ab = nullptr;
-    if (dalloc(h, &ab, (size_t)hc.nsys * ldab * n) || dalloc(h, &hc.ab32, (size_t)hc.nsys * ldab * n) ||
-        dalloc(h, &hc.ipiv, (size_t)hc.nsys * n) || dalloc(h, &hc.info, (size_t)hc.nsys) ||
-        up(h, &hc.sys, sys) || up(h, &hc.pen, pen))
-      return IW_ERR_NOMEM;
-    hc.ab = ab;
-    FactorArgs fa;
-    fa.sys = hc.sys;
-    fa.pen = hc.pen;
-    fa.ab = hc.ab;
-    fa.nsys = hc.nsys;
-    fa.D = h->dD;
-    fa.D2 = h->dD2;
-    fa.zh = h->dzh;
-    k_assemble_band<<<hc.nsys, 128, 0, h->st>>>(geo(h), fa);
-    launch_band_lu(h->st, hc.nsys, n, N, hc.ab, hc.ipiv, hc.info);
-    size_t tot = (size_t)hc.nsys * ldab * n;
-    k_convert<double, float><<<2048, 256, 0, h->st>>>(hc.ab, hc.ab32, tot);
-    CK(cudaGetLastError());
-  }
+  HelmEntry& E = it->second;
+  // k_helm_tc copies whole complex values: 16-byte aligned columns
+  const bool tc = mode == 0 && E.first < E.nsys && (((uintptr_t)rhs | (uintptr_t)sol) & 15) == 0;
   if (tc) {
+    if (int r = helm_blocks(h, E, bot, top)) return r;
     HelmTc H;
     memset(&H, 0, sizeof H);
-    H.ainv = hc.ainv;
-    H.lvec = hc.lvec;
-    H.minv = hc.minv;
-    H.pen = hc.pen2;
-    H.sys = hc.sys2;
+    H.ainv = E.ainv;
+    H.lvec = E.lvec;
+    H.minv = E.minv;
+    H.pen = E.pen;
+    H.sys = E.sys;
     H.D = h->dD;
     H.D2t = h->dD2t;
     H.zh = h->dzh;
-    H.tasks = hc.tasks;
-    H.order = hc.order;
+    H.tasks = E.tasks;
+    H.order = E.order;
     H.rhs = rhs;
     H.sol = sol;
     H.nb = h->nb;
     memcpy(H.bmap, h->bmap, sizeof H.bmap);
-    launch_helm_tc<double>(h, H, hc.ntask);
+    // the factors of the other systems first: after a failure nothing of the solution is written
+    if (E.nlist > 0)
+      if (int r = helm_lu(h, E, E.first, false, bot, top)) return r;
+    launch_helm_tc<double>(h, H, E.ntask);
     CK(cudaGetLastError());
+  } else if (int r = helm_lu(h, E, E.nsys, mode != 0, bot, top)) {
+    return r;
   }
-  const int nc = tc ? hc.nlist : ncol;
+  const int nc = tc ? E.nlist : ncol;
   const int warps = 4;
   const size_t sm32 = helm32_smem(n, N), smem = (size_t)warps * 6 * n * sizeof(double);
   // Mode 1 by the number of columns.  k_helm (a warp per column) is a short chain, k_helm32 (a lane per right-hand
@@ -3120,13 +3201,14 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
   if (mode != 0 && sm32 <= 200 * 1024 && rhs != sol && ncol > (N <= 33 ? 1 : 3) * wave) {
     // (the prefetch of the next factor column costs 6 NB registers; beyond 33 it spills)
     auto* kern = N <= 9 ? k_helm32<9> : N <= 17 ? k_helm32<17> : N <= 25 ? k_helm32<25> : N <= 33 ? k_helm32<33> : k_helm32<0>;
+    if (!E.order && up(h, &E.order, helm_order(E))) return IW_ERR_NOMEM;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
-    kern<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), hc, rhs, sol, ncol, h->dD2, h->dzh, hc.order);
+    kern<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), E.c, rhs, sol, ncol, h->dD2, h->dzh, E.order);
     CK(cudaGetLastError());
   } else if (nc > 0) {
     cudaFuncSetAttribute(k_helm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), hc, rhs, sol, nc, mode, h->dD2, h->dzh,
-                                                                  tc ? hc.list : nullptr);
+    k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), E.c, rhs, sol, nc, mode, h->dD2, h->dzh,
+                                                                  tc ? E.list : nullptr);
     CK(cudaGetLastError());
   }
   return 0;
@@ -3139,10 +3221,8 @@ static void helm_free(iw_handle* h) {
       ++it;
       continue;
     }
-    HelmCache& c = it->second;
-    for (void* p : {(void*)c.ab, (void*)c.ab32, (void*)c.ipiv, (void*)c.info, (void*)c.sys, (void*)c.pen, (void*)c.colsys,
-                    (void*)c.lam, (void*)c.pen2, (void*)c.sys2, (void*)c.ainv, (void*)c.lvec, (void*)c.minv, (void*)c.tasks, (void*)c.order, (void*)c.list})
-      cudaFree(p);
+    HelmEntry& E = it->second;
+    for (void* p : {(void*)E.c.colsys, (void*)E.lu, (void*)E.c.ab32, (void*)E.order, (void*)E.tcm}) cudaFree(p);
     it = g_helm.erase(it);
   }
 }
