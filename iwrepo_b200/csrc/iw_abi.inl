@@ -72,9 +72,70 @@ uint64_t xs_next(uint64_t& s) {
 // per-call device scratch of n doubles
 struct DBuf {
   double* p = nullptr;
-  explicit DBuf(size_t n) { cudaMalloc(&p, n * sizeof(double) + 16); }
+  explicit DBuf(size_t n) {
+    if (cudaMalloc(&p, n * sizeof(double) + 16) != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();
+      set_err(IW_ERR_NOMEM, "cudaMalloc");
+    }
+  }
   ~DBuf() { cudaFree(p); }
 };
+
+// Device scratch of n doubles for a routine on host fields: the handle's own, which stays
+// until iw_destroy, or an allocation of this call where another thread has it or n is beyond its bound.
+// cudaMalloc and cudaFree of a field (0.65 ms together, 9 MB) stall now and then for 10 to 600 ms;
+// copies of the same size do not, so a routine without them keeps its time from call to call.
+constexpr size_t kScratchMax = (size_t)32 << 20;  // 256 MB
+struct Scratch {
+  double* p = nullptr;
+  double* mine = nullptr;
+  std::unique_lock<std::mutex> lk;
+  Scratch(iw_handle* h, size_t n) : lk(h->scr_mu, std::try_to_lock) {
+    if (lk.owns_lock() && n <= kScratchMax) {
+      if (h->scr_n < n) {
+        h->bytes -= h->scr_n * sizeof(double);
+        cudaFree(h->scr);
+        h->scr_n = 0;
+        if (dalloc(h, &h->scr, n)) {
+          cudaGetLastError();
+          return;
+        }
+        h->scr_n = n;
+      }
+      p = h->scr;
+      return;
+    }
+    if (lk.owns_lock()) lk.unlock();
+    if (dalloc(h, &mine, n)) {
+      cudaGetLastError();
+      return;
+    }
+    h->bytes -= n * sizeof(double);  // (not kept)
+    p = mine;
+  }
+  ~Scratch() { cudaFree(mine); }
+  Scratch(const Scratch&) = delete;
+};
+// FP64 twiddles for the routines on host fields: the handle's, made by the first call of a mixed run
+bool twiddles64(iw_handle* h, FieldSet<double>& fs) {
+  const FieldSet<double>* src = &h->f64;
+  if (h->mixed) {
+    std::lock_guard<std::mutex> lk(h->tw_mu);
+    FieldSet<double>& t = h->tw64;
+    const int M = h->nx / 2;
+    if ((!t.Wm && up(h, &t.Wm, twiddles<double2>(M, M))) || (!t.Wn && up(h, &t.Wn, twiddles<double2>(h->nx, M + 1))) ||
+        (!t.Wy && up(h, &t.Wy, twiddles<double2>(h->ny, h->ny)))) {
+      cudaGetLastError();
+      return false;
+    }
+    src = &t;
+  }
+  fs.Wm = src->Wm;
+  fs.Wn = src->Wn;
+  fs.Wy = src->Wy;
+  return true;
+}
 
 iw_handle* bound() {
   if (!g_bound) set_err(IW_ERR_STATE, "no handle bound (iw_bind)");
@@ -189,38 +250,33 @@ void horfft_(double* b, const int* is, const int* nk) {
   iw_handle* h = bound();
   if (!h || !b || !is || !nk) return;
   size_t n = h->plane * (size_t)*nk;
-  DBuf d(n);
-  scopy(h, d.p, b, n * sizeof(double), cudaMemcpyHostToDevice);
+  Scratch d(h, n);
   FieldSet<double> tmp;
-  typedef double2 C;
-  int M = h->nx / 2;
-  auto wm = twiddles<C>(M, M);
-  auto wn = twiddles<C>(h->nx, M + 1);
-  auto wy = twiddles<C>(h->ny, h->ny);
-  if (up(h, &tmp.Wm, wm) || up(h, &tmp.Wn, wn) || up(h, &tmp.Wy, wy)) return;
+  if (!d.p || !twiddles64(h, tmp)) return;
+  scopy(h, d.p, b, n * sizeof(double), cudaMemcpyHostToDevice);
   horfft_dev<double>(h, tmp, d.p, *is, *nk);
   cudaStreamSynchronize(h->st);
   scopy(h, b, d.p, n * sizeof(double), cudaMemcpyDeviceToHost);
-  cudaFree(tmp.Wm);
-  cudaFree(tmp.Wn);
-  cudaFree(tmp.Wy);
 }
 
 void dpdz_(const double* a, double* b) {
   iw_handle* h = bound();
   if (!h || !a || !b) return;
-  DBuf da(h->ntot), db(h->ntot);
-  scopy(h, da.p, a, h->ntot * sizeof(double), cudaMemcpyHostToDevice);
-  k_dz_field<double><<<(unsigned)((h->ntot + 255) / 256), 256, 0, h->st>>>(geo(h), da.p, db.p);
+  Scratch d(h, 2 * h->ntot);
+  if (!d.p) return;
+  double* db = d.p + h->ntot;
+  scopy(h, d.p, a, h->ntot * sizeof(double), cudaMemcpyHostToDevice);
+  k_dz_field<double><<<(unsigned)((h->ntot + 255) / 256), 256, 0, h->st>>>(geo(h), d.p, db);
   cudaStreamSynchronize(h->st);
-  scopy(h, b, db.p, h->ntot * sizeof(double), cudaMemcpyDeviceToHost);
+  scopy(h, b, db, h->ntot * sizeof(double), cudaMemcpyDeviceToHost);
 }
 
 void filter_3dlegenfourier_(double* f, const int* ifourier, const int* ilegen, const int* iout) {
   (void)iout;
   iw_handle* h = bound();
   if (!h || !f) return;
-  DBuf d(h->ntot);
+  Scratch d(h, h->ntot);
+  if (!d.p) return;
   scopy(h, d.p, f, h->ntot * sizeof(double), cudaMemcpyHostToDevice);
   long total = (long)h->nxpp * h->ny * h->ns;
   k_filter_field<double><<<(unsigned)((total + 127) / 128), 128, 0, h->st>>>(geo(h), d.p, ifourier ? *ifourier : 1,
@@ -236,6 +292,7 @@ void filter_legenpen_(const double* fin, double* fout, const double* ybar, const
   iw_handle* h = bound();
   if (!h || !fin || !fout) return;
   DBuf d(h->N);
+  if (!d.p) return;
   scopy(h, d.p, fin, h->N * sizeof(double), cudaMemcpyHostToDevice);
   k_legen_one<<<1, 32, 0, h->st>>>(geo(h), h->dwg, h->dal, h->dsig, d.p, h->N);
   cudaStreamSynchronize(h->st);
@@ -246,16 +303,12 @@ void interface_avg3d_(double* f, int* ic) {
   iw_handle* h = bound();
   if (!h || !f) return;
   FieldSet<double> fs;
-  DBuf d(h->ntot), G(h->plane * 16 * (size_t)std::max(1, h->ns - 1));
-  typedef double2 C;
-  int M = h->nx / 2;
-  auto wm = twiddles<C>(M, M);
-  auto wn = twiddles<C>(h->nx, M + 1);
-  auto wy = twiddles<C>(h->ny, h->ny);
-  if (up(h, &fs.Wm, wm) || up(h, &fs.Wn, wn) || up(h, &fs.Wy, wy)) return;
+  const size_t at = (h->ntot + 31) & ~(size_t)31;  // of the planes next to interfaces: 16-byte copies
+  Scratch d(h, at + h->plane * 16 * (size_t)std::max(1, h->ns - 1));
+  if (!d.p || !twiddles64(h, fs)) return;
   scopy(h, d.p, f, h->ntot * sizeof(double), cudaMemcpyHostToDevice);
   for (int q = 0; q < 4; ++q) fs.F[q] = d.p;
-  fs.G = G.p;
+  fs.G = d.p + at;
   iface_avg<double>(h, fs, true, 1);
   cudaStreamSynchronize(h->st);
   scopy(h, f, d.p, h->ntot * sizeof(double), cudaMemcpyDeviceToHost);
@@ -266,10 +319,6 @@ void interface_avg3d_(double* f, int* ic) {
   }
   fs.F[0] = fs.F[1] = fs.F[2] = fs.F[3] = nullptr;
   fs.G = nullptr;
-  cudaFree(fs.Wm);
-  cudaFree(fs.Wn);
-  cudaFree(fs.Wy);
-  fs.Wm = fs.Wn = fs.Wy = nullptr;
 }
 
 void penalty_setup_(const double* epsilon) {
@@ -320,6 +369,11 @@ void penalty_main_(const double* epsilon, const int* ifuncreal, const double* bc
   int* dip;
   if (factor_dense_or_params(h, pen.data(), eps, *ifbcbot, *ifbctop, nullptr, &dab, &dip)) return;
   DBuf db(2 * (size_t)n);
+  if (!db.p) {
+    cudaFree(dab);
+    cudaFree(dip);
+    return;
+  }
   scopy(h, db.p, b.data(), b.size() * sizeof(double), cudaMemcpyHostToDevice);
   k_solve_one<<<1, 64, 2 * n * sizeof(double), h->st>>>(geo(h), dab, dip, db.p);
   cudaStreamSynchronize(h->st);
@@ -347,6 +401,11 @@ void bandlu_solve_(const double* ain, double* xr, double* xi, const int* ifuncre
     b[n + k] = xi ? xi[k] : 0.0;
   }
   DBuf db(2 * (size_t)n);
+  if (!db.p) {
+    cudaFree(dab);
+    cudaFree(dip);
+    return;
+  }
   scopy(h, db.p, b.data(), b.size() * sizeof(double), cudaMemcpyHostToDevice);
   k_solve_one<<<1, 32 * nr, (size_t)nr * n * sizeof(double), h->st>>>(geo(h), dab, dip, db.p);
   cudaStreamSynchronize(h->st);

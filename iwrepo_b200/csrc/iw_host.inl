@@ -364,6 +364,7 @@ struct iw_handle {
   bool err_ev_live = false;
   FftPlan plx, ply;
   FieldSet<double> f64;
+  FieldSet<double> tw64;  // twiddles only: FP64 transforms of host fields in a mixed run
   FieldSet<float> f32;
   // systems
   std::vector<double> akv;     // distinct kx^2+ky^2 values
@@ -391,6 +392,10 @@ struct iw_handle {
       *this = BI();
     }
   } bi[SYS_KINDS];
+  // device scratch and FP64 twiddles of the routines on host fields (iw_abi.inl)
+  double* scr = nullptr;
+  size_t scr_n = 0;
+  std::mutex scr_mu, tw_mu;
   int fail_alloc = 0;  // iw_fail_allocation: device allocations until one is refused
   bool use_bi = true;
   // grouped solve tasks per kind (columns sharing a system, <= G per task)
@@ -2363,6 +2368,8 @@ int iw_destroy(iw_handle* h) {
   if (h->out_ev) cudaEventDestroy(h->out_ev);
   free_fields(h->f64);
   free_fields(h->f32);
+  free_fields(h->tw64);
+  cudaFree(h->scr);
   for (double* p : {h->ddzinv, h->dpart, h->dDt, h->dD2t, h->dLt, h->dD, h->dD2, h->dL, h->dh, h->dxw, h->dyw, h->dcf, h->dzg, h->dzh, h->dwg, h->dal, h->dsig,
                     h->dmeang, h->dwnl, h->dwvr, h->dred})
     cudaFree(p);
