@@ -1917,12 +1917,17 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
     return ms;
   };
   const int save[4] = {h->tune_ytx, h->tune_a, h->tune_e, h->use_sys};
-  // y tiles: the 10-job inverse and the 4-job forward-with-fold launches
-  float best = 1e30f;
-  int besttx = 8;
+  // y tiles: the 10-job inverse and the 4-job forward-with-fold launches.  8 stands for the tiles taken by size (16
+  // columns where ny <= 128; narrower ones of two transforms that do not fit in shared memory); a narrower
+  // choice replaces it if its tiles differ and it is 2 % faster.
+  float best = 0.f;
+  int besttx = 8, seen1 = 0, seen2 = 0;
   for (int tx : {8, 4, 2}) {
     h->tune_ytx = tx;
-    if (ytx<T>(h, true) != tx) continue;  // does not fit in shared memory
+    const int w1 = ytx<T>(h, false), w2 = ytx<T>(h, true);
+    if (w1 == seen1 && w2 == seen2) continue;
+    seen1 = w1;
+    seen2 = w2;
     const float ms = timeit([&] {
       YJobs<T> ji, jf;
       memset(&ji, 0, sizeof ji);
@@ -1932,7 +1937,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
       launch_y<T>(h, ts, ji, 10, h->nz, false);
       launch_y<T>(h, ts, jf, 4, h->nz, true);
     });
-    if (ms < best) {
+    if (tx == 8 || ms < 0.98f * best) {
       best = ms;
       besttx = tx;
     }
