@@ -1754,7 +1754,9 @@ IW_INST_Z(extern, double)
 template <typename T>
 static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen, int cols = 0) {
   Geo g = geo(h);
-  const int warps = 4;
+  // a warp's right-hand sides (k_visc 4 columns of nz, k_press_g as many): four warps share a CTA while they fit in
+  // shared memory, two above nz = 1816 (nz <= 64 x 48)
+  const int warps = (size_t)4 * 4 * h->nz * sizeof(double) <= 227 * 1024 ? 4 : 2;
   const unsigned nblk = (unsigned)((h->ncol + warps - 1) / warps);
   const size_t smem = (size_t)warps * 4 * h->nz * sizeof(double);
   const int kstart = h->p.bc_variant == IW_BC_NOSLIP ? 1 : 0;
@@ -1764,7 +1766,7 @@ static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen, int cols = 0) 
   } else {
   {
     constexpr int G = 2;
-    const int wpb = 4;
+    const int wpb = warps;
     const size_t smp = (size_t)wpb * 2 * G * h->nz * sizeof(double);
     cudaFuncSetAttribute(k_press_g<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp);
     k_press_g<T, G><<<(h->ntask[SYS_P] + wpb - 1) / wpb, 32 * wpb, smp, h->st>>>(
