@@ -26,7 +26,7 @@ int phys_of(iw_handle* h, FieldSet<T>& fs, const T* src, T* dst, T* tmp, int op)
     k_mulikx<T><<<(unsigned)((h->ntot / 2 + 255) / 256), 256, 0, h->st>>>(g, dst);
   }
   k_xfft_field<T><<<h->ny * h->nz, 128, smem, h->st>>>(g, dst, h->nz, 1, h->plx, fs.Wm, fs.Wn);
-  CK(cudaGetLastError());
+  CK(launch_error());
   return 0;
 }
 
@@ -58,7 +58,7 @@ int horfft_dev(iw_handle* h, FieldSet<T>& fs, T* b, int is, int nk) {
     launch_y<T>(h, fs, jb, 1, nk, false);
     k_xfft_field<T><<<h->ny * nk, 128, smem, h->st>>>(g, b, nk, 1, h->plx, fs.Wm, fs.Wn);
   }
-  CK(cudaGetLastError());
+  CK(launch_error());
   return 0;
 }
 
@@ -97,20 +97,14 @@ struct Scratch {
         h->bytes -= h->scr_n * sizeof(double);
         cudaFree(h->scr);
         h->scr_n = 0;
-        if (dalloc(h, &h->scr, n)) {
-          cudaGetLastError();
-          return;
-        }
+        if (dalloc(h, &h->scr, n)) return;
         h->scr_n = n;
       }
       p = h->scr;
       return;
     }
     if (lk.owns_lock()) lk.unlock();
-    if (dalloc(h, &mine, n)) {
-      cudaGetLastError();
-      return;
-    }
+    if (dalloc(h, &mine, n)) return;
     h->bytes -= n * sizeof(double);  // (not kept)
     p = mine;
   }
@@ -125,10 +119,8 @@ bool twiddles64(iw_handle* h, FieldSet<double>& fs) {
     FieldSet<double>& t = h->tw64;
     const int M = h->nx / 2;
     if ((!t.Wm && up(h, &t.Wm, twiddles<double2>(M, M))) || (!t.Wn && up(h, &t.Wn, twiddles<double2>(h->nx, M + 1))) ||
-        (!t.Wy && up(h, &t.Wy, twiddles<double2>(h->ny, h->ny)))) {
-      cudaGetLastError();
+        (!t.Wy && up(h, &t.Wy, twiddles<double2>(h->ny, h->ny))))
       return false;
-    }
     src = &t;
   }
   fs.Wm = src->Wm;
@@ -571,7 +563,7 @@ static int stats_to_host(iw_handle* h, FieldSet<T>& fs, StatRows<T>& a, int n, i
   *nblk = std::max(1, std::min(most, (lines + kStatThreads / 32 - 1) / (kStatThreads / 32)));
   if (!h->hstat) CK(cudaHostAlloc((void**)&h->hstat, (kPartDoubles + 4) * sizeof(double), cudaHostAllocDefault));
   launch_xstats<T>(h, fs, a, n, *nblk);
-  CK(cudaGetLastError());
+  CK(launch_error());
   CK(cudaMemcpyAsync(h->hstat, h->dpart, (size_t)n * *nblk * kStatSlots * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   const int r = more();
   if (r) return r;
@@ -813,7 +805,7 @@ int iw_bandlu_solve_noalloc(const double* ain_dev, double* x_dev, int nzloc, int
   k_pack_band<<<64, 256, 0, st>>>(ain_dev, n, nzloc, ldab, ab, sd, info);
   launch_band_lu(st, 1, n, nzloc, ab, ipiv, info);
   k_solve_one<<<1, 32 * nrhs, (size_t)nrhs * n * sizeof(double), st>>>(g, ab, ipiv, x_dev);
-  CK(cudaGetLastError());
+  CK(launch_error());
   return IW_OK;
 }
 

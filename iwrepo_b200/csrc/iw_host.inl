@@ -510,7 +510,10 @@ static int dalloc(iw_handle* h, T** p, size_t n) {
   *p = nullptr;
   if (h->fail_alloc > 0 && --h->fail_alloc == 0) return set_err(IW_ERR_NOMEM, "allocation refused (iw_fail_allocation)");
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T) + 16);
-  if (e != cudaSuccess) return set_err(IW_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here: no later check finds it again
+    return set_err(IW_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   h->bytes += n * sizeof(T);
   return 0;
 }
@@ -694,7 +697,7 @@ static int build_sys_tasks(iw_handle* h, int kind, int nrefine) {
 // SGBTF2 of nsys assembled bands (k_band_lu)
 static void launch_band_lu(cudaStream_t st, int nsys, int n, int N, double* ab, int* ipiv, int* info) {
   const size_t sm = lu_smem(N);
-  cudaFuncSetAttribute(k_band_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  set_smem(k_band_lu, sm);
   k_band_lu<<<nsys, kLuThreads, sm, st>>>(n, N, ab, ipiv, info);
 }
 
@@ -769,7 +772,7 @@ static int build_factors(iw_handle* h, int kind) {
     fa.zh = h->dzh;
     k_assemble_band<<<nsys, 128, 0, h->st>>>(geo(h), fa);
     launch_band_lu(h->st, nsys, n, N, fa.ab, h->dipiv[kind], h->dinfo[kind]);
-    CK(cudaGetLastError());
+    CK(launch_error());
     // host copies must stay alive until the copies finish
     CK(cudaStreamSynchronize(h->st));
     std::vector<int> info(nsys);
@@ -815,9 +818,9 @@ static int build_systems(iw_handle* h, const double* dak, int nsys, double c0, i
   b.lvec = lvec;
   b.minv = minv;
   const size_t sm = build_smem(h->N, h->ns);
-  CK(cudaFuncSetAttribute(k_build_systems, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  set_smem(k_build_systems, sm);
   k_build_systems<<<nsys, 64 * kBuildGroups, sm, h->st>>>(b);
-  CK(cudaGetLastError());
+  CK(launch_error());
   return 0;
 }
 
@@ -1031,7 +1034,7 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
     const int blocks = z_grid(h, W, 1), v16 = (h->plane * sizeof(T)) % 16 == 0;
 #define IW_ETCASE(NT)                                                                                        \
   case NT:                                                                                                   \
-    cudaFuncSetAttribute(k_stageE_t<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);           \
+    set_smem(k_stageE_t<T, NT>, sm);           \
     k_stageE_t<T, NT><<<blocks, 32 * W, sm, h->st>>>(geo(h), a, h->c, cols, v16);                            \
     return;
     switch (tc_nt(h->N)) { IW_ETCASE(2) IW_ETCASE(3) IW_ETCASE(4) IW_ETCASE(5) }
@@ -1061,7 +1064,7 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
   if constexpr (sizeof(T) == 4) {
     k_stageE_f32<<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c);  // at most 39 KB
   } else {
-    cudaFuncSetAttribute(k_stageE<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  // > 48 KB from N = 42 on
+    set_smem(k_stageE<T>, smem);  // > 48 KB from N = 42 on
     k_stageE<T><<<grid, kTX * kTW, smem, h->st>>>(geo(h), a, h->c);
   }
 }
@@ -1094,7 +1097,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
     switch (p2 ? h->ny : 0) {
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
-    cudaFuncSetAttribute(k_yfft<T, TX, D, true, TWO, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    set_smem(k_yfft<T, TX, D, true, TWO, MC>, smem); \
     k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     return;
       IW_YCT(64, 8)
@@ -1107,7 +1110,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
     switch (p2 ? h->ny : 0) {
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
-    cudaFuncSetAttribute(k_yfft<T, TX, D, true, TWO, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    set_smem(k_yfft<T, TX, D, true, TWO, MC>, smem); \
     k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     return;
       IW_YCT(256, 8)
@@ -1121,7 +1124,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
 #define IW_YCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
     if constexpr ((TX < 16 || D == 4) && (TX >= 8 || !P)) { /* 16 columns only for ny <= 128 */              \
-      cudaFuncSetAttribute(k_yfft<T, TX, D, P, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      set_smem(k_yfft<T, TX, D, P, TWO>, smem); \
       k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     }                                                                                                        \
     break;
@@ -1200,7 +1203,7 @@ static bool launch_xrow_reg(iw_handle* h, FieldSet<T>& fs, const NLArgs<T>& a) {
 #define IW_XREG(R0, NB)                                                                                          \
   case R0 * NB: {                                                                                                \
     typedef XReg<T, R0, NB> X;                                                                                   \
-    cudaFuncSetAttribute(k_xrow_reg<T, R0, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X::smem);     \
+    set_smem(k_xrow_reg<T, R0, NB>, X::smem);     \
     k_xrow_reg<T, R0, NB><<<dim3((h->ny + X::YR - 1) / X::YR, h->nz), X::threads, X::smem, h->st>>>(geo(h), a, fs.Wm, \
                                                                                                     fs.Wn);      \
     return true;                                                                                                 \
@@ -1264,7 +1267,7 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
     switch (M) {  // compile-time plan
 #define IW_XCT(MC, D)                                                                                       \
   case MC:                                                                                                  \
-    cudaFuncSetAttribute(k_xrow_nl<T, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    set_smem(k_xrow_nl<T, D, true, MC>, smem); \
     k_xrow_nl<T, D, true, MC><<<grid, xthr, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn);                     \
     goto xrow_done;
       IW_XCT(512, 16)
@@ -1274,7 +1277,7 @@ void launch_xrow(iw_handle* h, FieldSet<T>& fs) {
     switch (fft_dpt(M) * (p2 ? 1 : -1)) {
 #define IW_XCASE(D, P)                                                                                   \
   case (P ? D : -D):                                                                                     \
-    cudaFuncSetAttribute(k_xrow_nl<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
+    set_smem(k_xrow_nl<T, D, P>, smem);   \
     k_xrow_nl<T, D, P><<<grid, xthr, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn);                        \
     break;
         IW_XCASE(4, true)
@@ -1303,7 +1306,7 @@ void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, i
   switch (p2 && M >= 32 && M <= 512 ? M : 0) {  // compile-time plans for power-of-two lengths
 #define IW_SCT(MC, D)                                                                                            \
   case MC:                                                                                                       \
-    cudaFuncSetAttribute(k_xrow_stats<T, D, true, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+    set_smem(k_xrow_stats<T, D, true, MC>, smem);  \
     k_xrow_stats<T, D, true, MC><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);     \
     return;
     IW_SCT(32, 8)
@@ -1317,7 +1320,7 @@ void launch_xstats(iw_handle* h, FieldSet<T>& fs, const StatRows<T>& a, int n, i
   switch (fft_dpt(M) * (p2 ? 1 : -1)) {
 #define IW_SCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
-    cudaFuncSetAttribute(k_xrow_stats<T, D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+    set_smem(k_xrow_stats<T, D, P>, smem);     \
     k_xrow_stats<T, D, P><<<grid, kStatThreads, smem, h->st>>>(g, a, h->plx, fs.Wm, fs.Wn, h->dpart);        \
     break;
     IW_SCASE(4, true)
@@ -1528,7 +1531,7 @@ static void launch_jobs_tc(iw_handle* h, const TcJobs<T>& jobs, int nblk, const 
   const size_t smem = tc_smem<T>(h->nz, h->N, h->ns, h->nb, false).total;
 #define IW_TC_CASE(NT)                                                                               \
   case NT:                                                                                           \
-    cudaFuncSetAttribute(k_solve_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    set_smem(k_solve_tc<T, NT>, smem); \
     k_solve_tc<T, NT><<<nblk, 32 * h->ns, smem, h->st>>>(g, jobs, order, h->dmeang);                 \
     break;
   switch (tc_nt(h->N)) { IW_TC_CASE(2) IW_TC_CASE(3) IW_TC_CASE(4) IW_TC_CASE(5) }
@@ -1543,7 +1546,7 @@ void launch_helm_tc(iw_handle* h, const HelmTc& H, int ntask) {
   const dim3 grid((unsigned)ntask, 2);
 #define IW_HT_CASE(NT)                                                                              \
   case NT:                                                                                          \
-    cudaFuncSetAttribute(k_helm_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    set_smem(k_helm_tc<NT>, smem);    \
     k_helm_tc<NT><<<grid, 32 * h->ns, smem, h->st>>>(g, H);                                         \
     break;
   switch (tc_nt(h->N)) { IW_HT_CASE(2) IW_HT_CASE(3) IW_HT_CASE(4) IW_HT_CASE(5) }
@@ -1573,7 +1576,7 @@ void launch_solve_tc(iw_handle* h, FieldSet<T>& fs, const int* roles, int nroles
     const dim3 grid((unsigned)h->ntask2[SYS_P], 2);
 #define IW_TC_CASE(NT)                                                                                             \
   case NT:                                                                                                         \
-    cudaFuncSetAttribute(k_press_tc<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
+    set_smem(k_press_tc<T, NT>, smem);               \
     k_press_tc<T, NT><<<grid, 32 * h->ns, smem, h->st>>>(g, bi, h->dtasks2[SYS_P], h->dcolorder, S[0], S[1], S[2], \
                                                          h->dDt, h->dwnl, h->dwvr, kstart, cols);                  \
     break;
@@ -1644,7 +1647,7 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
   }
   const double rd = role_rdiv(h, role);
   const int meanu = role == 0 ? h->p.meanu_damping : 0;
-  if (sm > 48 * 1024) cudaFuncSetAttribute(k_solve_cta<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (sm > 48 * 1024) set_smem(k_solve_cta<T, R>, sm);
   // refined prefix, then the rest
   // With the filter folded into ainv, the refined prefix uses the unfiltered
   // copy and the filter pass; the rest needs no filter pass.
@@ -1670,7 +1673,7 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
     if (us == 3) {
 #define IW_SYS2_LAUNCH(RL)                                                                                   \
   do {                                                                                                       \
-    cudaFuncSetAttribute(k_solve_sys2<T, RL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smsys);      \
+    set_smem(k_solve_sys2<T, RL>, smsys);      \
     k_solve_sys2<T, RL><<<h->ntask2[kind], nthr2, smsys, h->st>>>(g, bi, h->dtasks2[kind], h->dcolorder, F0, \
                                                                   F1, rd, meanu, mg, h->derr);              \
   } while (0)
@@ -1684,7 +1687,7 @@ void launch_solve_bi(iw_handle* h, FieldSet<T>& fs, int role, int cpen, int ksta
     } else {
 #define IW_SYS_LAUNCH(RL)                                                                                           \
   do {                                                                                                              \
-    cudaFuncSetAttribute(k_solve_sys<T, RL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smsys);              \
+    set_smem(k_solve_sys<T, RL>, smsys);              \
     k_solve_sys<T, RL><<<h->ntask2[kind], nthr, smsys, h->st>>>(g, bi, h->dtasks2[kind], h->dcolorder, F0, F1, F2, \
                                                                 rd, meanu, mg, h->dDt, h->dwnl, h->dwvr, kstart,   \
                                                                 h->derr);                                          \
@@ -1760,7 +1763,7 @@ static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen, int cols = 0) 
   const unsigned nblk = (unsigned)((h->ncol + warps - 1) / warps);
   const size_t smem = (size_t)warps * 4 * h->nz * sizeof(double);
   const int kstart = h->p.bc_variant == IW_BC_NOSLIP ? 1 : 0;
-  cudaFuncSetAttribute(k_visc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  set_smem(k_visc<T>, smem);
   if (h->use_bi) {
     launch_solve_bi<T>(h, fs, 3, cpen, kstart, cols, false);
   } else {
@@ -1768,7 +1771,7 @@ static int calcuvwt_impl(iw_handle* h, FieldSet<T>& fs, int cpen, int cols = 0) 
     constexpr int G = 2;
     const int wpb = warps;
     const size_t smp = (size_t)wpb * 2 * G * h->nz * sizeof(double);
-    cudaFuncSetAttribute(k_press_g<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp);
+    set_smem(k_press_g<T, G>, smp);
     k_press_g<T, G><<<(h->ntask[SYS_P] + wpb - 1) / wpb, 32 * wpb, smp, h->st>>>(
         g, solve_tabs(h, SYS_P), h->dtasks[SYS_P], h->ntask[SYS_P], fs.F[0], fs.F[1], fs.F[2], h->dwnl, h->dwvr, cpen,
         kstart);
@@ -1821,7 +1824,7 @@ static int iface_avg(iw_handle* h, FieldSet<T>& fs, bool count, int nf = 4) {
   {
     const int M = h->nx / 2;
     size_t smem = 2 * 4 * (size_t)M * sizeof(C);
-    cudaFuncSetAttribute(k_iface_rows<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    set_smem(k_iface_rows<T>, smem);
     dim3 grid(h->ny, ng);
     k_iface_rows<T><<<grid, 128, smem, h->st>>>(g, fs.G, h->plx, fs.Wm, fs.Wn, h->dcnt);
   }
@@ -1877,7 +1880,7 @@ static int full_step(iw_handle* h, FieldSet<T>& fs) {
   }
   if (h->npostp > 0 && h->istep % h->npostp == 0 && (r = postp_step<T>(h, fs))) return r;  // main.f:935-936
   prof_flush(h);
-  CK(cudaGetLastError());
+  CK(launch_error());
   return 0;
 }
 
@@ -2010,7 +2013,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  const cudaError_t err = cudaGetLastError();
+  const cudaError_t err = launch_error();
   if (err != cudaSuccess) {
     h->tune_ytx = save[0];
     h->tune_xthr = 0;
@@ -2092,7 +2095,7 @@ static int capture_step(iw_handle* const* hs, int n, cudaStream_t s0, cudaGraphE
   }
   if (g) cudaGraphDestroy(g);
   if (rc != IW_OK) {
-    cudaGetLastError();  // reported here; the next call starts without it
+    launch_error();  // reported here; the next call starts without it
     for (int i = 0; i < stepped; ++i) rotate_host(hs[i]);  // nothing ran: undo the host-side rotation
   }
   cudaEventDestroy(fork);
@@ -2427,7 +2430,7 @@ static int copy_level(iw_handle* h, int level, double* host, bool up_dir) {
           k_convert<float, double><<<1184, 256, 0, h->st>>>(dp + o, tmp, c);
           CK(cudaMemcpyAsync(host + q * n + o, tmp, c * sizeof(double), cudaMemcpyDeviceToHost, h->st));
         }
-        CK(cudaGetLastError());
+        CK(launch_error());
       }
     } else {
       double* const* L = level == 0 ? h->f64.F : level == 1 ? h->f64.Fn : level == 2 ? h->f64.Fnm : level == 3 ? h->f64.Sn : h->f64.Snm;
@@ -3078,7 +3081,7 @@ static int helm_lu(iw_handle* h, HelmEntry& E, int need, bool fp32, int bot, int
     if (dalloc(h, &E.c.ab32, E.nlu * band)) return IW_ERR_NOMEM;
     k_convert<double, float><<<2048, 256, 0, h->st>>>(E.c.ab, E.c.ab32, E.nlu * band);
   }
-  CK(cudaGetLastError());
+  CK(launch_error());
   return 0;
 }
 
@@ -3197,7 +3200,7 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     if (E.nlist > 0)
       if (int r = helm_lu(h, E, E.first, false, bot, top)) return r;
     launch_helm_tc<double>(h, H, E.ntask);
-    CK(cudaGetLastError());
+    CK(launch_error());
   } else if (int r = helm_lu(h, E, E.nsys, mode != 0, bot, top)) {
     return r;
   }
@@ -3216,14 +3219,14 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     // (the prefetch of the next factor column costs 6 NB registers; beyond 33 it spills)
     auto* kern = N <= 9 ? k_helm32<9> : N <= 17 ? k_helm32<17> : N <= 25 ? k_helm32<25> : N <= 33 ? k_helm32<33> : k_helm32<0>;
     if (!E.order && up(h, &E.order, helm_order(E))) return IW_ERR_NOMEM;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
+    set_smem(kern, sm32);
     kern<<<(ncol + 15) / 16, 32, sm32, h->st>>>(geo(h), E.c, rhs, sol, ncol, h->dD2, h->dzh, E.order);
-    CK(cudaGetLastError());
+    CK(launch_error());
   } else if (nc > 0) {
-    cudaFuncSetAttribute(k_helm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    set_smem(k_helm, smem);
     k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), E.c, rhs, sol, nc, mode, h->dD2, h->dzh,
                                                                   tc ? E.list : nullptr);
-    CK(cudaGetLastError());
+    CK(launch_error());
   }
   return 0;
 }

@@ -63,8 +63,33 @@ static int set_err(int code, const std::string& msg) {
 #define CK(x)                                                                            \
   do {                                                                                   \
     cudaError_t e_ = (x);                                                                \
-    if (e_ != cudaSuccess) return set_err(IW_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                             \
+      cudaGetLastError(); /* reported here: no later check finds it again */             \
+      return set_err(IW_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));      \
+    }                                                                                    \
   } while (0)
+
+// Launch errors.  A successful cudaFuncSetAttribute resets the runtime's record of a launch that failed
+// before it, so both go through set_smem, which keeps the first error of the thread until it is asked for.
+namespace iw {
+inline thread_local cudaError_t g_launch_error = cudaSuccess;
+}
+static inline void keep_launch_error(cudaError_t e) {  // (an event that is not ready yet is no error)
+  if (e != cudaSuccess && e != cudaErrorNotReady && g_launch_error == cudaSuccess) g_launch_error = e;
+}
+template <typename K>
+static inline void set_smem(K* kernel, size_t bytes) {  // dynamic shared memory that launches of the kernel may ask for
+  keep_launch_error(cudaGetLastError());
+  const cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) cudaGetLastError();
+  keep_launch_error(e);
+}
+static inline cudaError_t launch_error() {
+  keep_launch_error(cudaGetLastError());
+  const cudaError_t e = g_launch_error;
+  g_launch_error = cudaSuccess;
+  return e;
+}
 
 // ---------------------------------------------------------------------------
 // small device helpers

@@ -438,7 +438,7 @@ static int legspec_dump(iw_handle* h, FieldSet<T>& fs) {
     k_speclegen<T><<<dim3((unsigned)((h->nx + 127) / 128), (unsigned)h->ns), 128, 0, h->st>>>(
         geo(h), fs.Y12[0], jrow, h->dwg, h->dal, h->dlegspec + q * per);
   }
-  CK(cudaGetLastError());
+  CK(launch_error());
   CK(cudaMemcpyAsync(h->leg_host, h->dlegspec, 4 * per * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CK(cudaEventRecord(h->out_ev, h->st));
   fout::LegJob j;

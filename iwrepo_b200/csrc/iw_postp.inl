@@ -90,7 +90,7 @@ static int postp_impl(iw_handle* h, FieldSet<T>& fs, double* e18, double* w18) {
       phys_of<T>(h, fs, srcs[s], dst, tmp, op);
       k_row_dot<T><<<rg, 256, 0, h->st>>>(g, dst, dst, R + (8 + 3 * s + op - 1) * rows);
     }
-  CK(cudaGetLastError());
+  CK(launch_error());
   std::vector<double> hr(kPostpRows * rows);
   CK(cudaMemcpyAsync(hr.data(), R, hr.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
