@@ -308,23 +308,25 @@ __host__ __device__ __forceinline__ int fpadlen(int L) { return L > 0 ? fpad(L -
 
 // One pass over G rows, RS values apart: as many whole rows at a time as the warp's lanes hold
 // (M / R <= 32), or one row at a time in IT butterflies per lane (M / R <= 32 IT).  A lane keeps its
-// butterflies' indexes and twiddles over the rows.
-template <typename C, int R, int IT, int L>
-__device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns, float inb, float ins,
+// butterflies' indexes and twiddles over the rows; of a single row (ONE, G = 1) the twiddles are read where
+// they are used, which leaves their registers to the values.
+template <typename C, int R, int IT, int L, bool ONE>
+__device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns, float inb, float ins, int nssh,
                                            const C* __restrict__ W, bool inv, int lane) {
   const int nb = M / R, step = M / (Ns * R);
-  const int rpi = nb < 32 ? (int)(32.5f * inb) : 1;  // rows at a time
-  const int g = nb < 32 ? (int)(((float)lane + 0.5f) * inb) : 0, j0 = lane - g * nb;
-  const bool act = g < rpi;
+  const int rpi = !ONE && nb < 32 ? (int)(32.5f * inb) : 1;  // rows at a time
+  const int g = !ONE && nb < 32 ? (int)(((float)lane + 0.5f) * inb) : 0, j0 = lane - g * nb;
+  const bool act = ONE ? j0 < nb : g < rpi;
   // (values of idle lanes are set, or the compiler carries the registers of every radix through the
   // loop over the passes)
-  C tw[IT][R];
+  C tw[ONE ? 1 : IT][R];
   int jq[IT], jm[IT];
 #pragma unroll
   for (int q = 0; q < IT; ++q) {
     const int j = j0 + 32 * q;
-    jq[q] = (int)(((float)j + 0.5f) * ins);
+    jq[q] = nssh >= 0 ? j >> nssh : (int)(((float)j + 0.5f) * ins);
     jm[q] = j - jq[q] * Ns;
+    if (ONE) continue;
 #pragma unroll
     for (int r = 0; r < R; ++r) tw[q][r] = cmk<C>(1, 0);
     if (Ns > 1 && (q == 0 || j < nb)) {
@@ -337,20 +339,28 @@ __device__ __forceinline__ void fft_pass_w(C* base, int RS, int G, int M, int Ns
     }
   }
 #pragma unroll 1
-  for (int r0 = 0; r0 < G; r0 += rpi) {
+  for (int r0 = 0; r0 < (ONE ? 1 : G); r0 += rpi) {
     C* row = base + (r0 + g) * RS;
-    const bool on = act && r0 + g < G;
+    const bool on = act && (ONE || r0 + g < G);
     C v[IT][R];
 #pragma unroll
     for (int q = 0; q < IT; ++q) {
+      if (!ONE) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[q][r] = cmk<C>(0, 0);
+        for (int r = 0; r < R; ++r) v[q][r] = cmk<C>(0, 0);
+      }
       if (on && (q == 0 || j0 + 32 * q < nb)) {
 #pragma unroll
         for (int r = 0; r < R; ++r) v[q][r] = row[flay<L>(j0 + 32 * q + r * nb)];
         if (Ns > 1) {
 #pragma unroll
-          for (int r = 1; r < R; ++r) v[q][r] = cmul(v[q][r], tw[q][r]);
+          for (int r = 1; r < R; ++r) {
+            if (ONE) {
+              tw[0][r] = W[r * jm[q] * step];
+              if (inv) tw[0][r].y = -tw[0][r].y;
+            }
+            v[q][r] = cmul(v[q][r], tw[ONE ? 0 : q][r]);
+          }
         }
         dft_reg<C, R>(v[q], inv);
       }
@@ -372,25 +382,26 @@ __host__ __device__ constexpr int fft_rows_of(int M, int DPT) { return 32 * DPT 
 
 // In-place transform of G padded rows of M <= 32 DPT values by one warp (all lanes call
 // it).  POW2: the length is a power of two, so only radix 8, 4, 2 passes are
-// compiled (every compiled radix raises the register count of the kernel).
-template <typename C, int DPT, bool POW2, int L = 0>
+// compiled (every compiled radix raises the register count of the kernel).  ONE: G is 1.
+template <typename C, int DPT, bool POW2, int L = 0, bool ONE = false>
 __device__ __forceinline__ void fft_warp(C* base, int RS, int G, const FftPlan& pl, const C* __restrict__ W, bool inv,
                                          int lane) {
   for (int p = 0; p < pl.npass; ++p) {
     const int Ns = pl.ns[p];
     const float ib = pl.inb[p], is = pl.ins[p];
+    const int ss = ONE && POW2 ? pl.nssh[p] : -1;  // (a shift costs fewer instructions than two conversions)
     switch (pl.rad[p]) {
-      case 8: fft_pass_w<C, 8, (DPT + 7) / 8, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
-      case 4: fft_pass_w<C, 4, (DPT + 3) / 4, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
-      case 2: fft_pass_w<C, 2, (DPT + 1) / 2, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane); break;
+      case 8: fft_pass_w<C, 8, (DPT + 7) / 8, L, ONE>(base, RS, G, pl.M, Ns, ib, is, ss, W, inv, lane); break;
+      case 4: fft_pass_w<C, 4, (DPT + 3) / 4, L, ONE>(base, RS, G, pl.M, Ns, ib, is, ss, W, inv, lane); break;
+      case 2: fft_pass_w<C, 2, (DPT + 1) / 2, L, ONE>(base, RS, G, pl.M, Ns, ib, is, ss, W, inv, lane); break;
       default:
         if (!POW2) {
           if (pl.rad[p] == 3)
-            fft_pass_w<C, 3, (DPT + 2) / 3, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+            fft_pass_w<C, 3, (DPT + 2) / 3, L, ONE>(base, RS, G, pl.M, Ns, ib, is, ss, W, inv, lane);
           else if (pl.rad[p] == 6)
-            fft_pass_w<C, 6, (DPT + 5) / 6, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+            fft_pass_w<C, 6, (DPT + 5) / 6, L, ONE>(base, RS, G, pl.M, Ns, ib, is, ss, W, inv, lane);
           else
-            fft_pass_w<C, 5, (DPT + 4) / 5, L>(base, RS, G, pl.M, Ns, ib, is, W, inv, lane);
+            fft_pass_w<C, 5, (DPT + 4) / 5, L, ONE>(base, RS, G, pl.M, Ns, ib, is, ss, W, inv, lane);
         }
         break;
     }

@@ -1119,12 +1119,11 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
       default: break;
     }
   }
-  // narrow tiles serve long columns and the autotuner: one kernel for every radix
-  switch (fft_dpt(h->ny) * (p2 && TX >= 8 ? 1 : -1)) {
+  switch (fft_dpt(h->ny) * (p2 ? 1 : -1)) {
 #define IW_YCASE(D, P)                                                                                       \
   case (P ? D : -D):                                                                                         \
-    if constexpr ((TX < 16 || D == 4) && (TX >= 8 || !P)) { /* 16 columns only for ny <= 128 */              \
-      set_smem(k_yfft<T, TX, D, P, TWO>, smem); \
+    if constexpr (TX < 16 || D == 4) { /* 16 columns only for ny <= 128 */                                   \
+      set_smem(k_yfft<T, TX, D, P, TWO>, smem);                                                              \
       k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
     }                                                                                                        \
     break;

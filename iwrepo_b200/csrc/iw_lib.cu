@@ -280,15 +280,18 @@ struct YLay {
 
 // CTAs per SM: a single transform of a long column of the compile-time plans gains from a third CTA
 // (80 registers: 512^2 x 396 FP32 inverse 2.43 -> 2.13 ms, 256^2 x 200 FP64 561 -> 499 us); two
-// transforms (mode 3) lose by it (2.69 -> 2.94 ms, 580 -> 643 us with the other four).
-template <typename T, int DPT, bool POW2, int MC, bool TWO>
+// transforms (mode 3) lose by it (2.69 -> 2.94 ms, 580 -> 643 us with the other four).  Narrow tiles (a column per
+// warp) hold no twiddles over rows: four CTAs in FP64 for short columns (two: 72 -> 97 us, 64^2 x 68, 2 columns).
+template <typename T, int TX, int DPT, bool POW2, int MC, bool TWO>
 struct YOcc {
-  static constexpr int v = !TWO && MC > 0 && MC * (int)sizeof(T) >= 2048 && MC <= 512 && FftOcc<T, DPT, POW2>::v == 2
-                               ? 3
-                               : FftOcc<T, DPT, POW2>::v;
+  static constexpr int v =
+      TX < 8 ? (sizeof(T) == 4 ? (DPT <= 8 ? 4 : DPT <= 16 ? 2 : 1) : (DPT <= 4 ? 4 : DPT <= 8 ? 2 : 1))
+             : !TWO && MC > 0 && MC * (int)sizeof(T) >= 2048 && MC <= 512 && FftOcc<T, DPT, POW2>::v == 2
+                   ? 3
+                   : FftOcc<T, DPT, POW2>::v;
 };
 template <typename T, int TX, int DPT, bool POW2, bool TWO, int MC = 0>
-__global__ void __launch_bounds__(256, (YOcc<T, DPT, POW2, MC, TWO>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
+__global__ void __launch_bounds__(256, (YOcc<T, TX, DPT, POW2, MC, TWO>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
                                               const typename cplx_t<T>::type* __restrict__ Wy) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(256, (YOcc<T, DPT, POW2, MC, TWO>::v)) k_yfft(
       else if constexpr (MC > 0)
         fft_warp_ct<C, MC, YL>(row, RSY, G, Wy, !fwd, lane);
       else
-        fft_warp<C, DPT, POW2, YL>(row, RSY, G, pl, Wy, !fwd, lane);
+        fft_warp<C, DPT, POW2, YL, (TX < 8)>(row, RSY, G, pl, Wy, !fwd, lane);  // 8 warps: one column each
     }
   }
   __syncthreads();
