@@ -285,25 +285,24 @@ int iw_step(iw_handle *h);
 int iw_run(iw_handle *h, int nsteps, int use_graph);
 
 /* Not in the reference.  Times the launch candidates of this handle's step on
- * its device and keeps the fastest for the following steps: y-tile width (2, 4
- * or 8 columns), the stage-A and stage-E variants (register-column or tiled)
- * and the solve variant (system-grouped CTAs with the tables staged in shared
- * memory, their block products on the FP64 pipes or on the FP64 tensor cores,
- * or one CTA per task of <= 4 right-hand sides).  Candidates run on the
- * handle's scratch fields; the state is not changed (the solver tables are
- * built if no step has built them yet).  The stage-A variants and the solve
- * variants give the same bits; the stage-E variants round differently.
- * choices (optional, 4 ints): the y-tile width; for stage A and stage E
- * 1 = register-column, 0 = tiled, -1 = not applicable (stage E also 2 =
- * tiled with the input tiles staged by bulk copies, N <= 64); the pressure
- * solve's variant (1 = system-grouped, 2 = system-grouped on the tensor cores,
- * N <= 40, 0 = per task; each solve role keeps its own fastest). */
+ * its device and keeps the fastest for the following steps: the y tile, the
+ * stage-A and stage-E variants, the threads per x-row CTA and the solve variant
+ * of each role.  For nzloc <= 40 the stages and, where their tables fit in
+ * shared memory, the solves stay on the FP64 tensor cores.  Candidates run on
+ * the handle's scratch fields; the state is not changed (the solver tables are
+ * built if no step has built them yet).  The solve variants give the same bits.
+ * The stage-E variants round differently, and so does the tensor-core stage A
+ * of mixed precision (FP64 products) from its variants 0 and 1.
+ * choices (optional, 4 ints): the values of IW_LAUNCH_YTILE, IW_LAUNCH_STAGE_A,
+ * IW_LAUNCH_STAGE_E and IW_LAUNCH_SOLVE_PRESSURE that were kept; iw_set_launch
+ * takes them for another handle of the same sizes, as it takes all that
+ * iw_get_launch reads. */
 int iw_autotune(iw_handle *h, int *choices);
 
 /* Not in the reference.  Sets one launch choice of iw_autotune directly. */
 #define IW_LAUNCH_YTILE 0   /* columns per y tile: 0 (by size), 2, 4 or 8 (8 is 16 where ny <= 128) */
-#define IW_LAUNCH_STAGE_A 1 /* -1 (FP64 tensor cores, nzloc <= 40), 0 tiled, 1 register-column */
-#define IW_LAUNCH_STAGE_E 2 /* as stage A; 2 and 3 are the FP64 tensor cores too */
+#define IW_LAUNCH_STAGE_A 1 /* -1 (by size: FP64 tensor cores for nzloc <= 40, else tiled), 0 tiled, 1 register-column (nzloc <= 33) */
+#define IW_LAUNCH_STAGE_E 2 /* as stage A; 2 and 3 are the FP64 tensor cores too (nzloc <= 40) */
 #define IW_LAUNCH_SOLVE 3   /* 2 system-grouped on the FP64 tensor cores (default; 1 where it does not apply),
                                1 system-grouped on the FP64 pipes, 0 per task, 3 system-grouped with two rows
                                per thread (u/v, w, rho; the pressure takes 1).  All give the same bits. */

@@ -2024,7 +2024,7 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
   }
   if (choice) {
     choice[0] = h->tune_ytx;
-    choice[1] = h->tune_a < 0 && zop_bucket(h->N) ? 1 : h->tune_a;  // the tensor-core kernel's columns sit in registers too
+    choice[1] = h->tune_a;
     choice[2] = h->tune_e;
     choice[3] = h->sys_role[3] >= 0 ? h->sys_role[3] : h->use_sys;
   }
@@ -2246,6 +2246,7 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
   h->ncol = h->nxhp * h->ny;
   h->mixed = prm->precision == IW_PREC_MIXED;
   h->use_bi = prm->solver == 0 && d.nsubd <= 16;
+  if (h->N > kTcMaxN) h->use_sys = 1;
   h->plx = make_plan(h->nx / 2);
   h->ply = make_plan(h->ny);
   if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess ||
@@ -2526,8 +2527,7 @@ int iw_set_launch(iw_handle* h, int which, int value) {
       if (value < -1 || value > (which == IW_LAUNCH_STAGE_E ? 3 : 1))
         return set_err(IW_ERR_CONFIG, "stage variant: -1, 0, 1 (or 2, 3 for stage E)");
       if (value == 1 && !zop_bucket(h->N)) return set_err(IW_ERR_CONFIG, "register-column stages need N <= 33");
-      if (value >= 2 && (!zop_bucket(h->N) || h->plane * (h->mixed ? 4 : 8) % 16 != 0))
-        return set_err(IW_ERR_CONFIG, "bulk-staged stage E needs N <= 33 and whole 16-byte planes");
+      if (value >= 2 && h->N > kTcMaxN) return set_err(IW_ERR_CONFIG, "tensor-core stage E needs N <= 40");
       (which == IW_LAUNCH_STAGE_A ? h->tune_a : h->tune_e) = value;
       return IW_OK;
     case IW_LAUNCH_SOLVE:

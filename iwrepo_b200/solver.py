@@ -158,7 +158,13 @@ class Solver:
         names = {3: "tiled-bulk-constant-operators", 2: "tiled-bulk", 1: "register", 0: "tiled", -1: "n/a"}
         solve = {0: "per-task", 1: "system-grouped", 2: "system-grouped-tensor-core",
                  3: "system-grouped-two-rows"}
-        out = {"y_tile": ch[0], "stage_a": names[ch[1]], "stage_e": names[ch[2]], "solve": solve[ch[3]]}
+        # (stage_a and stage_e keep the names that callers compare with; z_kernels names what runs)
+        reg = ch[1] < 0 and self.cfg.nzloc <= 33
+        out = {"y_tile": ch[0], "stage_a": "register" if reg else names[ch[1]], "stage_e": names[ch[2]],
+               "solve": solve[ch[3]]}
+        tc = self.cfg.nzloc <= 40
+        out["z_kernels"] = {st: "tensor-core" if v not in (0, 1) and tc else "register" if v == 1 else "tiled"
+                            for st, v in (("stage_a", ch[1]), ("stage_e", ch[2]))}
         out["solve_roles"] = {role: solve.get(self.get_launch("solve_" + role), "n/a")
                               for role in ("uv", "w", "rho", "pressure")}
         out["x_row_threads"] = self.get_launch("x_row_threads")
