@@ -1805,7 +1805,7 @@ template <typename T>
 static int iface_avg(iw_handle* h, FieldSet<T>& fs, bool count, int nf = 4) {
   typedef typename cplx_t<T>::type C;
   Geo g = geo(h);
-  const dim3 pgrid((unsigned)((h->ny + 127) / 128), (unsigned)h->nz, (unsigned)(h->ns < 2 ? 4 : nf));
+  const dim3 pgrid((unsigned)((h->ny + 127) / 128), (unsigned)h->nz, (unsigned)nf);
   if (h->ns < 2) {
     k_project_planes<T><<<pgrid, 128, 0, h->st>>>(g, fs.F[0], fs.F[1], fs.F[2], fs.F[3], 0);
     return 0;
