@@ -3020,9 +3020,10 @@ static size_t carve(size_t& at, size_t bytes) {
 
 // the columns by system
 static std::vector<int> helm_order(const HelmEntry& E) {
-  std::vector<int> order(E.cs.size());
-  for (size_t c = 0; c < order.size(); ++c) order[c] = (int)c;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return E.cs[a] < E.cs[b]; });
+  std::vector<int> at(E.nsys + 1, 0), order(E.cs.size());
+  for (int u : E.cs) ++at[u + 1];
+  for (int u = 0; u < E.nsys; ++u) at[u + 1] += at[u];
+  for (size_t c = 0; c < order.size(); ++c) order[at[E.cs[c]]++] = (int)c;
   return order;
 }
 
@@ -3177,6 +3178,7 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
   HelmEntry& E = it->second;
   // k_helm_tc copies whole complex values: 16-byte aligned columns
   const bool tc = mode == 0 && E.first < E.nsys && (((uintptr_t)rhs | (uintptr_t)sol) & 15) == 0;
+  cudaStream_t st = h->st;  // of k_helm: beside k_helm_tc where the columns are split between them
   if (tc) {
     if (int r = helm_blocks(h, E, bot, top)) return r;
     HelmTc H;
@@ -3198,6 +3200,7 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     // the factors of the other systems first: after a failure nothing of the solution is written
     if (E.nlist > 0)
       if (int r = helm_lu(h, E, E.first, false, bot, top)) return r;
+    if (E.nlist > 0) st = side_fork(h);
     launch_helm_tc<double>(h, H, E.ntask);
     CK(launch_error());
   } else if (int r = helm_lu(h, E, E.nsys, mode != 0, bot, top)) {
@@ -3223,8 +3226,9 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     CK(launch_error());
   } else if (nc > 0) {
     set_smem(k_helm, smem);
-    k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, h->st>>>(geo(h), E.c, rhs, sol, nc, mode, h->dD2, h->dzh,
-                                                                  tc ? E.list : nullptr);
+    k_helm<<<(nc + warps - 1) / warps, 32 * warps, smem, st>>>(geo(h), E.c, rhs, sol, nc, mode, h->dD2, h->dzh,
+                                                               tc ? E.list : nullptr);
+    if (st != h->st) side_join(h);
     CK(launch_error());
   }
   return 0;
