@@ -698,7 +698,10 @@ static int build_sys_tasks(iw_handle* h, int kind, int nrefine) {
 static void launch_band_lu(cudaStream_t st, int nsys, int n, int N, double* ab, int* ipiv, int* info) {
   const size_t sm = lu_smem(N);
   set_smem(k_band_lu, sm);
-  k_band_lu<<<nsys, kLuThreads, sm, st>>>(n, N, ab, ipiv, info);
+  // A step's barrier costs more with eight warps than four, its update more with three warps than seven (us, 128 / 256
+  // threads; one system of 12 x 3 points 64 / 74, 17 x 4 107 / 125, penalty_main_ with 25 x 12 748 / 661;
+  // a first isolated solve of 2112 columns of 17 x 4 1089 / 1200).
+  k_band_lu<<<nsys, N <= 17 ? kLuThreads / 2 : kLuThreads, sm, st>>>(n, N, ab, ipiv, info);
 }
 
 // (re)build the factors of one kind for the current bdfv/dt

@@ -1614,7 +1614,7 @@ static __global__ void __launch_bounds__(kLuThreads) k_band_lu(int n, int N, dou
   extern __shared__ __align__(16) double sml[];
   __shared__ int sjp[2];
   const int kl = N, ku = N, kv = kl + ku, ldab = 2 * kl + ku + 1, W = lu_ring(N);
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = kLuThreads >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nth = blockDim.x, nw = nth >> 5;
   double* ab = abs_ + (size_t)blockIdx.x * ldab * n;
   int* ipiv = ipivs + (size_t)blockIdx.x * n;
   double* ring = sml;                    // column j at ring + (j % W) ldab
@@ -1624,7 +1624,7 @@ static __global__ void __launch_bounds__(kLuThreads) k_band_lu(int n, int N, dou
     if (c < n) {
       double* d = ring + (size_t)slot * ldab;
       const double* s = ab + (size_t)c * ldab;
-      for (int r = tid; r < ldab; r += kLuThreads) {
+      for (int r = tid; r < ldab; r += nth) {
         if (r < kl)
           d[r] = 0.0;
         else
@@ -1683,7 +1683,7 @@ static __global__ void __launch_bounds__(kLuThreads) k_band_lu(int n, int N, dou
         ipiv[j + 1] = j + 1 + (p >= 0 ? p : -1 - p) + 1;
       }
     }
-    for (int r = tid; r < ldab; r += kLuThreads) ab[(size_t)j * ldab + r] = cj[r];
+    for (int r = tid; r < ldab; r += nth) ab[(size_t)j * ldab + r] = cj[r];
     if (++sj >= W) sj -= W;
     if (++sf >= W) sf -= W;
   }
