@@ -1150,7 +1150,11 @@ void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int npla
     k_y1<T><<<dim3((unsigned)((nc + 255) / 256), (unsigned)njobs), 256, 0, h->st>>>(jobs, nc);
     return;
   }
-  const int tx = ytx<T>(h, four);
+  int tx = ytx<T>(h, four);
+  // FP32 columns of 16 or 32 rows in fewer tiles of 16 columns than SMs (one field of few planes, as in iw_postp): tiles of
+  // 4, a warp per column (iw_postp, 16 / 4 columns: 16 x 16 x 9 397 / 383 us, 32 x 32 x 18 484 / 448, 64 x 32 x 36 566 / 557;
+  // 180 tiles gain nothing, FP64 and 64 rows lose: 16 x 16 x 9 384 / 405, 16 x 64 x 18 601 / 649).  Same bits.
+  if (sizeof(T) == 4 && tx == 16 && (h->ny == 16 || h->ny == 32) && (h->nxhp + 15) / 16 * nplanes * njobs < h->nsm) tx = 4;
   const int ntile = (h->nxhp + tx - 1) / tx;
   dim3 grid(ntile, nplanes, njobs);
   const size_t smem = (four ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * sizeof(C);
