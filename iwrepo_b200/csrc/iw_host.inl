@@ -1044,11 +1044,7 @@ void launch_stageE(iw_handle* h, FieldSet<T>& fs, int cols) {
 #undef IW_ETCASE
   }
   const dim3 rgrid((unsigned)((h->plane + 127) / 128), (unsigned)h->ns, 4);
-  // The register-column stage E holds two columns per thread; past these sizes
-  // its register count costs more occupancy than the tiled kernel loses.
-  const int emax = sizeof(T) == 4 ? 25 : 17;
-  const bool reg = h->tune_e < 0 ? h->N <= emax : h->tune_e == 1;
-  switch (reg ? zop_bucket(h->N) : 0) {
+  switch (h->tune_e == 1 ? zop_bucket(h->N) : 0) {  // (a launch choice; else, N > 40, tiled)
 #define IW_ECASE(NM)                                                                          \
   case NM:                                                                                    \
     k_stageE_r<T, NM><<<rgrid, 128, 0, h->st>>>(geo(h), a, h->c, make_zop<T, NM>(h));         \
@@ -1092,7 +1088,7 @@ static int ytx(const iw_handle* h, bool two) {  // y-FFT tile width
 }
 
 template <typename T, int TX, bool TWO>
-static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, int nplanes,
+static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem,
                         const typename cplx_t<T>::type* Wy) {
   Geo g = geo(h);
   const bool p2 = (h->ny & (h->ny - 1)) == 0;
@@ -1101,7 +1097,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
     set_smem(k_yfft<T, TX, D, true, TWO, MC>, smem); \
-    k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+    k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, h->ply, Wy);                    \
     return;
       IW_YCT(64, 8)
       IW_YCT(128, 8)
@@ -1114,7 +1110,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
 #define IW_YCT(MC, D)                                                                                        \
   case MC:                                                                                                   \
     set_smem(k_yfft<T, TX, D, true, TWO, MC>, smem); \
-    k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+    k_yfft<T, TX, D, true, TWO, MC><<<grid, 256, smem, h->st>>>(g, jobs, h->ply, Wy);                    \
     return;
       IW_YCT(256, 8)
       IW_YCT(512, 16)
@@ -1127,7 +1123,7 @@ static void launch_y_tx(iw_handle* h, YJobs<T>& jobs, dim3 grid, size_t smem, in
   case (P ? D : -D):                                                                                         \
     if constexpr (TX < 16 || D == 4) { /* 16 columns only for ny <= 128 */                                   \
       set_smem(k_yfft<T, TX, D, P, TWO>, smem);                                                              \
-      k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, nplanes, h->ply, Wy);                    \
+      k_yfft<T, TX, D, P, TWO><<<grid, 256, smem, h->st>>>(g, jobs, h->ply, Wy);                    \
     }                                                                                                        \
     break;
     IW_YCASE(4, true)
@@ -1160,8 +1156,8 @@ void launch_y(iw_handle* h, FieldSet<T>& fs, YJobs<T>& jobs, int njobs, int npla
   const size_t smem = (four ? 2 : 1) * (size_t)tx * ystride_of<T>(h->ny, tx) * sizeof(C);
   switch (four ? -tx : tx) {
 #define IW_YTX(TX)                                                                        \
-  case TX: launch_y_tx<T, TX, false>(h, jobs, grid, smem, nplanes, fs.Wy); break;         \
-  case -TX: launch_y_tx<T, TX, true>(h, jobs, grid, smem, nplanes, fs.Wy); break;
+  case TX: launch_y_tx<T, TX, false>(h, jobs, grid, smem, fs.Wy); break;         \
+  case -TX: launch_y_tx<T, TX, true>(h, jobs, grid, smem, fs.Wy); break;
     IW_YTX(16)
     IW_YTX(8)
     IW_YTX(4)
@@ -2208,8 +2204,9 @@ int iw_init(const iw_dims* dims, const iw_params* prm, int device, iw_handle** o
   if (d.nsubd < 1 || d.nsubd > IW_MAX_SUBD) return set_err(IW_ERR_CONFIG, "nsubd outside [1,64]");
   {
     const size_t cs = prm->precision == IW_PREC_FP64 ? 16 : 8;
+    // (the row kernel holds 17 rows; lengths are accepted while 20 would fit)
     if (20 * (size_t)xstride(d.nx / 2) * cs > 227 * 1024 || d.nx / 2 > 1024)
-      return set_err(IW_ERR_CONFIG, "nx too large for the row kernel (20 rows of nx/2+1 values in shared memory)");
+      return set_err(IW_ERR_CONFIG, "nx too large: nx <= 2048, and 20 rows of nx/2+1 values within the 227 KB of shared memory");
     if ((size_t)ystride(d.ny) * cs > 110 * 1024 || d.ny > 1024)
       return set_err(IW_ERR_CONFIG, "ny too large for the y-transform kernel");
   }

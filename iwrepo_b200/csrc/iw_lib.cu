@@ -291,7 +291,7 @@ struct YOcc {
                    : FftOcc<T, DPT, POW2>::v;
 };
 template <typename T, int TX, int DPT, bool POW2, bool TWO, int MC = 0>
-__global__ void __launch_bounds__(256, (YOcc<T, TX, DPT, POW2, MC, TWO>::v)) k_yfft(Geo g, YJobs<T> jobs, int nplanes, FftPlan pl,
+__global__ void __launch_bounds__(256, (YOcc<T, TX, DPT, POW2, MC, TWO>::v)) k_yfft(Geo g, YJobs<T> jobs, FftPlan pl,
                                               const typename cplx_t<T>::type* __restrict__ Wy) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -306,7 +306,6 @@ __global__ void __launch_bounds__(256, (YOcc<T, TX, DPT, POW2, MC, TWO>::v)) k_y
   const int ii0 = blockIdx.x * TX;
   const bool fwd = jb.mode >= 2;
   constexpr bool two = TWO;  // mode 3
-  (void)nplanes;
   // load: column ii0+b, row j -> A[b*RSY + flay<YL>(j)] (all copies in flight at once).
   // With 256 threads and TX | 256 a thread keeps its column b and steps j by
   // JS = 256/TX, so both addresses advance by fixed strides.
