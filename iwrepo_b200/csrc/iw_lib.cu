@@ -3960,25 +3960,17 @@ __global__ void __launch_bounds__(512, 2) k_stageA_t(Geo g, const T* __restrict_
       }
       // non-finite values are looked for after the projection, which drops the imaginary part of
       // the x-Nyquist column (the derivative alone: in the raw values)
-      const bool pr = !PLAIN && special && proj > 0;
-      bool bad = false;
-      if (!pr) {
+      if (!PLAIN && special && proj > 0) {
 #pragma unroll
-        for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
+        for (int kt = 0; kt < 2 * NT; ++kt)
+          if (act && 4 * kt + lt < N) x[kt] = proj_val<T>(g, F, i, j, 4 * kt + lt);
       }
-      if (!PLAIN && special) {
-        const bool wzero = q == 2 && tt < 2;
+      bool bad = false;
 #pragma unroll
-        for (int kt = 0; kt < 2 * NT; ++kt) {
-          const int r = 4 * kt + lt;
-          if (act && r < N) {
-            if (pr) {
-              x[kt] = proj_val<T>(g, F, i, j, r);
-              bad |= !isfinite(x[kt]);
-            }
-            if (wzero) x[kt] = (T)0;
-          }
-        }
+      for (int kt = 0; kt < 2 * NT; ++kt) bad |= !isfinite(x[kt]);
+      if (!PLAIN && proj >= 0 && q == 2 && tt < 2) {  // the mean of w
+#pragma unroll
+        for (int kt = 0; kt < 2 * NT; ++kt) x[kt] = (T)0;
       }
       if (bad) err[0] = 1;  // the state of the last step holds a NaN or Inf
       if (proj >= 0) {
