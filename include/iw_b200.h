@@ -300,7 +300,8 @@ int iw_run(iw_handle *h, int nsteps, int use_graph);
 int iw_autotune(iw_handle *h, int *choices);
 
 /* Not in the reference.  Sets one launch choice of iw_autotune directly. */
-#define IW_LAUNCH_YTILE 0   /* columns per y tile: 0 (by size), 2, 4 or 8 (8 is 16 where ny <= 128) */
+#define IW_LAUNCH_YTILE 0   /* columns per y tile: 0 (by size), 2, 4 or 8 (8 is by size too: 16 where ny <= 128,
+                               4 for FP32 columns of 16 or 32 rows in few planes) */
 #define IW_LAUNCH_STAGE_A 1 /* -1 (by size: FP64 tensor cores for nzloc <= 40, else tiled), 0 tiled, 1 register-column (nzloc <= 33) */
 #define IW_LAUNCH_STAGE_E 2 /* as stage A; 2 and 3 are the FP64 tensor cores too (nzloc <= 40) */
 #define IW_LAUNCH_SOLVE 3   /* 2 system-grouped on the FP64 tensor cores (default; 1 where it does not apply),

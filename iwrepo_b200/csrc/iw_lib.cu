@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(256, (FftOcc<T, DPT, POW2>::v)) k_xrow_nl(Geo 
 // Measured against k_xrow_nl (which then also carried the three rows of d rho): 512^2 x 396 FP32
 // 5.56 -> 3.39 ms, 256^2 x 200 FP64 1.96 -> 0.96 ms, 192 x 120 x 110 FP32 401 -> 123 us, 64^2 x 68 FP64
 // 83 -> 29 us.  At 512^2 it moves its 21 fields at 2.6 TB/s, bound by instruction issue (2.6 per cycle)
-// and in FP64 by the L1 data path (twiddles and rows, 62 %).
+// and in FP64 by the L1 data path (twiddles and rows, 72 %).
 // Threads per SM: 512 in FP32 (128 registers; with 640 a thread of R0 = 8 spills: 3.39 -> 3.94 ms),
 // 384 in FP64 (168 registers: 1.02 against 1.05 ms with 256), but 256 for R0 < 6, whose rows are so
 // short that loads in flight count (64^2: 29 against 38 us).  From R0 = 6 on the indexes and twiddles
