@@ -1198,6 +1198,13 @@ static int legspec_dump(iw_handle* h, FieldSet<T>& fs);
 template <typename T>
 static int postp_step(iw_handle* h, FieldSet<T>& fs);
 
+// lengths nx / 2 with a kernel of their own (k_xrow_reg)
+static bool xrow_reg_length(int M) {
+  for (int nb : {8, 16, 32})
+    for (int r0 : {2, 4, 6, 8, 10})
+      if (M == r0 * nb && (nb == 8 || r0 >= 6)) return true;
+  return false;
+}
 // K_C for the lengths of k_xrow_reg; false for any other
 template <typename T>
 static bool launch_xrow_reg(iw_handle* h, FieldSet<T>& fs, const NLArgs<T>& a) {
@@ -1950,8 +1957,8 @@ static int tune_impl(iw_handle* h, FieldSet<T>& fs, int* choice) {
     }
   }
   h->tune_ytx = besttx;
-  // threads per x-row CTA (scratch rows in, scratch rows out)
-  {
+  // threads per x-row CTA (scratch rows in, scratch rows out), where the length's kernel has the choice
+  if (!xrow_reg_length(h->nx / 2)) {
     float bx = 0.f;
     int bestx = 256;
     for (int xt : {256, 128}) {

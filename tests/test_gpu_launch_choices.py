@@ -45,3 +45,15 @@ def test_reported_z_kernels():
         with iw.Solver(cf.Config(nx=16, ny=16, nzloc=nzloc, nsubd=2, dt=1e-3).validate()) as s:
             s.init_mode1(0.05, 1e-3, 11)
             assert s.autotune()["z_kernels"] == {"stage_a": kernel, "stage_e": kernel}
+
+
+@pytest.mark.parametrize("nx,own", [(32, True), (96, True), (640, True), (48, False), (512, True), (100, False), (1024, False)])
+def test_x_row_threads_where_the_length_has_the_choice(nx, own):
+    """Lengths with a kernel of their own leave the choice alone."""
+    import iwrepo_b200 as iw
+    cfg = cf.Config(nx=nx, ny=4, nzloc=5, nsubd=1, dt=1e-3, precision=cf.IW_PREC_MIXED).validate()
+    with iw.Solver(cfg) as s:
+        s.init_mode1(0.05, 1e-3, 11)
+        s.set_launch("x_row_threads", 256)
+        ch = s.autotune()["x_row_threads"]
+        assert ch == 256 if own else ch in (128, 256)
