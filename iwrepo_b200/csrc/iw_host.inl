@@ -2735,6 +2735,7 @@ struct HelmEntry {
   int* list = nullptr;
 };
 static std::map<std::pair<iw_handle*, std::string>, HelmEntry> g_helm;
+static std::mutex g_helm_mu;  // of the map: handles of other threads add entries and go away; an entry is its handle's alone
 
 // y = A x for the penalty matrix of system s (matrix-free, FP64)
 // row r; x(i): element i
@@ -3166,8 +3167,13 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
   snprintf(kb, sizeof kb, "%d|%d|%d|%llx", ncol, bot, top, (unsigned long long)hs);
   auto key = std::make_pair(h, std::string(kb));
   const int n = h->nz, N = h->N, ns = h->ns;
-  auto it = g_helm.find(key);
-  if (it == g_helm.end()) {
+  HelmEntry* found = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_helm_mu);
+    auto it = g_helm.find(key);
+    if (it != g_helm.end()) found = &it->second;
+  }
+  if (!found) {
     HelmEntry E;
     E.lam = lam;
     std::sort(E.lam.begin(), E.lam.end());
@@ -3184,9 +3190,10 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
     if (tc)
       while (E.first > 0 && E.lam[E.first - 1] > 0 && 1.0 + rho / E.lam[E.first - 1] <= kRefineCond) --E.first;
     if (up(h, &E.c.colsys, E.cs)) return IW_ERR_NOMEM;
-    it = g_helm.emplace(key, std::move(E)).first;
+    std::lock_guard<std::mutex> lk(g_helm_mu);
+    found = &g_helm.emplace(key, std::move(E)).first->second;
   }
-  HelmEntry& E = it->second;
+  HelmEntry& E = *found;
   // k_helm_tc copies whole complex values: 16-byte aligned columns
   const bool tc = mode == 0 && E.first < E.nsys && (((uintptr_t)rhs | (uintptr_t)sol) & 15) == 0;
   cudaStream_t st = h->st;  // of k_helm: beside k_helm_tc where the columns are split between them
@@ -3247,6 +3254,7 @@ static int helm_batched(iw_handle* h, const double* lam_dev, int ncol, int bot, 
 
 // the isolated-solve tables of a handle that goes away
 static void helm_free(iw_handle* h) {
+  std::lock_guard<std::mutex> lk(g_helm_mu);
   for (auto it = g_helm.begin(); it != g_helm.end();) {
     if (it->first.first != h) {
       ++it;
