@@ -41,6 +41,7 @@
 #include <string>
 #include <thread>
 #include <type_traits>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/iw_b200.h"
@@ -77,11 +78,28 @@ inline thread_local cudaError_t g_launch_error = cudaSuccess;
 static inline void keep_launch_error(cudaError_t e) {  // (an event that is not ready yet is no error)
   if (e != cudaSuccess && e != cudaErrorNotReady && g_launch_error == cudaSuccess) g_launch_error = e;
 }
+// Dynamic shared memory that launches of the kernel may ask for.  The limit is the kernel's, not the caller's: it only
+// grows, so that no thread lowers it between another thread's call and its launch.
+struct SmemLimits {
+  std::mutex mu;
+  std::unordered_map<const void*, size_t> set;
+};
+inline SmemLimits& smem_limits() {
+  static SmemLimits l;
+  return l;
+}
 template <typename K>
-static inline void set_smem(K* kernel, size_t bytes) {  // dynamic shared memory that launches of the kernel may ask for
+static inline void set_smem(K* kernel, size_t bytes) {
   keep_launch_error(cudaGetLastError());
-  const cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) cudaGetLastError();
+  SmemLimits& l = smem_limits();
+  std::lock_guard<std::mutex> lk(l.mu);
+  size_t& have = l.set[(const void*)kernel];
+  const size_t want = std::max(have, bytes);
+  const cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+  if (e == cudaSuccess)
+    have = want;
+  else
+    cudaGetLastError();
   keep_launch_error(e);
 }
 static inline cudaError_t launch_error() {
